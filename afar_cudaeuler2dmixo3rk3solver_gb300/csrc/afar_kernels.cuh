@@ -39,15 +39,17 @@ struct StepCtl {
 // sets each step with runTime.setDeltaT, cudaEuler2DmixO3RK3solver.cpp:44-48): with r the time to
 // the next write, n = floor(r/dt - small) + 1 steps of r/n, the change held within [dt/5, 2 dt].
 __device__ __forceinline__ double step_dt(const StepCtl* c) {
-  double dt = c->dt_fixed > 0.0 ? c->dt_fixed : __longlong_as_double((long long)c->dt_bits);
-  if (c->write_interval > 0.0) {
+  // (the tests as integers: thread 0 of every update block takes this way, and each FP64 comparison
+  // would hold its SM's FP64 pipe 16 clocks)
+  double dt = gt_zero(c->dt_fixed) ? c->dt_fixed : __longlong_as_double((long long)c->dt_bits);
+  if (gt_zero(c->write_interval)) {
     const double r = (double)(c->write_index + 1) * c->write_interval - c->t;
     if (r > 0.0) {
       const double nd = r / (floor(r / dt - 1e-15) + 1.0);
       dt = nd >= dt ? fmin(nd, 2.0 * dt) : fmax(nd, 0.2 * dt);
     }
   }
-  if (c->t_end > 0.0) dt = fmin(dt, c->t_end - c->t);
+  if (gt_zero(c->t_end)) dt = fmin(dt, c->t_end - c->t);
   return dt;
 }
 
@@ -69,7 +71,7 @@ struct StageArgs {
   const V2<double>* cellC;    // Nc+Nb cell centres, ghosts = boundary face centres
   const int2* on;             // Nf (owner, neighbour)
   const V4<G>* fd;            // Nf (xf-x_own, yf-y_own, xf-x_nei, yf-y_nei)
-  const V4<G>* fs;            // Nf+Nb (Sfx, Sfy, magSf, 0)
+  const V4<G>* fs;            // Nf+Nb (Sfx, Sfy, magSf, 1/magSf; ref: 0)
   const V2<double>* dtg;      // Nf (delta r, fraction) of the CFL estimate
   const V2<double>* bn;       // Nb unit normal of each boundary face
   const uint8_t* btype;       // Nb cudaEulerBCs label
@@ -98,6 +100,7 @@ struct StageArgs {
   StepCtl* ctl;
   V4<double>* res_dbg;        // optional residual dump (parity hook)
   double R, Cv, invR, gamma;
+  double Cp, gm1, gR;  // Cv + R, gamma - 1, gamma R (fp64)
   float gm1f, invRf;  // gamma - 1 and 1/R as floats (mixed)
   float Rf, Cvf, gRf;  // R, Cv and gamma*R as floats (mixed)
   double px, py;       // periods of a periodic mesh (0: none); setup kernels only
@@ -137,6 +140,40 @@ __device__ __forceinline__ void limiter_process_fast(float& limiter, float& phif
   const float d1 = phif < phic ? phiMin - phic : phiMax - phic;
   const float yy = fabsf(d2) >= 1e-5f ? fminf(2.f, __fdividef(0.5f * d1, d2 + (d2 >= 0.f ? 1e-10f : -1e-10f))) : 1.f;
   limiter = fminf(limiter, yy);
+}
+
+// limiterProcess for the fp64 policy: the face's ratio min(2, d1 / (2 (d2 +- 1e-10))) as a fraction
+// num/den of positive numbers (d1 and d2 have one sign), 1/1 where |d2| < 1e-5; the smaller of it and
+// the cell's smallest so far is kept, told apart by their FP32 quotients (20 bits of each operand), or
+// by cross-multiplication where those agree to 1e-5.  So a cell divides once for all variables
+// (limiter_ratios) instead of once per face and variable, and no comparison or selection takes the
+// FP64 pipe.  d2: the jump from the cell to phif.
+struct LimiterRatio {
+  double num, den;
+  float q;
+};
+__device__ __forceinline__ void limiter_process_ratio(LimiterRatio& r, double& phif, double& d2, const double phic,
+                                                      const double phiMax, const double phiMin, const double gx,
+                                                      const double gy, const double dx, const double dy) {
+  phif = phic + (gx * dx + gy * dy);
+  d2 = phif - phic;
+  const bool valid = abs_ge(d2, 1e-5);
+  const double num = valid ? dabs_((neg_(d2) ? phiMin : phiMax) - phic) : 1.0;
+  const double den = valid ? __fma_rn(2.0, dabs_(d2), 2e-10) : 1.0;
+  const float q = __fdividef(top_float(num), top_float(den));
+  bool less = q < r.q * 0.99999f;
+  if (!less && !(q > r.q * 1.00001f)) less = dbits(num * r.den) < dbits(r.num * den);
+  if (less) r = LimiterRatio{num, den, q};
+}
+// The four ratios of a cell from one reciprocal (simultaneous inversion, a few ulps from four
+// divisions).  Every den is 1, or 2 |d2| + 2e-10 >= 2e-5 with d2 a jump of the flow over a face: the
+// product of four stays far from the range limits of double.
+__device__ __forceinline__ V4<double> limiter_ratios(const LimiterRatio& a, const LimiterRatio& b,
+                                                     const LimiterRatio& c, const LimiterRatio& d) {
+  const double ab = a.den * b.den, cd = c.den * d.den;
+  const double inv = rcp64(ab * cd);
+  const double iab = inv * cd, icd = inv * ab;
+  return V4<double>{a.num * (iab * b.den), b.num * (iab * a.den), c.num * (icd * d.den), d.num * (icd * c.den)};
 }
 
 // Faces per cell: triangles and quadrilaterals, the only cells the reference's quadrature accepts
@@ -601,19 +638,17 @@ __device__ __forceinline__ void recon_tile_body(const StageArgs<P>& a, const int
   a.si[2 * c] = flag0;
 }
 
-// reconstruct for the FP64-heavy policies (ref, fp64): the stencil values are staged in shared
-// memory in batches (indices, then gathers), then each face side's O3 sum runs over the staged
-// values with its weights loaded eight at a time.  These policies are bound by the FP64 pipe, so
-// the kernel keeps the per-face loop (no work on missing face slots) and a small register set.
-template <class P>
-__device__ __forceinline__ void recon_staged_body(const StageArgs<P>& a, const int blk) {
+// reconstruct for the ref policy: the stencil values are staged in shared memory in batches (indices,
+// then gathers), then each face side's O3 sum runs over the staged values with its weights loaded
+// eight at a time.  The policy is bound by the FP64 pipe, so the kernel keeps the per-face loop (no
+// work on missing face slots) and a small register set.
+__device__ __forceinline__ void recon_ref_body(const StageArgs<PolicyRef>& a, const int blk) {
+  using P = PolicyRef;
   using S = typename P::S;
   using G = typename P::G;
   using WT = typename P::W;
-  // fp64 stages only the compact stencil (kCompact), ref the whole stencil
-  constexpr bool kCompact = P::id == PolicyFP64::id;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  V4<S>* sv = reinterpret_cast<V4<S>*>(smem_raw);  // [maxM or maxS][blockDim] staged stencil values
+  V4<S>* sv = reinterpret_cast<V4<S>*>(smem_raw);  // [maxS][blockDim] staged stencil values
   const int t = threadIdx.x, B = blockDim.x;
   const int c = blk * B + t;
   if (c >= a.Nc) return;
@@ -621,34 +656,17 @@ __device__ __forceinline__ void recon_staged_body(const StageArgs<P>& a, const i
   const int nS = a.nS[c], nM = a.nM[c];
   const V4<WT> wc = a.W[c];
   const S pc = (S)wc.x, uxc = (S)wc.y, uyc = (S)wc.z, tc = (S)wc.w;
-  // fp64: only the compact stencil (the face neighbours, at most kMaxFaces) is staged: the
-  // gradient, the min/max and the uniform-cell test need nothing else, and only cells that are not
-  // uniform read the rest of the stencil, in their O3 loop.  32-byte values make whole-stencil
-  // staging the occupancy limit (3 blocks an SM); with it, 4.  The ref policy's 16-byte values
-  // leave room for the whole stencil, which its smooth-flow cells reuse across faces.
-  if constexpr (!kCompact) {
-    constexpr int GB = 4;
-    for (int i0 = 0; i0 < nS; i0 += GB) {
-      int j[GB];
+  constexpr int GB = 4;
+  for (int i0 = 0; i0 < nS; i0 += GB) {
+    int j[GB];
 #pragma unroll
-      for (int u = 0; u < GB; ++u) j[u] = (i0 + u < nS) ? a.sten[(i0 + u) * ldc + c] : c;
-      V4<WT> wj[GB];
+    for (int u = 0; u < GB; ++u) j[u] = (i0 + u < nS) ? a.sten[(i0 + u) * ldc + c] : c;
+    V4<WT> wj[GB];
 #pragma unroll
-      for (int u = 0; u < GB; ++u) wj[u] = a.W[j[u]];
+    for (int u = 0; u < GB; ++u) wj[u] = a.W[j[u]];
 #pragma unroll
-      for (int u = 0; u < GB; ++u)
-        if (i0 + u < nS) sv[(i0 + u) * B + t] = V4<S>{(S)wj[u].x, (S)wj[u].y, (S)wj[u].z, (S)wj[u].w};
-    }
-  } else {
-    int j[kMaxFaces];
-#pragma unroll
-    for (int u = 0; u < kMaxFaces; ++u) j[u] = u < nM ? a.sten[u * ldc + c] : c;
-    V4<WT> wj[kMaxFaces];
-#pragma unroll
-    for (int u = 0; u < kMaxFaces; ++u) wj[u] = a.W[j[u]];
-#pragma unroll
-    for (int u = 0; u < kMaxFaces; ++u)
-      if (u < nM) sv[u * B + t] = V4<S>{(S)wj[u].x, (S)wj[u].y, (S)wj[u].z, (S)wj[u].w};
+    for (int u = 0; u < GB; ++u)
+      if (i0 + u < nS) sv[(i0 + u) * B + t] = V4<S>{(S)wj[u].x, (S)wj[u].y, (S)wj[u].z, (S)wj[u].w};
   }
 
   G gPx = 0, gPy = 0, gUxx = 0, gUxy = 0, gUyx = 0, gUyy = 0, gTx = 0, gTy = 0;
@@ -724,43 +742,14 @@ __device__ __forceinline__ void recon_staged_body(const StageArgs<P>& a, const i
       G uxf = wk * uxc;
       G uyf = wk * uyc;
       G tf = wk * tc;
-      // fp64: weights, stencil ids and the members past the compact stencil in batches of four
-      // (those from memory, the compact ones staged); ref: weights in batches of eight, every
-      // member staged.  Sums in stencil order either way.
-      if constexpr (!kCompact) {
-        for (int ci0 = 0; ci0 < nS; ci0 += 8) {
-          S wb[8];
+      for (int ci0 = 0; ci0 < nS; ci0 += 8) {
+        S wb[8];
 #pragma unroll
-          for (int u = 0; u < 8; ++u) wb[u] = (ci0 + u < nS) ? w[(size_t)(ci0 + u + 1) * ldc] : S(0);
+        for (int u = 0; u < 8; ++u) wb[u] = (ci0 + u < nS) ? w[(size_t)(ci0 + u + 1) * ldc] : S(0);
 #pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            if (ci0 + u < nS) {
-              const V4<S> v = sv[(ci0 + u) * B + t];
-              pf += wb[u] * v.x;
-              uxf += wb[u] * v.y;
-              uyf += wb[u] * v.z;
-              tf += wb[u] * v.w;
-            }
-          }
-        }
-      } else
-      for (int ci0 = 0; ci0 < nS; ci0 += 4) {
-        S wb[4];
-        int jj[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int ci = ci0 + u;
-          wb[u] = ci < nS ? w[(size_t)(ci + 1) * ldc] : S(0);
-          jj[u] = (ci < nS && ci >= nM) ? a.sten[ci * ldc + c] : c;
-        }
-        V4<WT> wv[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) wv[u] = a.W[jj[u]];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int ci = ci0 + u;
-          if (ci < nS) {
-            const V4<S> v = ci < nM ? sv[ci * B + t] : V4<S>{(S)wv[u].x, (S)wv[u].y, (S)wv[u].z, (S)wv[u].w};
+        for (int u = 0; u < 8; ++u) {
+          if (ci0 + u < nS) {
+            const V4<S> v = sv[(ci0 + u) * B + t];
             pf += wb[u] * v.x;
             uxf += wb[u] * v.y;
             uyf += wb[u] * v.z;
@@ -796,14 +785,163 @@ __device__ __forceinline__ void recon_staged_body(const StageArgs<P>& a, const i
   a.si[2 * c] = flag0;
 }
 
+// reconstruct for the fp64 policy.  The FP64 pipe bounds it (one warp instruction in 16 clocks of the
+// SM), so the kernel is laid out by its FP64 instructions: the O3 sums (4 products a member and face
+// side) are most of them, every comparison, minimum and selection runs on integers, and the limiter
+// divides once per cell (limiter_process_ratio).  Only the compact stencil (the face neighbours) is
+// staged in shared memory: the gradient, the min/max and the uniform-cell test need nothing else, and
+// the O3 loop of a cell that is not uniform reads the other members from memory.  500k triangles, no
+// uniform cells: 628 us a launch with FP64 comparisons and a division per face and variable, 352 now
+// (364 FP64 warp instructions, 180 of them the O3 sums; the pipe 86% busy).
+__device__ __forceinline__ void recon_fp64_body(const StageArgs<PolicyFP64>& a, const int blk) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  V4<double>* sv = reinterpret_cast<V4<double>*>(smem_raw);  // [maxM][blockDim] the face neighbours' states
+  const int t = threadIdx.x, B = blockDim.x;
+  const int c = blk * B + t;
+  if (c >= a.Nc) return;
+  const int ldc = a.ldc;
+  const int nS = a.nS[c], nM = a.nM[c];
+  const V4<double> wc = a.W[c];
+  {
+    int j[kMaxFaces];
+#pragma unroll
+    for (int u = 0; u < kMaxFaces; ++u) j[u] = u < nM ? a.sten[u * ldc + c] : c;
+    V4<double> wj[kMaxFaces];
+#pragma unroll
+    for (int u = 0; u < kMaxFaces; ++u) wj[u] = a.W[j[u]];
+#pragma unroll
+    for (int u = 0; u < kMaxFaces; ++u)
+      if (u < nM) sv[u * B + t] = wj[u];
+  }
+  // reference :148-169 (least-squares gradient) and :190-205 (min and max over the face neighbours)
+  double gPx = 0, gPy = 0, gUxx = 0, gUxy = 0, gUyx = 0, gUyy = 0, gTx = 0, gTy = 0;
+  V4<double> mx = wc, mn = wc;
+  for (int i = 0; i < nM; ++i) {
+    const V2<double> m = a.lsm[i * ldc + c];
+    const V4<double> v = sv[i * B + t];
+    double dphi = v.x - wc.x;
+    gPx += m.x * dphi;
+    gPy += m.y * dphi;
+    dphi = v.y - wc.y;
+    gUxx += m.x * dphi;
+    gUyx += m.y * dphi;
+    dphi = v.z - wc.z;
+    gUxy += m.x * dphi;
+    gUyy += m.y * dphi;
+    dphi = v.w - wc.w;
+    gTx += m.x * dphi;
+    gTy += m.y * dphi;
+    mx = V4<double>{dmax_(v.x, mx.x), dmax_(v.y, mx.y), dmax_(v.z, mx.z), dmax_(v.w, mx.w)};
+    mn = V4<double>{dmin_(v.x, mn.x), dmin_(v.y, mn.y), dmin_(v.z, mn.z), dmin_(v.w, mn.w)};
+  }
+  a.grad[2 * c] = V4<double>{gPx, gPy, gUxx, gUxy};
+  a.grad[2 * c + 1] = V4<double>{gUyx, gUyy, gTx, gTy};
+
+  V4<double> L{1.0, 1.0, 1.0, 1.0};
+  int8_t flag0 = 0;
+  const double rangeT = mx.w - mn.w;
+  const bool flat = abs_lt(rangeT, 1e-10);  // reference :208-233: linear face values, no limiting
+  // which variables take the O3 value (the reference's threshold on their range)
+  const bool o3x = abs_ge(mx.x - mn.x, 1e-5), o3y = abs_ge(mx.y - mn.y, 1e-5), o3z = abs_ge(mx.z - mn.z, 1e-5),
+             o3w = abs_ge(rangeT, 1e-5);
+  LimiterRatio lp{2.0, 1.0, 2.f}, lux = lp, luy = lp, lt = lp;
+  double smooth = 0.0;
+  bool notTrouble = true;
+  for (int fi = 0; fi < nM; ++fi) {
+    int f = a.cf[fi * ldc + c];
+    const bool isNei = (f < 0);
+    f = abs(f) - 1;
+    if (f >= a.Nf) continue;
+    const V2<double> d = a.sg[fi * ldc + c];
+    V4<double> o;
+    if (flat) {
+      o.x = wc.x + gPx * d.x + gPy * d.y;
+      o.y = wc.y + gUxx * d.x + gUyx * d.y;
+      o.z = wc.z + gUxy * d.x + gUyy * d.y;
+      o.w = wc.w + gTx * d.x + gTy * d.y;
+    } else {  // reference :235-314
+      const V2<double> rf = a.sr[fi * ldc + c];  // (1 / delta r, fraction)
+      const double* w = a.wts + (size_t)(fi * (a.maxS + 1)) * ldc + c;
+      const double w0 = w[0];
+      double pf = w0 * wc.x, uxf = w0 * wc.y, uyf = w0 * wc.z, tf = w0 * wc.w;
+      // weights, stencil ids and the members past the compact stencil in batches of four (those from
+      // memory, the compact ones staged); sums in stencil order
+      for (int ci0 = 0; ci0 < nS; ci0 += 4) {
+        double wb[4];
+        int jj[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int ci = ci0 + u;
+          wb[u] = ci < nS ? w[(size_t)(ci + 1) * ldc] : 0.0;
+          jj[u] = (ci < nS && ci >= nM) ? a.sten[ci * ldc + c] : c;
+        }
+        V4<double> wv[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) wv[u] = a.W[jj[u]];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int ci = ci0 + u;
+          if (ci < nS) {
+            const V4<double> v = ci < nM ? sv[ci * B + t] : wv[u];
+            pf += wb[u] * v.x;
+            uxf += wb[u] * v.y;
+            uyf += wb[u] * v.z;
+            tf += wb[u] * v.w;
+          }
+        }
+      }
+      const double pnb = sv[fi * B + t].x;
+      double phif, d2;
+      limiter_process_ratio(lp, phif, d2, wc.x, mx.x, mn.x, gPx, gPy, d.x, d.y);
+      o.x = o3x ? pf : phif;
+      // |(1 - w) p_c + w p_n - p_f| / delta r
+      double jump = dabs_(rf.y * (pnb - wc.x) - d2) * rf.x;
+      if (le_zero(pf) || le_zero(phif)) jump += le_zero(pf) && le_zero(phif) ? 2e20 : 1e20;
+      smooth = dnan_(jump) ? smooth : dbits(jump) > dbits(smooth) ? jump : smooth;
+      limiter_process_ratio(lux, phif, d2, wc.y, mx.y, mn.y, gUxx, gUyx, d.x, d.y);
+      o.y = o3y ? uxf : phif;
+      limiter_process_ratio(luy, phif, d2, wc.z, mx.z, mn.z, gUxy, gUyy, d.x, d.y);
+      o.z = o3z ? uyf : phif;
+      limiter_process_ratio(lt, phif, d2, wc.w, mx.w, mn.w, gTx, gTy, d.x, d.y);
+      o.w = o3w ? tf : phif;
+      notTrouble = gt_zero(phif);
+    }
+    a.fv[2 * f + isNei] = o;
+  }
+  if (!flat) {
+    if (notTrouble)
+      L = limiter_ratios(lp, lux, luy, lt);
+    else
+      L = V4<double>{0.0, 0.0, 0.0, 0.0};
+    const double scale = notTrouble ? 0.5 * (mx.x + mn.x) + 1e-10 : 1e-10;
+    flag0 = !neg_(scale) && dbits(smooth) > dbits(scale);  // smooth / scale > 1
+  }
+  a.lim[c] = L;
+  a.si[2 * c] = flag0;
+}
+
+__device__ __forceinline__ double mul64(const double a, const double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double add64(const double a, const double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double sub64(const double a, const double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ double fma64(const double a, const double b, const double c) { return __fma_rn(a, b, c); }
+// w + lim (ga dx + gb dy): the limited linear (TVD) value
+__device__ __forceinline__ double tvd64(const double w, const double lim, const double ga, const double gb,
+                                        const double dx, const double dy) {
+  return fma64(lim, fma64(ga, dx, mul64(gb, dy)), w);
+}
+
 // Limiter maps (reference cudaLimiter.h:14-32)
 template <class S>
 __device__ __forceinline__ S to_bj(const S y) {
-  return fmn(S(2) * y, S(1));
+  return gmn(S(2) * y, S(1));
 }
 template <class S>
 __device__ __forceinline__ S to_venkat(const S y) {
-  return fmn((y * y + y + AFAR_LIT(S, 1e-10)) / (y * y + S(0.5) + S(0.5) * y + AFAR_LIT(S, 1e-10)), S(1));
+  const S num = y * y + y + AFAR_LIT(S, 1e-10), den = y * y + S(0.5) + S(0.5) * y + AFAR_LIT(S, 1e-10);
+  if constexpr (std::is_same<S, double>::value)
+    return dmin_(num * rcp64(den), 1.0);
+  else
+    return fmn(num / den, S(1));
 }
 
 // BVDindicator (reference cudaLimiter.h:319-464): stencil flag counts, BVD test on T, final
@@ -861,10 +999,22 @@ __device__ __forceinline__ void bvd_body(const StageArgs<P>& a, const int blk) {
     const G tfCur = pick<P>(isNei, !isNei, tfNei, tfOwn);
     const G tfOther = pick<P>(!isNei, isNei, tfNei, tfOwn);
     const G lim = to_bj(L.w);
-    const G tfTVD = tc + lim * (gTx * d.x + gTy * d.y);
-    const int typeval = fab(tfTVD - tfOther) < AFAR_LIT(S, 0.5) * fab(tfCur - tfOther);
-    const int notFlat = fab(tfCur - tfOther) > AFAR_LIT(S, 1e-10);
-    const int limited = (lim < AFAR_LIT(S, 0.9)) + (shockTypeExt > 0);
+    G tfTVD;
+    if constexpr (P::id == PolicyFP64::id)
+      tfTVD = tvd64(tc, lim, gTx, gTy, d.x, d.y);
+    else
+      tfTVD = tc + lim * (gTx * d.x + gTy * d.y);
+    int typeval, notFlat, limited;
+    if constexpr (P::id == PolicyFP64::id) {  // the same comparisons on integers (L.w >= 0)
+      const double jump = dabs_(tfCur - tfOther);
+      typeval = dbits(dabs_(tfTVD - tfOther)) < dbits(0.5 * jump) && !dnan_(jump);
+      notFlat = !abs_lt(jump, 1e-10) && dbits(jump) != dbits(1e-10) && !dnan_(jump);
+      limited = (dbits(L.w) < dbits(0.45)) + (shockTypeExt > 0);
+    } else {
+      typeval = fab(tfTVD - tfOther) < AFAR_LIT(S, 0.5) * fab(tfCur - tfOther);
+      notFlat = fab(tfCur - tfOther) > AFAR_LIT(S, 1e-10);
+      limited = (lim < AFAR_LIT(S, 0.9)) + (shockTypeExt > 0);
+    }
     bvdType = max(bvdType, notFlat * limited * typeval);
   }
   const int finalType = (shockType > 0) * (shockTypeExt > 1) * (-2) + (bvdType > 0);
@@ -1016,9 +1166,7 @@ __device__ __forceinline__ void roe_flux(G& rhoFlux, G& rhoUxFlux, G& rhoUyFlux,
 // folded: p/rho as R T (the state's own equation of state), one reciprocal of magSf (precomputed
 // per face), of c^2 and of lambda, gamma and K computed once on the host, and the entropy fix's
 // division only on the faces that need it.  Equal to the reference's expressions up to rounding.
-__device__ __forceinline__ double fdiv(const double a, const double b) { return a / b; }
 __device__ __forceinline__ float fdiv(const float a, const float b) { return __fdividef(a, b); }
-__device__ __forceinline__ double rsqrt_(const double a) { return rsqrt(a); }
 __device__ __forceinline__ float rsqrt_(const float a) { return rsqrtf(a); }
 
 template <class D>
@@ -1102,6 +1250,154 @@ __device__ __forceinline__ void kfvs_flux_fast(D& rhoFlux, D& rhoUxFlux, D& rhoU
   rhoEFlux += trhoE * magSf - D(0.5) * rhoFlux * (Cv * tL + D(0.5) * (uxL * uxL + uyL * uyL) + R * tL) -
               D(0.5) * rhoFlux * (Cv * tR + D(0.5) * (uxR * uxR + uyR * uyR) + R * tR);
   rhoFlux += trho * magSf - D(0.5) * rhoL * (uxL * Sfx + uyL * Sfy) - D(0.5) * rhoR * (uxR * Sfx + uyR * Sfy);
+}
+
+// minimizeDeltaValue (min_delta) of doubles with the minima and the sign on integers.
+__device__ __forceinline__ double min_delta64(const double l, const double r, const double lT, const double rT) {
+  const double d = __dsub_rn(r, l);
+  double m = min_nonneg(dabs_(d), dabs_(__dsub_rn(r, lT)));
+  m = min_nonneg(m, dabs_(__dsub_rn(rT, l)));
+  m = min_nonneg(m, dabs_(__dsub_rn(rT, lT)));
+  return flip_sign(m, __double2hiint(d) & (int)0x80000000);
+}
+
+// One side of a face under the fp64 policy: the state that the flux uses.
+struct Side64 {
+  double p, ux, uy, T, rho;
+};
+
+// The flux of a face under the fp64 policy: central flux with the Roe dissipation, or the KFVS flux,
+// laid out by FP64 instructions: the two sides share their factors; the central flux takes Sf itself,
+// so that the fluxes of a uniform stream close over a cell as its face vectors do; the Roe weights
+// from one root and one reciprocal (sqrt(rhoL)/(sqrt(rhoL)+sqrt(rhoR)) = rhoL/(rhoL + sqrt(rhoL rhoR)));
+// the wave strengths summed before they multiply the eigenvectors; and the acoustic entropy fix, which
+// needs both sides' sound speeds, behind an FP32 look (20 bits of each operand, a margin of 1e-5 of
+// all speeds) at whether its waves are surely outside it, as all but the near-sonic ones are.
+// Every rounding is written out: the kernels of this policy (single and batched, of every block size,
+// face-centre and multi-point) then agree bit for bit whatever multiply-adds the compiler would fuse.
+// 750k faces: 426 us a launch before (244 FP64 instructions a face), 240 now (158 issued; the pipe 85%
+// busy); the stage-1 form with the Courant step 280.
+struct Gas64 {
+  double R, Cv, Cp, gm1, iR;
+  float gRf;
+};
+template <class A>
+__device__ __forceinline__ Gas64 gas64(const A& a) {
+  return Gas64{a.R, a.Cv, a.Cp, a.gm1, a.invR, a.gRf};
+}
+// The entropy fix of one wave: |lambda| below eps = 2 max(0, jump) becomes (lambda^2 + eps^2)/(2 eps).
+__device__ __forceinline__ double entropy_fix64(const double l, const double jump) {
+  const double eps = gt_zero(jump) ? add64(jump, jump) : 0.0;
+  if (!(dbits(l) < dbits(eps))) return l;
+  return mul64(fma64(l, l, mul64(eps, eps)), rcp64(fma64(2.0, eps, 1e-30)));
+}
+// One side's kinetic moments (reference cudaRiemannSolver.h:16-68): the half-range fluxes of mass,
+// normal and tangential momentum and energy per unit area; sign +1 from the left, -1 from the right.
+__device__ __forceinline__ V4<double> kinetic_side64(const Side64& q, const double sign, const double u, const double v,
+                                                     const double R, const double K) {
+  const double il = mul64(add64(R, R), q.T);  // 1/lambda = 2 p / rho
+  const double lam = rcp64(il), rs = rsq64(lam);
+  const double m0 = mul64(0.5, erfc(mul64(-sign, mul64(mul64(lam, rs), u))));
+  const double ex = mul64(mul64(sign * 0.28209479177387814, rs), exp(mul64(mul64(-lam, u), u)));  // 1/(2 sqrt(pi))
+  const double m1 = fma64(u, m0, ex);
+  const double m2 = fma64(u, m1, mul64(mul64(0.5, m0), il));
+  const double m3 = fma64(u, m2, mul64(m1, il));
+  const double e = fma64(m1, fma64(v, v, mul64(mul64(0.5, il), add64(1.0, K))), m3);
+  const double rm1 = mul64(q.rho, m1);
+  return V4<double>{rm1, mul64(q.rho, m2), mul64(rm1, v), mul64(mul64(0.5, q.rho), e)};
+}
+__device__ __forceinline__ V4<double> face_flux64(const Side64& l, const Side64& r, const double pLT, const double pRT,
+                                                  const double rhoLT, const double rhoRT, const bool isShock,
+                                                  const Gas64& k, const V4<double>& fs) {
+  const double Sfx = fs.x, Sfy = fs.y, nx = mul64(Sfx, fs.w), ny = mul64(Sfy, fs.w);
+  const double unL = fma64(l.uy, Sfy, mul64(l.ux, Sfx)), unR = fma64(r.uy, Sfy, mul64(r.ux, Sfx));  // times |Sf|
+  const double cvL = mul64(unL, fs.w), cvR = mul64(unR, fs.w);
+  if (isShock) {
+    const double K = fma64(mul64(2.0, k.Cv), k.iR, -2.0);
+    const V4<double> a = kinetic_side64(l, 1.0, cvL, fma64(l.uy, nx, mul64(-l.ux, ny)), k.R, K);
+    const V4<double> b = kinetic_side64(r, -1.0, cvR, fma64(r.uy, nx, mul64(-r.ux, ny)), k.R, K);
+    const double tn = add64(a.y, b.y), tt = add64(a.z, b.z);
+    return V4<double>{mul64(add64(a.x, b.x), fs.z), fma64(tn, Sfx, mul64(-tt, Sfy)), fma64(tn, Sfy, mul64(tt, Sfx)),
+                      mul64(add64(a.w, b.w), fs.z)};
+  }
+  const double kL = fma64(l.uy, l.uy, mul64(l.ux, l.ux)), kR = fma64(r.uy, r.uy, mul64(r.ux, r.ux));
+  const double hL = fma64(0.5, kL, mul64(k.Cp, l.T)), hR = fma64(0.5, kR, mul64(k.Cp, r.T));  // p/rho = R T
+  const double M = fma64(r.rho, unR, mul64(l.rho, unL)), hF = mul64(0.25, M), hp = mul64(0.5, add64(l.p, r.p));
+  const double dP = min_delta64(l.p, r.p, pLT, pRT), dRho = min_delta64(l.rho, r.rho, rhoLT, rhoRT);
+  const double tiny = 1e-20;
+  const double rl = dmax_(l.rho, tiny), rr = dmax_(r.rho, tiny);
+  const double rho2 = mul64(rl, rr);
+  const double rhoT = mul64(rho2, rsq64(rho2));
+  const double wL = mul64(rl, rcp64(add64(rl, rhoT)));
+  const double dUx = sub64(r.ux, l.ux), dUy = sub64(r.uy, l.uy);
+  const double uxT = fma64(-wL, dUx, r.ux), uyT = fma64(-wL, dUy, r.uy);
+  const double hT = fma64(-wL, sub64(hR, hL), hR);
+  const double kT = mul64(0.5, fma64(uyT, uyT, mul64(uxT, uxT)));
+  const double cT2 = dmax_(mul64(k.gm1, sub64(hT, kT)), tiny);
+  const double rcT = rsq64(cT2);
+  const double cT = mul64(cT2, rcT), ic2 = mul64(rcT, rcT);
+  const double cvT = fma64(uyT, ny, mul64(uxT, nx));
+  const double dCv = fma64(dUy, ny, mul64(dUx, nx));
+  const double rc = mul64(mul64(rhoT, cT), dCv), hic2 = mul64(0.5, ic2);
+  double l1 = dabs_(sub64(cvT, cT)), l3 = dabs_(add64(cvT, cT));
+  const double l2 = entropy_fix64(dabs_(cvT), sub64(cvR, cvL));
+  {
+    const float uL = top_float(cvL), uR = top_float(cvR), c = top_float(cT);
+    const float cL = sqrtf(k.gRf * top_float(l.T)), cR = sqrtf(k.gRf * top_float(r.T));
+    const float margin = 1e-5f * (fabsf(uL) + fabsf(uR) + cL + cR + c);
+    const bool clear1 = top_float(l1) > 2.f * fmaxf(0.f, (uR - cR) - (uL - cL)) + margin;
+    const bool clear3 = top_float(l3) > 2.f * fmaxf(0.f, (uR + cR) - (uL + cL)) + margin;
+    if (!(clear1 && clear3)) {
+      const double xL = dmax_(mul64(k.gm1, mul64(k.Cp, l.T)), tiny), xR = dmax_(mul64(k.gm1, mul64(k.Cp, r.T)), tiny);
+      const double sL = mul64(xL, rsq64(xL)), sR = mul64(xR, rsq64(xR));
+      l1 = entropy_fix64(l1, sub64(sub64(cvR, sR), sub64(cvL, sL)));
+      l3 = entropy_fix64(l3, sub64(add64(cvR, sR), add64(cvL, sL)));
+    }
+  }
+  const double a1 = mul64(mul64(sub64(dP, rc), hic2), l1), a3 = mul64(mul64(add64(dP, rc), hic2), l3);
+  const double a2 = mul64(fma64(-dP, ic2, dRho), l2);
+  const double s13 = add64(a1, a3), s = add64(s13, a2), b = mul64(sub64(a3, a1), cT);
+  const double gt = mul64(mul64(l2, rhoT), fma64(dUy, nx, mul64(-dUx, ny)));  // the shear wave
+  const double h = mul64(-0.5, fs.z);
+  const double d1 = fma64(-gt, ny, fma64(b, nx, mul64(s, uxT)));
+  const double d2 = fma64(gt, nx, fma64(b, ny, mul64(s, uyT)));
+  const double d3 = fma64(gt, fma64(uyT, nx, mul64(-uxT, ny)), fma64(a2, kT, fma64(b, cvT, mul64(s13, hT))));
+  return V4<double>{fma64(h, s, mul64(0.5, M)), fma64(h, d1, fma64(hp, Sfx, mul64(hF, add64(l.ux, r.ux)))),
+                    fma64(h, d2, fma64(hp, Sfy, mul64(hF, add64(l.uy, r.uy)))), fma64(h, d3, mul64(hF, add64(hL, hR)))};
+}
+// The densities of a face's two states and their two TVD states (p/(R T)) from one reciprocal
+// (simultaneous inversion of the four temperatures, a few ulps from four divisions; their product
+// neither overflows nor underflows).
+__device__ __forceinline__ void densities64(double& rhoL, double& rhoR, double& rhoLT, double& rhoRT, const double pL,
+                                            const double pR, const double pLT, const double pRT, const double tL,
+                                            const double tR, const double tLT, const double tRT, const double iR) {
+  const double tt = mul64(tL, tR), ttT = mul64(tLT, tRT);
+  const double inv = mul64(iR, rcp64(mul64(tt, ttT)));
+  const double itt = mul64(inv, ttT), ittT = mul64(inv, tt);  // 1/(R tL tR), 1/(R tLT tRT)
+  rhoL = mul64(pL, mul64(itt, tR));
+  rhoR = mul64(pR, mul64(itt, tL));
+  rhoLT = mul64(pLT, mul64(ittT, tRT));
+  rhoRT = mul64(pRT, mul64(ittT, tLT));
+}
+// The Courant step of one face in FP64 for the fp64 policy (setDeltaT, reference
+// cudaFieldOperation.h:140-157).  Every rounding is written out, so the fused stage-1 flux and the
+// separate pass give the same bits.
+__device__ __forceinline__ double courant_dt64(const double CFL, const double gR, const V2<double> g,
+                                               const V4<double>& fs, const V4<double>& Wo, const V4<double>& Wn) {
+  const double w1 = g.y, w0 = __dadd_rn(1.0, -w1);
+  const double unL = dabs_(__fma_rn(Wo.y, fs.x, __dmul_rn(Wo.z, fs.y)));
+  const double unR = dabs_(__fma_rn(Wn.y, fs.x, __dmul_rn(Wn.z, fs.y)));
+  const double c2 = __dmul_rn(gR, __fma_rn(w0, Wo.w, __dmul_rn(w1, Wn.w)));
+  const double c = __dmul_rn(c2, rsq64(c2));
+  const double den = __fma_rn(c, fs.z, __fma_rn(w0, unL, __dmul_rn(w1, unR)));
+  return __dmul_rn(__dmul_rn(__dmul_rn(CFL, g.x), fs.z), rcp64(den));
+}
+// The same to about 1e-5 in FP32, from 20 bits of each operand and without the Courant number.
+__device__ __forceinline__ float courant_estimate(const float gRf, const V2<double> g, const V4<double>& fs,
+                                                  const V4<double>& Wo, const V4<double>& Wn) {
+  const float w1 = top_float(g.y), w0 = 1.f - w1, i = top_float(fs.w), x = i * top_float(fs.x), y = i * top_float(fs.y);
+  const float uL = fabsf(top_float(Wo.y) * x + top_float(Wo.z) * y), uR = fabsf(top_float(Wn.y) * x + top_float(Wn.z) * y);
+  return __fdividef(top_float(g.x), w0 * uL + w1 * uR + sqrtf(gRf * (w0 * top_float(Wo.w) + w1 * top_float(Wn.w))));
 }
 
 // ---------------------------------------------------------------- ref policy: face flux
@@ -1240,12 +1536,34 @@ __device__ __forceinline__ void flux_body(const StageArgs<P>& a, const int blk) 
     }
     __syncthreads();
   }
-  double dtf = 1e5;
   float dtf32 = 1e5f;
+  float est = __int_as_float(0x7F800000);  // fp64: the face's Courant step over the Courant number
   if (id < a.Nf) {
     if constexpr (P::id == PolicyRef::id) {
       static_assert(!DT, "under the ref policy the Courant step is a kernel of its own, as in the reference");
       flux_ref_face(a, id);
+    } else if constexpr (P::id == PolicyFP64::id) {
+      const int2 on = a.on[id];
+      const V4<double> fd = a.fd[id], fs = a.fs[id];
+      const int8_t sL = a.si[2 * on.x + 1], sR = a.si[2 * on.y + 1];
+      const V4<double> Wo = a.W[on.x], Wn = a.W[on.y];
+      const V4<double> go0 = a.grad[2 * on.x], go1 = a.grad[2 * on.x + 1];
+      const V4<double> gn0 = a.grad[2 * on.y], gn1 = a.grad[2 * on.y + 1];
+      const V4<double> lo = a.lim[on.x], ln = a.lim[on.y];
+      const V4<double> fo = a.fv[2 * id], fn = a.fv[2 * id + 1];
+      const double pLT = tvd64(Wo.x, lo.x, go0.x, go0.y, fd.x, fd.y), tLT = tvd64(Wo.w, lo.w, go1.z, go1.w, fd.x, fd.y);
+      const double pRT = tvd64(Wn.x, ln.x, gn0.x, gn0.y, fd.z, fd.w), tRT = tvd64(Wn.w, ln.w, gn1.z, gn1.w, fd.z, fd.w);
+      Side64 l{fo.x, fo.y, fo.z, fo.w, 0.0}, r{fn.x, fn.y, fn.z, fn.w, 0.0};
+      if (sL != 0)  // the TVD velocities only where the switch asks for them
+        l = Side64{pLT, tvd64(Wo.y, lo.y, go0.z, go1.x, fd.x, fd.y), tvd64(Wo.z, lo.z, go0.w, go1.y, fd.x, fd.y), tLT, 0.0};
+      if (sR != 0)
+        r = Side64{pRT, tvd64(Wn.y, ln.y, gn0.z, gn1.x, fd.z, fd.w), tvd64(Wn.z, ln.z, gn0.w, gn1.y, fd.z, fd.w), tRT, 0.0};
+      double rhoLT, rhoRT;
+      densities64(l.rho, r.rho, rhoLT, rhoRT, l.p, r.p, pLT, pRT, l.T, r.T, tLT, tRT, a.invR);
+      a.flux[id] = face_flux64(l, r, pLT, pRT, rhoLT, rhoRT, sL < 0 || sR < 0, gas64(a), fs);
+      if constexpr (DT) {
+        est = courant_estimate(a.gRf, a.dtg[id], fs, Wo, Wn);
+      }
     } else {
       const int2 on = a.on[id];
       const int own = on.x, nei = on.y;
@@ -1256,18 +1574,7 @@ __device__ __forceinline__ void flux_body(const StageArgs<P>& a, const int blk) 
       const bool isShock = sL < 0 || sR < 0;
       const V4<G> fs = a.fs[id];
       const G Sfx = fs.x, Sfy = fs.y, magSf = fs.z;
-      G R, Cv, iR, gam;
-      if constexpr (kF32) {
-        R = a.Rf;
-        Cv = a.Cvf;
-        iR = a.invRf;
-        gam = a.gm1f + 1.f;
-      } else {
-        R = (G)a.R;
-        Cv = (G)a.Cv;
-        iR = (G)a.invR;
-        gam = (G)a.gamma;
-      }
+      const G R = a.Rf, Cv = a.Cvf, iR = a.invRf, gam = a.gm1f + 1.f;
       const V4<typename P::W> Wo = a.W[own], Wn = a.W[nei];
       const V4<G> go0 = a.grad[2 * own], go1 = a.grad[2 * own + 1];
       const V4<G> gn0 = a.grad[2 * nei], gn1 = a.grad[2 * nei + 1];
@@ -1292,25 +1599,9 @@ __device__ __forceinline__ void flux_body(const StageArgs<P>& a, const int blk) 
         const G uxR = pick<P>(!tvdR, tvdR, fn.y, uxRT);
         const G uyR = pick<P>(!tvdR, tvdR, fn.z, uyRT);
         const G tR = pick<P>(!tvdR, tvdR, fn.w, tRT);
-        G rhoLT, rhoRT, rhoL, rhoR;  // p / (R T) of the four states
-        if constexpr (kF32) {
-          rhoLT = fdiv(pLT * iR, tLT);
-          rhoRT = fdiv(pRT * iR, tRT);
-          rhoL = fdiv(pL * iR, tL);
-          rhoR = fdiv(pR * iR, tR);
-        } else {
-          // FP64: the four reciprocal temperatures from one division (Montgomery's simultaneous
-          // inversion, a few ulps from four divisions); a double division is among the dearest
-          // operations of GB300's FP64 pipe, which bounds this kernel.  Temperatures stay far from
-          // the range limits of double (their product of four neither overflows nor underflows).
-          const G tt = tL * tR, ttT = tLT * tRT;
-          const G inv = G(1) / (tt * ttT);
-          const G itt = inv * ttT, ittT = inv * tt;  // 1/(tL tR), 1/(tLT tRT)
-          rhoL = pL * iR * (itt * tR);
-          rhoR = pR * iR * (itt * tL);
-          rhoLT = pLT * iR * (ittT * tRT);
-          rhoRT = pRT * iR * (ittT * tLT);
-        }
+        // p / (R T) of the four states
+        const G rhoLT = fdiv(pLT * iR, tLT), rhoRT = fdiv(pRT * iR, tRT);
+        const G rhoL = fdiv(pL * iR, tL), rhoR = fdiv(pR * iR, tR);
         dP = min_delta<D, G>(pL, pR, pLT, pRT);
         dRho = min_delta<D, G>(rhoL, rhoR, rhoLT, rhoRT);
         const G h = G(0.5);
@@ -1332,22 +1623,10 @@ __device__ __forceinline__ void flux_body(const StageArgs<P>& a, const int blk) 
                          dRho, R, Cv, gam, magSf, nfx, nfy);
       a.flux[id] = V4<typename P::F>{(typename P::F)rhoFlux, (typename P::F)rhoUxFlux, (typename P::F)rhoUyFlux,
                                      (typename P::F)rhoEFlux};
-      if constexpr (DT && kF32) {
+      if constexpr (DT) {
         if (s_cfl_step) {  // setDeltaT, cudaFieldOperation.h:140-157, as an FP32 estimate
           const V2<float> g = a.dtgf[id];
           dtf32 = courant_dt_f32(s_cfl, g.x, magSf, courant_den_f32(g.y, magSf, Sfx, Sfy, Wo, Wn, a.gRf));
-        }
-      } else if (DT) {
-        const StepCtl* ctl = a.ctl;
-        if (!(ctl->dt_fixed > 0.0)) {  // setDeltaT, cudaFieldOperation.h:140-157
-          const V2<double> g = a.dtg[id];
-          const double deltaR = g.x, fraction = g.y;
-          const double sfx = (double)Sfx, sfy = (double)Sfy, msf = (double)magSf;
-          const double CFL = ctl->cfl, Rd = a.R, Cvd = a.Cv;
-          dtf = CFL * deltaR * msf /
-                ((1.0 - fraction) * fabs((double)Wo.y * sfx + (double)Wo.z * sfy) +
-                 fraction * fabs((double)Wn.y * sfx + (double)Wn.z * sfy) +
-                 sqrt((Rd / Cvd + 1.0) * Rd * ((1.0 - fraction) * (double)Wo.w + fraction * (double)Wn.w)) * msf);
         }
       }
     }
@@ -1393,24 +1672,34 @@ __device__ __forceinline__ void flux_body(const StageArgs<P>& a, const int blk) 
           m >= 0x7F800000u ? 0x7FF0000000000000ull : (unsigned long long)__double_as_longlong((double)mf);
       atomicMin(&a.ctl->dt_bits, bits);
     }
-  } else if (DT) {
-    // block min (warp shuffles) then one atomicMin per block on the bit pattern; non-negative
-    // doubles order like their bit patterns, and NaN patterns sort above +inf.
-    unsigned long long v = (unsigned long long)__double_as_longlong(dtf);
-    if (!(dtf >= 0.0)) v = 0x7FF0000000000000ull;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long u = __shfl_xor_sync(0xffffffffu, v, o);
-      v = u < v ? u : v;
-    }
-    __shared__ unsigned long long wmin[8];
+  } else if constexpr (DT) {
+    // fp64: only the smallest step counts, so a face is evaluated in FP64 only where its FP32 estimate
+    // is within 1e-3 (the estimates' error is below 1e-4) of the block's smallest and of the smallest
+    // step of any block so far -- a few faces of a few blocks instead of 25 FP64 instructions a face.
+    // The minimum is that over all faces, exactly.  (An estimate that is not a number is evaluated.)
+    __shared__ unsigned wmin[8];
+    __shared__ float s_prior;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned v = __float_as_uint(est);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
     if (lane == 0) wmin[warp] = v;
-    __syncthreads();
     if (threadIdx.x == 0) {
-      unsigned long long m = wmin[0];
-      for (int k = 1; k < (int)(blockDim.x >> 5); ++k) m = wmin[k] < m ? wmin[k] : m;
-      atomicMin(&a.ctl->dt_bits, m);
+      const StepCtl* ctl = a.ctl;
+      const unsigned long long prior = *(const volatile unsigned long long*)&ctl->dt_bits;
+      s_prior = ctl->dt_fixed > 0.0 ? -1.f : __fdividef((float)__longlong_as_double((long long)prior), (float)ctl->cfl);
+    }
+    __syncthreads();
+    if (s_prior < 0.f) return;  // a fixed step
+    unsigned b = wmin[0];
+    for (int k = 1; k < (int)(blockDim.x >> 5); ++k) b = min(b, wmin[k]);
+    const float limit = 1.001f * fminf(__uint_as_float(b), s_prior);
+    if (id < a.Nf && !(est > limit)) {
+      const int2 on = a.on[id];
+      const V4<G> fs = a.fs[id];
+      const double dt = courant_dt64(a.ctl->cfl, a.gR, a.dtg[id], fs, a.W[on.x], a.W[on.y]);
+      const unsigned long long bits = dbits(dt);
+      atomicMin(&a.ctl->dt_bits, bits > kInfBits ? kInfBits : bits);  // not a number, negative: no step from here
     }
   }
 }
@@ -1526,12 +1815,13 @@ __device__ __forceinline__ void update_body(const StageArgs<P>& a, const int blk
   // Block constants, computed once by thread 0 (a block never spans two solves): the step size,
   // whether the step is live, and for mixed beta3*dt as a float.  Per-thread code then makes no
   // FP64 operation in the mixed policy (on GB300 even an FP64 comparison costs FP64-pipe time).
-  __shared__ double s_dt;
+  __shared__ double s_dt, s_nb3dt;  // the step; -beta3 times the step
   __shared__ int s_go;
   __shared__ float s_bdt;
   if (threadIdx.x == 0) {
     s_dt = step_dt(a.ctl);
-    s_go = s_dt > 0.0;  // past t_end: the step is a no-op
+    s_nb3dt = -k.b3 * s_dt;
+    s_go = gt_zero(s_dt);  // past t_end: the step is a no-op
     if constexpr (P::id == PolicyMixed::id) s_bdt = (float)(k.b3 * s_dt);
   }
   const int c = blk * blockDim.x + threadIdx.x;
@@ -1543,7 +1833,7 @@ __device__ __forceinline__ void update_body(const StageArgs<P>& a, const int blk
   if (c >= a.Nc || !s_go) return;
   const double beta1 = k.b1, beta2 = k.b2, beta3 = k.b3;
   const int last_stage = k.last;
-  const double deltaT = s_dt;
+  const double deltaT = s_dt, nb3dt = s_nb3dt;
   const int ldc = a.ldc;
   const int nM = a.nM[c];
   double Rrho = 0.0, RrhoUx = 0.0, RrhoUy = 0.0, RrhoE = 0.0;
@@ -1558,23 +1848,24 @@ __device__ __forceinline__ void update_body(const StageArgs<P>& a, const int blk
 #pragma unroll
     for (int u = 0; u < MB; ++u) {
       if (f0 + u < nM) {
-        const int direction = (fid[u] > 0) - (fid[u] < 0);
-        Rrho += direction * (double)fl[u].x;
-        RrhoUx += direction * (double)fl[u].y;
-        RrhoUy += direction * (double)fl[u].z;
-        RrhoE += direction * (double)fl[u].w;
+        // the neighbour's sign as a flip of the sign bit: no conversion or product on the FP64 pipe
+        const int flip = fid[u] & (int)0x80000000;
+        Rrho += flip_sign(fl[u].x, flip);
+        RrhoUx += flip_sign(fl[u].y, flip);
+        RrhoUy += flip_sign(fl[u].z, flip);
+        RrhoE += flip_sign(fl[u].w, flip);
       }
     }
   }
   if (a.res_dbg) a.res_dbg[c] = V4<double>{Rrho, RrhoUx, RrhoUy, RrhoE};
   const V4<double> o = a.U0[c];
-  const V4<double> u = a.U[c];
-  const double R = a.R;
-  const double gamma = a.gamma;  // R/Cv + 1, computed once on the host like GPUevolve.cu:222
   using WT = typename P::W;
   V4<double> un;
   V4<WT> wn;
   if constexpr (P::exact_blend) {  // the reference's eight divisions (cudaFieldOperation.h:229-242)
+    const V4<double> u = a.U[c];
+    const double R = a.R;
+    const double gamma = a.gamma;  // R/Cv + 1, computed once on the host like GPUevolve.cu:222
     const double V = a.vol[c];
     const double rho = beta1 * o.x + beta2 * u.x + beta3 * deltaT * (-Rrho / V);
     const double rhoUx = beta1 * o.y + beta2 * u.y + beta3 * deltaT * (-RrhoUx / V);
@@ -1583,16 +1874,18 @@ __device__ __forceinline__ void update_body(const StageArgs<P>& a, const int blk
     un = V4<double>{rho, rhoUx, rhoUy, rhoE};
     const double p = (gamma - 1.0) * (rhoE - 0.5 * (rhoUx * rhoUx + rhoUy * rhoUy) / rho);
     wn = V4<WT>{(WT)p, (WT)(rhoUx / rho), (WT)(rhoUy / rho), (WT)(p / (R * rho))};
-  } else {  // FP64 is scarce on GB300: 1/V precomputed, one division for 1/rho
-    const double s3 = -beta3 * deltaT * a.vinv[c];
-    const double rho = beta1 * o.x + beta2 * u.x + s3 * Rrho;
-    const double rhoUx = beta1 * o.y + beta2 * u.y + s3 * RrhoUx;
-    const double rhoUy = beta1 * o.z + beta2 * u.z + s3 * RrhoUy;
-    const double rhoE = beta1 * o.w + beta2 * u.w + s3 * RrhoE;
-    un = V4<double>{rho, rhoUx, rhoUy, rhoE};
-    const double ir = 1.0 / rho;
-    const double ux = rhoUx * ir, uy = rhoUy * ir;
-    const double p = (gamma - 1.0) * (rhoE - 0.5 * (rhoUx * ux + rhoUy * uy));
+  } else {  // FP64 is scarce on GB300: 1/V precomputed, one reciprocal for 1/rho
+    const double s3 = nb3dt * a.vinv[c];
+    if (k.first) {  // beta1 = 1, beta2 = 0: U is not read
+      un = V4<double>{o.x + s3 * Rrho, o.y + s3 * RrhoUx, o.z + s3 * RrhoUy, o.w + s3 * RrhoE};
+    } else {
+      const V4<double> u = a.U[c];
+      un = V4<double>{beta1 * o.x + beta2 * u.x + s3 * Rrho, beta1 * o.y + beta2 * u.y + s3 * RrhoUx,
+                      beta1 * o.z + beta2 * u.z + s3 * RrhoUy, beta1 * o.w + beta2 * u.w + s3 * RrhoE};
+    }
+    const double ir = rcp64(un.x);
+    const double ux = un.y * ir, uy = un.z * ir;
+    const double p = a.gm1 * (un.w - 0.5 * (un.y * ux + un.z * uy));
     wn = V4<WT>{(WT)p, (WT)ux, (WT)uy, (WT)(p * ir * a.invR)};
   }
   a.U[c] = un;
@@ -1622,12 +1915,12 @@ __global__ void __launch_bounds__(kTile, 4) k_reconstruct_tile(StageArgs<P> a) {
 }
 template <class P>
 __global__ void __launch_bounds__(128) k_reconstruct_staged(StageArgs<P> a) {
-  recon_staged_body<P>(a, blockIdx.x);
+  recon_ref_body(a, blockIdx.x);
 }
 // fp64: its compact staging leaves room for 4 blocks an SM, which 128 registers a thread allow
 template <>
 __global__ void __launch_bounds__(128, 4) k_reconstruct_staged<PolicyFP64>(StageArgs<PolicyFP64> a) {
-  recon_staged_body<PolicyFP64>(a, blockIdx.x);
+  recon_fp64_body(a, blockIdx.x);
 }
 template <class P>
 __global__ void __launch_bounds__(128) k_bvd(StageArgs<P> a) {
@@ -1677,36 +1970,79 @@ __global__ void __launch_bounds__(128) k_reconstruct_gauss(StageArgs<P> a) {
   S pMax = pc, pMin = pc, uxMax = uxc, uxMin = uxc, uyMax = uyc, uyMin = uyc, tMax = tc, tMin = tc;
   for (int i = 0; i < nM; ++i) {
     const V4<WT> v = a.W[a.sten[i * ldc + c]];
-    pMax = fmx((S)v.x, pMax);
-    pMin = fmn((S)v.x, pMin);
-    uxMax = fmx((S)v.y, uxMax);
-    uxMin = fmn((S)v.y, uxMin);
-    uyMax = fmx((S)v.z, uyMax);
-    uyMin = fmn((S)v.z, uyMin);
-    tMax = fmx((S)v.w, tMax);
-    tMin = fmn((S)v.w, tMin);
+    pMax = gmx((S)v.x, pMax);
+    pMin = gmn((S)v.x, pMin);
+    uxMax = gmx((S)v.y, uxMax);
+    uxMin = gmn((S)v.y, uxMin);
+    uyMax = gmx((S)v.z, uyMax);
+    uyMin = gmn((S)v.z, uyMin);
+    tMax = gmx((S)v.w, tMax);
+    tMin = gmn((S)v.w, tMin);
   }
   const V4<G> g0 = a.grad[2 * c], g1 = a.grad[2 * c + 1];  // (px py uxx uxy), (uyx uyy tx ty)
   const S SMALL = AFAR_LIT(S, 1e-5), VSMALL = AFAR_LIT(S, 1e-10);
-  const bool flat = fab(tMax - tMin) < VSMALL;
-  const bool o3p = !flat && fab(pMax - pMin) >= SMALL, o3ux = !flat && fab(uxMax - uxMin) >= SMALL;
-  const bool o3uy = !flat && fab(uyMax - uyMin) >= SMALL, o3t = !flat && fab(tMax - tMin) >= SMALL;
+  const bool flat = abs_lt(tMax - tMin, VSMALL);
+  const bool o3p = !flat && abs_ge(pMax - pMin, SMALL), o3ux = !flat && abs_ge(uxMax - uxMin, SMALL);
+  const bool o3uy = !flat && abs_ge(uyMax - uyMin, SMALL), o3t = !flat && abs_ge(tMax - tMin, SMALL);
   for (int fi = 0; fi < nM; ++fi) {
     const int fid = a.cf[fi * ldc + c];
     const int f = abs(fid) - 1;
     if (f >= a.Nf) continue;
     const int side = fid < 0;
-    for (int k = 0; k < ng; ++k) {
-      const V2<G> d = a.sgk[(fi * ng + k) * ldc + c];
-      V4<G> o;
-      o.x = (G)pc + g0.x * d.x + g0.y * d.y;
-      o.y = (G)uxc + g0.z * d.x + g1.x * d.y;
-      o.z = (G)uyc + g0.w * d.x + g1.y * d.y;
-      o.w = (G)tc + g1.z * d.x + g1.w * d.y;
-      if (o3p || o3ux || o3uy || o3t) {
-        const S* w = a.wg + (size_t)((fi * ng + k) * wrow) * ldc + c;
-        G sp, sux, suy, st;
-        if constexpr (std::is_same<G, float>::value) {  // mixed: the difference form of recon_tile_body
+    V4<G>* const out = a.fvg + (size_t)(2 * f + side) * ng;
+    const bool all3 = o3p && o3ux && o3uy && o3t, any3 = o3p || o3ux || o3uy || o3t;
+    if constexpr (std::is_same<G, double>::value) {
+      // two points at a time: each member's state is read once for both, and the linear values are
+      // formed only in a cell with a variable that takes them
+      for (int k0 = 0; k0 < ng; k0 += 2) {
+        const int n2 = min(2, ng - k0);
+        V4<double> o[2];
+        if (any3) {
+          const double* w = a.wg + (size_t)((fi * ng + k0) * wrow) * ldc + c;
+          const size_t next = n2 > 1 ? (size_t)wrow * ldc : 0;  // a single point twice
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const double w0 = w[q * next];
+            o[q] = V4<double>{w0 * pc, w0 * uxc, w0 * uyc, w0 * tc};
+          }
+          for (int j = 0; j < nS; ++j) {
+            const V4<double> v = a.W[a.sten[j * ldc + c]];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              if (q < n2) {
+                const double wj = w[q * next + (size_t)(j + 1) * ldc];
+                o[q].x += wj * v.x;
+                o[q].y += wj * v.y;
+                o[q].z += wj * v.z;
+                o[q].w += wj * v.w;
+              }
+            }
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          if (q >= n2) break;
+          if (!all3) {
+            const V2<double> d = a.sgk[(fi * ng + k0 + q) * ldc + c];
+            if (!o3p) o[q].x = pc + g0.x * d.x + g0.y * d.y;
+            if (!o3ux) o[q].y = uxc + g0.z * d.x + g1.x * d.y;
+            if (!o3uy) o[q].z = uyc + g0.w * d.x + g1.y * d.y;
+            if (!o3t) o[q].w = tc + g1.z * d.x + g1.w * d.y;
+          }
+          out[k0 + q] = o[q];
+        }
+      }
+    } else {
+      for (int k = 0; k < ng; ++k) {
+        const V2<G> d = a.sgk[(fi * ng + k) * ldc + c];
+        V4<G> o;
+        o.x = (G)pc + g0.x * d.x + g0.y * d.y;
+        o.y = (G)uxc + g0.z * d.x + g1.x * d.y;
+        o.z = (G)uyc + g0.w * d.x + g1.y * d.y;
+        o.w = (G)tc + g1.z * d.x + g1.w * d.y;
+        if (any3) {  // the difference form of recon_tile_body
+          const S* w = a.wg + (size_t)((fi * ng + k) * wrow) * ldc + c;
+          G sp, sux, suy, st;
           sp = sux = suy = st = G(0);
           for (int j = 0; j < nS; ++j) {
             const S wj = w[(size_t)(j + 1) * ldc];
@@ -1720,27 +2056,13 @@ __global__ void __launch_bounds__(128) k_reconstruct_gauss(StageArgs<P> a) {
           sux += (G)uxc;
           suy += (G)uyc;
           st += (G)tc;
-        } else {  // fp64: the plain sum, the cell itself first
-          const S w0 = w[0];
-          sp = w0 * pc;
-          sux = w0 * uxc;
-          suy = w0 * uyc;
-          st = w0 * tc;
-          for (int j = 0; j < nS; ++j) {
-            const S wj = w[(size_t)(j + 1) * ldc];
-            const V4<WT> v = a.W[a.sten[j * ldc + c]];
-            sp += wj * (S)v.x;
-            sux += wj * (S)v.y;
-            suy += wj * (S)v.z;
-            st += wj * (S)v.w;
-          }
+          if (o3p) o.x = sp;
+          if (o3ux) o.y = sux;
+          if (o3uy) o.z = suy;
+          if (o3t) o.w = st;
         }
-        if (o3p) o.x = sp;
-        if (o3ux) o.y = sux;
-        if (o3uy) o.z = suy;
-        if (o3t) o.w = st;
+        out[k] = o;
       }
-      a.fvg[(2 * f + side) * ng + k] = o;
     }
   }
 }
@@ -1775,48 +2097,78 @@ __global__ void __launch_bounds__(256) k_flux_gauss(StageArgs<P> a) {
     const G gam = std::is_same<G, float>::value ? (G)(a.gm1f + 1.f) : (G)a.gamma;
     const G K = G(2) * Cv * iR - G(2);
     G acc[4] = {G(0), G(0), G(0), G(0)};
-    for (int k = 0; k < a.ng; ++k) {
-      const V2<G> off = a.fgk[id * a.ng + k];
-      G st[2][4], T[2][4], rho[2], rhoT[2];
+    if constexpr (std::is_same<G, double>::value) {
+      for (int k = 0; k < a.ng; ++k) {
+        const V2<double> off = a.fgk[(size_t)id * a.ng + k];
+        Side64 st[2];
+        double pT[2], tT[2];
 #pragma unroll
-      for (int sd = 0; sd < 2; ++sd) {
-        const int c = cell[sd];
-        const G dx = (sd ? fd.z : fd.x) + off.x, dy = (sd ? fd.w : fd.y) + off.y;
-        const V4<typename P::W> w = a.W[c];
-        const V4<G> g0 = a.grad[2 * c], g1 = a.grad[2 * c + 1];
-        const V4<S> l = a.lim[c];
-        T[sd][0] = (G)w.x + l.x * (g0.x * dx + g0.y * dy);
-        T[sd][1] = (G)w.y + l.y * (g0.z * dx + g1.x * dy);
-        T[sd][2] = (G)w.z + l.z * (g0.w * dx + g1.y * dy);
-        T[sd][3] = (G)w.w + l.w * (g1.z * dx + g1.w * dy);
-        const V4<G> o3 = a.fvg[(2 * id + sd) * a.ng + k];
-        const bool tvd = sw[sd] != 0;
-        st[sd][0] = tvd ? T[sd][0] : o3.x;
-        st[sd][1] = tvd ? T[sd][1] : o3.y;
-        st[sd][2] = tvd ? T[sd][2] : o3.z;
-        st[sd][3] = tvd ? T[sd][3] : o3.w;
-        rho[sd] = fdiv(st[sd][0] * iR, st[sd][3]);
-        rhoT[sd] = fdiv(T[sd][0] * iR, T[sd][3]);
+        for (int sd = 0; sd < 2; ++sd) {
+          const int c = cell[sd];
+          const double dx = (sd ? fd.z : fd.x) + off.x, dy = (sd ? fd.w : fd.y) + off.y;
+          const V4<double> w = a.W[c], g0 = a.grad[2 * c], g1 = a.grad[2 * c + 1], l = a.lim[c];
+          pT[sd] = tvd64(w.x, l.x, g0.x, g0.y, dx, dy);
+          tT[sd] = tvd64(w.w, l.w, g1.z, g1.w, dx, dy);
+          if (sw[sd] != 0) {
+            st[sd] = Side64{pT[sd], tvd64(w.y, l.y, g0.z, g1.x, dx, dy), tvd64(w.z, l.z, g0.w, g1.y, dx, dy), tT[sd], 0.0};
+          } else {
+            const V4<double> o3 = a.fvg[(size_t)(2 * id + sd) * a.ng + k];
+            st[sd] = Side64{o3.x, o3.y, o3.z, o3.w, 0.0};
+          }
+        }
+        double rhoLT, rhoRT;
+        densities64(st[0].rho, st[1].rho, rhoLT, rhoRT, st[0].p, st[1].p, pT[0], pT[1], st[0].T, st[1].T, tT[0], tT[1], iR);
+        const V4<double> F = face_flux64(st[0], st[1], pT[0], pT[1], rhoLT, rhoRT, isShock, gas64(a), fs);
+        const double wk = a.gw[k];
+        acc[0] += wk * F.x;
+        acc[1] += wk * F.y;
+        acc[2] += wk * F.z;
+        acc[3] += wk * F.w;
       }
-      const G dP = min_delta<G, G>(st[0][0], st[1][0], T[0][0], T[1][0]);
-      const G dRho = min_delta<G, G>(rho[0], rho[1], rhoT[0], rhoT[1]);
-      const G h = G(0.5);
-      G F0 = h * rho[0] * (st[0][1] * Sfx + st[0][2] * Sfy) + h * rho[1] * (st[1][1] * Sfx + st[1][2] * Sfy);
-      G F1 = h * (F0 * st[0][1] + st[0][0] * Sfx) + h * (F0 * st[1][1] + st[1][0] * Sfx);
-      G F2 = h * (F0 * st[0][2] + st[0][0] * Sfy) + h * (F0 * st[1][2] + st[1][0] * Sfy);
-      G F3 = h * F0 * (Cv * st[0][3] + h * (st[0][1] * st[0][1] + st[0][2] * st[0][2]) + R * st[0][3]) +
-             h * F0 * (Cv * st[1][3] + h * (st[1][1] * st[1][1] + st[1][2] * st[1][2]) + R * st[1][3]);
-      if (isShock)
-        kfvs_flux_fast<G>(F0, F1, F2, F3, rho[0], rho[1], st[0][0], st[1][0], st[0][1], st[1][1], st[0][2], st[1][2],
-                          st[0][3], st[1][3], R, Cv, K, magSf, nfx, nfy);
-      else
-        roe_flux_fast<G>(F0, F1, F2, F3, rho[0], rho[1], st[0][1], st[1][1], st[0][2], st[1][2], st[0][3], st[1][3],
-                         dP, dRho, R, Cv, gam, magSf, nfx, nfy);
-      const G wk = a.gw[k];
-      acc[0] += wk * F0;
-      acc[1] += wk * F1;
-      acc[2] += wk * F2;
-      acc[3] += wk * F3;
+    } else {
+      for (int k = 0; k < a.ng; ++k) {
+        const V2<G> off = a.fgk[id * a.ng + k];
+        G st[2][4], T[2][4], rho[2], rhoT[2];
+  #pragma unroll
+        for (int sd = 0; sd < 2; ++sd) {
+          const int c = cell[sd];
+          const G dx = (sd ? fd.z : fd.x) + off.x, dy = (sd ? fd.w : fd.y) + off.y;
+          const V4<typename P::W> w = a.W[c];
+          const V4<G> g0 = a.grad[2 * c], g1 = a.grad[2 * c + 1];
+          const V4<S> l = a.lim[c];
+          T[sd][0] = (G)w.x + l.x * (g0.x * dx + g0.y * dy);
+          T[sd][1] = (G)w.y + l.y * (g0.z * dx + g1.x * dy);
+          T[sd][2] = (G)w.z + l.z * (g0.w * dx + g1.y * dy);
+          T[sd][3] = (G)w.w + l.w * (g1.z * dx + g1.w * dy);
+          const V4<G> o3 = a.fvg[(2 * id + sd) * a.ng + k];
+          const bool tvd = sw[sd] != 0;
+          st[sd][0] = tvd ? T[sd][0] : o3.x;
+          st[sd][1] = tvd ? T[sd][1] : o3.y;
+          st[sd][2] = tvd ? T[sd][2] : o3.z;
+          st[sd][3] = tvd ? T[sd][3] : o3.w;
+          rho[sd] = fdiv(st[sd][0] * iR, st[sd][3]);
+          rhoT[sd] = fdiv(T[sd][0] * iR, T[sd][3]);
+        }
+        const G dP = min_delta<G, G>(st[0][0], st[1][0], T[0][0], T[1][0]);
+        const G dRho = min_delta<G, G>(rho[0], rho[1], rhoT[0], rhoT[1]);
+        const G h = G(0.5);
+        G F0 = h * rho[0] * (st[0][1] * Sfx + st[0][2] * Sfy) + h * rho[1] * (st[1][1] * Sfx + st[1][2] * Sfy);
+        G F1 = h * (F0 * st[0][1] + st[0][0] * Sfx) + h * (F0 * st[1][1] + st[1][0] * Sfx);
+        G F2 = h * (F0 * st[0][2] + st[0][0] * Sfy) + h * (F0 * st[1][2] + st[1][0] * Sfy);
+        G F3 = h * F0 * (Cv * st[0][3] + h * (st[0][1] * st[0][1] + st[0][2] * st[0][2]) + R * st[0][3]) +
+               h * F0 * (Cv * st[1][3] + h * (st[1][1] * st[1][1] + st[1][2] * st[1][2]) + R * st[1][3]);
+        if (isShock)
+          kfvs_flux_fast<G>(F0, F1, F2, F3, rho[0], rho[1], st[0][0], st[1][0], st[0][1], st[1][1], st[0][2], st[1][2],
+                            st[0][3], st[1][3], R, Cv, K, magSf, nfx, nfy);
+        else
+          roe_flux_fast<G>(F0, F1, F2, F3, rho[0], rho[1], st[0][1], st[1][1], st[0][2], st[1][2], st[0][3], st[1][3],
+                           dP, dRho, R, Cv, gam, magSf, nfx, nfy);
+        const G wk = a.gw[k];
+        acc[0] += wk * F0;
+        acc[1] += wk * F1;
+        acc[2] += wk * F2;
+        acc[3] += wk * F3;
+      }
     }
     a.flux[id] = V4<typename P::F>{(typename P::F)acc[0], (typename P::F)acc[1], (typename P::F)acc[2],
                                    (typename P::F)acc[3]};
@@ -1860,17 +2212,10 @@ __global__ void __launch_bounds__(kTile, 4) kb_reconstruct_tile(const StageArgs<
   const int2 m = map[blockIdx.x];
   recon_tile_body<P, NF>(member_args(tab, m.x), m.y, sm);
 }
-template <class P>
-__global__ void __launch_bounds__(128) kb_reconstruct_staged(const StageArgs<P>* __restrict__ tab,
-                                                             const int2* __restrict__ map) {
+__global__ void __launch_bounds__(128, 4) kb_reconstruct_fp64(const StageArgs<PolicyFP64>* __restrict__ tab,
+                                                              const int2* __restrict__ map) {
   const int2 m = map[blockIdx.x];
-  recon_staged_body<P>(member_args(tab, m.x), m.y);
-}
-template <>
-__global__ void __launch_bounds__(128, 4) kb_reconstruct_staged<PolicyFP64>(const StageArgs<PolicyFP64>* __restrict__ tab,
-                                                                            const int2* __restrict__ map) {
-  const int2 m = map[blockIdx.x];
-  recon_staged_body<PolicyFP64>(member_args(tab, m.x), m.y);
+  recon_fp64_body(member_args(tab, m.x), m.y);
 }
 // the register-pass reconstruct of the mixed policy over the members the autotuner gave it
 template <class P>
@@ -1940,11 +2285,15 @@ __global__ void __launch_bounds__(256) k_delta_t(StageArgs<P> a, double CFL, uns
     const V4<typename P::G> fs = a.fs[id];
     const double sfx = (double)fs.x, sfy = (double)fs.y, msf = (double)fs.z;
     const V2<double> g = a.dtg[id];
-    const double deltaR = g.x, fraction = g.y, Rd = a.R, Cvd = a.Cv;
-    dtf = CFL * deltaR * msf /
-          ((1.0 - fraction) * fabs((double)Wo.y * sfx + (double)Wo.z * sfy) +
-           fraction * fabs((double)Wn.y * sfx + (double)Wn.z * sfy) +
-           sqrt((Rd / Cvd + 1.0) * Rd * ((1.0 - fraction) * (double)Wo.w + fraction * (double)Wn.w)) * msf);
+    if constexpr (P::id == PolicyFP64::id) {
+      dtf = courant_dt64(CFL, a.gR, g, fs, Wo, Wn);
+    } else {
+      const double deltaR = g.x, fraction = g.y, Rd = a.R, Cvd = a.Cv;
+      dtf = CFL * deltaR * msf /
+            ((1.0 - fraction) * fabs((double)Wo.y * sfx + (double)Wo.z * sfy) +
+             fraction * fabs((double)Wn.y * sfx + (double)Wn.z * sfy) +
+             sqrt((Rd / Cvd + 1.0) * Rd * ((1.0 - fraction) * (double)Wo.w + fraction * (double)Wn.w)) * msf);
+    }
   }
   unsigned long long v = (unsigned long long)__double_as_longlong(dtf);
   if (!(dtf >= 0.0)) v = 0x7FF0000000000000ull;
@@ -2047,7 +2396,7 @@ __global__ void k_setup_slot_geom(StageArgs<P> a, const V4<double>* faceXY) {
       const float fraction = sqrt(dx * dx + dy * dy) / deltaR;
       if (P::id == PolicyFP64::id) {
         const double dRd = hypot(nx, ny);
-        dR = (S)dRd;
+        dR = (S)(1.0 / dRd);  // its kernel multiplies by the reciprocal
         fr = (S)(sqrt(dx * dx + dy * dy) / dRd);
       } else {
         dR = (S)deltaR;

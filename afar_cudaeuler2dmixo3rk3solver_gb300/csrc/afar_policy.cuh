@@ -86,6 +86,91 @@ __device__ __forceinline__ double erfc_(double a) { return erfc(a); }
 __device__ __forceinline__ float exp_(float a) { return expf(a); }
 __device__ __forceinline__ double exp_(double a) { return exp(a); }
 
+// ---------------------------------------------------------------- sparing the FP64 pipe
+// GB300 issues two FP64 lanes a clock and SM: one FP64 warp instruction takes the pipe 16 clocks, in
+// which the four schedulers issue 64 others.  Comparisons, minima, conversions and the compiler's
+// division and root sequences all run on that pipe, so the fp64 policy compares doubles as integers,
+// and starts reciprocals from the FP32 approximation, refined by one third-order step in FP64.
+__device__ __forceinline__ unsigned long long dbits(const double x) {
+  return (unsigned long long)__double_as_longlong(x);
+}
+constexpr unsigned long long kInfBits = 0x7FF0000000000000ull;
+// by the high word: as a mask on all 64 bits the compiler makes it an addition on the FP64 pipe
+__device__ __forceinline__ double dabs_(const double x) {
+  return __hiloint2double(__double2hiint(x) & 0x7FFFFFFF, __double2loint(x));
+}
+// by the high word alone (every NaN that arithmetic produces has a high fraction bit set): as a test
+// on all 64 bits the compiler makes it a comparison on the FP64 pipe
+__device__ __forceinline__ bool dnan_(const double x) { return (__double2hiint(x) & 0x7FFFFFFF) > 0x7FF00000; }
+// |x| < c and |x| >= c for a constant c > 0; false on NaN, as the comparisons are.
+__device__ __forceinline__ bool abs_lt(const double x, const double c) { return dbits(dabs_(x)) < dbits(c); }
+__device__ __forceinline__ bool abs_ge(const double x, const double c) {
+  return dbits(dabs_(x)) - dbits(c) <= kInfBits - dbits(c);
+}
+__device__ __forceinline__ bool abs_lt(const float x, const float c) { return fabsf(x) < c; }
+__device__ __forceinline__ bool abs_ge(const float x, const float c) { return fabsf(x) >= c; }
+__device__ __forceinline__ bool gt_zero(const double x) { return dbits(x) - 1ull < kInfBits; }
+__device__ __forceinline__ bool le_zero(const double x) {
+  return dbits(x) == 0ull || dbits(x) - 0x8000000000000000ull <= kInfBits;
+}
+__device__ __forceinline__ double flip_sign(const double x, const int bit) {
+  return __hiloint2double(__double2hiint(x) ^ bit, __double2loint(x));
+}
+__device__ __forceinline__ bool neg_(const double x) { return (long long)dbits(x) < 0; }  // the sign bit
+// fmin of two doubles without a sign (NaN loses, as in fmin)
+__device__ __forceinline__ double min_nonneg(const double a, const double b) { return dbits(b) < dbits(a) ? b : a; }
+// fmax and fmin for any operands (of two zeros either; NaN loses): the bits of a double, its lower 63
+// flipped where it is negative, order like the numbers.
+__device__ __forceinline__ long long dkey(const double x) {
+  const long long b = __double_as_longlong(x);
+  return b ^ ((b >> 63) & 0x7FFFFFFFFFFFFFFFll);
+}
+__device__ __forceinline__ double dmax_(const double a, const double b) {
+  return dnan_(a) || (dkey(b) > dkey(a) && !dnan_(b)) ? b : a;
+}
+__device__ __forceinline__ double dmin_(const double a, const double b) {
+  return dnan_(a) || (dkey(b) < dkey(a) && !dnan_(b)) ? b : a;
+}
+// the policy's larger and smaller of two: fmaxf, fminf, or the integer forms
+__device__ __forceinline__ float gmx(const float a, const float b) { return fmaxf(a, b); }
+__device__ __forceinline__ float gmn(const float a, const float b) { return fminf(a, b); }
+__device__ __forceinline__ double gmx(const double a, const double b) { return dmax_(a, b); }
+__device__ __forceinline__ double gmn(const double a, const double b) { return dmin_(a, b); }
+// x as a float to 20 bits from its high word (zero below the range of float), for estimates
+__device__ __forceinline__ float top_float(const double x) {
+  const int hi = __double2hiint(x), a = hi & 0x7FFFFFFF;
+  const unsigned m = a < 0x38100000 ? 0u : a >= 0x47F00000 ? 0x7F800000u : (unsigned)(a - 0x38000000) << 3;
+  return __uint_as_float(m | ((unsigned)hi & 0x80000000u));
+}
+// 1/x: y0 to 23 bits from the mantissa's FP32 reciprocal, then y0 (1 + e + e^2) with e = 1 - x y0,
+// whose remainder e^3 is below 2^-66: three FP64 operations, within an ulp.  Zeros, subnormals,
+// infinities, NaN and reciprocals that are subnormal take the division.
+__device__ __forceinline__ double rcp64(const double x) {
+  const int hi = __double2hiint(x), lo = __double2loint(x);
+  const int e = (hi >> 20) & 0x7FF;
+  if ((unsigned)(e - 1) > 2042u) return 1.0 / x;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__int_as_float(0x3F800000 | ((hi & 0xFFFFF) << 3) | ((unsigned)lo >> 29))));
+  const int rb = __float_as_int(r);
+  const double y0 = __hiloint2double(((rb >> 3) + (896 + 1023 - e) * (1 << 20)) | (hi & (int)0x80000000), rb << 29);
+  const double d = __fma_rn(-x, y0, 1.0);
+  return __fma_rn(y0, __fma_rn(d, d, d), y0);
+}
+// 1/sqrt(x): y0 the same way from x scaled by an even power of two into [1, 4), then
+// y0 (1 + e/2 + 3/8 e^2) with e = 1 - x y0^2 (Halley's step): five FP64 operations.
+__device__ __forceinline__ double rsq64(const double x) {
+  const int hi = __double2hiint(x), lo = __double2loint(x);
+  const int e = hi >> 20;  // the sign bit makes it negative
+  if ((unsigned)(e - 1) > 2045u) return rsqrt(x);
+  const int k = (e - 1023) >> 1;
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__int_as_float(((e - 896 - 2 * k) << 23) | ((hi & 0xFFFFF) << 3) | ((unsigned)lo >> 29))));
+  const int rb = __float_as_int(r);
+  const double y0 = __hiloint2double((rb >> 3) + ((896 - k) << 20), rb << 29);
+  const double d = __fma_rn(-__dmul_rn(x, y0), y0, 1.0);
+  return __fma_rn(__dmul_rn(y0, d), __fma_rn(0.375, d, 0.5), y0);
+}
+
 // Bulk global->shared copies (cp.async.bulk, the TMA unit's untiled form) completing on an
 // mbarrier.  Both addresses 16-byte aligned, size a multiple of 16.
 __device__ __forceinline__ unsigned smem_addr(const void* p) {

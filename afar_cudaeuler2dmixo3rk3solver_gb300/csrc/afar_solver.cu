@@ -45,6 +45,7 @@ namespace {
 constexpr int kCellBlock = 128;
 constexpr size_t kMaxDynamicSmem = 227 * 1024;  // per CTA on sm_103a
 constexpr int kFaceBlock = 256;
+constexpr int kFaceBlock64 = 128;  // ref and fp64: smaller blocks, an evener last wave over the SMs' FP64 pipes
 // GPUevolve.cu:223-225: the reference's truncated SSP-RK3 coefficients
 constexpr double kBeta1[3] = {1.0, 0.75, 0.333333};
 constexpr double kBeta2[3] = {0.0, 0.25, 0.666667};
@@ -311,7 +312,10 @@ StageArgs<P> make_args(afar_solver* s) {
   a.Cv = s->Cv;
   a.invR = s->R > 0.0 ? 1.0 / s->R : 0.0;
   a.gamma = s->Cv > 0.0 ? s->R / s->Cv + 1.0 : 0.0;
-  a.gm1f = (float)(a.gamma - 1.0);
+  a.Cp = s->Cv + s->R;
+  a.gm1 = a.gamma - 1.0;
+  a.gR = a.gamma * s->R;
+  a.gm1f = (float)a.gm1;
   a.invRf = (float)a.invR;
   a.vinvf = s->vinvf;
   a.Rf = (float)s->R;
@@ -344,13 +348,27 @@ afar_status raise_smem_limit(K kernel, int device, size_t bytes) {
   return AFAR_OK;
 }
 
+// Threads a block of the single-solve kernels over n cells or faces.  The ref and fp64 kernels are
+// bound by each SM's FP64 pipe, so a mesh too small to give every SM two full blocks is cut into
+// smaller ones until it reaches all SMs: the pipe's time on the busiest SM is the kernel's (fp64,
+// 1,754 cells: 55 blocks of 32 instead of 14 of 128, the step 317 -> 182 us with the kernels' other
+// changes; whole meshes of 250k cells and more are past the line and keep the full block).
+template <class P>
+int block_for(long long n, int full) {
+  if constexpr (P::id == PolicyMixed::id) return full;
+  constexpr long long kSMs = 152;
+  int b = full;
+  while (b > 32 && n < 2 * kSMs * b) b /= 2;
+  return b;
+}
+
 // Dynamic shared memory of the reconstruct: the mixed policy stages a whole 128-cell tile of
 // operator rows (recon_tile_layout); ref stages the stencil values, fp64 the compact stencil's.
 template <class P>
-size_t recon_smem(const afar_solver* s) {
+size_t recon_smem(const afar_solver* s, int block = kCellBlock) {
   if constexpr (P::id == PolicyMixed::id) return recon_tile_layout(s->maxM, s->maxS).bytes;
   const int rows = P::id == PolicyFP64::id ? s->maxM : s->maxS;  // fp64 stages the compact stencil only
-  return (size_t)(rows > 0 ? rows : 1) * kCellBlock * sizeof(V4<typename P::S>);
+  return (size_t)(rows > 0 ? rows : 1) * block * sizeof(V4<typename P::S>);
 }
 
 // One solve's stage launches, arguments by value.  The ref policy reconstructs in the staged
@@ -359,7 +377,8 @@ template <class P>
 struct Stage {
   afar_solver* s;
   StageArgs<P> a;
-  int gc() const { return grid_for(s->Nc, kCellBlock); }
+  int bc() const { return block_for<P>(s->Nc, kCellBlock); }
+  int gc() const { return grid_for(s->Nc, bc()); }
 
   void reconstruct() const {
     if constexpr (P::id == PolicyMixed::id) {
@@ -370,33 +389,34 @@ struct Stage {
       else
         k_reconstruct_tile<P, 4><<<gc(), kTile, recon_smem<P>(s), s->stream>>>(a);
     } else
-      k_reconstruct_staged<P><<<gc(), kCellBlock, recon_smem<P>(s), s->stream>>>(a);
+      k_reconstruct_staged<P><<<gc(), bc(), recon_smem<P>(s, bc()), s->stream>>>(a);
     if constexpr (P::id != PolicyRef::id) {
-      if (s->ng > 0) k_reconstruct_gauss<P><<<gc(), kCellBlock, 0, s->stream>>>(a);
+      if (s->ng > 0) k_reconstruct_gauss<P><<<gc(), bc(), 0, s->stream>>>(a);
     }
   }
-  void bvd() const { k_bvd<P><<<gc(), kCellBlock, 0, s->stream>>>(a); }
+  void bvd() const { k_bvd<P><<<gc(), bc(), 0, s->stream>>>(a); }
   // The face flux.  The ref policy computes the CFL step as a kernel of its own before the first
   // stage's flux, like the reference's setDeltaT; the other policies fuse it into that flux.
   void flux(bool dt_stage) const {
-    const int gf = grid_for((long long)s->Nf + s->Nb, kFaceBlock);
+    const int bf = block_for<P>((long long)s->Nf + s->Nb, P::id == PolicyMixed::id ? kFaceBlock : kFaceBlock64);
+    const int gf = grid_for((long long)s->Nf + s->Nb, bf);
     if constexpr (P::id == PolicyRef::id) {
       if (dt_stage && s->Nf > 0)
-        k_delta_t<P><<<grid_for(s->Nf, kFaceBlock), kFaceBlock, 0, s->stream>>>(a, 0.0, &s->ctl->dt_bits, s->ctl);
-      k_flux<P, false><<<gf, kFaceBlock, 0, s->stream>>>(a);
+        k_delta_t<P><<<grid_for(s->Nf, bf), bf, 0, s->stream>>>(a, 0.0, &s->ctl->dt_bits, s->ctl);
+      k_flux<P, false><<<gf, bf, 0, s->stream>>>(a);
     } else if (s->ng > 0) {  // the multi-point face flux; the Courant step as a kernel of its own
       if (dt_stage && s->Nf > 0)
-        k_delta_t<P><<<grid_for(s->Nf, kFaceBlock), kFaceBlock, 0, s->stream>>>(a, 0.0, &s->ctl->dt_bits, s->ctl);
-      k_flux_gauss<P><<<gf, kFaceBlock, 0, s->stream>>>(a);
+        k_delta_t<P><<<grid_for(s->Nf, bf), bf, 0, s->stream>>>(a, 0.0, &s->ctl->dt_bits, s->ctl);
+      k_flux_gauss<P><<<gf, bf, 0, s->stream>>>(a);
     } else {
       if (dt_stage)
-        k_flux<P, true><<<gf, kFaceBlock, 0, s->stream>>>(a);
+        k_flux<P, true><<<gf, bf, 0, s->stream>>>(a);
       else
-        k_flux<P, false><<<gf, kFaceBlock, 0, s->stream>>>(a);
+        k_flux<P, false><<<gf, bf, 0, s->stream>>>(a);
     }
   }
   void update(int k) const {
-    k_update<P><<<gc(), kCellBlock, 0, s->stream>>>(a, stage_coef(k));
+    k_update<P><<<gc(), bc(), 0, s->stream>>>(a, stage_coef(k));
   }
 };
 
@@ -1096,8 +1116,7 @@ extern "C" afar_status afar_adjustTimeStep(afar_solver* s, int facesNum, double 
       }
       case AFAR_POLICY_FP64: {
         StageArgs<PolicyFP64> a = make_args<PolicyFP64>(s);
-        a.R = R;
-        a.Cv = Cv;
+        a.gR = (R / Cv + 1.0) * R;
         k_delta_t<PolicyFP64><<<gf, kFaceBlock, 0, s->stream>>>(a, CFL, s->dt_bits, nullptr);
         break;
       }
@@ -1708,7 +1727,7 @@ afar_status batch_build(afar_batch* b) {
   int nfmax = 3;
   for (afar_solver* s : b->members) nfmax = std::max(nfmax, s->maxM);
   if constexpr (P::id != PolicyMixed::id) {
-    if ((st = raise_smem_limit(kb_reconstruct_staged<P>, b->device, smem))) return st;
+    if ((st = raise_smem_limit(kb_reconstruct_fp64, b->device, smem))) return st;
   } else {
     if ((st = raise_smem_limit(kb_reconstruct_tile<P, 3>, b->device, smem))) return st;
     if ((st = raise_smem_limit(kb_reconstruct_tile<P, 4>, b->device, smem))) return st;
@@ -1736,7 +1755,7 @@ afar_status batch_build(afar_batch* b) {
       }
       if (b->n_reg) kb_reconstruct_reg<P><<<b->n_reg, kCellBlock, 0, b->stream>>>(t, b->maps + o_reg);
     } else
-      kb_reconstruct_staged<P><<<b->n_cell, kCellBlock, b->smem, b->stream>>>(t, b->maps + o_cell);
+      kb_reconstruct_fp64<<<b->n_cell, kCellBlock, b->smem, b->stream>>>(t, b->maps + o_cell);
   };
 
   if (timed) {
