@@ -39,4 +39,7 @@ struct RbfInputs {
 // bit-identical to the host stage's.  Returns AFAR_OK or AFAR_ERR_CUDA (message set).
 afar_status rbf_stage_device(int device, const RbfInputs& in, float* RBFbasis, double* rbf64);
 
+// afar_set_gas without the step graphs, for a solver that is only stepped in a batch (afar_solver.cu).
+afar_status set_gas_batched(afar_solver* s, double R, double Cv);
+
 }  // namespace afar

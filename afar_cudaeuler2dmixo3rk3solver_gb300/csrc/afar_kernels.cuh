@@ -2343,7 +2343,8 @@ __device__ __forceinline__ double wrapd(const double d, const double L) { return
 // calcLeastSquareMatrix (reference cudaFieldOperation.h:91-120) into the slot-major matrix, in
 // FP64 math, stored in the policy's operator type.
 template <class P>
-__global__ void k_setup_lsm(StageArgs<P> a, V2<typename P::S>* lsm, float* lsm_ref_layout, int maxM_ref) {
+__global__ void k_setup_lsm(StageArgs<P> a, V2<typename P::S>* lsm, float* lsm_ref_layout, int maxM_ref,
+                            const int* perm) {
   using S = typename P::S;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= a.Nc) return;
@@ -2364,8 +2365,9 @@ __global__ void k_setup_lsm(StageArgs<P> a, V2<typename P::S>* lsm, float* lsm_r
     const S m2 = (-Sxy * dx + Sxx * dy) / (Sxx * Syy - Sxy * Sxy);
     lsm[i * a.ldc + c] = V2<S>{m1, m2};
     if (lsm_ref_layout) {
-      lsm_ref_layout[2 * (size_t)maxM_ref * c + 2 * i] = (float)m1;
-      lsm_ref_layout[2 * (size_t)maxM_ref * c + 2 * i + 1] = (float)m2;
+      const size_t row = perm ? perm[c] : c;  // the caller's cell
+      lsm_ref_layout[2 * (size_t)maxM_ref * row + 2 * i] = (float)m1;
+      lsm_ref_layout[2 * (size_t)maxM_ref * row + 2 * i + 1] = (float)m2;
     }
   }
 }
@@ -2438,7 +2440,7 @@ __global__ void k_setup_face_geom(StageArgs<P> a, const V4<double>* faceXY, cons
 // weights at the points (its side's row of rbfg [face][side][point][maxS+1]; zeros past the stencil
 // and for boundary faces) and the points minus the cell centre (nearest periodic image).
 template <class P>
-__global__ void k_setup_gauss(StageArgs<P> a, const double* rbfg, const double* pts) {
+__global__ void k_setup_gauss(StageArgs<P> a, const double* rbfg, const double* pts, const int* fperm) {
   using S = typename P::S;
   using G = typename P::G;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2453,21 +2455,23 @@ __global__ void k_setup_gauss(StageArgs<P> a, const double* rbfg, const double* 
     if (f >= a.Nf) continue;
     const int side = fid < 0;
     for (int k = 0; k < ng; ++k) {
-      const double px = pts[2 * ((size_t)f * ng + k)], py = pts[2 * ((size_t)f * ng + k) + 1];
+      const size_t hf = fperm ? fperm[f] : f;  // the caller's face
+      const double px = pts[2 * (hf * ng + k)], py = pts[2 * (hf * ng + k) + 1];
       sgk[(fi * ng + k) * ldc + c] = V2<G>{(G)wrapd(px - x0, a.px), (G)wrapd(py - y0, a.py)};
-      const double* src = rbfg + (((size_t)f * 2 + side) * ng + k) * nmax;
+      const double* src = rbfg + ((hf * 2 + side) * ng + k) * nmax;
       for (int j = 0; j <= a.nS[c]; ++j) wg[(size_t)((fi * ng + k) * nmax + j) * ldc + c] = (S)src[j];
     }
   }
 }
 template <class P>
-__global__ void k_setup_gauss_faces(StageArgs<P> a, const double* pts, const V4<double>* faceXY) {
+__global__ void k_setup_gauss_faces(StageArgs<P> a, const double* pts, const V4<double>* faceXY, const int* fperm) {
   using G = typename P::G;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.Nf * a.ng) return;
   const int f = i / a.ng;
   const V4<double> xy = faceXY[f];
-  const_cast<V2<G>*>(a.fgk)[i] = V2<G>{(G)wrapd(pts[2 * (size_t)i] - xy.x, a.px), (G)wrapd(pts[2 * (size_t)i + 1] - xy.y, a.py)};
+  const size_t h = (size_t)(fperm ? fperm[f] : f) * a.ng + i % a.ng;  // the caller's face and point
+  const_cast<V2<G>*>(a.fgk)[i] = V2<G>{(G)wrapd(pts[2 * h] - xy.x, a.px), (G)wrapd(pts[2 * h + 1] - xy.y, a.py)};
 }
 
 }  // namespace afar

@@ -93,7 +93,7 @@ struct afar_server {
                                             z.maxStencilSize, z.maxCompactStencilSize, z.maxLocalBlockStencilSize,
                                             z.maxCompactLocalBlockStencilSize)))
       return fail(r, e, "stencil upload"), false;
-    if ((e = afar_set_gas(s, q.R, q.Cv))) return fail(r, e, "gas"), false;
+    if ((e = afar::set_gas_batched(s, q.R, q.Cv))) return fail(r, e, "gas"), false;
     if ((e = afar_set_step_params(s, 0.0, q.CFL, q.tEnd > 0.0 ? q.tEnd : 0.0))) return fail(r, e, "step"), false;
     if ((e = afar_device_bytes(s, &r->bytes))) return fail(r, e, "bytes"), false;
     double t, dt;
