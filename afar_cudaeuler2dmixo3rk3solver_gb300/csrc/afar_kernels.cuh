@@ -31,6 +31,7 @@ struct StepCtl {
   unsigned err;  // bit 0: a bounded device wait gave up (the stage's results are not valid)
   double write_interval;  // > 0: land on its multiples like OpenFOAM's adjustableRunTime
   long long write_index;  // write times passed
+  unsigned tiles_done;    // tiles of the last stage that are through (fused tail)
 };
 
 // The step of the current RK step: fixed or CFL, spread over the steps left to the next write time
@@ -106,6 +107,17 @@ struct StageArgs {
   double px, py;       // periods of a periodic mesh (0: none); setup kernels only
   const V2<float>* dtgf;  // Nf (delta r, fraction) as floats (mixed Courant estimate)
   // the optional multi-point face flux (ng > 0 points per face; 0: the face-centre flux)
+  // mixed: the fused stage tail (tail_body)
+  const struct TailTile* tail;   // the tiles of 192 cells
+  const int* thalo;              // [tile][kTailHalo] the cells across each tile's border
+  const int* thcode;             // [tile][4][kTailHalo] the faces of their slots (see tail_body)
+  const V2<typename P::G>* thsg; // [tile][4][kTailHalo] and sg of each
+  const int* textra;             // [tile][kTailExtra] the tile's faces past its own
+  const uint16_t* tlf;           // [maxM][ldc] local face of a cell's slot; bit 15: its neighbour side
+  const int* tlist;              // [tile][kTailList] the 128-cell tiles its stencils reach
+  unsigned* wflag;               // a bit for each cell: troubled (written by the reconstruct)
+  V4<typename P::W>* W3[3];      // the state's buffers: W, and the outputs of the first two stages
+  int nTail, tailT;              // its tiles and the cells of one
   int ng;
   const S* wg;       // [(maxM*ng)*(maxS+1)][ldc] O3 weights at the face Gauss points, per cell slot
   const V2<G>* sgk;  // [maxM*ng][ldc] point minus cell centre, per cell slot
@@ -180,6 +192,77 @@ __device__ __forceinline__ V4<double> limiter_ratios(const LimiterRatio& a, cons
 // (d2GaussQuadrature.C:65-148); the stencil upload rejects larger compact stencils.
 constexpr int kMaxFaces = 4;
 
+// The mixed policy's FP32 Courant estimate of one internal face (setDeltaT, reference
+// cudaFieldOperation.h:140-157): dt = CFL deltaR |Sf| / ((1-w)|U_o.Sf| + w|U_n.Sf| + c |Sf|),
+// c = sqrt(gamma R ((1-w) T_o + w T_n)).  Every rounding is written out, so the fused stage-1 flux
+// and the separate pass (afar_adjustTimeStep) give the same bits wherever the compiler places them.
+__device__ __forceinline__ float courant_den_f32(const float fraction, const float magSf, const float Sfx,
+                                                 const float Sfy, const V4<float>& Wo, const V4<float>& Wn,
+                                                 const float gRf) {
+  const float w0 = __fadd_rn(1.f, -fraction);
+  const float unL = fabsf(__fmaf_rn(Wo.y, Sfx, __fmul_rn(Wo.z, Sfy)));
+  const float unR = fabsf(__fmaf_rn(Wn.y, Sfx, __fmul_rn(Wn.z, Sfy)));
+  const float c = __fsqrt_rn(__fmul_rn(gRf, __fmaf_rn(w0, Wo.w, __fmul_rn(fraction, Wn.w))));
+  return __fmaf_rn(c, magSf, __fmaf_rn(w0, unL, __fmul_rn(fraction, unR)));
+}
+__device__ __forceinline__ float courant_dt_f32(const float cfl, const float deltaR, const float magSf,
+                                                const float den) {
+  return __fdiv_rn(__fmul_rn(__fmul_rn(cfl, deltaR), magSf), den);
+}
+
+// What the mixed reconstructs add for the fused stage tail (tail_body).
+// The lanes of a warp of consecutive cells that have one.
+__device__ __forceinline__ unsigned cell_lanes(const int c, const int Nc) {
+  const int n = Nc - (c & ~31);
+  return n >= 32 ? 0xffffffffu : (1u << n) - 1u;
+}
+// Troubled-cell flags as bits, a word for each warp's cells.
+template <class P>
+__device__ __forceinline__ void put_troubled(const StageArgs<P>& a, const int c, const int8_t flag) {
+  const unsigned b = __ballot_sync(cell_lanes(c, a.Nc), flag != 0);
+  if ((threadIdx.x & 31) == 0 && a.wflag) a.wflag[c >> 5] = b;
+}
+// DT (first stage): the Courant step's minimum over the internal faces that the warp's cells own, from
+// the states at the start of the step: the cell's and, across each face, the stencil member of that
+// face's slot.  The same estimate, to the bit, as in the stage-1 flux.  The geometry is loaded ahead
+// (courant_load); one atomic a warp, which nothing waits for.
+template <int NF>
+struct CourantFaces {
+  V4<float> fs[NF];
+  V2<float> g[NF];
+  float cfl;  // < 0: a fixed step
+};
+template <int NF, class P>
+__device__ __forceinline__ void courant_load(CourantFaces<NF>& q, const StageArgs<P>& a, const int* fid,
+                                             const bool* inner) {
+  q.cfl = gt_zero(a.ctl->dt_fixed) ? -1.f : (float)a.ctl->cfl;
+#pragma unroll
+  for (int fi = 0; fi < NF; ++fi)
+    if (inner[fi] && fid[fi] > 0) {
+      q.fs[fi] = a.fs[fid[fi] - 1];
+      q.g[fi] = a.dtgf[fid[fi] - 1];
+    }
+}
+template <int NF, class P>
+__device__ __forceinline__ void courant_min(const CourantFaces<NF>& q, const StageArgs<P>& a, const int c,
+                                            const int* fid, const bool* inner, const V4<float>& wc,
+                                            const V4<float>* wj) {
+  if (q.cfl < 0.f) return;
+  unsigned m = 0x7F800000u;
+#pragma unroll
+  for (int fi = 0; fi < NF; ++fi) {
+    if (inner[fi] && fid[fi] > 0) {
+      const V4<float> fs = q.fs[fi];
+      const float dt =
+          courant_dt_f32(q.cfl, q.g[fi].x, fs.z, courant_den_f32(q.g[fi].y, fs.z, fs.x, fs.y, wc, wj[fi], a.gRf));
+      if (dt >= 0.f) m = min(m, __float_as_uint(dt));
+    }
+  }
+  m = __reduce_min_sync(cell_lanes(c, a.Nc), m);
+  if ((threadIdx.x & 31) == 0 && m < 0x7F800000u)
+    atomicMin(&a.ctl->dt_bits, (unsigned long long)__double_as_longlong((double)__uint_as_float(m)));
+}
+
 // reconstruct, register-pass variant for the mixed policy (the autotuner's alternative to the
 // tile-staged kernel): LS gradient, stencil min/max, raw limiter, O3 RBF face values of this
 // cell's side of each internal face, troubled-cell flag.
@@ -188,8 +271,8 @@ constexpr int kMaxFaces = 4;
 // loads of a batch of members (indices, gathers, weights) are issued together, so several are in
 // flight per thread; no shared memory, so occupancy is set by registers alone.  Every sum is
 // still accumulated in stencil order, as in the reference.
-template <class P>
-__device__ __forceinline__ void recon_reg_body(const StageArgs<P>& a, const int blk) {
+template <class P, bool DT>
+__device__ __forceinline__ void recon_reg_body(const StageArgs<P>& a, const V4<typename P::W>* W, const int blk) {
   using S = typename P::S;
   using G = typename P::G;
   using WT = typename P::W;
@@ -207,7 +290,7 @@ __device__ __forceinline__ void recon_reg_body(const StageArgs<P>& a, const int 
     inner[fi] = fi < nM && abs(fid[fi]) - 1 < a.Nf;
     lm[fi] = fi < nM ? a.lsm[fi * ldc + c] : V2<S>{S(0), S(0)};
   }
-  const V4<WT> wc = a.W[c];
+  const V4<WT> wc = W[c];
   const S pc = (S)wc.x, uxc = (S)wc.y, uyc = (S)wc.z, tc = (S)wc.w;
   // O3 sums in difference form: sum_i w_i phi_i = phi_c + sum_{i>0} w_i (phi_i - phi_c), since the
   // weights of every face side sum to one.  In FP32 this drops the error phi_c * (sum of the float
@@ -225,7 +308,12 @@ __device__ __forceinline__ void recon_reg_body(const StageArgs<P>& a, const int 
     for (int u = 0; u < kMaxFaces; ++u) j[u] = u < nS ? a.sten[u * ldc + c] : c;
     V4<WT> wj[kMaxFaces];
 #pragma unroll
-    for (int u = 0; u < kMaxFaces; ++u) wj[u] = a.W[j[u]];
+    for (int u = 0; u < kMaxFaces; ++u) wj[u] = W[j[u]];
+    if constexpr (DT) {
+      CourantFaces<kMaxFaces> cour;
+      courant_load<kMaxFaces>(cour, a, fid, inner);
+      courant_min<kMaxFaces>(cour, a, c, fid, inner, wc, wj);
+    }
     S wv[kMaxFaces][kMaxFaces];
 #pragma unroll
     for (int u = 0; u < kMaxFaces; ++u)
@@ -274,7 +362,7 @@ __device__ __forceinline__ void recon_reg_body(const StageArgs<P>& a, const int 
     for (int u = 0; u < U; ++u) j[u] = (ci0 + u < nS) ? a.sten[(ci0 + u) * ldc + c] : c;
     V4<WT> wj[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) wj[u] = a.W[j[u]];
+    for (int u = 0; u < U; ++u) wj[u] = W[j[u]];
     S wv[U][kMaxFaces];
 #pragma unroll
     for (int u = 0; u < U; ++u)
@@ -357,6 +445,7 @@ __device__ __forceinline__ void recon_reg_body(const StageArgs<P>& a, const int 
   }
   a.lim[c] = L;
   a.si[2 * c] = flag0;
+  put_troubled(a, c, flag0);
 }
 
 // ---------------------------------------------------------------- mixed reconstruct, tile-staged
@@ -435,7 +524,8 @@ __host__ __device__ inline ReconTile recon_tile_layout(const int maxM, const int
 // in.  Smem rows hold 128 cells: face ids [maxM][128], stencil ids [S][128], LS and geometry
 // [maxM][128] pairs, weights [maxM][S][128] (S = the tile's largest stencil).
 template <class P>
-__device__ __forceinline__ void recon_tile_fetch(const StageArgs<P>& a, const int blk, const ReconTile& L,
+__device__ __forceinline__ void recon_tile_fetch(const StageArgs<P>& a, const V4<typename P::W>* W, const int blk,
+                                                 const ReconTile& L,
                                                  unsigned char* sm, unsigned long long* bar) {
   const int lane = threadIdx.x;
   const int c0 = blk * kTile;
@@ -450,7 +540,7 @@ __device__ __forceinline__ void recon_tile_fetch(const StageArgs<P>& a, const in
   switch (lane) {
     case 0: tma_load_2d(sm + L.off_cf, &tm->cf, c0, 0, bar); break;
     case 1: tma_load_2d(sm + L.off_sten, &tm->sten[S - 1], c0, 0, bar); break;
-    case 2: bulk_to_smem(sm + L.off_w, a.W + c0, (unsigned)min(kTile, a.Nc - c0) * 16u, bar); break;
+    case 2: bulk_to_smem(sm + L.off_w, W + c0, (unsigned)min(kTile, a.Nc - c0) * 16u, bar); break;
     case 3: tma_load_2d(sm + L.off_lsm, &tm->lsm, 2 * c0, 0, bar + 1); break;
     case 4: tma_load_2d(sm + L.off_sg, &tm->sg, 2 * c0, 0, bar + 1); break;
     case 5: tma_load_2d(sm + L.off_sr, &tm->sr, 2 * c0, 0, bar + 1); break;
@@ -465,8 +555,9 @@ __device__ __forceinline__ void recon_tile_fetch(const StageArgs<P>& a, const in
 // batches of 8, all in flight) and feeds the gradient and min/max (compact members) and the O3 sums
 // of every face side; every sum is accumulated in stencil order, as in the reference.  NF: the
 // largest number of faces of a cell (3 on all-triangle meshes, else 4).
-template <class P, int NF>
-__device__ __forceinline__ void recon_tile_body(const StageArgs<P>& a, const int blk, unsigned char* sm) {
+template <class P, int NF, bool DT>
+__device__ __forceinline__ void recon_tile_body(const StageArgs<P>& a, const V4<typename P::W>* W, const int blk,
+                                                unsigned char* sm) {
   using S = typename P::S;
   using G = typename P::G;
   using WT = typename P::W;
@@ -478,7 +569,7 @@ __device__ __forceinline__ void recon_tile_body(const StageArgs<P>& a, const int
     mbar_init(bar + 1, 1);
   }
   __syncthreads();
-  if (t < 32) recon_tile_fetch(a, blk, L, sm, bar);
+  if (t < 32) recon_tile_fetch(a, W, blk, L, sm, bar);
   const int c = blk * kTile + t;
   const int nS = c < a.Nc ? a.nS[c] : 0, nM = c < a.Nc ? a.nM[c] : 0;
   const long long limit = g_tile_wait_limit;
@@ -515,8 +606,11 @@ __device__ __forceinline__ void recon_tile_body(const StageArgs<P>& a, const int
   V4<WT> wj[U];  // the first batch of stencil states, gathered before the weights have landed
 #pragma unroll
   for (int u = 0; u < U; ++u)
-    if (u < nS) wj[u] = a.W[s_sten[u * kTile + t]];
+    if (u < nS) wj[u] = W[s_sten[u * kTile + t]];
+  CourantFaces<NF> cour;
+  if constexpr (DT) courant_load<NF>(cour, a, fid, inner);
   if (!mbar_wait_bounded(bar + 1, 0, limit)) return give_up();
+  if constexpr (DT) courant_min<NF>(cour, a, c, fid, inner, wc, wj);
   // O3 weights of boundary-face and missing slots are zero in the operator rows (setup), so only
   // slots past this mesh's largest cell (a batch may stage fewer rows than NF) are skipped
   const int nfm = a.maxM;
@@ -532,7 +626,7 @@ __device__ __forceinline__ void recon_tile_body(const StageArgs<P>& a, const int
     if (ci0 > 0) {
 #pragma unroll
       for (int u = 0; u < U; ++u)
-        if (ci0 + u < nS) wj[u] = a.W[s_sten[(ci0 + u) * kTile + t]];
+        if (ci0 + u < nS) wj[u] = W[s_sten[(ci0 + u) * kTile + t]];
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -636,6 +730,7 @@ __device__ __forceinline__ void recon_tile_body(const StageArgs<P>& a, const int
   }
   a.lim[c] = Lm;
   a.si[2 * c] = flag0;
+  put_troubled(a, c, flag0);
 }
 
 // reconstruct for the ref policy: the stencil values are staged in shared memory in batches (indices,
@@ -1039,24 +1134,6 @@ __device__ __forceinline__ void bvd_body(const StageArgs<P>& a, const int blk) {
   a.lim[c] = L;
 }
 
-// The mixed policy's FP32 Courant estimate of one internal face (setDeltaT, reference
-// cudaFieldOperation.h:140-157): dt = CFL deltaR |Sf| / ((1-w)|U_o.Sf| + w|U_n.Sf| + c |Sf|),
-// c = sqrt(gamma R ((1-w) T_o + w T_n)).  Every rounding is written out, so the fused stage-1 flux
-// and the separate pass (afar_adjustTimeStep) give the same bits wherever the compiler places them.
-__device__ __forceinline__ float courant_den_f32(const float fraction, const float magSf, const float Sfx,
-                                                 const float Sfy, const V4<float>& Wo, const V4<float>& Wn,
-                                                 const float gRf) {
-  const float w0 = __fadd_rn(1.f, -fraction);
-  const float unL = fabsf(__fmaf_rn(Wo.y, Sfx, __fmul_rn(Wo.z, Sfy)));
-  const float unR = fabsf(__fmaf_rn(Wn.y, Sfx, __fmul_rn(Wn.z, Sfy)));
-  const float c = __fsqrt_rn(__fmul_rn(gRf, __fmaf_rn(w0, Wo.w, __fmul_rn(fraction, Wn.w))));
-  return __fmaf_rn(c, magSf, __fmaf_rn(w0, unL, __fmul_rn(fraction, unR)));
-}
-__device__ __forceinline__ float courant_dt_f32(const float cfl, const float deltaR, const float magSf,
-                                                const float den) {
-  return __fdiv_rn(__fmul_rn(__fmul_rn(cfl, deltaR), magSf), den);
-}
-
 // minimizeDeltaValue (reference cudaRiemannSolver.h:7-14)
 template <class D, class G>
 __device__ __forceinline__ D min_delta(const G l, const G r, const G lT, const G rT) {
@@ -1250,6 +1327,167 @@ __device__ __forceinline__ void kfvs_flux_fast(D& rhoFlux, D& rhoUxFlux, D& rhoU
   rhoEFlux += trhoE * magSf - D(0.5) * rhoFlux * (Cv * tL + D(0.5) * (uxL * uxL + uyL * uyL) + R * tL) -
               D(0.5) * rhoFlux * (Cv * tR + D(0.5) * (uxR * uxR + uyR * uyR) + R * tR);
   rhoFlux += trho * magSf - D(0.5) * rhoL * (uxL * Sfx + uyL * Sfy) - D(0.5) * rhoR * (uxR * Sfx + uyR * Sfy);
+}
+
+// One side of a face: the state that the flux uses, and p and T of its TVD state.
+struct MixedSide {
+  float p, ux, uy, T, pT, tT;
+};
+// The mixed policy's flux of an internal face (reference cudaRiemannSolver.h:16-251): central flux with the
+// Roe dissipation, or the KFVS flux; the expressions of roe_flux_fast and kfvs_flux_fast.  Every rounding
+// is written out, in the pattern in which the compiler fuses those expressions in the separate flux
+// kernel (found by comparing results: each candidate rounding on 65k random faces, equal to the bit), so
+// that the kernels that call it agree bit for bit whatever the code around the call.  E: the energy flux's
+// sum of two products fused, as the compiler has it in the batched stage-1 flux (DT) and nowhere else.
+__device__ __forceinline__ float fm_(const float a, const float b, const float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float ml_(const float a, const float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float ad_(const float a, const float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float dot_(const float a, const float b, const float c, const float d) {  // a b + c d
+  return fm_(a, b, ml_(c, d));
+}
+// w + lim (ga dx + gb dy): the limited linear (TVD) value
+__device__ __forceinline__ float tvd_mixed(const float w, const float lim, const float ga, const float gb,
+                                           const V2<float> d) {
+  return fm_(lim, dot_(ga, d.x, gb, d.y), w);
+}
+// __fdividef(a, b) is a times this, to the bit, for |b| up to 2^126 (checked on 2.7e9 pairs); it also spends
+// four instructions on larger ones
+__device__ __forceinline__ float rcp_(const float x) {
+  float y;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// The density p/(R T) as the product it is, for the differences that round the product away
+struct MixedRho {
+  float num, rcp, rho;
+};
+__device__ __forceinline__ MixedRho mixed_rho(const float p, const float iR, const float T) {
+  MixedRho r;
+  r.num = ml_(p, iR);
+  r.rcp = rcp_(T);
+  r.rho = ml_(r.num, r.rcp);
+  return r;
+}
+// minimizeDeltaValue's last step: the smallest jump d >= 0 with the sign of r - l
+__device__ __forceinline__ float signed_jump(const float d, const float l, const float r) { return r >= l ? d : -d; }
+__device__ __forceinline__ void entropy_fix_mixed(float& l, const float jump) {
+  const float eps = ml_(2.f, fmaxf(0.f, jump));
+  if (l < eps) l = ml_(fm_(eps, eps, ml_(l, l)), rcp_(fm_(2.f, eps, 1e-30f)));
+}
+// One side's kinetic moments: the half-range fluxes of mass, normal momentum and energy moments.
+struct MixedKinetic {
+  float m1, m2, m3;
+};
+__device__ __forceinline__ MixedKinetic mixed_kinetic(const bool left, const float u, const float lam, const float il) {
+  const float su = ml_(sqrtf(lam), u);
+  const float m0 = ml_(0.5f, erfcf(left ? -su : su));
+  const float ex = ml_(0.5f, expf(ml_(ml_(-lam, u), u))), rs = rsqrtf(ml_(3.141593f, lam));
+  MixedKinetic q;
+  q.m1 = left ? fm_(ex, rs, ml_(u, m0)) : fm_(u, m0, ml_(-ex, rs));
+  q.m2 = fm_(ml_(0.5f, m0), il, ml_(u, q.m1));
+  q.m3 = fm_(q.m1, il, ml_(u, q.m2));
+  return q;
+}
+template <bool E>
+__device__ __forceinline__ V4<float> mixed_flux(const MixedSide& l, const MixedSide& r, const bool isShock,
+                                                const V4<float>& fs, const float R, const float Cv, const float iR,
+                                                const float gam) {
+  const float h = 0.5f, Sfx = fs.x, Sfy = fs.y, magSf = fs.z;
+  const MixedRho dl = mixed_rho(l.p, iR, l.T), dr = mixed_rho(r.p, iR, r.T);
+  const float rhoL = dl.rho, rhoR = dr.rho;
+  // central flux
+  const float unL = dot_(l.ux, Sfx, l.uy, Sfy), unR = dot_(r.ux, Sfx, r.uy, Sfy);
+  const float F0 = dot_(ml_(h, rhoL), unL, ml_(h, rhoR), unR);
+  const float F1 = dot_(h, dot_(l.p, Sfx, F0, l.ux), h, dot_(r.p, Sfx, F0, r.ux));
+  const float F2 = dot_(h, dot_(l.p, Sfy, F0, l.uy), h, dot_(r.p, Sfy, F0, r.uy));
+  const float kkL = dot_(l.ux, l.ux, l.uy, l.uy), kkR = dot_(r.ux, r.ux, r.uy, r.uy);
+  const float hF = ml_(h, F0);
+  const float htL = fm_(R, l.T, fm_(Cv, l.T, ml_(h, kkL))), htR = fm_(R, r.T, fm_(Cv, r.T, ml_(h, kkR)));
+  const float F3 = E ? dot_(hF, htL, hF, htR) : ad_(ml_(hF, htL), ml_(hF, htR));
+  const float nfx = ml_(Sfx, fs.w), nfy = ml_(Sfy, fs.w);  // fs.w = 1/|Sf| (setup)
+  const float cvL = dot_(l.ux, nfx, l.uy, nfy), cvR = dot_(r.ux, nfx, r.uy, nfy);
+  if (isShock) {
+    const float K = fm_(ml_(2.f, Cv), iR, -2.f);
+    const float Gx = ml_(nfx, magSf), Gy = ml_(nfy, magSf);
+    const float vL = dot_(l.uy, nfx, -l.ux, nfy), vR = dot_(r.uy, nfx, -r.ux, nfy);
+    const float ilL = ml_(ml_(2.f, R), l.T), ilR = ml_(ml_(2.f, R), r.T);  // 1/lambda = 2 p / rho
+    const MixedKinetic a = mixed_kinetic(true, cvL, rcp_(ilL), ilL);
+    const MixedKinetic b = mixed_kinetic(false, cvR, rcp_(ilR), ilR);
+    const float rmL = ml_(rhoL, a.m1), rmR = ml_(rhoR, b.m1);
+    const float t0 = ad_(rmL, rmR), tx = dot_(rhoL, a.m2, rhoR, b.m2), ty = dot_(rmL, vL, rmR, vR);
+    const float hrL = ml_(h, rhoL), hrR = ml_(h, rhoR);
+    const float enL = fm_(ml_(ml_(a.m1, K), h), ilL, fm_(a.m1, fm_(vL, vL, ml_(h, ilL)), a.m3));
+    const float enR = fm_(ml_(ml_(b.m1, K), h), ilR, fm_(b.m1, fm_(vR, vR, ml_(h, ilR)), b.m3));
+    const float t3 = dot_(hrL, enL, hrR, enR);
+    const float x1 = fm_(-h, dot_(r.p, Gx, F0, r.ux), fm_(-h, dot_(l.p, Gx, F0, l.ux), dot_(tx, Gx, -ty, Gy)));
+    const float x2 = fm_(-h, dot_(r.p, Gy, F0, r.uy), fm_(-h, dot_(l.p, Gy, F0, l.uy), dot_(ty, Gx, tx, Gy)));
+    const float x3 = E ? fm_(-hF, htR, fm_(t3, magSf, -ml_(hF, htL))) : ad_(fm_(t3, magSf, -ml_(hF, htL)), -ml_(hF, htR));
+    const float x0 = fm_(-hrR, dot_(r.ux, Gx, r.uy, Gy), fm_(t0, magSf, ml_(-hrL, dot_(l.ux, Gx, l.uy, Gy))));
+    return V4<float>{ad_(F0, x0), ad_(F1, x1), ad_(F2, x2), ad_(F3, x3)};
+  }
+  const MixedRho dlT = mixed_rho(l.pT, iR, l.tT), drT = mixed_rho(r.pT, iR, r.tT);
+  float dP = fabsf(ad_(r.p, -l.p));
+  dP = fminf(dP, fabsf(ad_(r.p, -l.pT)));
+  dP = fminf(dP, fabsf(ad_(r.pT, -l.p)));
+  dP = fminf(dP, fabsf(ad_(r.pT, -l.pT)));
+  dP = signed_jump(dP, l.p, r.p);
+  float dRho = fabsf(ad_(rhoR, -rhoL));
+  dRho = fminf(dRho, fabsf(fm_(-dlT.num, dlT.rcp, rhoR)));
+  dRho = fminf(dRho, fabsf(fm_(drT.num, drT.rcp, -rhoL)));
+  dRho = fminf(dRho, fabsf(fm_(drT.num, drT.rcp, -dlT.rho)));
+  dRho = signed_jump(dRho, rhoL, rhoR);
+  const float kL = ml_(h, kkL), kR = ml_(h, kkR);
+  const float hL = fm_(R, l.T, fm_(Cv, l.T, kL)), hR = fm_(R, r.T, fm_(Cv, r.T, kR));
+  const float tiny = 1e-20f;
+  const float sL = sqrtf(fmaxf(rhoL, tiny)), sR = sqrtf(fmaxf(rhoR, tiny));
+  const float rhoT = ml_(sL, sR);  // sqrt(rhoL rhoR) from the two roots the weights need anyway
+  const float wL = ml_(sL, rcp_(ad_(sL, sR))), wR = ad_(1.f, -wL);
+  const float uxT = dot_(l.ux, wL, r.ux, wR), uyT = dot_(l.uy, wL, r.uy, wR), hT = dot_(hL, wL, hR, wR);
+  const float q2 = dot_(uxT, uxT, uyT, uyT), gm1 = ad_(gam, -1.f);
+  const float cT2 = fmaxf(ml_(gm1, fm_(-h, q2, hT)), tiny);
+  const float rcT = rsqrtf(cT2);  // 1/cT: the speed and 1/cT^2 from one reciprocal root
+  const float cT = ml_(cT2, rcT), ic2 = ml_(rcT, rcT);
+  const float cvT = dot_(uxT, nfx, uyT, nfy);
+  const float dUx = ad_(r.ux, -l.ux), dUy = ad_(r.uy, -l.uy);
+  const float dCv = dot_(dUx, nfx, dUy, nfy);
+  const float rc = ml_(rhoT, cT), hic2 = ml_(h, ic2);
+  const float r1 = ml_(fm_(-rc, dCv, dP), hic2), r2 = fm_(-dP, ic2, dRho), r3 = ml_(fm_(rc, dCv, dP), hic2);
+  float l1 = fabsf(ad_(cvT, -cT)), l2 = fabsf(cvT), l3 = fabsf(ad_(cvT, cT));
+  entropy_fix_mixed(l2, ad_(cvR, -cvL));
+  {  // the acoustic waves: the sides' sound speeds exactly only where approximate ones do not rule the fix out
+    const float xL = fmaxf(ml_(gm1, ad_(hL, -kL)), tiny), xR = fmaxf(ml_(gm1, ad_(hR, -kR)), tiny);
+    float cL, cR;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(cL) : "f"(xL));
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(cR) : "f"(xR));
+    const float margin = 1e-5f * (fabsf(cvL) + fabsf(cvR) + cL + cR + cT), dcv = cvR - cvL, dc = cR - cL;
+    if (!(l1 > fmaxf(0.f, 2.f * (dcv - dc)) + margin && l3 > fmaxf(0.f, 2.f * (dcv + dc)) + margin)) {
+      cL = sqrtf(xL);
+      cR = sqrtf(xR);
+      entropy_fix_mixed(l1, ad_(ad_(cvR, -cR), -ad_(cvL, -cL)));
+      entropy_fix_mixed(l3, ad_(ad_(cvR, cR), -ad_(cvL, cL)));
+    }
+  }
+  const float a1 = ml_(l1, r1), a3 = ml_(l3, r3);
+  const float s0 = ad_(a3, fm_(l2, r2, a1));
+  const float s1 = fm_(a3, fm_(cT, nfx, uxT),
+                       dot_(a1, fm_(-cT, nfx, uxT), l2, dot_(rhoT, fm_(-dCv, nfx, dUx), r2, uxT)));
+  const float s2 = fm_(a3, fm_(cT, nfy, uyT),
+                       dot_(a1, fm_(-cT, nfy, uyT), l2, dot_(rhoT, fm_(-dCv, nfy, dUy), r2, uyT)));
+  const float shear = fm_(-cvT, dCv, dot_(uxT, dUx, uyT, dUy));
+  const float s3 = fm_(a3, fm_(cT, cvT, hT), dot_(a1, fm_(-cT, cvT, hT), l2, dot_(ml_(r2, h), q2, rhoT, shear)));
+  return V4<float>{fm_(-ml_(h, s0), magSf, F0), fm_(-ml_(h, s1), magSf, F1), fm_(-ml_(h, s2), magSf, F2),
+                   fm_(-ml_(h, s3), magSf, F3)};
+}
+// The Euler flux of a boundary face's ghost state, its roundings written out as the compiler fuses them in
+// flux_body (the separate flux kernels), so that both forms of the stage give the same bits.
+__device__ __forceinline__ V4<float> mixed_boundary_flux(const V4<float>& wb, const V4<float>& fs, const float R,
+                                                         const float Cv) {
+  const float rho = wb.x / __fmul_rn(R, wb.w);
+  const float rhoFlux = __fmul_rn(rho, __fmaf_rn(wb.y, fs.x, __fmul_rn(wb.z, fs.y)));
+  const float ke2 = __fmaf_rn(wb.y, wb.y, __fmul_rn(wb.z, wb.z));
+  const float h = __fadd_rn(__fmaf_rn(0.5f, ke2, __fmul_rn(Cv, wb.w)), wb.x / rho);
+  return V4<float>{rhoFlux, __fmaf_rn(wb.x, fs.x, __fmul_rn(rhoFlux, wb.y)),
+                   __fmaf_rn(wb.x, fs.y, __fmul_rn(rhoFlux, wb.z)), __fmul_rn(rhoFlux, h)};
 }
 
 // minimizeDeltaValue (min_delta) of doubles with the minima and the sign on integers.
@@ -1518,7 +1756,7 @@ __device__ __forceinline__ void flux_ref_face(const StageArgs<PolicyRef>& a, con
 // boundary face (ids Nf..Nf+Nb-1; the reference's grid covers boundary faces b < 128*ceil(Nf/128)
 // only, which holds on every mesh with Nf >= Nb).  DT: also reduce the CFL step of the reference's
 // setDeltaT (cudaFieldOperation.h:124-180) from the state at the start of the step.
-template <class P, bool DT>
+template <class P, bool DT, bool BATCH = false>
 __device__ __forceinline__ void flux_body(const StageArgs<P>& a, const int blk) {
   using S = typename P::S;
   using G = typename P::G;
@@ -1571,58 +1809,24 @@ __device__ __forceinline__ void flux_body(const StageArgs<P>& a, const int blk) 
       const G dxL = fd.x, dyL = fd.y, dxR = fd.z, dyR = fd.w;
       const int8_t sL = a.si[2 * own + 1], sR = a.si[2 * nei + 1];
       const bool tvdL = sL != 0, tvdR = sR != 0;
-      const bool isShock = sL < 0 || sR < 0;
       const V4<G> fs = a.fs[id];
-      const G Sfx = fs.x, Sfy = fs.y, magSf = fs.z;
-      const G R = a.Rf, Cv = a.Cvf, iR = a.invRf, gam = a.gm1f + 1.f;
       const V4<typename P::W> Wo = a.W[own], Wn = a.W[nei];
       const V4<G> go0 = a.grad[2 * own], go1 = a.grad[2 * own + 1];
       const V4<G> gn0 = a.grad[2 * nei], gn1 = a.grad[2 * nei + 1];
       const V4<S> lo = a.lim[own], ln = a.lim[nei];
       const V4<G> fo = a.fv[2 * id], fn = a.fv[2 * id + 1];
-      G rhoFlux, rhoUxFlux, rhoUyFlux, rhoEFlux;
-      D pLf, uxLf, uyLf, tLf, rhoLf, pRf, uxRf, uyRf, tRf, rhoRf, dP, dRho;
-      {
-        const G pLT = (G)Wo.x + lo.x * (go0.x * dxL + go0.y * dyL);
-        const G uxLT = (G)Wo.y + lo.y * (go0.z * dxL + go1.x * dyL);
-        const G uyLT = (G)Wo.z + lo.z * (go0.w * dxL + go1.y * dyL);
-        const G tLT = (G)Wo.w + lo.w * (go1.z * dxL + go1.w * dyL);
-        const G pRT = (G)Wn.x + ln.x * (gn0.x * dxR + gn0.y * dyR);
-        const G uxRT = (G)Wn.y + ln.y * (gn0.z * dxR + gn1.x * dyR);
-        const G uyRT = (G)Wn.z + ln.z * (gn0.w * dxR + gn1.y * dyR);
-        const G tRT = (G)Wn.w + ln.w * (gn1.z * dxR + gn1.w * dyR);
-        const G pL = pick<P>(!tvdL, tvdL, fo.x, pLT);
-        const G uxL = pick<P>(!tvdL, tvdL, fo.y, uxLT);
-        const G uyL = pick<P>(!tvdL, tvdL, fo.z, uyLT);
-        const G tL = pick<P>(!tvdL, tvdL, fo.w, tLT);
-        const G pR = pick<P>(!tvdR, tvdR, fn.x, pRT);
-        const G uxR = pick<P>(!tvdR, tvdR, fn.y, uxRT);
-        const G uyR = pick<P>(!tvdR, tvdR, fn.z, uyRT);
-        const G tR = pick<P>(!tvdR, tvdR, fn.w, tRT);
-        // p / (R T) of the four states
-        const G rhoLT = fdiv(pLT * iR, tLT), rhoRT = fdiv(pRT * iR, tRT);
-        const G rhoL = fdiv(pL * iR, tL), rhoR = fdiv(pR * iR, tR);
-        dP = min_delta<D, G>(pL, pR, pLT, pRT);
-        dRho = min_delta<D, G>(rhoL, rhoR, rhoLT, rhoRT);
-        const G h = G(0.5);
-        rhoFlux = h * rhoL * (uxL * Sfx + uyL * Sfy) + h * rhoR * (uxR * Sfx + uyR * Sfy);
-        rhoUxFlux = h * (rhoFlux * uxL + pL * Sfx) + h * (rhoFlux * uxR + pR * Sfx);
-        rhoUyFlux = h * (rhoFlux * uyL + pL * Sfy) + h * (rhoFlux * uyR + pR * Sfy);
-        rhoEFlux = h * rhoFlux * (Cv * tL + h * (uxL * uxL + uyL * uyL) + R * tL) +  // p/rho = R T
-                   h * rhoFlux * (Cv * tR + h * (uxR * uxR + uyR * uyR) + R * tR);
-        pLf = pL; uxLf = uxL; uyLf = uyL; tLf = tL; rhoLf = rhoL;
-        pRf = pR; uxRf = uxR; uyRf = uyR; tRf = tR; rhoRf = rhoR;
-      }
-      static_assert(std::is_same<D, G>::value, "fp64 and mixed run the dissipation in their face-value type");
-      const G nfx = Sfx * fs.w, nfy = Sfy * fs.w;  // fs.w = 1/|Sf| (setup)
-      if (isShock)
-        kfvs_flux_fast<G>(rhoFlux, rhoUxFlux, rhoUyFlux, rhoEFlux, rhoLf, rhoRf, pLf, pRf, uxLf, uxRf, uyLf, uyRf, tLf,
-                          tRf, R, Cv, G(2) * Cv * iR - G(2), magSf, nfx, nfy);
-      else
-        roe_flux_fast<G>(rhoFlux, rhoUxFlux, rhoUyFlux, rhoEFlux, rhoLf, rhoRf, uxLf, uxRf, uyLf, uyRf, tLf, tRf, dP,
-                         dRho, R, Cv, gam, magSf, nfx, nfy);
-      a.flux[id] = V4<typename P::F>{(typename P::F)rhoFlux, (typename P::F)rhoUxFlux, (typename P::F)rhoUyFlux,
-                                     (typename P::F)rhoEFlux};
+      const G pLT = Wo.x + lo.x * (go0.x * dxL + go0.y * dyL);
+      const G uxLT = Wo.y + lo.y * (go0.z * dxL + go1.x * dyL);
+      const G uyLT = Wo.z + lo.z * (go0.w * dxL + go1.y * dyL);
+      const G tLT = Wo.w + lo.w * (go1.z * dxL + go1.w * dyL);
+      const G pRT = Wn.x + ln.x * (gn0.x * dxR + gn0.y * dyR);
+      const G uxRT = Wn.y + ln.y * (gn0.z * dxR + gn1.x * dyR);
+      const G uyRT = Wn.z + ln.z * (gn0.w * dxR + gn1.y * dyR);
+      const G tRT = Wn.w + ln.w * (gn1.z * dxR + gn1.w * dyR);
+      const MixedSide l{tvdL ? pLT : fo.x, tvdL ? uxLT : fo.y, tvdL ? uyLT : fo.z, tvdL ? tLT : fo.w, pLT, tLT};
+      const MixedSide r{tvdR ? pRT : fn.x, tvdR ? uxRT : fn.y, tvdR ? uyRT : fn.z, tvdR ? tRT : fn.w, pRT, tRT};
+      const G Sfx = fs.x, Sfy = fs.y, magSf = fs.z;
+      a.flux[id] = mixed_flux<BATCH && DT>(l, r, sL < 0 || sR < 0, fs, a.Rf, a.Cvf, a.invRf, a.gm1f + 1.f);
       if constexpr (DT) {
         if (s_cfl_step) {  // setDeltaT, cudaFieldOperation.h:140-157, as an FP32 estimate
           const V2<float> g = a.dtgf[id];
@@ -1732,13 +1936,51 @@ __device__ __forceinline__ void two_sum(float& s, float& e, const float a, const
   e = (a - (s - bp)) + (b - bp);
 }
 
+// The RK combine of one cell of the mixed policy from its residual (hi + lo) and its Un and U (from0, from):
+// U (and Un after the last stage) are stored, the new primitive state returned.
+__device__ __forceinline__ V4<float> advance_mixed(const StageArgs<PolicyMixed>& a, const int c, const StageCoef& k,
+                                                   const float bdt, const float* hi, const float* lo,
+                                                   const DF4* from0, const DF4* from) {
+  const float s3 = -bdt * a.vinvf[c];
+  DF4* const U = reinterpret_cast<DF4*>(a.U);
+  DF4* const U0 = reinterpret_cast<DF4*>(a.U0);
+  const DF4 o = *from0;
+  DF base[4] = {{o.hi.x, o.lo.x}, {o.hi.y, o.lo.y}, {o.hi.z, o.lo.z}, {o.hi.w, o.lo.w}};
+  if (!k.first) {  // stages 2, 3: beta1 Un + beta2 U (stage 1 is Un + increment, U not read)
+    const DF4 u = *from;
+    const DF b1{k.b1h, k.b1l}, b2{k.b2h, k.b2l};
+    const DF uu[4] = {{u.hi.x, u.lo.x}, {u.hi.y, u.lo.y}, {u.hi.z, u.lo.z}, {u.hi.w, u.lo.w}};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) base[q] = df_add(df_mul(b1, base[q]), df_mul(b2, uu[q]));
+  }
+  DF un[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) un[q] = df_add(base[q], __fmul_rn(s3, __fadd_rn(hi[q], lo[q])));
+  const DF4 st{{un[0].hi, un[1].hi, un[2].hi, un[3].hi}, {un[0].lo, un[1].lo, un[2].lo, un[3].lo}};
+  U[c] = st;
+  if (k.last) U0[c] = st;
+  float irf = __fdividef(1.f, un[0].hi);  // 1/rho: fast reciprocal + one Newton step (~1 ulp)
+  irf = __fmaf_rn(irf, __fmaf_rn(-un[0].hi, irf, 1.f), irf);
+  const DF ke2 = df_div(df_add(df_sqr(un[1]), df_sqr(un[2])), un[0], irf);  // |rhoU|^2 / rho
+  const DF e = df_add(un[3], DF{-0.5f * ke2.hi, -0.5f * ke2.lo});
+  const float pf = a.gm1f * __fadd_rn(e.hi, e.lo);
+  return V4<float>{pf, un[1].hi * irf, un[2].hi * irf, pf * irf * a.invRf};
+}
+// The ghost of boundary face b from its cell's new state.
+__device__ __forceinline__ void ghost_mixed(const StageArgs<PolicyMixed>& a, const int b, const V4<float>& wn,
+                                            V4<float>* W) {
+  if (a.btype[b] == AFAR_BC_FIXED_INITIAL) return;  // the ghost keeps its uploaded state
+  const V4<double> g =
+      boundary_value(a.btype[b], V4<double>{(double)wn.x, (double)wn.y, (double)wn.z, (double)wn.w}, a.bn[b]);
+  W[a.Nc + b] = V4<float>{(float)g.x, (float)g.y, (float)g.z, (float)g.w};
+}
+
 // The mixed policy's gather + update, with no FP64 arithmetic on the path (GB300's FP64 pipe is
 // 1/53 of FP32): the residual of the float fluxes is summed error-free as a float pair, the
 // conserved state U, Un is stored and combined as float pairs (DF4, ~48 bits), and the pressure is
 // the float-pair difference rhoE - |rhoU|^2/(2 rho) (the cancellation at high Mach costs no
 // precision), rounded once to float.  k = {beta3*dt, beta1 (hi, lo), beta2 (hi, lo)} of the stage.
-template <class P>
-__device__ __forceinline__ void update_mixed(const StageArgs<P>& a, const int c, const StageCoef& k,
+__device__ __forceinline__ void update_mixed(const StageArgs<PolicyMixed>& a, const int c, const StageCoef& k,
                                              const int* s_go, const float* s_bdt) {
   const int ldc = a.ldc;
   const bool live = c < a.Nc;
@@ -1751,7 +1993,7 @@ __device__ __forceinline__ void update_mixed(const StageArgs<P>& a, const int c,
     for (int u = 0; u < MB; ++u) fid[u] = (f0 + u < nM) ? a.cf[(f0 + u) * ldc + c] : 1;
     V4<float> fl[MB];
 #pragma unroll
-    for (int u = 0; u < MB; ++u) fl[u] = reinterpret_cast<const V4<float>*>(a.flux)[abs(fid[u]) - 1];
+    for (int u = 0; u < MB; ++u) fl[u] = a.flux[abs(fid[u]) - 1];
 #pragma unroll
     for (int u = 0; u < MB; ++u) {
       if (f0 + u < nM) {
@@ -1770,39 +2012,12 @@ __device__ __forceinline__ void update_mixed(const StageArgs<P>& a, const int c,
   if (!live || !*s_go) return;
   if (a.res_dbg) a.res_dbg[c] = V4<double>{(double)hi[0] + lo[0], (double)hi[1] + lo[1], (double)hi[2] + lo[2],
                                           (double)hi[3] + lo[3]};
-  const float s3 = -*s_bdt * a.vinvf[c];
-  DF4* const U = reinterpret_cast<DF4*>(a.U);
-  DF4* const U0 = reinterpret_cast<DF4*>(a.U0);
-  const DF4 o = U0[c];
-  DF base[4] = {{o.hi.x, o.lo.x}, {o.hi.y, o.lo.y}, {o.hi.z, o.lo.z}, {o.hi.w, o.lo.w}};
-  if (!k.first) {  // stages 2, 3: beta1 Un + beta2 U (stage 1 is Un + increment, U not read)
-    const DF4 u = U[c];
-    const DF b1{k.b1h, k.b1l}, b2{k.b2h, k.b2l};
-    const DF uu[4] = {{u.hi.x, u.lo.x}, {u.hi.y, u.lo.y}, {u.hi.z, u.lo.z}, {u.hi.w, u.lo.w}};
-#pragma unroll
-    for (int q = 0; q < 4; ++q) base[q] = df_add(df_mul(b1, base[q]), df_mul(b2, uu[q]));
-  }
-  DF un[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) un[q] = df_add(base[q], __fmul_rn(s3, __fadd_rn(hi[q], lo[q])));
-  const DF4 st{{un[0].hi, un[1].hi, un[2].hi, un[3].hi}, {un[0].lo, un[1].lo, un[2].lo, un[3].lo}};
-  U[c] = st;
-  if (k.last) U0[c] = st;
-  float irf = __fdividef(1.f, un[0].hi);  // 1/rho: fast reciprocal + one Newton step (~1 ulp)
-  irf = __fmaf_rn(irf, __fmaf_rn(-un[0].hi, irf, 1.f), irf);
-  const DF ke2 = df_div(df_add(df_sqr(un[1]), df_sqr(un[2])), un[0], irf);  // |rhoU|^2 / rho
-  const DF e = df_add(un[3], DF{-0.5f * ke2.hi, -0.5f * ke2.lo});
-  const float pf = a.gm1f * __fadd_rn(e.hi, e.lo);
-  const V4<float> wn{pf, un[1].hi * irf, un[2].hi * irf, pf * irf * a.invRf};
-  reinterpret_cast<V4<float>*>(a.W)[c] = wn;
+  const V4<float> wn = advance_mixed(a, c, k, *s_bdt, hi, lo, reinterpret_cast<const DF4*>(a.U0) + c,
+                                     reinterpret_cast<const DF4*>(a.U) + c);
+  a.W[c] = wn;
   for (int fi = 0; fi < nM; ++fi) {
     const int f = abs(a.cf[fi * ldc + c]) - 1;
-    if (f < a.Nf) continue;
-    const int b = f - a.Nf;
-    if (a.btype[b] == AFAR_BC_FIXED_INITIAL) continue;  // the ghost keeps its uploaded state
-    const V4<double> g = boundary_value(a.btype[b], V4<double>{(double)wn.x, (double)wn.y, (double)wn.z, (double)wn.w},
-                                        a.bn[b]);
-    reinterpret_cast<V4<float>*>(a.W)[a.Nc + b] = V4<float>{(float)g.x, (float)g.y, (float)g.z, (float)g.w};
+    if (f >= a.Nf) ghost_mixed(a, f - a.Nf, wn, a.W);
   }
 }
 
@@ -1827,8 +2042,7 @@ __device__ __forceinline__ void update_body(const StageArgs<P>& a, const int blk
   const int c = blk * blockDim.x + threadIdx.x;
   if constexpr (P::id == PolicyMixed::id) {
     update_mixed(a, c, k, &s_go, &s_bdt);  // synchronises the block after its flux gather
-    return;
-  }
+  } else {
   __syncthreads();
   if (c >= a.Nc || !s_go) return;
   const double beta1 = k.b1, beta2 = k.b2, beta3 = k.b3;
@@ -1900,18 +2114,484 @@ __device__ __forceinline__ void update_body(const StageArgs<P>& a, const int blk
         boundary_value(a.btype[b], V4<double>{(double)wn.x, (double)wn.y, (double)wn.z, (double)wn.w}, a.bn[b]);
     a.W[a.Nc + b] = V4<WT>{(WT)g.x, (WT)g.y, (WT)g.z, (WT)g.w};
   }
+  }
 }
+
+// Closes a step: advance time, record the step, re-arm the CFL minimum for the next step.
+__device__ __forceinline__ void finish_one(StepCtl* ctl) {
+  const double dt = step_dt(ctl);
+  if (dt > 0.0) {
+    ctl->t += dt;
+    ctl->steps += 1;
+    ctl->last_dt = dt;
+    if (ctl->write_interval > 0.0)  // passed a write time (within rounding): aim at the next one
+      for (int k = 0; k < 4 && ctl->t >= (double)(ctl->write_index + 1) * ctl->write_interval * (1.0 - 1e-12); ++k)
+        ctl->write_index += 1;
+  }
+  ctl->dt_bits = (unsigned long long)__double_as_longlong(1e5);
+}
+// ---------------------------------------------------------------- mixed: the stage after the reconstruct
+// BVD switch, face flux, residual and RK update of a tile of consecutive cells in one kernel.  As three
+// kernels these pass limiters, switches and fluxes through memory and gather the cells' states and
+// gradients at random (504 of the 903 B a cell and stage of the four kernels).  Here the two O3 states of
+// the tile's faces come into shared memory; a cell's thread decides its switch from them and adds its
+// side's TVD state; a face's thread makes the flux; the cell's thread sums its fluxes and advances.  Cells
+// across the tile's border (the tiles are compact patches of the Hilbert order: about 50 for 192
+// triangles) have their switch decided in every tile that needs it and a border face its flux in both its
+// tiles, by the same instructions on the same inputs: the same bits.  The new states go to another buffer
+// than the one read (three in turn, so a step of three stages ends where it began).
+//
+// What bounds it is the chain of waits of a tile, so its loads start at once: the tile's own faces (first
+// cell in the tile: a contiguous range) and conserved states by bulk copies, its own cells' operands into
+// registers, border and boundary faces by the threads.  The stencils' troubled-cell flags are read only
+// where a 128-cell tile that they reach holds one (words of 32 flags, written by the reconstruct).
+// 256 threads: with its halo a tile of 192 triangles or 152 quads is mostly one pass of the block.  Four
+// blocks a SM (64 registers); five spilled and lost 8%.  us a step, separate kernels / fused: 986 quads 54 / 42,
+// 65k quads 66 / 52, 500k triangles 380 / 345, 2.0M triangles 1165 / 1026, 4.0M quads 2460 / 2297
+// (the tail itself 437 us a step at 2.0M triangles: 1.5 TB/s; its blocks wait, on the halo's gathers and at
+// their two barriers).
+constexpr int kTailThreads = 256, kTailBlocks = 4;
+constexpr int kTailHalo = 128, kTailExtra = 192, kTailList = 32;  // most of each that a tile may have
+struct TailTile {
+  int fstart;  // the tile's own faces are fstart .. fstart + nOwn - 1
+  int nOwn;
+  int nFace;  // with the extra ones: faces of earlier tiles' cells, boundary faces
+  int nHalo;  // cells across the border; in the upper half the number of 128-cell tiles in tlist (0xFFFF: too many)
+};
+// Shared memory of a tile of nf faces: O3 and TVD states of both sides, face vectors, Un and U of the
+// cells, the sides' switches, two mbarriers.
+struct TailSmem {
+  unsigned tv, tu, fs, u0, u, sw, bar, bytes;
+};
+__host__ __device__ inline TailSmem tail_smem(const int nf, const int cells) {
+  TailSmem L;
+  L.tv = nf * 32;
+  L.tu = L.tv + nf * 16;
+  L.fs = L.tu + nf * 16;
+  L.u0 = L.fs + nf * 16;
+  L.u = L.u0 + cells * 32;
+  L.sw = L.u + cells * 32;
+  L.bar = L.sw + (nf * 2 + 15) / 16 * 16;
+  L.bytes = L.bar + 16;
+  return L;
+}
+
+// A halo cell's slot: its local face with the neighbour side in bit 15 where the face is one of the tile's,
+// kNoFace, kWall for a boundary face, else 2 f + side of the face, from kElsewhere on.
+constexpr int kNoFace = -1, kWall = -2, kElsewhere = 0x10000;
+
+template <int NF, bool E>
+__device__ __forceinline__ void tail_body(const StageArgs<PolicyMixed>& a, const V4<float>* __restrict__ Win,
+                                          V4<float>* __restrict__ Wout, const int blk, const StageCoef& k,
+                                          unsigned char* sm) {
+  __shared__ int s_go, s_extra[kTailExtra];
+  __shared__ float s_bdt;
+  const int tid = threadIdx.x, ldc = a.ldc;
+  const int T = a.tailT;  // cells a tile
+  const int c0 = blk * T, nc = min(T, a.Nc - c0);
+  const bool own0 = tid < T;  // this thread has an own cell first, else a halo cell
+  // Loads that need no other's result, all issued before the first wait: the tile's header and lists, an
+  // own cell's operands, a halo cell's id and slots.
+  const int4 hdr = reinterpret_cast<const int4*>(a.tail)[blk];
+  const int xid = tid < kTailExtra ? a.textra[(size_t)blk * kTailExtra + tid] : 0;
+  const int reach = tid < kTailList ? a.tlist[(size_t)blk * kTailList + tid] : 0;
+  int c = c0 + (own0 && tid < nc ? tid : 0), nM = 0, nS = 0;
+  int lf[NF];
+  V2<float> d[NF];
+  float wp, wT, Lp, LT;
+  V2<float> gp, gT;
+  // what the switch and the TVD p and T need of a cell; the velocities' part is read where it is used
+  auto load_cell = [&]() {
+    wp = Win[c].x;
+    wT = Win[c].w;
+    gp = reinterpret_cast<const V2<float>*>(a.grad)[4 * (size_t)c];
+    gT = reinterpret_cast<const V2<float>*>(a.grad)[4 * (size_t)c + 3];
+    Lp = a.lim[c].x;
+    LT = a.lim[c].w;
+  };
+  auto load_slots = [&](const int h) {  // of halo cell h
+#pragma unroll
+    for (int fi = 0; fi < NF; ++fi) {
+      lf[fi] = a.thcode[((size_t)blk * 4 + fi) * kTailHalo + h];
+      d[fi] = a.thsg[((size_t)blk * 4 + fi) * kTailHalo + h];
+    }
+  };
+  if (own0) {
+#pragma unroll
+    for (int fi = 0; fi < NF; ++fi) {
+      if (fi >= 3 && a.maxM < 4) continue;  // (a member of triangles in a batch with quads)
+      lf[fi] = a.tlf[(size_t)fi * ldc + c];
+      d[fi] = a.sg[(size_t)fi * ldc + c];  // (rows past a cell's faces hold something)
+    }
+    nM = a.nM[c];
+    nS = a.nS[c];
+    load_cell();
+  } else {
+    c = a.thalo[(size_t)blk * kTailHalo + (tid - T)];
+    load_slots(tid - T);
+  }
+  const int fstart = hdr.x, nOwn = hdr.y, nF = hdr.z, nX = nF - nOwn, nHalo = hdr.w & 0xFFFF, nReach = (int)((unsigned)hdr.w >> 16);
+  const TailSmem S = tail_smem(nF, T);
+  V4<float>* const st = reinterpret_cast<V4<float>*>(sm);          // [2 nF] O3 state of each side; then the flux
+  V2<float>* const tv = reinterpret_cast<V2<float>*>(sm + S.tv);   // [2 nF] TVD p and T
+  V2<float>* const tu = reinterpret_cast<V2<float>*>(sm + S.tu);   // [2 nF] TVD velocity, where the switch asks
+  V4<float>* const sfs = reinterpret_cast<V4<float>*>(sm + S.fs);  // [nF] face vectors
+  const DF4* const su0 = reinterpret_cast<const DF4*>(sm + S.u0);
+  const DF4* const su = reinterpret_cast<const DF4*>(sm + S.u);
+  int8_t* const sw = reinterpret_cast<int8_t*>(sm + S.sw);         // [2 nF] switch of each side's cell
+  unsigned long long* const bar = reinterpret_cast<unsigned long long*>(sm + S.bar);
+  const long long limit = g_tile_wait_limit;
+  if (tid == 0) {
+    mbar_init(bar, 1);
+    mbar_init(bar + 1, 1);
+    mbar_arrive_expect_tx(bar, (unsigned)nOwn * 48u);
+    if (nOwn) {
+      bulk_to_smem(st, a.fv + 2 * (size_t)fstart, (unsigned)nOwn * 32u, bar);
+      bulk_to_smem(sfs, a.fs + fstart, (unsigned)nOwn * 16u, bar);
+    }
+    mbar_arrive_expect_tx(bar + 1, (unsigned)nc * (k.first ? 32u : 64u));
+    bulk_to_smem(sm + S.u0, a.U0 + c0, (unsigned)nc * 32u, bar + 1);
+    if (!k.first) bulk_to_smem(sm + S.u, a.U + c0, (unsigned)nc * 32u, bar + 1);
+  }
+  // the last tile of the last stage to finish closes the step: every tile has read the step control by then
+  auto done = [&]() {
+    if (!k.last || tid != kTailThreads - 1) return;
+    __threadfence();
+    if (atomicAdd(&a.ctl->tiles_done, 1u) == (unsigned)a.nTail - 1u) {
+      a.ctl->tiles_done = 0;
+      finish_one(a.ctl);
+    }
+  };
+  // Loads that needed those: border and boundary faces, the flags of the 128-cell tiles that the stencils
+  // reach, a halo cell's operands, the T values of its faces elsewhere.
+  V4<float> xfs, xl, xr;
+  if (tid < nX) {
+    xfs = a.fs[xid];
+    xl = xid < a.Nf ? a.fv[2 * xid] : Win[a.Nc + (xid - a.Nf)];
+    if (xid < a.Nf) xr = a.fv[2 * xid + 1];
+  }
+  int near = nReach == 0xFFFF;  // does any stencil of the tile reach a troubled cell?
+  if (!near && tid < nReach) {
+    const uint4 w = reinterpret_cast<const uint4*>(a.wflag)[reach];
+    near = (w.x | w.y | w.z | w.w) != 0;
+  }
+  float tCur[NF], tOther[NF];
+  auto load_elsewhere = [&]() {
+#pragma unroll
+    for (int fi = 0; fi < NF; ++fi)
+      if (lf[fi] >= kElsewhere) {
+        tCur[fi] = a.fv[lf[fi] - kElsewhere].w;
+        tOther[fi] = a.fv[(lf[fi] - kElsewhere) ^ 1].w;
+      }
+  };
+  bool live = own0 ? tid < nc : tid - T < nHalo;
+  if (!own0 && live) {
+    load_cell();
+    load_elsewhere();
+  }
+#pragma unroll
+  for (int fi = 0; fi < NF; ++fi)
+    if (!live || (own0 && fi >= nM)) lf[fi] = kNoFace;
+  if (tid < nX) {
+    const int j = nOwn + tid;
+    s_extra[tid] = xid;
+    sfs[j] = xfs;
+    st[2 * j] = xl;
+    if (xid < a.Nf) st[2 * j + 1] = xr;
+  }
+  if (tid == kTailThreads - 1) {  // the block's step, as in update_body
+    const double dt = step_dt(a.ctl);
+    s_go = gt_zero(dt);
+    s_bdt = (float)(k.b3 * dt);
+  }
+  if (tid == 0 && !mbar_wait_bounded(bar, 0, limit)) near = 1;  // one thread polls, the block's barrier tells
+  near = __syncthreads_or(near);
+  int lfs[NF];  // of this thread's own cell: local face of each slot, bit 15: the neighbour side; -1: none
+#pragma unroll
+  for (int fi = 0; fi < NF; ++fi) lfs[fi] = kNoFace;
+  // first the own cells and the halo's first, then the rest of the halo
+  for (int h0 = -T; h0 < nHalo; h0 += kTailThreads) {
+    const int h = h0 + tid;
+    const bool own = h < 0;
+    if (h0 >= 0) {
+      live = h < nHalo;
+      if (live) {
+        c = a.thalo[(size_t)blk * kTailHalo + h];
+        load_slots(h);
+        load_cell();
+        load_elsewhere();
+      } else {
+#pragma unroll
+        for (int fi = 0; fi < NF; ++fi) lf[fi] = kNoFace;
+      }
+    }
+    // the switch (bvd_body)
+    int shockType = 0, shockTypeExt = 0;
+    if (near && live) {
+      if (!own) {
+        nS = a.nS[c];
+        nM = a.nM[c];
+      }
+      shockType = (a.wflag[c >> 5] >> (c & 31)) & 1;
+      shockTypeExt = shockType;
+      for (int q0 = 0; q0 < nS; q0 += 10) {
+        int j[10];
+#pragma unroll
+        for (int u = 0; u < 10; ++u) j[u] = (q0 + u < nS) ? a.sten[(size_t)(q0 + u) * ldc + c] : a.Nc;
+#pragma unroll
+        for (int u = 0; u < 10; ++u) {
+          const int fl = j[u] < a.Nc ? (a.wflag[j[u] >> 5] >> (j[u] & 31)) & 1 : 0;  // ghosts carry no flags
+          if (q0 + u < nM) shockType += fl;
+          shockTypeExt += fl;
+        }
+      }
+    }
+    int bvdType = 0, walls = 0;
+    const float lim = to_bj(LT);
+#pragma unroll
+    for (int fi = 0; fi < NF; ++fi) {
+      if (lf[fi] == kNoFace) continue;
+      const int l = lf[fi] & 0x7FFF;
+      if (own && l >= nOwn && s_extra[l - nOwn] >= a.Nf) lf[fi] |= 0x40000;  // a boundary face of its own
+      if (lf[fi] == kWall || (own && lf[fi] >= 0x40000)) {
+        walls += 1;
+        if (walls >= 2) bvdType = 1;  // corner cell: low order
+        continue;
+      }
+      if (lf[fi] < kElsewhere) {
+        const int side = (lf[fi] >> 15) & 1;
+        tCur[fi] = st[2 * l + side].w;
+        tOther[fi] = st[2 * l + (side ^ 1)].w;
+      }
+      const float tfTVD = tvd_mixed(wT, lim, gT.x, gT.y, d[fi]);
+      const int typeval = fab(ad_(tfTVD, -tOther[fi])) < ml_(0.5f, fab(ad_(tCur[fi], -tOther[fi])));
+      const int notFlat = fab(ad_(tCur[fi], -tOther[fi])) > 1e-10f;
+      const int limited = (lim < 0.9f) + (shockTypeExt > 0);
+      bvdType = max(bvdType, notFlat * limited * typeval);
+    }
+    const int type = (shockType > 0) * (shockTypeExt > 1) * (-2) + (bvdType > 0);
+    if (own && live) a.si[2 * c + 1] = (int8_t)type;
+    Lp = type < 0 ? to_venkat(Lp) : to_bj(Lp);
+    LT = type < 0 ? to_venkat(LT) : to_bj(LT);
+    V2<float> wu, gx, gy, Lu;  // Ux, Uy: state, gradients (d/dx, d/dy of each), limiters
+    if (type != 0 && live) {
+      wu = V2<float>{Win[c].y, Win[c].z};
+      const V4<float> g0 = a.grad[2 * c], g1 = a.grad[2 * c + 1];
+      gx = V2<float>{g0.z, g0.w};
+      gy = V2<float>{g1.x, g1.y};
+      const V4<float> L = a.lim[c];
+      Lu = type < 0 ? V2<float>{to_venkat(L.y), to_venkat(L.z)} : V2<float>{to_bj(L.y), to_bj(L.z)};
+    }
+    // the TVD states of its faces
+#pragma unroll
+    for (int fi = 0; fi < NF; ++fi) {
+      if (lf[fi] >= 0 && lf[fi] < kElsewhere) {
+        const int at = 2 * (lf[fi] & 0x7FFF) + ((lf[fi] >> 15) & 1);
+        tv[at] = V2<float>{tvd_mixed(wp, Lp, gp.x, gp.y, d[fi]), tvd_mixed(wT, LT, gT.x, gT.y, d[fi])};
+        if (type != 0)
+          tu[at] = V2<float>{tvd_mixed(wu.x, Lu.x, gx.x, gy.x, d[fi]), tvd_mixed(wu.y, Lu.y, gx.y, gy.y, d[fi])};
+        sw[at] = (int8_t)type;
+      }
+    }
+    if (own) {
+#pragma unroll
+      for (int fi = 0; fi < NF; ++fi) lfs[fi] = lf[fi];
+    }
+  }
+  bool ok = true;
+  if (tid == 0) ok = mbar_wait_bounded(bar, 0, 1) && mbar_wait_bounded(bar + 1, 0, limit);
+  if (!__syncthreads_and(ok)) {  // a bulk copy did not arrive: wait (bounded) once more for both, leave
+    if (tid == 0) atomicOr(&a.ctl->err, 1u);
+    mbar_wait_bounded(bar, 0, limit);
+    mbar_wait_bounded(bar + 1, 0, limit);
+    return done();
+  }
+  // the faces' fluxes, each in the place of its first side's state
+  for (int j = tid; j < nF; j += kTailThreads) {
+    const V4<float> fs = sfs[j];
+    V4<float> sl = st[2 * j], F;
+    if (j < nOwn || s_extra[j - nOwn] < a.Nf) {
+      V4<float> sr = st[2 * j + 1];
+      const V4<float> t = reinterpret_cast<const V4<float>*>(tv)[j];  // both sides' p and T
+      const char2 w = reinterpret_cast<const char2*>(sw)[j];
+      if (w.x) sl = V4<float>{t.x, tu[2 * j].x, tu[2 * j].y, t.y};
+      if (w.y) sr = V4<float>{t.z, tu[2 * j + 1].x, tu[2 * j + 1].y, t.w};
+      const MixedSide l{sl.x, sl.y, sl.z, sl.w, t.x, t.y}, r{sr.x, sr.y, sr.z, sr.w, t.z, t.w};
+      F = mixed_flux<E>(l, r, (signed char)w.x < 0 || (signed char)w.y < 0, fs, a.Rf, a.Cvf, a.invRf, a.gm1f + 1.f);
+    } else {
+      F = mixed_boundary_flux(sl, fs, a.Rf, a.Cvf);
+    }
+    st[2 * j] = F;
+  }
+  __syncthreads();
+  if (tid < nc) {
+    const int c = c0 + tid;
+    if (s_go) {
+      float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int fi = 0; fi < NF; ++fi) {
+        if (lfs[fi] >= 0) {
+          const V4<float> F = st[2 * (lfs[fi] & 0x7FFF)];
+          const float sgn = (lfs[fi] & 0x8000) ? -1.f : 1.f;
+          const float x[4] = {sgn * F.x, sgn * F.y, sgn * F.z, sgn * F.w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            if (fi == 0) {  // (every cell has a first face)
+              hi[q] = x[q];
+            } else {
+              const DF t = df_two_sum(hi[q], x[q]);
+              hi[q] = t.hi;
+              lo[q] = __fadd_rn(lo[q], t.lo);
+            }
+          }
+        }
+      }
+      const V4<float> wn = advance_mixed(a, c, k, s_bdt, hi, lo, su0 + tid, su + tid);
+      Wout[c] = wn;
+#pragma unroll
+      for (int fi = 0; fi < NF; ++fi)
+        if (lfs[fi] >= 0x40000) ghost_mixed(a, s_extra[(lfs[fi] & 0x7FFF) - nOwn] - a.Nf, wn, Wout);
+    } else {  // past t_end: the step is a no-op, the state moves on to the next buffer
+      Wout[c] = Win[c];
+#pragma unroll
+      for (int fi = 0; fi < NF; ++fi) {
+        if (lfs[fi] < 0x40000) continue;
+        const int g = a.Nc + s_extra[(lfs[fi] & 0x7FFF) - nOwn] - a.Nf;
+        Wout[g] = Win[g];
+      }
+    }
+  }
+  done();
+}
+
+// ---- the tiles' lists (set-up; one block of 128 threads a tile)
+constexpr int kTailHash = 512;  // halo cells of a tile in shared memory: open addressing
+__device__ __forceinline__ int tail_hash_find(int* key, const int c, const bool insert) {
+  for (int i = 0; i < kTailHash; ++i) {
+    const int at = (int)(((unsigned)c * 2654435761u >> 7) + i) & (kTailHash - 1);
+    const int was = insert ? atomicCAS(&key[at], -1, c) : key[at];
+    if (was == c || (insert && was == -1)) return at;
+    if (was == -1) return -1;
+  }
+  return -1;
+}
+// limits[0]: the most faces of a tile; limits[1]: set when a tile has more cells or faces than it may
+__global__ void __launch_bounds__(128) k_tail_tiles(StageArgs<PolicyMixed> a, const int* start, TailTile* tiles,
+                                                    int* halo, int* hcode, V2<float>* hsg, int* extra, uint16_t* lfo,
+                                                    int* limits) {
+  __shared__ int key[kTailHash], idx[kTailHash], nH, nX, bad;
+  const int blk = blockIdx.x, tid = threadIdx.x, ldc = a.ldc;
+  const int c0 = blk * a.tailT, c1 = min(c0 + a.tailT, a.Nc);
+  const int f0 = start[c0], f1 = c1 < a.Nc ? start[c1] : a.Nf, nOwn = f1 - f0;
+  for (int i = tid; i < kTailHash; i += 128) key[i] = -1;
+  if (tid == 0) nH = nX = bad = 0;
+  __syncthreads();
+  for (int c = c0 + tid; c < c1; c += 128)
+    for (int fi = 0; fi < a.nM[c]; ++fi) {
+      const int fid = a.cf[(size_t)fi * ldc + c], f = abs(fid) - 1;
+      int l = f - f0;
+      if (f >= a.Nf || f < f0 || f >= f1) {
+        const int x = atomicAdd(&nX, 1);
+        if (x < kTailExtra)
+          extra[(size_t)blk * kTailExtra + x] = f;
+        else
+          bad = 1;
+        l = nOwn + x;
+      }
+      lfo[(size_t)fi * ldc + c] = (uint16_t)(min(l, 0x7FFE) | (fid < 0 ? 0x8000 : 0));
+      if (f < a.Nf) {
+        const int o = fid > 0 ? a.on[f].y : a.on[f].x;
+        if ((o < c0 || o >= c1) && tail_hash_find(key, o, true) < 0) bad = 1;
+      }
+    }
+  __syncthreads();
+  for (int i = tid; i < kTailHash; i += 128)
+    if (key[i] >= 0) {
+      idx[i] = atomicAdd(&nH, 1);
+      if (idx[i] < kTailHalo) halo[(size_t)blk * kTailHalo + idx[i]] = key[i];
+    }
+  __syncthreads();
+  if (nH <= kTailHalo && nX <= kTailExtra && !bad) {
+    for (int i = tid; i < 4 * nH; i += 128) {  // the halo's slots as faces elsewhere
+      const int h = i >> 2, q = i & 3, o = halo[(size_t)blk * kTailHalo + h];
+      const size_t at = ((size_t)blk * 4 + q) * kTailHalo + h;
+      int code = kNoFace;
+      if (q < a.nM[o]) {
+        const int fid = a.cf[(size_t)q * ldc + o], f = abs(fid) - 1;
+        code = f < a.Nf ? kElsewhere + 2 * f + (fid < 0) : kWall;
+        hsg[at] = a.sg[(size_t)q * ldc + o];
+      }
+      hcode[at] = code;
+    }
+    __syncthreads();  // (the condition is the block's)
+    for (int c = c0 + tid; c < c1; c += 128)  // those that are the tile's
+      for (int fi = 0; fi < a.nM[c]; ++fi) {
+        const int fid = a.cf[(size_t)fi * ldc + c], f = abs(fid) - 1;
+        if (f >= a.Nf) continue;
+        const int o = fid > 0 ? a.on[f].y : a.on[f].x;
+        if (o >= c0 && o < c1) continue;
+        const int h = idx[tail_hash_find(key, o, false)];
+        for (int q = 0; q < a.nM[o]; ++q)
+          if (a.cf[(size_t)q * ldc + o] == -fid)
+            hcode[((size_t)blk * 4 + q) * kTailHalo + h] =
+                (lfo[(size_t)fi * ldc + c] & 0x7FFF) | (fid > 0 ? 0x8000 : 0);
+      }
+  }
+  if (tid == 0) {
+    if (nH > kTailHalo || nX > kTailExtra || bad || nOwn + nX > 0x7FF0) atomicExch(limits + 1, 1);
+    atomicMax(limits, nOwn + nX);
+    tiles[blk] = TailTile{f0, nOwn, nOwn + min(nX, kTailExtra), min(nH, kTailHalo)};
+  }
+}
+// The 128-cell tiles that the stencils of a tile's cells and halo reach.
+__global__ void __launch_bounds__(128) k_tail_lists(StageArgs<PolicyMixed> a, TailTile* tiles, const int* halo,
+                                                    int* list) {
+  __shared__ int set[128], n, many;
+  const int blk = blockIdx.x, tid = threadIdx.x;
+  const int c0 = blk * a.tailT, nc = min(a.tailT, a.Nc - c0), nLoc = nc + tiles[blk].nHalo;
+  set[tid] = -1;
+  if (tid == 0) n = many = 0;
+  __syncthreads();
+  for (int i = tid; i < nLoc; i += 128) {
+    const int c = i < nc ? c0 + i : halo[(size_t)blk * kTailHalo + (i - nc)];
+    for (int q = -1; q < a.nS[c]; ++q) {  // the cell itself and its stencil
+      const int j = q < 0 ? c : a.sten[(size_t)q * a.ldc + c];
+      if (j >= a.Nc) continue;  // ghosts carry no flags
+      const int t = j >> 7;
+      int p = 0;
+      for (; p < 128; ++p) {
+        const int at = (t + p) & 127;
+        const int was = atomicCAS(&set[at], -1, t);
+        if (was == -1 || was == t) break;
+      }
+      if (p == 128) many = 1;
+    }
+  }
+  __syncthreads();
+  if (set[tid] >= 0) {
+    const int at = atomicAdd(&n, 1);
+    if (at < kTailList) list[(size_t)blk * kTailList + at] = set[tid];
+  }
+  __syncthreads();
+  if (tid == 0) tiles[blk].nHalo |= (n > kTailList || many ? 0xFFFF : n) << 16;
+}
+
 
 // ------------------------------------------------------------------------- single-solve kernels
 // One solve per launch, arguments by value (read from the parameter bank).
-template <class P>
+template <class P, bool DT>
 __global__ void __launch_bounds__(128, 5) k_reconstruct_reg(StageArgs<P> a) {
-  recon_reg_body<P>(a, blockIdx.x);
+  recon_reg_body<P, DT>(a, a.W, blockIdx.x);
 }
-template <class P, int NF>
+template <class P, int NF, bool DT>
 __global__ void __launch_bounds__(kTile, 4) k_reconstruct_tile(StageArgs<P> a) {
   extern __shared__ __align__(128) unsigned char sm[];
-  recon_tile_body<P, NF>(a, blockIdx.x, sm);
+  recon_tile_body<P, NF, DT>(a, a.W, blockIdx.x, sm);
+}
+template <int NF>
+__global__ void __launch_bounds__(kTailThreads, kTailBlocks) k_tail(StageArgs<PolicyMixed> a, V4<float>* Wout, const StageCoef k) {
+  extern __shared__ __align__(128) unsigned char sm[];
+  tail_body<NF, false>(a, a.W, Wout, blockIdx.x, k, sm);
 }
 template <class P>
 __global__ void __launch_bounds__(128) k_reconstruct_staged(StageArgs<P> a) {
@@ -2210,19 +2890,61 @@ __global__ void __launch_bounds__(kTile, 4) kb_reconstruct_tile(const StageArgs<
                                                                 const int2* __restrict__ map) {
   extern __shared__ __align__(128) unsigned char sm[];
   const int2 m = map[blockIdx.x];
-  recon_tile_body<P, NF>(member_args(tab, m.x), m.y, sm);
+  const StageArgs<P>& a = member_args(tab, m.x);
+  recon_tile_body<P, NF, false>(a, a.W, m.y, sm);
+}
+// The two kernels of the fused stage over up to kMembers solves, whose arguments are the launch's own
+// parameters: the block finds its member from its index alone, so every pointer and constant of the
+// body is an operand in the parameter bank, as in the single solve.  With the arguments staged in
+// shared memory (member_args) the body keeps them in registers: the tail spilled 132 bytes a thread
+// (64 registers) and took 260 us a stage at 2.0M quads, and the whole step was no faster than the separate
+// kernels.  us a step, separate kernels (64-cell BVD blocks, 128-face flux blocks) / shared memory /
+// parameters: 10 members of 160k quads 1110 / 1105 / 974, 8 of 90k 572 / 550 / 488, 4 of 40k
+// 146 / 154 / 136, 4 of 4k 63 / 52 / 48; 12 members of 121k triangles 963 / 863 / 760, 4 of 6k 64 / 49 / 47.
+template <class P>
+struct MemberTable {
+  static constexpr int kMembers = 48;  // what fits the 32 KB of a launch's parameters
+  int n;                      // members
+  int first[kMembers + 1];    // member i has blocks [first[i], first[i + 1]) of the launch
+  StageArgs<P> m[kMembers];
+};
+template <class P>
+__device__ __forceinline__ int member_of(const MemberTable<P>& t) {
+  int lo = 0, hi = t.n;  // first[lo] <= block < first[hi]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if ((int)blockIdx.x >= t.first[mid]) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+static_assert(sizeof(MemberTable<PolicyMixed>) + sizeof(StageCoef) + 16 <= 32764, "a launch's parameters");
+template <int NF, bool DT>
+__global__ void __launch_bounds__(kTile, 4)
+    kp_reconstruct_tile(const __grid_constant__ MemberTable<PolicyMixed> t, const int buf) {
+  extern __shared__ __align__(128) unsigned char sm[];
+  const int i = member_of(t);
+  recon_tile_body<PolicyMixed, NF, DT>(t.m[i], t.m[i].W3[buf], blockIdx.x - t.first[i], sm);
+}
+template <int NF, bool FIRST>
+__global__ void __launch_bounds__(kTailThreads, kTailBlocks)
+    kp_tail(const __grid_constant__ MemberTable<PolicyMixed> t, const int buf, const StageCoef k) {
+  extern __shared__ __align__(128) unsigned char sm[];
+  const int i = member_of(t);
+  tail_body<NF, FIRST>(t.m[i], t.m[i].W3[buf], t.m[i].W3[buf == 2 ? 0 : buf + 1], blockIdx.x - t.first[i], k, sm);
 }
 __global__ void __launch_bounds__(128, 4) kb_reconstruct_fp64(const StageArgs<PolicyFP64>* __restrict__ tab,
                                                               const int2* __restrict__ map) {
   const int2 m = map[blockIdx.x];
   recon_fp64_body(member_args(tab, m.x), m.y);
 }
-// the register-pass reconstruct of the mixed policy over the members the autotuner gave it
+// the register-pass reconstruct of the mixed policy over the members that ask for it
 template <class P>
 __global__ void __launch_bounds__(128, 5) kb_reconstruct_reg(const StageArgs<P>* __restrict__ tab,
                                                             const int2* __restrict__ map) {
   const int2 m = map[blockIdx.x];
-  recon_reg_body<P>(member_args(tab, m.x), m.y);
+  const StageArgs<P>& a = member_args(tab, m.x);
+  recon_reg_body<P, false>(a, a.W, m.y);
 }
 // BVD and flux in blocks of B threads (the batch autotuner's choice; the map's blocks are B cells
 // or faces of one member).  mixed BVD: 32 registers, the full 64 warps per SM; fp64: 40 warps.
@@ -2235,7 +2957,7 @@ __global__ void __launch_bounds__(B, (P::id == PolicyMixed::id ? 2048 : 1280) / 
 template <class P, bool DT, int B>
 __global__ void __launch_bounds__(B) kb_flux(const StageArgs<P>* __restrict__ tab, const int2* __restrict__ map) {
   const int2 m = map[blockIdx.x];
-  flux_body<P, DT>(member_args(tab, m.x), m.y);
+  flux_body<P, DT, true>(member_args(tab, m.x), m.y);
 }
 template <class P>
 __global__ void __launch_bounds__(128) kb_update(const StageArgs<P>* __restrict__ tab, const int2* __restrict__ map,
@@ -2244,19 +2966,6 @@ __global__ void __launch_bounds__(128) kb_update(const StageArgs<P>* __restrict_
   update_body<P>(member_args(tab, m.x), m.y, k);
 }
 
-// Closes a step: advance time, record the step, re-arm the CFL minimum for the next step.
-__device__ __forceinline__ void finish_one(StepCtl* ctl) {
-  const double dt = step_dt(ctl);
-  if (dt > 0.0) {
-    ctl->t += dt;
-    ctl->steps += 1;
-    ctl->last_dt = dt;
-    if (ctl->write_interval > 0.0)  // passed a write time (within rounding): aim at the next one
-      for (int k = 0; k < 4 && ctl->t >= (double)(ctl->write_index + 1) * ctl->write_interval * (1.0 - 1e-12); ++k)
-        ctl->write_index += 1;
-  }
-  ctl->dt_bits = (unsigned long long)__double_as_longlong(1e5);
-}
 template <class P>
 __global__ void kb_finish_step(const StageArgs<P>* __restrict__ tab, const int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

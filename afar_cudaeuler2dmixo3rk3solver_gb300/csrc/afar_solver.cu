@@ -10,6 +10,7 @@
 #include <cstring>
 #include <algorithm>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <system_error>
 #include <thread>
@@ -150,6 +151,7 @@ __global__ void k_init_ctl(StepCtl* ctl) {
     ctl->err = 0;
     ctl->write_interval = 0.0;
     ctl->write_index = 0;
+    ctl->tiles_done = 0;
   }
 }
 
@@ -193,11 +195,15 @@ __global__ void k_convert2(int n, const V2<A>* in, V2<B>* out) {
 }
 
 // the primitive state (cells, then ghosts) into the device's cell order and out of it
-__global__ void k_state_in(int Nc, int n, const V4<double>* in, V4<float>* out, DeviceOrder o) {
+// (the ghosts also into the state's other buffers: those of label 6 are never written again)
+__global__ void k_state_in(int Nc, int n, const V4<double>* in, V4<float>* out, V4<float>* b, V4<float>* c,
+                           DeviceOrder o) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const V4<double> v = in[i < Nc ? o.cell(i) : i];
-  out[i] = V4<float>{(float)v.x, (float)v.y, (float)v.z, (float)v.w};
+  const V4<float> w{(float)v.x, (float)v.y, (float)v.z, (float)v.w};
+  out[i] = w;
+  if (i >= Nc) b[i] = c[i] = w;
 }
 __global__ void k_state_out(int Nc, int n, const V4<float>* in, V4<double>* out, DeviceOrder o) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -254,11 +260,25 @@ struct afar_solver {
   // head_pending: the head ran on the current state and nothing has touched the solver since.
   cudaGraphExec_t graph_head = nullptr, graph_tail = nullptr;
   bool head_pending = false;
+  // The fused stage leaves the limiter untransformed, and its head the switch types of the step
+  // before: the state buffer of the last stage whose BVD the accessors still have to run (-1: none).
+  int bvd_pending = -1;
   float tune_ms[2] = {0.f, 0.f};  // the autotuner's measured launch times (0: decision from the cache)
   void* xfer = nullptr;    // mixed: staging for double <-> device-format copies, 32 B x (Nc + Nb)
   // The mixed policy keeps its cells along a Hilbert curve, its internal faces by their first cell in
   // that order (see setup_cell_order); everything that crosses the boundary is in the caller's order.
   DeviceOrder order;
+  // The fused stage tail (tail_body) of the mixed policy: its tiles, the state's other two buffers, and
+  // whether the mesh has it (`tail_faces` the most faces of a tile).
+  TailTile* tail = nullptr;
+  int *thalo = nullptr, *textra = nullptr, *tlist = nullptr;
+  int* thcode = nullptr;
+  V2<float>* thsg = nullptr;
+  uint16_t* tlf = nullptr;
+  unsigned* wflag = nullptr;
+  void* Wb[2] = {nullptr, nullptr};
+  bool fused = false;
+  int tail_faces = 0;
   int2* on = nullptr;
   uint8_t* btype = nullptr;
   uint8_t* nS = nullptr;
@@ -357,6 +377,12 @@ void reorder(afar_solver* s, T* a, size_t n) {
   k_gather<<<grid_for((long long)n, 256), 256, 0, s->stream>>>((int)n, s->order.perm, static_cast<const T*>(s->xfer), a);
 }
 
+// Cells of a tile of the fused stage tail: as many as its 256 threads take with the halo in one pass (192
+// triangles, 152 quads), fewer quads where the mesh has no block for every SM and a block's time is the
+// kernel's.  us a step at 96 / 152 / 192 cells: triangles 1.1k 41 / 43 / 41, 99k 72 / 73 / 68, 998k 588 / 512 / 497;
+// quads 1.0k 42 / 45 / 58, 10k 46.5 / 47.2 / 61, 66k 70 / 62 / 72, 1.0M 670 / 584 / 631.
+int tail_cells(const afar_solver* s) { return s->maxM <= 3 ? 192 : s->Nc <= 152 * 96 ? 96 : 152; }
+
 template <class P>
 StageArgs<P> make_args(afar_solver* s) {
   StageArgs<P> a;
@@ -413,6 +439,18 @@ StageArgs<P> make_args(afar_solver* s) {
   a.dtgf = s->dtgf;
   a.px = s->px;
   a.py = s->py;
+  a.tail = s->tail;
+  a.thalo = s->thalo;
+  a.thcode = s->thcode;
+  a.thsg = reinterpret_cast<const V2<G>*>(s->thsg);
+  a.textra = s->textra;
+  a.tlf = s->tlf;
+  a.tlist = s->tlist;
+  a.wflag = s->wflag;
+  a.W3[0] = a.W;
+  for (int i = 0; i < 2; ++i) a.W3[i + 1] = static_cast<V4<typename P::W>*>(s->Wb[i]);
+  a.tailT = tail_cells(s);
+  a.nTail = (s->Nc + a.tailT - 1) / a.tailT;
   a.ng = s->ng;
   a.wg = static_cast<const S*>(s->wg);
   a.sgk = static_cast<const V2<G>*>(s->sgk);
@@ -460,6 +498,9 @@ size_t recon_smem(const afar_solver* s, int block = kCellBlock) {
   return (size_t)(rows > 0 ? rows : 1) * block * sizeof(V4<typename P::S>);
 }
 
+// mixed: the step runs as the fused stage (see enqueue_step)
+inline bool fused_step(const afar_solver* s) { return s->fused && s->ng == 0; }
+
 // One solve's stage launches, arguments by value.  The ref policy reconstructs in the staged
 // kernel and runs the reference-layout flux; fp64 reconstructs staged, mixed in registers.
 template <class P>
@@ -469,18 +510,34 @@ struct Stage {
   int bc() const { return block_for<P>(s->Nc, kCellBlock); }
   int gc() const { return grid_for(s->Nc, bc()); }
 
-  void reconstruct() const {
+  // dt (mixed): also reduce the Courant step
+  void reconstruct(bool dt = false) const {
     if constexpr (P::id == PolicyMixed::id) {
+      const auto tile = s->maxM <= 3 ? (dt ? k_reconstruct_tile<P, 3, true> : k_reconstruct_tile<P, 3, false>)
+                                     : (dt ? k_reconstruct_tile<P, 4, true> : k_reconstruct_tile<P, 4, false>);
+      const auto reg = dt ? k_reconstruct_reg<P, true> : k_reconstruct_reg<P, false>;
       if (s->recon_variant == 1)
-        k_reconstruct_reg<P><<<gc(), kCellBlock, 0, s->stream>>>(a);
-      else if (s->maxM <= 3)
-        k_reconstruct_tile<P, 3><<<gc(), kTile, recon_smem<P>(s), s->stream>>>(a);
+        reg<<<gc(), kCellBlock, 0, s->stream>>>(a);
       else
-        k_reconstruct_tile<P, 4><<<gc(), kTile, recon_smem<P>(s), s->stream>>>(a);
+        tile<<<gc(), kTile, recon_smem<P>(s), s->stream>>>(a);
     } else
       k_reconstruct_staged<P><<<gc(), bc(), recon_smem<P>(s, bc()), s->stream>>>(a);
     if constexpr (P::id != PolicyRef::id) {
       if (s->ng > 0) k_reconstruct_gauss<P><<<gc(), bc(), 0, s->stream>>>(a);
+    }
+  }
+  // mixed: everything after the reconstruct in one kernel where the mesh has its tiles
+  bool fused() const { return P::id == PolicyMixed::id && fused_step(s); }
+  // the reconstruct and the rest of stage k with the state in the k-th buffer
+  Stage<P> at(int k) const {
+    Stage<P> r = *this;
+    r.a.W = a.W3[k];
+    return r;
+  }
+  void tail(int k) const {
+    if constexpr (P::id == PolicyMixed::id) {
+      const auto f = s->maxM <= 3 ? k_tail<3> : k_tail<4>;
+      f<<<a.nTail, kTailThreads, tail_smem(s->tail_faces, tail_cells(s)).bytes, s->stream>>>(a, a.W3[(k + 1) % 3], stage_coef(k));
     }
   }
   void bvd() const { k_bvd<P><<<gc(), bc(), 0, s->stream>>>(a); }
@@ -518,15 +575,25 @@ afar_status make_stage(afar_solver* s, bool debug, Stage<P>* out) {
   return AFAR_OK;
 }
 
-// A step is its head (stage 1 up to the flux, which also reduces the Courant step) and its tail.
+// A step is its head (stage 1 as far as the Courant step) and its tail.  Fused (mixed): two kernels a
+// stage, the head the first reconstruct.
 template <class P>
 void enqueue_head(const Stage<P>& st) {
-  st.reconstruct();
+  st.reconstruct(st.fused());
+  if (st.fused()) return;
   st.bvd();
   st.flux(true);
 }
 template <class P>
 void enqueue_tail(const Stage<P>& st) {
+  if (st.fused()) {
+    st.tail(0);
+    for (int k = 1; k < 3; ++k) {
+      st.at(k).reconstruct();
+      st.at(k).tail(k);
+    }
+    return;
+  }
   st.update(0);
   for (int k = 1; k < 3; ++k) {
     st.reconstruct();
@@ -536,6 +603,21 @@ void enqueue_tail(const Stage<P>& st) {
   }
   k_finish_step<<<1, 32, 0, st.s->stream>>>(st.s->ctl);
 }
+
+// What the separate BVD kernel leaves behind, after a fused stage: for the accessors of the limiter and
+// of the switch types.  A pending head no longer fits its tail then (the tail transforms the limiter).
+afar_status settle_bvd(afar_solver* s) {
+  if (s->bvd_pending < 0) return AFAR_OK;
+  Stage<PolicyMixed> st;
+  if (afar_status r = make_stage<PolicyMixed>(s, false, &st)) return r;
+  st.at(s->bvd_pending).bvd();
+  s->bvd_pending = -1;
+  s->head_pending = false;
+  AFAR_CUDA(cudaGetLastError());
+  AFAR_CUDA(cudaStreamSynchronize(s->stream));
+  return AFAR_OK;
+}
+
 template <class P>
 void enqueue_step(const Stage<P>& st) {
   enqueue_head(st);
@@ -587,8 +669,10 @@ afar_status setup_operators(afar_solver* s, const afar_fieldPointer* h, void* sc
       set_error("stencil too large for the reconstruct tile: %zu bytes of shared memory", recon_smem<P>(s));
       return AFAR_ERR_LIMIT;
     }
-    if ((st = raise_smem_limit(k_reconstruct_tile<P, 3>, s->device, recon_smem<P>(s)))) return st;
-    return raise_smem_limit(k_reconstruct_tile<P, 4>, s->device, recon_smem<P>(s));
+    if ((st = raise_smem_limit(k_reconstruct_tile<P, 3, false>, s->device, recon_smem<P>(s)))) return st;
+    if ((st = raise_smem_limit(k_reconstruct_tile<P, 3, true>, s->device, recon_smem<P>(s)))) return st;
+    if ((st = raise_smem_limit(k_reconstruct_tile<P, 4, false>, s->device, recon_smem<P>(s)))) return st;
+    return raise_smem_limit(k_reconstruct_tile<P, 4, true>, s->device, recon_smem<P>(s));
   }
 }
 
@@ -715,7 +799,9 @@ static afar_status put_state(afar_solver* s, const afar_basicFieldData* FD, cons
       AFAR_CUDA(cudaMemcpyAsync(s->xfer, FD, sizeof(V4<double>) * (Nc + Nb), cudaMemcpyHostToDevice, s->stream));
       k_state_in<<<grid_for(Nc + Nb, 256), 256, 0, s->stream>>>((int)Nc, (int)(Nc + Nb),
                                                                 static_cast<const V4<double>*>(s->xfer),
-                                                                static_cast<V4<float>*>(s->W), s->order);
+                                                                static_cast<V4<float>*>(s->W),
+                                                                static_cast<V4<float>*>(s->Wb[0]),
+                                                                static_cast<V4<float>*>(s->Wb[1]), s->order);
     } else {
       AFAR_CUDA(cudaMemcpyAsync(s->W, FD, sizeof(V4<double>) * (Nc + Nb), cudaMemcpyHostToDevice, s->stream));
     }
@@ -763,6 +849,9 @@ static afar_status get_state(afar_solver* s, afar_basicFieldData* FD, afar_conse
     }
   }
   if (si) {
+    if (s->bvd_pending == 0) {  // a fused head: its stage's types
+      if (afar_status st = settle_bvd(s)) return st;
+    }
     const int8_t* from = s->si;
     if (mixed) {
       if (cFD) AFAR_CUDA(cudaStreamSynchronize(s->stream));  // xfer is reused
@@ -944,6 +1033,8 @@ extern "C" afar_status afar_setDeviceFieldData(afar_solver* s, const afar_fieldP
            if ((st = dalloc(s, &s->xfer, std::max(sizeof(V4<double>) * (Nc + Nb), order_scratch(cellsNum))))) return st;
            if ((st = dalloc_t(s, &perm, Nc))) return st;
            if ((st = dalloc_t(s, &inv, Nc))) return st;
+           for (void*& w : s->Wb)
+             if ((st = dalloc(s, &w, sizeof(V4<float>) * (Nc + Nb)))) return st;
          }
          if ((st = dalloc_t(s, &s->U, Nc))) return st;
          if ((st = dalloc_t(s, &s->U0, Nc))) return st;
@@ -1048,6 +1139,7 @@ extern "C" afar_status afar_setDeviceFieldDataStencil(afar_solver* s, const afar
       set_error("cell %d: stencil sizes %d/%d exceed the declared maxima", c, h->stencilSize[c], h->compactStencilSize[c]);
       return AFAR_ERR_ARGUMENT;
     }
+    int across[kMaxFaces] = {-1, -1, -1, -1};  // the cell across each internal face: the slot's stencil member
     for (int i = 0; i < h->compactStencilSize[c]; ++i) {
       const int fid = h->cellFaces[(size_t)maxCompactStencilSize * c + i];
       const int f = (fid < 0 ? -fid : fid) - 1;
@@ -1060,6 +1152,7 @@ extern "C" afar_status afar_setDeviceFieldDataStencil(afar_solver* s, const afar
         if (h->neighbour[2 * (size_t)f + (fid < 0)] != c) *paired = false;
         for (int k = 0; k < i; ++k)
           if (h->cellFaces[(size_t)maxCompactStencilSize * c + k] == fid) *paired = false;
+        across[i] = h->neighbour[2 * (size_t)f + (fid > 0)];
       }
     }
     const int blk = c / AFAR_BLOCKDIM;
@@ -1075,10 +1168,11 @@ extern "C" afar_status afar_setDeviceFieldDataStencil(afar_solver* s, const afar
         set_error("cell %d: stencil member %d out of range", c, g);
         return AFAR_ERR_ARGUMENT;
       }
+      if (i < kMaxFaces && across[i] >= 0 && across[i] != g) *paired = false;
     }
     return AFAR_OK;
   };
-  bool paired = true;  // every internal face is in the lists of both its cells, with the right sign
+  bool paired = true;  // every internal face is in the lists of both its cells, with the right sign and stencil member
   {
     std::mutex mu;
     int bad = Nc;
@@ -1121,6 +1215,7 @@ extern "C" afar_status afar_setDeviceFieldDataStencil(afar_solver* s, const afar
   const size_t ldc = s->ldc;
   const size_t wS = s->policy == AFAR_POLICY_FP64 ? 8 : 4, wG = s->policy == AFAR_POLICY_MIXED ? 4 : 8;
   const int ntile = (Nc + kTile - 1) / kTile;
+  const size_t ntail = grid_for(Nc, tail_cells(s));
   int *fperm = nullptr, *finv = nullptr;
   afar_status st;
   if ((st = alloc_all(s, [&]() -> afar_status {
@@ -1144,6 +1239,14 @@ extern "C" afar_status afar_setDeviceFieldDataStencil(afar_solver* s, const afar
            if ((st = dalloc_t(s, &s->tmaps, 1))) return st;
            if ((st = dalloc_t(s, &fperm, (size_t)Nf))) return st;
            if ((st = dalloc_t(s, &finv, (size_t)Nf))) return st;
+           if ((st = dalloc_t(s, &s->tail, ntail))) return st;
+           if ((st = dalloc_t(s, &s->thalo, ntail * kTailHalo))) return st;
+           if ((st = dalloc_t(s, &s->thcode, ntail * 4 * kTailHalo))) return st;
+           if ((st = dalloc_t(s, &s->thsg, ntail * 4 * kTailHalo))) return st;
+           if ((st = dalloc_t(s, &s->textra, ntail * kTailExtra))) return st;
+           if ((st = dalloc_t(s, &s->tlf, (size_t)s->maxM * ldc))) return st;
+           if ((st = dalloc_t(s, &s->tlist, ntail * kTailList))) return st;
+           if ((st = dalloc_t(s, &s->wflag, (size_t)ntile * 4))) return st;
          }
          return AFAR_OK;
        })))
@@ -1154,6 +1257,7 @@ extern "C" afar_status afar_setDeviceFieldDataStencil(afar_solver* s, const afar
   const size_t n_dls = (sizeof(uint16_t) * (size_t)s->maxS * Nc + 15) / 16 * 16, n_dext = (sizeof(int) * next + 15) / 16 * 16;
   const size_t nrbf = 2 * (size_t)(s->maxS + 1) * Nf;
   const size_t n_lists = n_dls + n_dext + (sizeof(int) * (size_t)s->maxM * Nc + 15) / 16 * 16;
+  int tail_limits[2] = {0, 1};  // the most faces of a tile; a tile past the limits
   Scratch scratch;
   AFAR_CUDA(cudaMalloc(&scratch.p, std::max({n_lists + sizeof(int2) * (size_t)Nf, nrbf * wS,
                                              2 * sizeof(V4<double>) * (size_t)(Nf + Nb + 1)})));
@@ -1196,6 +1300,9 @@ extern "C" afar_status afar_setDeviceFieldDataStencil(afar_solver* s, const afar
     k_setup_lists<<<grid_for(Nc, kCellBlock), kCellBlock, 0, s->stream>>>(Nc, Nf, s->ldc, s->maxS, s->maxM, s->maxLB,
                                                                            s->nS, s->nM, dls, dext, dcf, s->sten, s->cf,
                                                                            s->order);
+    if (s->policy == AFAR_POLICY_MIXED) {
+      AFAR_CUDA(cudaMemsetAsync(s->wflag, 0, sizeof(unsigned) * (size_t)ntile * 4, s->stream));
+    }
     AFAR_CUDA(cudaGetLastError());
   }
   switch (s->policy) {
@@ -1204,7 +1311,27 @@ extern "C" afar_status afar_setDeviceFieldDataStencil(afar_solver* s, const afar
     default: st = setup_operators<PolicyMixed>(s, h, scratch.p); break;
   }
   if (st) return st;
+  if (s->policy == AFAR_POLICY_MIXED && paired && Nf > 0 && s->maxM >= 3) {
+    int* start = static_cast<int*>(s->xfer);  // (of k_face_order)
+    int* limits = start + Nc;
+    StageArgs<PolicyMixed> a = make_args<PolicyMixed>(s);
+    AFAR_CUDA(cudaMemsetAsync(limits, 0, 2 * sizeof(int), s->stream));
+    k_tail_tiles<<<(int)ntail, 128, 0, s->stream>>>(a, start, s->tail, s->thalo, s->thcode, s->thsg, s->textra, s->tlf,
+                                                    limits);
+    k_tail_lists<<<(int)ntail, 128, 0, s->stream>>>(a, s->tail, s->thalo, s->tlist);
+    AFAR_CUDA(cudaMemcpyAsync(tail_limits, limits, 2 * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  }
+  AFAR_CUDA(cudaGetLastError());
   AFAR_CUDA(cudaStreamSynchronize(s->stream));
+  // meshes whose tiles are past the limits of the fused stage tail, or whose faces are not in the lists of
+  // both their cells, or of cells with one or two faces, keep the separate kernels
+  s->bvd_pending = -1;
+  s->fused = tail_limits[1] == 0 && tail_smem(tail_limits[0], tail_cells(s)).bytes <= kMaxDynamicSmem - 2048;
+  s->tail_faces = tail_limits[0];
+  if (s->fused) {
+    if ((st = raise_smem_limit(k_tail<3>, s->device, tail_smem(s->tail_faces, tail_cells(s)).bytes))) return st;
+    if ((st = raise_smem_limit(k_tail<4>, s->device, tail_smem(s->tail_faces, tail_cells(s)).bytes))) return st;
+  }
   if (s->policy == AFAR_POLICY_MIXED && (st = build_tile_maps(s))) return st;
   if (s->policy == AFAR_POLICY_MIXED && (st = tune_reconstruct(s))) return st;
   s->have_stencil = true;
@@ -1244,6 +1371,7 @@ extern "C" afar_status afar_adjustTimeStep(afar_solver* s, int facesNum, double 
       k_set_ctl<<<1, 32, 0, s->stream>>>(s->ctl, 0.0, CFL, 0.0);
       AFAR_CUDA(cudaMemcpyAsync(&s->ctl->dt_bits, &init, sizeof(init), cudaMemcpyHostToDevice, s->stream));
       AFAR_CUDA(cudaGraphLaunch(s->graph_head, s->stream));
+      s->bvd_pending = fused_step(s) ? 0 : -1;
       StepCtl c;
       AFAR_CUDA(cudaMemcpyAsync(&c, s->ctl, sizeof(c), cudaMemcpyDeviceToHost, s->stream));
       AFAR_CUDA(cudaStreamSynchronize(s->stream));
@@ -1306,6 +1434,7 @@ static afar_status run_impl(afar_solver* s, int nSteps, double dt, double CFL, d
   if ((st = ensure_graph(s, kGraphStep))) return st;
   k_set_ctl<<<1, 32, 0, s->stream>>>(s->ctl, dt > 0.0 ? dt : 0.0, CFL, tEnd);
   for (int i = 0; i < nSteps; ++i) AFAR_CUDA(cudaGraphLaunch(s->graph, s->stream));
+  if (nSteps > 0) s->bvd_pending = fused_step(s) ? 2 : -1;
   AFAR_CUDA(cudaGetLastError());
   if (wait) return check_device_error(s);
   return AFAR_OK;
@@ -1335,6 +1464,7 @@ extern "C" afar_status afar_GPUevolve(afar_solver* s, double R, double Cv, doubl
     // for: a device-side error of the step surfaces at the next call that waits.
     k_set_ctl<<<1, 32, 0, s->stream>>>(s->ctl, deltaT, 1.0, 0.0);
     AFAR_CUDA(cudaGraphLaunch(s->graph_tail, s->stream));
+    s->bvd_pending = fused_step(s) ? 2 : -1;
     AFAR_CUDA(cudaGetLastError());
     return AFAR_OK;
   }
@@ -1384,6 +1514,7 @@ extern "C" afar_status afar_run_timed(afar_solver* s, int nSteps, double dt, dou
   k_set_ctl<<<1, 32, 0, s->stream>>>(s->ctl, dt > 0.0 ? dt : 0.0, CFL, tEnd);
   AFAR_CUDA(cudaEventRecord(e0, s->stream));
   for (int i = 0; i < nSteps; ++i) AFAR_CUDA(cudaGraphLaunch(s->graph, s->stream));
+  if (nSteps > 0) s->bvd_pending = fused_step(s) ? 2 : -1;
   AFAR_CUDA(cudaEventRecord(e1, s->stream));
   AFAR_CUDA(cudaEventSynchronize(e1));
   AFAR_CUDA(cudaEventElapsedTime(ms, e0, e1));
@@ -1414,6 +1545,14 @@ extern "C" afar_status afar_profile_step(afar_solver* s, double dt, double CFL, 
     if (r) return r;
     mark(-1);
     for (int k = 0; k < 3; ++k) {
+      if (sg.fused()) {
+        sg.at(k).reconstruct(k == 0);
+        mark(0);
+        sg.at(k).tail(k);
+        mark(3);
+        s->bvd_pending = k;
+        continue;
+      }
       sg.reconstruct();
       mark(0);
       sg.bvd();
@@ -1423,8 +1562,10 @@ extern "C" afar_status afar_profile_step(afar_solver* s, double dt, double CFL, 
       sg.update(k);
       mark(3);
     }
-    k_finish_step<<<1, 32, 0, s->stream>>>(s->ctl);
-    mark(4);
+    if (!sg.fused()) {
+      k_finish_step<<<1, 32, 0, s->stream>>>(s->ctl);
+      mark(4);
+    }
     return AFAR_OK;
   };
   switch (s->policy) {
@@ -1497,6 +1638,7 @@ extern "C" afar_status afar_stage_debug(afar_solver* s, int stage, double deltaT
     Stage<P> sg;
     afar_status r = make_stage<P>(s, true, &sg);
     if (r) return r;
+    s->bvd_pending = -1;
     sg.reconstruct();
     sg.bvd();
     sg.flux(false);
@@ -1559,6 +1701,7 @@ extern "C" afar_status afar_debug_limiter64(afar_solver* s, double* lim) {
   afar_status st = check_ready(s);
   if (st) return st;
   if (!lim) return (set_error("null output"), AFAR_ERR_ARGUMENT);
+  if ((st = settle_bvd(s))) return st;
   const size_t Nc = s->Nc;
   if (s->policy == AFAR_POLICY_FP64) {
     AFAR_CUDA(cudaMemcpy(lim, s->lim, Nc * sizeof(V4<double>), cudaMemcpyDeviceToHost));
@@ -1619,6 +1762,10 @@ extern "C" afar_status afar_state_snapshot(afar_solver* s, int op) {
     else
       AFAR_CUDA(cudaMemcpyAsync(src[i], dst[i], n[i], cudaMemcpyDeviceToDevice, s->stream));
   }
+  if (op == AFAR_SNAPSHOT_RESTORE && s->policy == AFAR_POLICY_MIXED && s->Nb)  // the ghosts in every buffer
+    for (void* b : s->Wb)
+      AFAR_CUDA(cudaMemcpyAsync(static_cast<V4<float>*>(b) + s->Nc, static_cast<V4<float>*>(s->W) + s->Nc,
+                                sizeof(V4<float>) * (size_t)s->Nb, cudaMemcpyDeviceToDevice, s->stream));
   AFAR_CUDA(cudaStreamSynchronize(s->stream));
   return AFAR_OK;
 }
@@ -1682,6 +1829,7 @@ extern "C" afar_status afar_switch_counts(afar_solver* s, long long counts[4]) {
   afar_status st = check_ready(s);
   if (st) return st;
   if (!counts) return (set_error("null output"), AFAR_ERR_ARGUMENT);
+  if (s->bvd_pending == 0 && (st = settle_bvd(s))) return st;  // a fused head: its stage's types
   unsigned long long* d = nullptr;
   AFAR_CUDA(cudaMalloc(&d, 4 * sizeof(unsigned long long)));
   AFAR_CUDA(cudaMemsetAsync(d, 0, 4 * sizeof(unsigned long long), s->stream));
@@ -1779,6 +1927,7 @@ struct afar_batch {
   size_t maps_n = 0;
   int n_tile = 0, n_reg = 0, n_cell = 0, n_bvd = 0, n_face = 0;
   size_t smem = 0;  // dynamic shared memory of the staged reconstruct (largest member)
+  bool fused = false;  // mixed: the fused stage (two kernels a stage)
   BatchSchedule sched;
   int forced_bvd = 0, forced_flux = 0;  // afar_batch_set_schedule (0: autotune)
   cudaGraphExec_t graph = nullptr;
@@ -1823,6 +1972,66 @@ void launch_flux(int block, int nblocks, const StageArgs<P>* t, const int2* map,
 std::mutex g_batch_tune_mu;
 std::map<std::tuple<int, int, int, int>, std::pair<int, int>> g_batch_tune;
 
+// One fused step of a batch as a graph: a chain of six kernels for every MemberTable's worth of
+// members.  The chains do not depend on one another.
+afar_status capture_fused(afar_batch* b, const std::vector<StageArgs<PolicyMixed>>& tab, int nfmax, size_t smem,
+                          size_t tail_bytes, cudaGraph_t* graph) {
+  using Table = MemberTable<PolicyMixed>;
+  const bool tri = nfmax <= 3;
+  const auto recon = tri ? kp_reconstruct_tile<3, false> : kp_reconstruct_tile<4, false>;
+  const auto recon_dt = tri ? kp_reconstruct_tile<3, true> : kp_reconstruct_tile<4, true>;
+  const auto tail_1 = tri ? kp_tail<3, true> : kp_tail<4, true>;
+  const auto tail_23 = tri ? kp_tail<3, false> : kp_tail<4, false>;
+  afar_status st;
+  if ((st = raise_smem_limit(recon, b->device, smem))) return st;
+  if ((st = raise_smem_limit(recon_dt, b->device, smem))) return st;
+  if ((st = raise_smem_limit(tail_1, b->device, tail_bytes))) return st;
+  if ((st = raise_smem_limit(tail_23, b->device, tail_bytes))) return st;
+
+  AFAR_CUDA(cudaGraphCreate(graph, 0));
+  auto build = [&]() -> afar_status {
+    std::unique_ptr<Table> cells(new Table), tiles(new Table);
+    for (size_t i0 = 0; i0 < tab.size(); i0 += Table::kMembers) {
+      const int n = (int)std::min<size_t>(Table::kMembers, tab.size() - i0);
+      cells->n = tiles->n = n;
+      cells->first[0] = tiles->first[0] = 0;
+      for (int i = 0; i < n; ++i) {
+        const StageArgs<PolicyMixed>& m = tab[i0 + i];
+        cells->m[i] = tiles->m[i] = m;
+        cells->first[i + 1] = cells->first[i] + grid_for(m.Nc, kTile);
+        tiles->first[i + 1] = tiles->first[i] + m.nTail;
+      }
+      cudaGraphNode_t last = nullptr;
+      for (int k = 0; k < 3; ++k) {
+        StageCoef coef = stage_coef(k);
+        void* recon_args[] = {cells.get(), &k};
+        void* tail_args[] = {tiles.get(), &k, &coef};
+        cudaKernelNodeParams np{};
+        np.func = reinterpret_cast<void*>(k == 0 ? recon_dt : recon);
+        np.gridDim = dim3(cells->first[n]);
+        np.blockDim = dim3(kTile);
+        np.sharedMemBytes = (unsigned)smem;
+        np.kernelParams = recon_args;
+        cudaGraphNode_t node;
+        AFAR_CUDA(cudaGraphAddKernelNode(&node, *graph, last ? &last : nullptr, last ? 1 : 0, &np));
+        np.func = reinterpret_cast<void*>(k == 0 ? tail_1 : tail_23);
+        np.gridDim = dim3(tiles->first[n]);
+        np.blockDim = dim3(kTailThreads);
+        np.sharedMemBytes = (unsigned)tail_bytes;
+        np.kernelParams = tail_args;
+        AFAR_CUDA(cudaGraphAddKernelNode(&last, *graph, &node, 1, &np));
+      }
+    }
+    return AFAR_OK;
+  };
+  st = build();
+  if (st) {
+    cudaGraphDestroy(*graph);
+    *graph = nullptr;
+  }
+  return st;
+}
+
 template <class P>
 afar_status batch_build(afar_batch* b) {
   std::vector<StageArgs<P>> tab;
@@ -1844,6 +2053,17 @@ afar_status batch_build(afar_batch* b) {
       is_tile[i] = !is_reg[i];
     }
   }
+  // mixed: the fused stage (two kernels a stage) where every member has it, unless a member forces
+  // the register pass or block sizes of the separate BVD and flux kernels are asked for; the same
+  // bits either way
+  bool fused = P::id == PolicyMixed::id && !b->forced_bvd && !b->forced_flux && !tab.empty();
+  size_t tail_bytes = 0;
+  for (size_t i = 0; i < b->members.size(); ++i) {
+    const afar_solver* s = b->members[i];
+    fused = fused && fused_step(s) && is_tile[i];
+    if (fused) tail_bytes = std::max<size_t>(tail_bytes, tail_smem(s->tail_faces, tail_cells(s)).bytes);
+  }
+  b->fused = fused;
   int lc = 0, lm = 0;
   while ((1ll << (lc + 1)) <= cells) ++lc;
   while ((1ll << (lm + 1)) <= (long long)b->members.size()) ++lm;
@@ -1851,7 +2071,9 @@ afar_status batch_build(afar_batch* b) {
   BatchSchedule sc;
   for (size_t i = 0; i < b->members.size(); ++i) sc.tile_members += is_tile[i], sc.reg_members += is_reg[i];
   bool timed = true;
-  if (b->forced_bvd || b->forced_flux) {
+  if (fused) {
+    timed = false;  // neither kernel runs: the schedule keeps its defaults
+  } else if (b->forced_bvd || b->forced_flux) {
     sc.bvd_block = b->forced_bvd ? b->forced_bvd : 128;
     sc.flux_block = b->forced_flux ? b->forced_flux : 256;
     timed = false;
@@ -1873,9 +2095,9 @@ afar_status batch_build(afar_batch* b) {
   const int bvd_sizes[3] = {64, 128, 256}, flux_sizes[2] = {128, 256};
   std::vector<int2> mp_bvd[3], mp_face[2];
   for (int k = 0; k < 3; ++k)
-    if (timed || bvd_sizes[k] == sc.bvd_block) batch_map(b->members, bvd_sizes[k], false, nullptr, mp_bvd[k]);
+    if (timed || (!fused && bvd_sizes[k] == sc.bvd_block)) batch_map(b->members, bvd_sizes[k], false, nullptr, mp_bvd[k]);
   for (int k = 0; k < 2; ++k)
-    if (timed || flux_sizes[k] == sc.flux_block) batch_map(b->members, flux_sizes[k], true, nullptr, mp_face[k]);
+    if (timed || (!fused && flux_sizes[k] == sc.flux_block)) batch_map(b->members, flux_sizes[k], true, nullptr, mp_face[k]);
   std::vector<int2> all;
   auto append = [&](const std::vector<int2>& v) {
     const size_t o = all.size();
@@ -1927,14 +2149,10 @@ afar_status batch_build(afar_batch* b) {
     return AFAR_OK;
   }
   const StageArgs<P>* t = static_cast<const StageArgs<P>*>(b->tab);
-  auto reconstruct = [&]() {
+  auto reconstruct = [&] {
     if constexpr (P::id == PolicyMixed::id) {
-      if (b->n_tile) {
-        if (nfmax <= 3)
-          kb_reconstruct_tile<P, 3><<<b->n_tile, kTile, b->smem, b->stream>>>(t, b->maps + o_tile);
-        else
-          kb_reconstruct_tile<P, 4><<<b->n_tile, kTile, b->smem, b->stream>>>(t, b->maps + o_tile);
-      }
+      const auto f = nfmax <= 3 ? kb_reconstruct_tile<P, 3> : kb_reconstruct_tile<P, 4>;
+      if (b->n_tile) f<<<b->n_tile, kTile, b->smem, b->stream>>>(t, b->maps + o_tile);
       if (b->n_reg) kb_reconstruct_reg<P><<<b->n_reg, kCellBlock, 0, b->stream>>>(t, b->maps + o_reg);
     } else
       kb_reconstruct_fp64<<<b->n_cell, kCellBlock, b->smem, b->stream>>>(t, b->maps + o_cell);
@@ -1987,18 +2205,25 @@ afar_status batch_build(afar_batch* b) {
 
   // capture one step of the whole batch
   cudaGraph_t g = nullptr;
-  AFAR_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-  for (int k = 0; k < 3; ++k) {
-    reconstruct();
-    launch_bvd<P>(sc.bvd_block, b->n_bvd, t, bmap, b->stream);
-    if (k == 0)
-      launch_flux<P, true>(sc.flux_block, b->n_face, t, fmap, b->stream);
-    else
-      launch_flux<P, false>(sc.flux_block, b->n_face, t, fmap, b->stream);
-    kb_update<P><<<b->n_cell, kCellBlock, 0, b->stream>>>(t, b->maps + o_cell, stage_coef(k));
+  if constexpr (P::id == PolicyMixed::id) {
+    if (fused) {
+      if ((st = capture_fused(b, tab, nfmax, smem, tail_bytes, &g))) return st;
+    }
   }
-  kb_finish_step<P><<<grid_for((long long)tab.size(), 128), 128, 0, b->stream>>>(t, (int)tab.size());
-  AFAR_CUDA(cudaStreamEndCapture(b->stream, &g));
+  if (!fused) {
+    AFAR_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+    for (int k = 0; k < 3; ++k) {
+      reconstruct();
+      launch_bvd<P>(sc.bvd_block, b->n_bvd, t, bmap, b->stream);
+      if (k == 0)
+        launch_flux<P, true>(sc.flux_block, b->n_face, t, fmap, b->stream);
+      else
+        launch_flux<P, false>(sc.flux_block, b->n_face, t, fmap, b->stream);
+      kb_update<P><<<b->n_cell, kCellBlock, 0, b->stream>>>(t, b->maps + o_cell, stage_coef(k));
+    }
+    kb_finish_step<P><<<grid_for((long long)tab.size(), 128), 128, 0, b->stream>>>(t, (int)tab.size());
+    AFAR_CUDA(cudaStreamEndCapture(b->stream, &g));
+  }
   const cudaError_t e = cudaGraphInstantiate(&b->graph, g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) {
@@ -2088,6 +2313,7 @@ extern "C" afar_status afar_batch_run(afar_batch* b, int nSteps, float* ms) {
   AFAR_CUDA(cudaEventCreate(&e1));
   AFAR_CUDA(cudaEventRecord(e0, b->stream));
   for (int i = 0; i < nSteps; ++i) AFAR_CUDA(cudaGraphLaunch(b->graph, b->stream));
+  for (afar_solver* m : b->members) m->bvd_pending = b->fused ? 2 : -1;
   AFAR_CUDA(cudaEventRecord(e1, b->stream));
   AFAR_CUDA(cudaEventSynchronize(e1));
   if (ms) AFAR_CUDA(cudaEventElapsedTime(ms, e0, e1));

@@ -507,6 +507,9 @@ def run_ours(args, dist: Dist):
             for k, v in s.profile_step().items():
                 acc[k] = acc.get(k, 0.0) + v / PROFILE_STEPS
         results[pol]["kernels_ms"] = acc
+        # a step without BVD and flux kernels is the fused one: reconstruct and stage tail, three times
+        if acc["bvd"] == 0.0 and acc["flux"] == 0.0:
+            results[pol]["launches"] = 6
         results[pol]["device_bytes"] = s.device_bytes()
         if pol == "mixed":
             results[pol]["tuning"] = s.tuning()
@@ -1116,7 +1119,7 @@ def run_batch(args, dist: Dist):
     compression ramps, cells log-uniform in [5k, 200k] (quads, 2:1 channel), inflow Mach U[1.5, 4]
     through a label-6 inflow patch, ramp angle U[5, 20] degrees, an isentropic vortex of strength
     U[0, 5] carried in the stream; mixed policy, CFL 0.3; all stepped together --batch-steps RK3
-    steps by one afar_batch (13 launches per step for the whole batch).  Compared with stepping
+    steps by one afar_batch (six launches per step for every 48 members).  Compared with stepping
     the same solves one after another (afar_run_timed, 40 steps each)."""
     from afar_cudaeuler2dmixo3rk3solver_gb300 import Batch, CaseConfig, CudaSolver, mesh, precompute
     from afar_cudaeuler2dmixo3rk3solver_gb300 import build as b
@@ -1142,6 +1145,11 @@ def run_batch(args, dist: Dist):
         s.restore()
         solo_ms += s.run_timed(40) / 40.0
         s.restore()
+    # the fused step: reconstruct and stage tail, three times, for every 48 members (see the single solve)
+    fused = all(s.profile_step()["flux"] == 0.0 for s in solvers)
+    for s in solvers:
+        s.restore()
+    launches = 6 if fused else 13
     batch = Batch("mixed", device=dist.local)
     for s in solvers:
         s.set_step_params()
@@ -1164,11 +1172,11 @@ def run_batch(args, dist: Dist):
         "n_gpus": dist.world, "higher_is_better": True, "ms_per_step": ms / args.batch_steps,
         "data": "synthetic (compression ramps 5k-200k quads, Mach 1.5-4, 5-20 deg, vortex 0-5, seeded)",
         "config": {"workload": "batch_wedges", "solves": args.batch_solves, "cells": int(cells.sum()),
-                   "steps": args.batch_steps, "policy": "mixed", "launches_per_step": 13, "setup_s": round(setup_s, 1)},
+                   "steps": args.batch_steps, "policy": "mixed", "launches_per_step": 6 * -(-len(solvers) // 48) if fused else 13, "setup_s": round(setup_s, 1)},
         "schedule": schedule,
         "one_after_another": None if args.batch_no_solo else {
             "value": float(cells.sum()) / (solo_ms * 1e-3), "ms_per_step": solo_ms,
-            "launches_per_step": 13 * args.batch_solves},
+            "launches_per_step": launches * args.batch_solves},
         "finite": finite,
     }), flush=True)
 

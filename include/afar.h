@@ -313,7 +313,8 @@ afar_status afar_run_timed(afar_solver* solver, int nSteps, double deltaT, doubl
 /* Runs one step kernel by kernel (not as a graph) with events between the kernels and returns
  * the device time of each kind summed over the three stages: ms[0] reconstruct, ms[1] BVD switch,
  * ms[2] face flux (with the CFL kernel where the policy runs one), ms[3] gather + RK update,
- * ms[4] step bookkeeping. */
+ * ms[4] step bookkeeping.  The mixed policy's fused step has two kernels a stage: the reconstruct, and
+ * the rest of the stage as ms[3]; ms[1], ms[2] and ms[4] are then 0. */
 afar_status afar_profile_step(afar_solver* solver, double deltaT, double CFL, float ms[5]);
 
 /* Simulated time, last step size and number of steps taken on the device. */
@@ -354,10 +355,10 @@ afar_status afar_set_write_interval(afar_solver* solver, double writeInterval);
 afar_status afar_set_periodic(afar_solver* solver, double periodX, double periodY);
 
 /* ---- batches: many independent solves stepped by the same kernel launches ------------------- */
-/* A batch steps all of its member solvers with one launch per stage kernel (13 per RK3 step,
- * replayed as one CUDA graph): every block works on one member, so meshes of uneven size share the
- * GPU without padding.  Each member keeps its own device data, time step (fixed or CFL, with its
- * own step params), end time and step count.  A member's result does not depend on which other
+/* A batch steps all of its member solvers with one launch per stage kernel (13 per RK3 step; the
+ * mixed policy's fused stage: six for every 48 members; replayed as one CUDA graph): every block works
+ * on one member, so meshes of uneven size share the GPU without padding.  Each member keeps its own
+ * device data, time step (fixed or CFL, with its own step params), end time and step count.  A member's result does not depend on which other
  * solves share its batch (bitwise); it agrees with afar_run of the same solve to the policy's
  * rounding (the batched kernels read their arguments from a device table, afar_run's from kernel
  * parameters, and the compiler may fuse a multiply-add differently in the two).  Members join and
@@ -380,7 +381,8 @@ afar_status afar_batch_destroy(afar_batch* batch);
  * member's result never depends on its batch-mates), and the BVD and flux kernels run in the block
  * size that timed fastest on the whole batch (BVD 64, 128 or 256 cells, flux 128 or 256 faces;
  * best of three launches each), cached per device, policy and batch shape (cells and members, each
- * to a factor of two).  Block sizes do not change results.  afar_batch_get_schedule reports the
+ * to a factor of two).  A mixed batch whose members all have the fused
+ * stage, and force neither, runs that and times nothing.  Block sizes do not change results.  afar_batch_get_schedule reports the
  * members on each reconstruct, the block sizes and the launch times measured (ms: BVD at 64, 128,
  * 256, flux at 128, 256; zeros when the decision came from the cache or was forced);
  * afar_batch_set_schedule forces block sizes (0: autotune). */
@@ -515,7 +517,8 @@ afar_status afar_debug_wait_injection(int device, unsigned extraBytes, long long
 afar_status afar_set_face_gauss_flux(afar_solver* solver, int nPoints, const double* points,
                                      const double* pointWeights, const double* rbfGauss);
 
-/* Number of kernel launches one afar_run step issues on this solver (for accounting). */
+/* Number of kernel launches of one step as separate stage kernels (for accounting).  The mixed
+ * policy's fused step (see afar_profile_step) issues six instead of its 13. */
 int afar_launches_per_step(afar_solver* solver);
 
 #ifdef __cplusplus
