@@ -126,12 +126,12 @@ struct StageArgs {
   G gw[4];           // the points' weights, normalised to sum to one
 };
 
-// limiterProcess (reference cudaLimiter.h:35-50)
-template <class S, class G>
-__device__ __forceinline__ void limiter_process(S& limiter, S& phif, const S phic, const S phiMax, const S phiMin,
-                                                const G gx, const G gy, const G dx, const G dy) {
-  phif = phic;
-  phif += gx * dx + gy * dy;
+// limiterProcess (reference cudaLimiter.h:35-50), ref policy
+__device__ __forceinline__ void limiter_process(float& limiter, float& phif, const float phic, const float phiMax,
+                                                const float phiMin, const double gx, const double gy, const double dx,
+                                                const double dy) {
+  using S = float;
+  phif = to_float(to_double(phic) + (gx * dx + gy * dy));
   const S d2 = phif - phic;
   const S d1 = (phif < phic) * (phiMin - phic) + (phif >= phic) * (phiMax - phic);
   S yy = fmn(S(2), S(0.5) * d1 / (d2 + (d2 >= S(0)) * AFAR_LIT(S, 1e-10) - (d2 < S(0)) * AFAR_LIT(S, 1e-10)));
@@ -750,7 +750,7 @@ __device__ __forceinline__ void recon_ref_body(const StageArgs<PolicyRef>& a, co
   const int ldc = a.ldc;
   const int nS = a.nS[c], nM = a.nM[c];
   const V4<WT> wc = a.W[c];
-  const S pc = (S)wc.x, uxc = (S)wc.y, uyc = (S)wc.z, tc = (S)wc.w;
+  const S pc = to_float(wc.x), uxc = to_float(wc.y), uyc = to_float(wc.z), tc = to_float(wc.w);
   constexpr int GB = 4;
   for (int i0 = 0; i0 < nS; i0 += GB) {
     int j[GB];
@@ -761,7 +761,7 @@ __device__ __forceinline__ void recon_ref_body(const StageArgs<PolicyRef>& a, co
     for (int u = 0; u < GB; ++u) wj[u] = a.W[j[u]];
 #pragma unroll
     for (int u = 0; u < GB; ++u)
-      if (i0 + u < nS) sv[(i0 + u) * B + t] = V4<S>{(S)wj[u].x, (S)wj[u].y, (S)wj[u].z, (S)wj[u].w};
+      if (i0 + u < nS) sv[(i0 + u) * B + t] = V4<S>{to_float(wj[u].x), to_float(wj[u].y), to_float(wj[u].z), to_float(wj[u].w)};
   }
 
   G gPx = 0, gPy = 0, gUxx = 0, gUxy = 0, gUyx = 0, gUyy = 0, gTx = 0, gTy = 0;
@@ -770,17 +770,17 @@ __device__ __forceinline__ void recon_ref_body(const StageArgs<PolicyRef>& a, co
     const S M1 = m.x, M2 = m.y;
     const V4<S> v = sv[i * B + t];
     S dphi = v.x - pc;
-    gPx += M1 * dphi;
-    gPy += M2 * dphi;
+    gPx += to_double(M1 * dphi);
+    gPy += to_double(M2 * dphi);
     dphi = v.y - uxc;
-    gUxx += M1 * dphi;
-    gUyx += M2 * dphi;
+    gUxx += to_double(M1 * dphi);
+    gUyx += to_double(M2 * dphi);
     dphi = v.z - uyc;
-    gUxy += M1 * dphi;
-    gUyy += M2 * dphi;
+    gUxy += to_double(M1 * dphi);
+    gUyy += to_double(M2 * dphi);
     dphi = v.w - tc;
-    gTx += M1 * dphi;
-    gTy += M2 * dphi;
+    gTx += to_double(M1 * dphi);
+    gTy += to_double(M2 * dphi);
   }
   a.grad[2 * c] = V4<G>{gPx, gPy, gUxx, gUxy};
   a.grad[2 * c + 1] = V4<G>{gUyx, gUyy, gTx, gTy};
@@ -811,10 +811,10 @@ __device__ __forceinline__ void recon_ref_body(const StageArgs<PolicyRef>& a, co
       const V2<G> d = a.sg[fi * ldc + c];
       const G dx = d.x, dy = d.y;
       V4<G> o;
-      o.x = (G)(pc) + gPx * dx + gPy * dy;
-      o.y = (G)(uxc) + gUxx * dx + gUyx * dy;
-      o.z = (G)(uyc) + gUxy * dx + gUyy * dy;
-      o.w = (G)(tc) + gTx * dx + gTy * dy;
+      o.x = to_double(pc) + gPx * dx + gPy * dy;
+      o.y = to_double(uxc) + gUxx * dx + gUyx * dy;
+      o.z = to_double(uyc) + gUxy * dx + gUyy * dy;
+      o.w = to_double(tc) + gTx * dx + gTy * dy;
       a.fv[2 * f + isNei] = o;
     }
     flag0 = 0;
@@ -833,10 +833,10 @@ __device__ __forceinline__ void recon_ref_body(const StageArgs<PolicyRef>& a, co
       const S deltaR = rf.x, fraction = rf.y;
       const S* w = a.wts + (size_t)(fi * (a.maxS + 1)) * ldc + c;
       S wk = w[0];
-      G pf = wk * pc;
-      G uxf = wk * uxc;
-      G uyf = wk * uyc;
-      G tf = wk * tc;
+      G pf = to_double(wk * pc);
+      G uxf = to_double(wk * uxc);
+      G uyf = to_double(wk * uyc);
+      G tf = to_double(wk * tc);
       for (int ci0 = 0; ci0 < nS; ci0 += 8) {
         S wb[8];
 #pragma unroll
@@ -845,10 +845,10 @@ __device__ __forceinline__ void recon_ref_body(const StageArgs<PolicyRef>& a, co
         for (int u = 0; u < 8; ++u) {
           if (ci0 + u < nS) {
             const V4<S> v = sv[(ci0 + u) * B + t];
-            pf += wb[u] * v.x;
-            uxf += wb[u] * v.y;
-            uyf += wb[u] * v.z;
-            tf += wb[u] * v.w;
+            pf += to_double(wb[u] * v.x);
+            uxf += to_double(wb[u] * v.y);
+            uyf += to_double(wb[u] * v.z);
+            tf += to_double(wb[u] * v.w);
           }
         }
       }
@@ -856,16 +856,16 @@ __device__ __forceinline__ void recon_ref_body(const StageArgs<PolicyRef>& a, co
       S phif;
       V4<G> o;
       limiter_process(lp, phif, pc, pMax, pMin, gPx, gPy, dx, dy);
-      o.x = pick<P>(fab(pMax - pMin) >= SMALL, fab(pMax - pMin) < SMALL, pf, phif);
+      o.x = blend64(fab(pMax - pMin) >= SMALL, fab(pMax - pMin) < SMALL, pf, to_double(phif));
       notTrouble = phif > S(0);
-      smooth = fmx(smooth, fab((S(1) - fraction) * pc + fraction * pnb - phif) / deltaR + (pf <= S(0)) * AFAR_LIT(S, 1e20) +
+      smooth = fmx(smooth, fab((S(1) - fraction) * pc + fraction * pnb - phif) / deltaR + le_zero(pf) * AFAR_LIT(S, 1e20) +
                                (phif <= S(0)) * AFAR_LIT(S, 1e20));
       limiter_process(lux, phif, uxc, uxMax, uxMin, gUxx, gUyx, dx, dy);
-      o.y = pick<P>(fab(uxMax - uxMin) >= SMALL, fab(uxMax - uxMin) < SMALL, uxf, phif);
+      o.y = blend64(fab(uxMax - uxMin) >= SMALL, fab(uxMax - uxMin) < SMALL, uxf, to_double(phif));
       limiter_process(luy, phif, uyc, uyMax, uyMin, gUxy, gUyy, dx, dy);
-      o.z = pick<P>(fab(uyMax - uyMin) >= SMALL, fab(uyMax - uyMin) < SMALL, uyf, phif);
+      o.z = blend64(fab(uyMax - uyMin) >= SMALL, fab(uyMax - uyMin) < SMALL, uyf, to_double(phif));
       limiter_process(lt, phif, tc, tMax, tMin, gTx, gTy, dx, dy);
-      o.w = pick<P>(fab(tMax - tMin) >= SMALL, fab(tMax - tMin) < SMALL, tf, phif);
+      o.w = blend64(fab(tMax - tMin) >= SMALL, fab(tMax - tMin) < SMALL, tf, to_double(phif));
       notTrouble = phif > S(0);
       a.fv[2 * f + isNei] = o;
     }
@@ -1071,7 +1071,9 @@ __device__ __forceinline__ void bvd_body(const StageArgs<P>& a, const int blk) {
     }
   }
 
-  const S tc = (S)a.W[c].w;
+  S tc;
+  if constexpr (P::id == PolicyRef::id) tc = to_float(a.W[c].w);
+  else tc = (S)a.W[c].w;
   const V4<G> g1 = a.grad[2 * c + 1];
   const G gTx = g1.z, gTy = g1.w;
   V4<S> L = a.lim[c];
@@ -1091,24 +1093,31 @@ __device__ __forceinline__ void bvd_body(const StageArgs<P>& a, const int blk) {
     const V2<G> d = a.sg[fi * ldc + c];
     const G tfOwn = a.fv[2 * f].w;
     const G tfNei = a.fv[2 * f + 1].w;
-    const G tfCur = pick<P>(isNei, !isNei, tfNei, tfOwn);
-    const G tfOther = pick<P>(!isNei, isNei, tfNei, tfOwn);
-    const G lim = to_bj(L.w);
-    G tfTVD;
-    if constexpr (P::id == PolicyFP64::id)
-      tfTVD = tvd64(tc, lim, gTx, gTy, d.x, d.y);
-    else
-      tfTVD = tc + lim * (gTx * d.x + gTy * d.y);
     int typeval, notFlat, limited;
-    if constexpr (P::id == PolicyFP64::id) {  // the same comparisons on integers (L.w >= 0)
-      const double jump = dabs_(tfCur - tfOther);
+    if constexpr (P::id == PolicyMixed::id) {
+      const G tfCur = isNei ? tfNei : tfOwn, tfOther = isNei ? tfOwn : tfNei;
+      const G lim = to_bj(L.w);
+      const G tfTVD = tc + lim * (gTx * d.x + gTy * d.y);
+      typeval = fab(tfTVD - tfOther) < 0.5f * fab(tfCur - tfOther);
+      notFlat = fab(tfCur - tfOther) > 1e-10f;
+      limited = (lim < 0.9f) + (shockTypeExt > 0);
+    } else {  // the comparisons on integers
+      double jump, tfTVD, tfOther;
+      if constexpr (P::id == PolicyFP64::id) {
+        tfOther = isNei ? tfOwn : tfNei;
+        jump = dabs_((isNei ? tfNei : tfOwn) - tfOther);
+        tfTVD = tvd64(tc, to_bj(L.w), gTx, gTy, d.x, d.y);
+        limited = (dbits(L.w) < dbits(0.45)) + (shockTypeExt > 0);  // (L.w >= 0)
+      } else {
+        tfOther = blend64(!isNei, isNei, tfNei, tfOwn);
+        jump = dabs_(blend64(isNei, !isNei, tfNei, tfOwn) - tfOther);
+        const S lim = to_bj(L.w);
+        tfTVD = to_double(tc) + to_double(lim) * (gTx * d.x + gTy * d.y);
+        limited = (lim < 0.9f) + (shockTypeExt > 0);
+      }
+      const double flat = AFAR_LIT(S, 1e-10);
       typeval = dbits(dabs_(tfTVD - tfOther)) < dbits(0.5 * jump) && !dnan_(jump);
-      notFlat = !abs_lt(jump, 1e-10) && dbits(jump) != dbits(1e-10) && !dnan_(jump);
-      limited = (dbits(L.w) < dbits(0.45)) + (shockTypeExt > 0);
-    } else {
-      typeval = fab(tfTVD - tfOther) < AFAR_LIT(S, 0.5) * fab(tfCur - tfOther);
-      notFlat = fab(tfCur - tfOther) > AFAR_LIT(S, 1e-10);
-      limited = (lim < AFAR_LIT(S, 0.9)) + (shockTypeExt > 0);
+      notFlat = dbits(jump) > dbits(flat) && !dnan_(jump);
     }
     bvdType = max(bvdType, notFlat * limited * typeval);
   }
@@ -1186,19 +1195,21 @@ __device__ __forceinline__ void kfvs_flux(G& rhoFlux, G& rhoUxFlux, G& rhoUyFlux
 }
 
 // RoeFlux (reference cudaRiemannSolver.h:71-136): Roe dissipation with a Harten-type entropy fix.
-template <class D, class RC, class G>
-__device__ __forceinline__ void roe_flux(G& rhoFlux, G& rhoUxFlux, G& rhoUyFlux, G& rhoEFlux, const D& rhoL,
-                                         const D& rhoR, const D& pL, const D& pR, const D& uxL, const D& uxR,
-                                         const D& uyL, const D& uyR, const D& tL, const D& tR, const D& deltaP,
-                                         const D& deltaRho, const RC& R, const RC& Cv, const D magSf, const D Sfx,
-                                         const D Sfy) {
-  const D gamma = (Cv + R) / Cv;
+// R and Cv are double in it, the rest float; conversions and the division by Cv off the FP64 pipe.
+__device__ __forceinline__ void roe_flux(double& rhoFlux, double& rhoUxFlux, double& rhoUyFlux, double& rhoEFlux,
+                                         const float& rhoL, const float& rhoR, const float& pL, const float& pR,
+                                         const float& uxL, const float& uxR, const float& uyL, const float& uyR,
+                                         const float& tL, const float& tR, const float& deltaP, const float& deltaRho,
+                                         const double& R, const double& Cv, const float magSf, const float Sfx,
+                                         const float Sfy) {
+  using D = float;
+  const D gamma = to_float(div64(Cv + R, Cv));
   const D nfx = Sfx / magSf;
   const D nfy = Sfy / magSf;
   const D cvL = uxL * nfx + uyL * nfy;
   const D cvR = uxR * nfx + uyR * nfy;
-  const D hL = Cv * tL + D(0.5) * (uxL * uxL + uyL * uyL) + pL / rhoL;
-  const D hR = Cv * tR + D(0.5) * (uxR * uxR + uyR * uyR) + pR / rhoR;
+  const D hL = to_float(Cv * to_double(tL) + to_double(D(0.5) * (uxL * uxL + uyL * uyL)) + to_double(pL / rhoL));
+  const D hR = to_float(Cv * to_double(tR) + to_double(D(0.5) * (uxR * uxR + uyR * uyR)) + to_double(pR / rhoR));
   const D tiny = AFAR_LIT(D, 1e-20);
   const D rhoT = sqr_(fmx(rhoL * rhoR, tiny));
   const D wL = sqr_(fmx(rhoL, tiny)) / (sqr_(fmx(rhoL, tiny)) + sqr_(fmx(rhoR, tiny)));
@@ -1229,13 +1240,13 @@ __device__ __forceinline__ void roe_flux(G& rhoFlux, G& rhoUxFlux, G& rhoUyFlux,
   eps = D(2) * fmx(D(0), (UR + cR) - (UL + cL));
   D l3 = fab(cvT + cT);
   l3 = (l3 >= eps) * l3 + (l3 < eps) * ((l3 * l3 + eps * eps) / (D(2) * eps + eps0));
-  rhoFlux -= D(0.5) * (l1 * r1 + l2 * r2 + l3 * r3) * magSf;
-  rhoUxFlux -= D(0.5) * (l1 * r1 * (uxT - cT * nfx) + l2 * (r2 * uxT + rhoT * (dUx - dCv * nfx)) + l3 * r3 * (uxT + cT * nfx)) * magSf;
-  rhoUyFlux -= D(0.5) * (l1 * r1 * (uyT - cT * nfy) + l2 * (r2 * uyT + rhoT * (dUy - dCv * nfy)) + l3 * r3 * (uyT + cT * nfy)) * magSf;
-  rhoEFlux -= D(0.5) *
+  rhoFlux -= to_double(D(0.5) * (l1 * r1 + l2 * r2 + l3 * r3) * magSf);
+  rhoUxFlux -= to_double(D(0.5) * (l1 * r1 * (uxT - cT * nfx) + l2 * (r2 * uxT + rhoT * (dUx - dCv * nfx)) + l3 * r3 * (uxT + cT * nfx)) * magSf);
+  rhoUyFlux -= to_double(D(0.5) * (l1 * r1 * (uyT - cT * nfy) + l2 * (r2 * uyT + rhoT * (dUy - dCv * nfy)) + l3 * r3 * (uyT + cT * nfy)) * magSf);
+  rhoEFlux -= to_double(D(0.5) *
               (l1 * r1 * (hT - cT * cvT) + l2 * (r2 * D(0.5) * q2 + rhoT * (uxT * dUx + uyT * dUy - cvT * dCv)) +
                l3 * r3 * (hT + cT * cvT)) *
-              magSf;
+              magSf);
 }
 
 // ---------------------------------------------------------------- dissipation, fp64 and mixed
@@ -1630,12 +1641,64 @@ __device__ __forceinline__ double courant_dt64(const double CFL, const double gR
   const double den = __fma_rn(c, fs.z, __fma_rn(w0, unL, __dmul_rn(w1, unR)));
   return __dmul_rn(__dmul_rn(__dmul_rn(CFL, g.x), fs.z), rcp64(den));
 }
-// The same to about 1e-5 in FP32, from 20 bits of each operand and without the Courant number.
-__device__ __forceinline__ float courant_estimate(const float gRf, const V2<double> g, const V4<double>& fs,
-                                                  const V4<double>& Wo, const V4<double>& Wn) {
-  const float w1 = top_float(g.y), w0 = 1.f - w1, i = top_float(fs.w), x = i * top_float(fs.x), y = i * top_float(fs.y);
-  const float uL = fabsf(top_float(Wo.y) * x + top_float(Wo.z) * y), uR = fabsf(top_float(Wn.y) * x + top_float(Wn.z) * y);
-  return __fdividef(top_float(g.x), w0 * uL + w1 * uR + sqrtf(gRf * (w0 * top_float(Wo.w) + w1 * top_float(Wn.w))));
+// Bounds of a face's step over the Courant number in FP32, from 20 bits of each operand (i: 1/|Sf|):
+// every operand's error counts against the largest term, so a velocity across the face that is the
+// difference of large components, or a sound speed far below them, widens the bounds.  A bound that
+// cannot be had is 0 below and infinite above.
+struct CourantBounds {
+  float lo, hi;
+};
+__device__ __forceinline__ CourantBounds courant_bounds(const float gR, const V2<double> g, const V4<double>& fs,
+                                                        const float i, const V4<double>& Wo, const V4<double>& Wn) {
+  const float inf = __int_as_float(0x7F800000);
+  const float w1 = top_float(g.y), w0 = 1.f - w1, ws = fabsf(w0) + fabsf(w1);
+  const float x = i * top_float(fs.x), y = i * top_float(fs.y), dr = top_float(g.x);
+  const float ax = top_float(Wo.y) * x, ay = top_float(Wo.z) * y, bx = top_float(Wn.y) * x, by = top_float(Wn.z) * y;
+  const float tL = top_float(Wo.w), tR = top_float(Wn.w);
+  const float un = w0 * fabsf(ax + ay) + w1 * fabsf(bx + by);
+  const float eu = 1e-5f * ws * fmaxf(fabsf(ax) + fabsf(ay), fabsf(bx) + fabsf(by));
+  const float c2 = gR * (w0 * tL + w1 * tR), e2 = 1e-5f * gR * ws * fmaxf(fabsf(tL), fabsf(tR));
+  const float most = un + eu + sqrtf(c2 + e2), least = un - eu + sqrtf(fmaxf(c2 - e2, 0.f));
+  CourantBounds r;
+  r.lo = most > 1e-18f ? 0.9999f * __fdividef(dr, most) : 0.f;  // (0 where it is not a number either)
+  r.hi = least > 1e-18f && least < 1e37f ? 1.0001f * __fdividef(dr, least) : inf;
+  return r;
+}
+
+// The smallest Courant step of a block's faces into *bits: only the smallest counts, so a face is
+// evaluated in FP64 only where its lower bound is not above the smallest upper bound of the block and
+// the smallest step of any block so far -- a few faces of a few blocks of a flow that varies instead of
+// 25 to 45 FP64 instructions a face.  The minimum is that over all faces, exactly.  All threads of the
+// block take part.
+template <class Exact>
+__device__ __forceinline__ void courant_block_min(const CourantBounds est, const double cfl, unsigned long long* bits,
+                                                  const bool face, Exact exact) {
+  __shared__ unsigned wmin[8];
+  __shared__ float s_prior;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned v = __float_as_uint(est.hi);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if (lane == 0) wmin[warp] = v;
+  if (threadIdx.x == 0)
+    s_prior = 1.0001f *
+              __fdividef((float)__longlong_as_double((long long)*(const volatile unsigned long long*)bits), (float)cfl);
+  __syncthreads();
+  unsigned b = wmin[0];
+  for (int k = 1; k < (int)(blockDim.x >> 5); ++k) b = min(b, wmin[k]);
+  const bool near = face && !(est.lo > fminf(__uint_as_float(b), s_prior));
+  if (!__any_sync(0xffffffffu, near)) return;
+  unsigned long long d = kInfBits;
+  if (near) {
+    d = dbits(exact());
+    if (d > kInfBits) d = kInfBits;  // not a number, negative: no step from here
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long u = __shfl_xor_sync(0xffffffffu, d, o);
+    d = u < d ? u : d;
+  }
+  if (lane == 0 && d < *(const volatile unsigned long long*)bits) atomicMin(bits, d);
 }
 
 // ---------------------------------------------------------------- ref policy: face flux
@@ -1663,10 +1726,10 @@ struct RefSide {
 };
 __device__ __forceinline__ double ref_tvd(const double w, const float lim, const double ga, const double gb,
                                           const double dx, const double dy) {
-  return __fma_rn((double)lim, __fma_rn(ga, dx, __dmul_rn(gb, dy)), w);  // w + lim (ga dx + gb dy)
+  return __fma_rn(to_double(lim), __fma_rn(ga, dx, __dmul_rn(gb, dy)), w);  // w + lim (ga dx + gb dy)
 }
 __device__ __forceinline__ double ref_blend(const bool tvd, const double o3, const double t) {
-  return __dadd_rn(__dmul_rn((double)(1 - tvd), o3), __dmul_rn((double)tvd, t));
+  return blend64(!tvd, tvd, o3, t);
 }
 __device__ __forceinline__ RefSide ref_face_side(const StageArgs<PolicyRef>& a, const int c, const int slot,
                                                  const double dx, const double dy, const bool tvd) {
@@ -1681,18 +1744,30 @@ __device__ __forceinline__ RefSide ref_face_side(const StageArgs<PolicyRef>& a, 
   const double tT = ref_tvd(w.w, lm.w, g1.z, g1.w, dx, dy);
   RefSide s;
   s.pT = pT;
-  s.rhoT = pT / __dmul_rn(R, tT);
+  s.rhoT = div64(pT, __dmul_rn(R, tT));
   s.p = ref_blend(tvd, o3.x, pT);
   s.ux = ref_blend(tvd, o3.y, uxT);
   s.uy = ref_blend(tvd, o3.z, uyT);
   s.T = ref_blend(tvd, o3.w, tT);
-  s.rho = s.p / __dmul_rn(R, s.T);
+  s.rho = div64(s.p, __dmul_rn(R, s.T));
   return s;
 }
 // Cv T + |u|^2 / 2 + p / rho of a side (its total enthalpy per unit mass)
 __device__ __forceinline__ double ref_enthalpy(const RefSide& s, const double Cv) {
-  return __dadd_rn(__dadd_rn(__dmul_rn(Cv, s.T), __dmul_rn(0.5, __fma_rn(s.ux, s.ux, __dmul_rn(s.uy, s.uy)))),
-                   s.p / s.rho);
+  return __dadd_rn(__dadd_rn(__dmul_rn(Cv, s.T), half64(__fma_rn(s.ux, s.ux, __dmul_rn(s.uy, s.uy)))),
+                   div64(s.p, s.rho));
+}
+
+// min_delta of doubles, kept in a float: rounding keeps the order, so the minima are taken after it
+__device__ __forceinline__ float ref_min_delta(const double l, const double r, const double lT, const double rT) {
+  const double j = r - l;
+  float d = fabsf(to_float(j));
+  d = fminf(d, fabsf(to_float(r - lT)));
+  d = fminf(d, fabsf(to_float(rT - l)));
+  d = fminf(d, fabsf(to_float(rT - lT)));
+  bool lt = neg_(j) && (dbits(j) << 1) != 0ull, ge = !lt;
+  if (dnan_(j)) ge = r >= l, lt = r < l;
+  return ge * d - lt * d;
 }
 
 // The float dissipation of the ref policy: adds the Roe dissipation, or replaces the central flux
@@ -1707,7 +1782,7 @@ __device__ __noinline__ void ref_roe(double& rhoFlux, double& rhoUxFlux, double&
                                      const float& tL, const float& tR, const float& dP, const float& dRho,
                                      const double& R, const double& Cv, const float magSf, const float Sfx,
                                      const float Sfy) {
-  roe_flux<float, double, double>(rhoFlux, rhoUxFlux, rhoUyFlux, rhoEFlux, rhoL, rhoR, pL, pR, uxL, uxR, uyL, uyR, tL,
+  roe_flux(rhoFlux, rhoUxFlux, rhoUyFlux, rhoEFlux, rhoL, rhoR, pL, pR, uxL, uxR, uyL, uyR, tL,
                                   tR, dP, dRho, R, Cv, magSf, Sfx, Sfy);
 }
 __device__ __noinline__ void ref_kfvs(double& rhoFlux, double& rhoUxFlux, double& rhoUyFlux, double& rhoEFlux,
@@ -1723,6 +1798,9 @@ __device__ __noinline__ void ref_kfvs(double& rhoFlux, double& rhoUxFlux, double
 // evaluateFlux of internal face f under the ref policy (reference cudaRiemannSolver.h:171-251):
 // both sides' states, the minimised jumps of p and rho, the central flux in double, then the float
 // Roe dissipation, or the KFVS flux where either cell is a shock cell.
+// The FP64 pipe bounds it, so what need not run there does not: selections and conversions on integers,
+// divisions by div64, minima of the jumps as floats, with the same bits.  129 FP64 instructions a face
+// now; 121k triangles 108 -> 88 us a launch (the pipe 79% busy), the update 33 -> 26, the BVD 19 -> 14.
 __device__ __forceinline__ void flux_ref_face(const StageArgs<PolicyRef>& a, const int f) {
   const int2 on = a.on[f];
   const V4<double> d = a.fd[f];   // face centre - owner centre, face centre - neighbour centre
@@ -1731,24 +1809,25 @@ __device__ __forceinline__ void flux_ref_face(const StageArgs<PolicyRef>& a, con
   const RefSide L = ref_face_side(a, on.x, 2 * f, d.x, d.y, swL != 0);
   const RefSide Rs = ref_face_side(a, on.y, 2 * f + 1, d.z, d.w, swR != 0);
   const double Sfx = sf.x, Sfy = sf.y, magSf = sf.z, Cv = a.Cv, R = a.R;
-  const float dP = min_delta<float, double>(L.p, Rs.p, L.pT, Rs.pT);
-  const float dRho = min_delta<float, double>(L.rho, Rs.rho, L.rhoT, Rs.rhoT);
+  const float dP = ref_min_delta(L.p, Rs.p, L.pT, Rs.pT);
+  const float dRho = ref_min_delta(L.rho, Rs.rho, L.rhoT, Rs.rhoT);
   // central flux: the mean of the two sides' Euler fluxes through Sf
   double F0, F1, F2, F3;
   const double unL = __fma_rn(L.ux, Sfx, __dmul_rn(L.uy, Sfy)), unR = __fma_rn(Rs.ux, Sfx, __dmul_rn(Rs.uy, Sfy));
-  F0 = __fma_rn(__dmul_rn(0.5, L.rho), unL, __dmul_rn(__dmul_rn(0.5, Rs.rho), unR));
-  F1 = __dadd_rn(__dmul_rn(0.5, __fma_rn(L.p, Sfx, __dmul_rn(F0, L.ux))),
-                 __dmul_rn(0.5, __fma_rn(Rs.p, Sfx, __dmul_rn(F0, Rs.ux))));
-  F2 = __dadd_rn(__dmul_rn(0.5, __fma_rn(L.p, Sfy, __dmul_rn(F0, L.uy))),
-                 __dmul_rn(0.5, __fma_rn(Rs.p, Sfy, __dmul_rn(F0, Rs.uy))));
-  const double half = __dmul_rn(0.5, F0);
+  F0 = __fma_rn(half64(L.rho), unL, __dmul_rn(half64(Rs.rho), unR));
+  F1 = __dadd_rn(half64(__fma_rn(L.p, Sfx, __dmul_rn(F0, L.ux))),
+                 half64(__fma_rn(Rs.p, Sfx, __dmul_rn(F0, Rs.ux))));
+  F2 = __dadd_rn(half64(__fma_rn(L.p, Sfy, __dmul_rn(F0, L.uy))),
+                 half64(__fma_rn(Rs.p, Sfy, __dmul_rn(F0, Rs.uy))));
+  const double half = half64(F0);
   F3 = __fma_rn(half, ref_enthalpy(L, Cv), __dmul_rn(half, ref_enthalpy(Rs, Cv)));
   // the dissipation sees the states, face vector and jumps as floats; R and Cv stay double
-  const float rhoL = L.rho, rhoR = Rs.rho, pL = L.p, pR = Rs.p, uxL = L.ux, uxR = Rs.ux, uyL = L.uy, uyR = Rs.uy,
-              tL = L.T, tR = Rs.T;
+  const float rhoL = to_float(L.rho), rhoR = to_float(Rs.rho), pL = to_float(L.p), pR = to_float(Rs.p),
+              uxL = to_float(L.ux), uxR = to_float(Rs.ux), uyL = to_float(L.uy), uyR = to_float(Rs.uy),
+              tL = to_float(L.T), tR = to_float(Rs.T);
   const RefDissipation diss = (swL < 0 || swR < 0) ? ref_kfvs : ref_roe;
-  diss(F0, F1, F2, F3, rhoL, rhoR, pL, pR, uxL, uxR, uyL, uyR, tL, tR, dP, dRho, R, Cv, (float)magSf, (float)Sfx,
-       (float)Sfy);
+  diss(F0, F1, F2, F3, rhoL, rhoR, pL, pR, uxL, uxR, uyL, uyR, tL, tR, dP, dRho, R, Cv, to_float(magSf),
+       to_float(Sfx), to_float(Sfy));
   a.flux[f] = V4<double>{F0, F1, F2, F3};
 }
 
@@ -1775,7 +1854,7 @@ __device__ __forceinline__ void flux_body(const StageArgs<P>& a, const int blk) 
     __syncthreads();
   }
   float dtf32 = 1e5f;
-  float est = __int_as_float(0x7F800000);  // fp64: the face's Courant step over the Courant number
+  CourantBounds est{__int_as_float(0x7F800000), __int_as_float(0x7F800000)};  // fp64: of the face's Courant step
   if (id < a.Nf) {
     if constexpr (P::id == PolicyRef::id) {
       static_assert(!DT, "under the ref policy the Courant step is a kernel of its own, as in the reference");
@@ -1800,7 +1879,7 @@ __device__ __forceinline__ void flux_body(const StageArgs<P>& a, const int blk) 
       densities64(l.rho, r.rho, rhoLT, rhoRT, l.p, r.p, pLT, pRT, l.T, r.T, tLT, tRT, a.invR);
       a.flux[id] = face_flux64(l, r, pLT, pRT, rhoLT, rhoRT, sL < 0 || sR < 0, gas64(a), fs);
       if constexpr (DT) {
-        est = courant_estimate(a.gRf, a.dtg[id], fs, Wo, Wn);
+        est = courant_bounds(a.gRf, a.dtg[id], fs, top_float(fs.w), Wo, Wn);
       }
     } else {
       const int2 on = a.on[id];
@@ -1877,34 +1956,11 @@ __device__ __forceinline__ void flux_body(const StageArgs<P>& a, const int blk) 
       atomicMin(&a.ctl->dt_bits, bits);
     }
   } else if constexpr (DT) {
-    // fp64: only the smallest step counts, so a face is evaluated in FP64 only where its FP32 estimate
-    // is within 1e-3 (the estimates' error is below 1e-4) of the block's smallest and of the smallest
-    // step of any block so far -- a few faces of a few blocks instead of 25 FP64 instructions a face.
-    // The minimum is that over all faces, exactly.  (An estimate that is not a number is evaluated.)
-    __shared__ unsigned wmin[8];
-    __shared__ float s_prior;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned v = __float_as_uint(est);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (lane == 0) wmin[warp] = v;
-    if (threadIdx.x == 0) {
-      const StepCtl* ctl = a.ctl;
-      const unsigned long long prior = *(const volatile unsigned long long*)&ctl->dt_bits;
-      s_prior = ctl->dt_fixed > 0.0 ? -1.f : __fdividef((float)__longlong_as_double((long long)prior), (float)ctl->cfl);
-    }
-    __syncthreads();
-    if (s_prior < 0.f) return;  // a fixed step
-    unsigned b = wmin[0];
-    for (int k = 1; k < (int)(blockDim.x >> 5); ++k) b = min(b, wmin[k]);
-    const float limit = 1.001f * fminf(__uint_as_float(b), s_prior);
-    if (id < a.Nf && !(est > limit)) {
+    if (gt_zero(a.ctl->dt_fixed)) return;  // (the same in every thread)
+    courant_block_min(est, a.ctl->cfl, &a.ctl->dt_bits, id < a.Nf, [&] {
       const int2 on = a.on[id];
-      const V4<G> fs = a.fs[id];
-      const double dt = courant_dt64(a.ctl->cfl, a.gR, a.dtg[id], fs, a.W[on.x], a.W[on.y]);
-      const unsigned long long bits = dbits(dt);
-      atomicMin(&a.ctl->dt_bits, bits > kInfBits ? kInfBits : bits);  // not a number, negative: no step from here
-    }
+      return courant_dt64(a.ctl->cfl, a.gR, a.dtg[id], a.fs[id], a.W[on.x], a.W[on.y]);
+    });
   }
 }
 
@@ -2081,13 +2137,16 @@ __device__ __forceinline__ void update_body(const StageArgs<P>& a, const int blk
     const double R = a.R;
     const double gamma = a.gamma;  // R/Cv + 1, computed once on the host like GPUevolve.cu:222
     const double V = a.vol[c];
-    const double rho = beta1 * o.x + beta2 * u.x + beta3 * deltaT * (-Rrho / V);
-    const double rhoUx = beta1 * o.y + beta2 * u.y + beta3 * deltaT * (-RrhoUx / V);
-    const double rhoUy = beta1 * o.z + beta2 * u.z + beta3 * deltaT * (-RrhoUy / V);
-    const double rhoE = beta1 * o.w + beta2 * u.w + beta3 * deltaT * (-RrhoE / V);
+    constexpr int kSign = (int)0x80000000;
+    const double rV = rcp64(V);
+    const double rho = beta1 * o.x + beta2 * u.x + beta3 * deltaT * flip_sign(div64(Rrho, V, rV), kSign);
+    const double rhoUx = beta1 * o.y + beta2 * u.y + beta3 * deltaT * flip_sign(div64(RrhoUx, V, rV), kSign);
+    const double rhoUy = beta1 * o.z + beta2 * u.z + beta3 * deltaT * flip_sign(div64(RrhoUy, V, rV), kSign);
+    const double rhoE = beta1 * o.w + beta2 * u.w + beta3 * deltaT * flip_sign(div64(RrhoE, V, rV), kSign);
     un = V4<double>{rho, rhoUx, rhoUy, rhoE};
-    const double p = (gamma - 1.0) * (rhoE - 0.5 * (rhoUx * rhoUx + rhoUy * rhoUy) / rho);
-    wn = V4<WT>{(WT)p, (WT)(rhoUx / rho), (WT)(rhoUy / rho), (WT)(p / (R * rho))};
+    const double rr = rcp64(rho);
+    const double p = (gamma - 1.0) * (rhoE - div64(half64(rhoUx * rhoUx + rhoUy * rhoUy), rho, rr));
+    wn = V4<WT>{(WT)p, (WT)div64(rhoUx, rho, rr), (WT)div64(rhoUy, rho, rr), (WT)div64(p, R * rho)};
   } else {  // FP64 is scarce on GB300: 1/V precomputed, one reciprocal for 1/rho
     const double s3 = nb3dt * a.vinv[c];
     if (k.first) {  // beta1 = 1, beta2 = 0: U is not read
@@ -2987,31 +3046,49 @@ __global__ void __launch_bounds__(256) k_delta_t(StageArgs<P> a, double CFL, uns
     CFL = ctl->cfl;
   }
   const int id = blockIdx.x * blockDim.x + threadIdx.x;
-  double dtf = 1e5;
-  if (id < a.Nf) {
-    const int2 on = a.on[id];
-    const V4<typename P::W> Wo = a.W[on.x], Wn = a.W[on.y];
-    const V4<typename P::G> fs = a.fs[id];
-    const double sfx = (double)fs.x, sfy = (double)fs.y, msf = (double)fs.z;
-    const V2<double> g = a.dtg[id];
-    if constexpr (P::id == PolicyFP64::id) {
-      dtf = courant_dt64(CFL, a.gR, g, fs, Wo, Wn);
-    } else {
+  if constexpr (P::id == PolicyMixed::id) {  // (the mixed policy's multi-point flux: in FP64 all the same)
+    double dtf = 1e5;
+    if (id < a.Nf) {
+      const int2 on = a.on[id];
+      const V4<float> Wo = a.W[on.x], Wn = a.W[on.y], fs = a.fs[id];
+      const double sfx = (double)fs.x, sfy = (double)fs.y, msf = (double)fs.z;
+      const V2<double> g = a.dtg[id];
       const double deltaR = g.x, fraction = g.y, Rd = a.R, Cvd = a.Cv;
       dtf = CFL * deltaR * msf /
             ((1.0 - fraction) * fabs((double)Wo.y * sfx + (double)Wo.z * sfy) +
              fraction * fabs((double)Wn.y * sfx + (double)Wn.z * sfy) +
              sqrt((Rd / Cvd + 1.0) * Rd * ((1.0 - fraction) * (double)Wo.w + fraction * (double)Wn.w)) * msf);
     }
-  }
-  unsigned long long v = (unsigned long long)__double_as_longlong(dtf);
-  if (!(dtf >= 0.0)) v = 0x7FF0000000000000ull;
+    unsigned long long v = (unsigned long long)__double_as_longlong(dtf);
+    if (!(dtf >= 0.0)) v = 0x7FF0000000000000ull;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long u = __shfl_xor_sync(0xffffffffu, v, o);
-    v = u < v ? u : v;
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long u = __shfl_xor_sync(0xffffffffu, v, o);
+      v = u < v ? u : v;
+    }
+    if ((threadIdx.x & 31) == 0) atomicMin(bits, v);
+  } else {
+    CourantBounds est{__int_as_float(0x7F800000), __int_as_float(0x7F800000)};
+    if (id < a.Nf) {
+      const int2 on = a.on[id];
+      const V4<double> fs = a.fs[id];
+      const float i = P::id == PolicyFP64::id ? top_float(fs.w) : __fdividef(1.f, top_float(fs.z));
+      est = courant_bounds((float)a.gR, a.dtg[id], fs, i, a.W[on.x], a.W[on.y]);
+    }
+    courant_block_min(est, CFL, bits, id < a.Nf, [&] {
+      const int2 on = a.on[id];
+      const V4<double> fs = a.fs[id], Wo = a.W[on.x], Wn = a.W[on.y];
+      const V2<double> g = a.dtg[id];
+      if constexpr (P::id == PolicyFP64::id) {
+        return courant_dt64(CFL, a.gR, g, fs, Wo, Wn);
+      } else {
+        const double deltaR = g.x, fraction = g.y, Rd = a.R, Cvd = a.Cv;
+        return CFL * deltaR * fs.z /
+               ((1.0 - fraction) * fabs(Wo.y * fs.x + Wo.z * fs.y) + fraction * fabs(Wn.y * fs.x + Wn.z * fs.y) +
+                sqrt((Rd / Cvd + 1.0) * Rd * ((1.0 - fraction) * Wo.w + fraction * Wn.w)) * fs.z);
+      }
+    });
   }
-  if ((threadIdx.x & 31) == 0) atomicMin(bits, v);
 }
 
 // The Courant step of the mixed policy for afar_adjustTimeStep: the FP32 estimate of its fused

@@ -171,6 +171,64 @@ __device__ __forceinline__ double rsq64(const double x) {
   return __fma_rn(__dmul_rn(y0, d), __fma_rn(0.375, d, 0.5), y0);
 }
 
+// float to double and double to float (to nearest, ties to even) on integers: as conversions they take
+// the FP64 pipe.  Whatever is not a normal float or zero on the float's side takes the conversion.
+__device__ __forceinline__ double to_double(const float x) {
+  const unsigned b = __float_as_uint(x), m = b & 0x7FFFFFFFu;
+  if (m - 0x00800000u < 0x7F000000u || m == 0u)
+    return __hiloint2double((int)((b & 0x80000000u) | (m ? (m >> 3) + 0x38000000u : 0u)), (int)(m << 29));
+  double y;
+  asm volatile("cvt.f64.f32 %0, %1;" : "=d"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float to_float(const double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), m = hi & 0x7FFFFFFFu;
+  if (m - 0x38100000u < 0x47EFFFFFu - 0x38100000u || (m | lo) == 0u) {  // below the largest float
+    const unsigned t = m ? __funnelshift_l(lo, m - 0x38000000u, 3) : 0u;
+    const unsigned up = ((lo & 0x1FFFFFFFu) + 0x0FFFFFFFu + (t & 1u)) >> 29;
+    return __uint_as_float((hi & 0x80000000u) | (t + up));
+  }
+  float y;
+  asm volatile("cvt.rn.f32.f64 %0, %1;" : "=f"(y) : "d"(x));
+  return y;
+}
+// a/b rounded to nearest from r = rcp64(b): q = a r is within two ulp, its remainder a - b q comes out of
+// the fused multiply-add and corrects it (Markstein 1990) to 2^-103 before the last rounding.  Operands
+// far from the ends of the range, or a = 0; others take the division.
+__device__ __forceinline__ bool div64_range(const double x) {
+  return ((unsigned)__double2hiint(x) & 0x7FFFFFFFu) - 0x26F00000u < 0x32000000u;  // 2^-400 to 2^400
+}
+__device__ __forceinline__ double div64(const double a, const double b, const double r) {
+  const bool zero = (dbits(a) << 1) == 0ull;
+  if (!div64_range(b) || !(zero || div64_range(a))) return a / b;
+  const double q = __dmul_rn(a, r);
+  const double c = __fma_rn(__fma_rn(-b, q, a), r, q);
+  return zero ? q : c;  // (a zero keeps its sign)
+}
+__device__ __forceinline__ double div64(const double a, const double b) { return div64(a, b, rcp64(b)); }
+// x/2 by the exponent
+__device__ __forceinline__ double half64(const double x) {
+  const int hi = __double2hiint(x);
+  if ((((unsigned)hi & 0x7FFFFFFFu) - 0x00200000u) < 0x7FC00000u) return __hiloint2double(hi - 0x00100000, __double2loint(x));
+  double y;  // zeros, subnormals, halves that are, and what is not finite
+  asm volatile("mul.rn.f64 %0, %1, 0d3FE0000000000000;" : "=d"(y) : "d"(x));
+  return y;
+}
+// c1*a + c2*b of two conditions, one true: the chosen one, as the sum leaves it (a negative zero stays
+// one only next to a negative operand); anything not finite takes the sum.
+__device__ __noinline__ double blend64_sum(const bool c1, const bool c2, const double a, const double b) {
+  return __dadd_rn(__dmul_rn((double)c1, a), __dmul_rn((double)c2, b));
+}
+__device__ __forceinline__ double blend64(const bool c1, const bool c2, const double a, const double b) {
+  const unsigned ha = (unsigned)__double2hiint(a), hb = (unsigned)__double2hiint(b);
+  if (c1 == c2 || (ha & 0x7FF00000u) == 0x7FF00000u || (hb & 0x7FF00000u) == 0x7FF00000u)
+    return blend64_sum(c1, c2, a, b);
+  unsigned hi = c1 ? ha : hb;
+  const unsigned lo = (unsigned)(c1 ? __double2loint(a) : __double2loint(b)), other = c1 ? hb : ha;
+  if (hi == 0x80000000u && lo == 0u) hi &= other;
+  return __hiloint2double((int)hi, (int)lo);
+}
+
 // Bulk global->shared copies (cp.async.bulk, the TMA unit's untiled form) completing on an
 // mbarrier.  Both addresses 16-byte aligned, size a multiple of 16.
 __device__ __forceinline__ unsigned smem_addr(const void* p) {

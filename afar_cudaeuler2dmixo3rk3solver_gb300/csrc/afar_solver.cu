@@ -476,16 +476,16 @@ afar_status raise_smem_limit(K kernel, int device, size_t bytes) {
 }
 
 // Threads a block of the single-solve kernels over n cells or faces.  The ref and fp64 kernels are
-// bound by each SM's FP64 pipe, so a mesh too small to give every SM two full blocks is cut into
-// smaller ones until it reaches all SMs: the pipe's time on the busiest SM is the kernel's (fp64,
-// 1,754 cells: 55 blocks of 32 instead of 14 of 128, the step 317 -> 182 us with the kernels' other
-// changes; whole meshes of 250k cells and more are past the line and keep the full block).
+// bound by each SM's FP64 pipe, so a mesh too small to give every SM eight full blocks is cut into
+// smaller ones until it reaches all SMs evenly: the pipe's time on the busiest SM is the kernel's.  us a
+// step in blocks of 128 / 64 / 32: fp64, 41k triangles 267 / 242 / 237, 121k 553 / 545 / 550, 500k 1980 /
+// 1966 / 1972; ref, 41k 333 / 294 / 281, 250k quads 1027 / 1022 / 1018.
 template <class P>
 int block_for(long long n, int full) {
   if constexpr (P::id == PolicyMixed::id) return full;
   constexpr long long kSMs = 152;
   int b = full;
-  while (b > 32 && n < 2 * kSMs * b) b /= 2;
+  while (b > 32 && n < 8 * kSMs * b) b /= 2;
   return b;
 }
 
@@ -1395,6 +1395,7 @@ extern "C" afar_status afar_adjustTimeStep(afar_solver* s, int facesNum, double 
         StageArgs<PolicyRef> a = make_args<PolicyRef>(s);
         a.R = R;
         a.Cv = Cv;
+        a.gR = (R / Cv + 1.0) * R;
         k_delta_t<PolicyRef><<<gf, kFaceBlock, 0, s->stream>>>(a, CFL, s->dt_bits, nullptr);
         break;
       }
