@@ -273,6 +273,7 @@ __device__ __forceinline__ void courant_min(const CourantFaces<NF>& q, const Sta
 // still accumulated in stencil order, as in the reference.
 template <class P, bool DT>
 __device__ __forceinline__ void recon_reg_body(const StageArgs<P>& a, const V4<typename P::W>* W, const int blk) {
+  pdl_wait();
   using S = typename P::S;
   using G = typename P::G;
   using WT = typename P::W;
@@ -383,6 +384,7 @@ __device__ __forceinline__ void recon_reg_body(const StageArgs<P>& a, const V4<t
       }
     }
   }
+  pdl_next();
   a.grad[2 * c] = V4<G>{gPx, gPy, gUxx, gUxy};
   a.grad[2 * c + 1] = V4<G>{gUyx, gUyy, gTx, gTy};
 
@@ -523,7 +525,7 @@ __host__ __device__ inline ReconTile recon_tile_layout(const int maxM, const int
 // face geometry and O3 weights, so the first gathers are in flight while the weights still stream
 // in.  Smem rows hold 128 cells: face ids [maxM][128], stencil ids [S][128], LS and geometry
 // [maxM][128] pairs, weights [maxM][S][128] (S = the tile's largest stencil).
-template <class P>
+template <bool EARLY, class P>
 __device__ __forceinline__ void recon_tile_fetch(const StageArgs<P>& a, const V4<typename P::W>* W, const int blk,
                                                  const ReconTile& L,
                                                  unsigned char* sm, unsigned long long* bar) {
@@ -540,7 +542,10 @@ __device__ __forceinline__ void recon_tile_fetch(const StageArgs<P>& a, const V4
   switch (lane) {
     case 0: tma_load_2d(sm + L.off_cf, &tm->cf, c0, 0, bar); break;
     case 1: tma_load_2d(sm + L.off_sten, &tm->sten[S - 1], c0, 0, bar); break;
-    case 2: bulk_to_smem(sm + L.off_w, W + c0, (unsigned)min(kTile, a.Nc - c0) * 16u, bar); break;
+    case 2:  // (the one copy of what the kernel before has written)
+      pdl_wait<EARLY>();
+      bulk_to_smem(sm + L.off_w, W + c0, (unsigned)min(kTile, a.Nc - c0) * 16u, bar);
+      break;
     case 3: tma_load_2d(sm + L.off_lsm, &tm->lsm, 2 * c0, 0, bar + 1); break;
     case 4: tma_load_2d(sm + L.off_sg, &tm->sg, 2 * c0, 0, bar + 1); break;
     case 5: tma_load_2d(sm + L.off_sr, &tm->sr, 2 * c0, 0, bar + 1); break;
@@ -555,7 +560,7 @@ __device__ __forceinline__ void recon_tile_fetch(const StageArgs<P>& a, const V4
 // batches of 8, all in flight) and feeds the gradient and min/max (compact members) and the O3 sums
 // of every face side; every sum is accumulated in stencil order, as in the reference.  NF: the
 // largest number of faces of a cell (3 on all-triangle meshes, else 4).
-template <class P, int NF, bool DT>
+template <class P, int NF, bool DT, bool EARLY = true>
 __device__ __forceinline__ void recon_tile_body(const StageArgs<P>& a, const V4<typename P::W>* W, const int blk,
                                                 unsigned char* sm) {
   using S = typename P::S;
@@ -569,9 +574,10 @@ __device__ __forceinline__ void recon_tile_body(const StageArgs<P>& a, const V4<
     mbar_init(bar + 1, 1);
   }
   __syncthreads();
-  if (t < 32) recon_tile_fetch(a, W, blk, L, sm, bar);
+  if (t < 32) recon_tile_fetch<EARLY>(a, W, blk, L, sm, bar);
   const int c = blk * kTile + t;
   const int nS = c < a.Nc ? a.nS[c] : 0, nM = c < a.Nc ? a.nM[c] : 0;
+  pdl_wait<EARLY>();
   const long long limit = g_tile_wait_limit;
   // leaving: every copy into this block's shared memory must have landed first
   auto give_up = [&]() {
@@ -668,6 +674,7 @@ __device__ __forceinline__ void recon_tile_body(const StageArgs<P>& a, const V4<
       }
     }
   }
+  pdl_next<EARLY>();
   a.grad[2 * c] = V4<G>{gPx, gPy, gUxx, gUxy};
   a.grad[2 * c + 1] = V4<G>{gUyx, gUyy, gTx, gTy};
 
@@ -2239,7 +2246,7 @@ __host__ __device__ inline TailSmem tail_smem(const int nf, const int cells) {
 // kNoFace, kWall for a boundary face, else 2 f + side of the face, from kElsewhere on.
 constexpr int kNoFace = -1, kWall = -2, kElsewhere = 0x10000;
 
-template <int NF, bool E>
+template <int NF, bool E, bool EARLY = true>
 __device__ __forceinline__ void tail_body(const StageArgs<PolicyMixed>& a, const V4<float>* __restrict__ Win,
                                           V4<float>* __restrict__ Wout, const int blk, const StageCoef& k,
                                           unsigned char* sm) {
@@ -2250,7 +2257,7 @@ __device__ __forceinline__ void tail_body(const StageArgs<PolicyMixed>& a, const
   const int c0 = blk * T, nc = min(T, a.Nc - c0);
   const bool own0 = tid < T;  // this thread has an own cell first, else a halo cell
   // Loads that need no other's result, all issued before the first wait: the tile's header and lists, an
-  // own cell's operands, a halo cell's id and slots.
+  // own cell's operands, a halo cell's id and slots; first those that no kernel writes.
   const int4 hdr = reinterpret_cast<const int4*>(a.tail)[blk];
   const int xid = tid < kTailExtra ? a.textra[(size_t)blk * kTailExtra + tid] : 0;
   const int reach = tid < kTailList ? a.tlist[(size_t)blk * kTailList + tid] : 0;
@@ -2284,11 +2291,12 @@ __device__ __forceinline__ void tail_body(const StageArgs<PolicyMixed>& a, const
     }
     nM = a.nM[c];
     nS = a.nS[c];
-    load_cell();
   } else {
     c = a.thalo[(size_t)blk * kTailHalo + (tid - T)];
     load_slots(tid - T);
   }
+  pdl_wait<EARLY>();
+  if (own0) load_cell();
   const int fstart = hdr.x, nOwn = hdr.y, nF = hdr.z, nX = nF - nOwn, nHalo = hdr.w & 0xFFFF, nReach = (int)((unsigned)hdr.w >> 16);
   const TailSmem S = tail_smem(nF, T);
   V4<float>* const st = reinterpret_cast<V4<float>*>(sm);          // [2 nF] O3 state of each side; then the flux
@@ -2465,6 +2473,7 @@ __device__ __forceinline__ void tail_body(const StageArgs<PolicyMixed>& a, const
     mbar_wait_bounded(bar + 1, 0, limit);
     return done();
   }
+  pdl_next<EARLY>();
   // the faces' fluxes, each in the place of its first side's state
   for (int j = tid; j < nF; j += kTailThreads) {
     const V4<float> fs = sfs[j];
@@ -2950,7 +2959,7 @@ __global__ void __launch_bounds__(kTile, 4) kb_reconstruct_tile(const StageArgs<
   extern __shared__ __align__(128) unsigned char sm[];
   const int2 m = map[blockIdx.x];
   const StageArgs<P>& a = member_args(tab, m.x);
-  recon_tile_body<P, NF, false>(a, a.W, m.y, sm);
+  recon_tile_body<P, NF, false, false>(a, a.W, m.y, sm);
 }
 // The two kernels of the fused stage over up to kMembers solves, whose arguments are the launch's own
 // parameters: the block finds its member from its index alone, so every pointer and constant of the
@@ -2978,19 +2987,20 @@ __device__ __forceinline__ int member_of(const MemberTable<P>& t) {
   return lo;
 }
 static_assert(sizeof(MemberTable<PolicyMixed>) + sizeof(StageCoef) + 16 <= 32764, "a launch's parameters");
-template <int NF, bool DT>
+// (EARLY: launched as programmatic dependents; the two instructions alone cost ten members of 160k quads 1%)
+template <int NF, bool DT, bool EARLY>
 __global__ void __launch_bounds__(kTile, 4)
     kp_reconstruct_tile(const __grid_constant__ MemberTable<PolicyMixed> t, const int buf) {
   extern __shared__ __align__(128) unsigned char sm[];
   const int i = member_of(t);
-  recon_tile_body<PolicyMixed, NF, DT>(t.m[i], t.m[i].W3[buf], blockIdx.x - t.first[i], sm);
+  recon_tile_body<PolicyMixed, NF, DT, EARLY>(t.m[i], t.m[i].W3[buf], blockIdx.x - t.first[i], sm);
 }
-template <int NF, bool FIRST>
+template <int NF, bool FIRST, bool EARLY>
 __global__ void __launch_bounds__(kTailThreads, kTailBlocks)
     kp_tail(const __grid_constant__ MemberTable<PolicyMixed> t, const int buf, const StageCoef k) {
   extern __shared__ __align__(128) unsigned char sm[];
   const int i = member_of(t);
-  tail_body<NF, FIRST>(t.m[i], t.m[i].W3[buf], t.m[i].W3[buf == 2 ? 0 : buf + 1], blockIdx.x - t.first[i], k, sm);
+  tail_body<NF, FIRST, EARLY>(t.m[i], t.m[i].W3[buf], t.m[i].W3[buf == 2 ? 0 : buf + 1], blockIdx.x - t.first[i], k, sm);
 }
 __global__ void __launch_bounds__(128, 4) kb_reconstruct_fp64(const StageArgs<PolicyFP64>* __restrict__ tab,
                                                               const int2* __restrict__ map) {

@@ -229,6 +229,18 @@ __device__ __forceinline__ double blend64(const bool c1, const bool c2, const do
   return __hiloint2double((int)hi, (int)lo);
 }
 
+// Programmatic dependent launch: a kernel that says pdl_next() in every block lets the one after it on
+// the stream start, whose pdl_wait() returns when the first is complete and its writes are visible.
+// Neither does anything in a launch without that attribute.
+template <bool EARLY = true>
+__device__ __forceinline__ void pdl_next() {
+  if constexpr (EARLY) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <bool EARLY = true>
+__device__ __forceinline__ void pdl_wait() {
+  if constexpr (EARLY) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Bulk global->shared copies (cp.async.bulk, the TMA unit's untiled form) completing on an
 // mbarrier.  Both addresses 16-byte aligned, size a multiple of 16.
 __device__ __forceinline__ unsigned smem_addr(const void* p) {

@@ -378,10 +378,10 @@ void reorder(afar_solver* s, T* a, size_t n) {
 }
 
 // Cells of a tile of the fused stage tail: as many as its 256 threads take with the halo in one pass (192
-// triangles, 152 quads), fewer quads where the mesh has no block for every SM and a block's time is the
-// kernel's.  us a step at 96 / 152 / 192 cells: triangles 1.1k 41 / 43 / 41, 99k 72 / 73 / 68, 998k 588 / 512 / 497;
-// quads 1.0k 42 / 45 / 58, 10k 46.5 / 47.2 / 61, 66k 70 / 62 / 72, 1.0M 670 / 584 / 631.
-int tail_cells(const afar_solver* s) { return s->maxM <= 3 ? 192 : s->Nc <= 152 * 96 ? 96 : 152; }
+// triangles, 152 quads), fewer quads where a mesh is a few blocks and a block's time is the kernel's.  us a
+// step at 96 / 152 / 192 cells: triangles 1.1k 41 / 43 / 41, 99k 72 / 73 / 68, 998k 588 / 512 / 497; quads 1.0k 42 / 45 / 58,
+// 10k 46.5 / 47.2 / 61, 66k 70 / 62 / 72, 1.0M 670 / 584 / 631; six members of 10k quads in a batch 73 / 65.
+int tail_cells(const afar_solver* s) { return s->maxM <= 3 ? 192 : s->Nc <= 4096 ? 96 : 152; }
 
 template <class P>
 StageArgs<P> make_args(afar_solver* s) {
@@ -503,10 +503,37 @@ inline bool fused_step(const afar_solver* s) { return s->fused && s->ng == 0; }
 
 // One solve's stage launches, arguments by value.  The ref policy reconstructs in the staged
 // kernel and runs the reference-layout flux; fp64 reconstructs staged, mixed in registers.
+// The fused stage's kernels start before the one ahead is complete (pdl_next near its end): their
+// barriers, lists and operator rows are on the way when its results are there.  us a step, without / with:
+// 1k quads 43.6 / 39.2, 10k 47 / 41, 250k 191 / 186; 10k triangles 46 / 40, 202k 130 / 121, 2.0M 946 / 937.  (Saying
+// pdl_next first thing: 4.0M quads 2308, 2.0M triangles 1003: the next kernel's waiting blocks take the places
+// of blocks that have work.)  Not meshes of many quads (4.0M 2167 / 2164), and not the tail where a quad mesh's
+// reconstruct is one wave of 2.5 to 4 blocks a SM: its blocks crowd where that ends first (65k quads 62.7 with
+// both early, 59.5 with the reconstruct alone; 48k 55.6 against 55.5 and 78k 67.6 against 70.5 on either side).
+inline bool quads_one_wave(int maxM, long long reconBlocks) { return maxM > 3 && reconBlocks > 380 && reconBlocks <= 608; }
+inline bool stage_early(int maxM, long long reconBlocks) { return maxM <= 3 || reconBlocks <= 4000; }
+
+// Launches a kernel, with pdl as the programmatic dependent of the one before it on the stream.
+template <class... A, class... B>
+void launch(void (*kernel)(A...), int grid, int block, size_t smem, cudaStream_t stream, bool pdl, const B&... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = pdl ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, A(args)...);
+}
+
 template <class P>
 struct Stage {
   afar_solver* s;
   StageArgs<P> a;
+  bool pdl = false;  // the launch may start before the one ahead of it is complete
   int bc() const { return block_for<P>(s->Nc, kCellBlock); }
   int gc() const { return grid_for(s->Nc, bc()); }
 
@@ -517,9 +544,9 @@ struct Stage {
                                      : (dt ? k_reconstruct_tile<P, 4, true> : k_reconstruct_tile<P, 4, false>);
       const auto reg = dt ? k_reconstruct_reg<P, true> : k_reconstruct_reg<P, false>;
       if (s->recon_variant == 1)
-        reg<<<gc(), kCellBlock, 0, s->stream>>>(a);
+        launch(reg, gc(), kCellBlock, 0, s->stream, pdl, a);
       else
-        tile<<<gc(), kTile, recon_smem<P>(s), s->stream>>>(a);
+        launch(tile, gc(), kTile, recon_smem<P>(s), s->stream, pdl, a);
     } else
       k_reconstruct_staged<P><<<gc(), bc(), recon_smem<P>(s, bc()), s->stream>>>(a);
     if constexpr (P::id != PolicyRef::id) {
@@ -537,7 +564,8 @@ struct Stage {
   void tail(int k) const {
     if constexpr (P::id == PolicyMixed::id) {
       const auto f = s->maxM <= 3 ? k_tail<3> : k_tail<4>;
-      f<<<a.nTail, kTailThreads, tail_smem(s->tail_faces, tail_cells(s)).bytes, s->stream>>>(a, a.W3[(k + 1) % 3], stage_coef(k));
+      launch(f, a.nTail, kTailThreads, tail_smem(s->tail_faces, tail_cells(s)).bytes, s->stream, pdl, a,
+             a.W3[(k + 1) % 3], stage_coef(k));
     }
   }
   void bvd() const { k_bvd<P><<<gc(), bc(), 0, s->stream>>>(a); }
@@ -587,10 +615,12 @@ void enqueue_head(const Stage<P>& st) {
 template <class P>
 void enqueue_tail(const Stage<P>& st) {
   if (st.fused()) {
-    st.tail(0);
-    for (int k = 1; k < 3; ++k) {
-      st.at(k).reconstruct();
-      st.at(k).tail(k);
+    Stage<P> d = st;
+    for (int k = 0; k < 3; ++k) {
+      d.pdl = stage_early(st.s->maxM, d.gc());
+      if (k > 0) d.at(k).reconstruct();
+      d.pdl = d.pdl && !quads_one_wave(st.s->maxM, d.gc());
+      d.at(k).tail(k);
     }
     return;
   }
@@ -1973,59 +2003,73 @@ void launch_flux(int block, int nblocks, const StageArgs<P>* t, const int2* map,
 std::mutex g_batch_tune_mu;
 std::map<std::tuple<int, int, int, int>, std::pair<int, int>> g_batch_tune;
 
-// One fused step of a batch as a graph: a chain of six kernels for every MemberTable's worth of
-// members.  The chains do not depend on one another.
+// A chain of six kernels in a graph for up to a MemberTable's worth of members of a fused batch.
+template <int NF, bool EARLY>
+afar_status add_fused_chain(cudaGraph_t graph, int device, const MemberTable<PolicyMixed>& cells,
+                            const MemberTable<PolicyMixed>& tiles, size_t smem, size_t tail_bytes) {
+  const auto recon = kp_reconstruct_tile<NF, false, EARLY>, recon_dt = kp_reconstruct_tile<NF, true, EARLY>;
+  const auto tail_1 = kp_tail<NF, true, EARLY>, tail_23 = kp_tail<NF, false, EARLY>;
+  afar_status st;
+  if ((st = raise_smem_limit(recon, device, smem))) return st;
+  if ((st = raise_smem_limit(recon_dt, device, smem))) return st;
+  if ((st = raise_smem_limit(tail_1, device, tail_bytes))) return st;
+  if ((st = raise_smem_limit(tail_23, device, tail_bytes))) return st;
+  cudaGraphEdgeData edge{};
+  if (EARLY) {
+    edge.from_port = cudaGraphKernelNodePortProgrammatic;
+    edge.type = cudaGraphDependencyTypeProgrammatic;
+  }
+  cudaGraphNode_t last = nullptr;
+  for (int k = 0; k < 3; ++k) {
+    StageCoef coef = stage_coef(k);
+    void* recon_args[] = {const_cast<MemberTable<PolicyMixed>*>(&cells), &k};
+    void* tail_args[] = {const_cast<MemberTable<PolicyMixed>*>(&tiles), &k, &coef};
+    cudaKernelNodeParams np{};
+    cudaGraphNode_t node;
+    np.func = reinterpret_cast<void*>(k == 0 ? recon_dt : recon);
+    np.gridDim = dim3(cells.first[cells.n]);
+    np.blockDim = dim3(kTile);
+    np.sharedMemBytes = (unsigned)smem;
+    np.kernelParams = recon_args;
+    AFAR_CUDA(cudaGraphAddKernelNode(&node, graph, nullptr, 0, &np));
+    if (last) AFAR_CUDA(cudaGraphAddDependencies(graph, &last, &node, &edge, 1));
+    np.func = reinterpret_cast<void*>(k == 0 ? tail_1 : tail_23);
+    np.gridDim = dim3(tiles.first[tiles.n]);
+    np.blockDim = dim3(kTailThreads);
+    np.sharedMemBytes = (unsigned)tail_bytes;
+    np.kernelParams = tail_args;
+    AFAR_CUDA(cudaGraphAddKernelNode(&last, graph, nullptr, 0, &np));
+    AFAR_CUDA(cudaGraphAddDependencies(graph, &node, &last, &edge, 1));
+  }
+  return AFAR_OK;
+}
+
+// One fused step of a batch as a graph.  The chains do not depend on one another.  Early starts (see
+// stage_early) where the members together are no more than 4000 blocks of 128 cells; us a step without / with:
+// four members of 4k quads 48 / 43, twelve of 41k triangles 296 / 292, twelve of 121k 727 / 731.
 afar_status capture_fused(afar_batch* b, const std::vector<StageArgs<PolicyMixed>>& tab, int nfmax, size_t smem,
                           size_t tail_bytes, cudaGraph_t* graph) {
   using Table = MemberTable<PolicyMixed>;
-  const bool tri = nfmax <= 3;
-  const auto recon = tri ? kp_reconstruct_tile<3, false> : kp_reconstruct_tile<4, false>;
-  const auto recon_dt = tri ? kp_reconstruct_tile<3, true> : kp_reconstruct_tile<4, true>;
-  const auto tail_1 = tri ? kp_tail<3, true> : kp_tail<4, true>;
-  const auto tail_23 = tri ? kp_tail<3, false> : kp_tail<4, false>;
-  afar_status st;
-  if ((st = raise_smem_limit(recon, b->device, smem))) return st;
-  if ((st = raise_smem_limit(recon_dt, b->device, smem))) return st;
-  if ((st = raise_smem_limit(tail_1, b->device, tail_bytes))) return st;
-  if ((st = raise_smem_limit(tail_23, b->device, tail_bytes))) return st;
-
   AFAR_CUDA(cudaGraphCreate(graph, 0));
-  auto build = [&]() -> afar_status {
-    std::unique_ptr<Table> cells(new Table), tiles(new Table);
-    for (size_t i0 = 0; i0 < tab.size(); i0 += Table::kMembers) {
-      const int n = (int)std::min<size_t>(Table::kMembers, tab.size() - i0);
-      cells->n = tiles->n = n;
-      cells->first[0] = tiles->first[0] = 0;
-      for (int i = 0; i < n; ++i) {
-        const StageArgs<PolicyMixed>& m = tab[i0 + i];
-        cells->m[i] = tiles->m[i] = m;
-        cells->first[i + 1] = cells->first[i] + grid_for(m.Nc, kTile);
-        tiles->first[i + 1] = tiles->first[i] + m.nTail;
-      }
-      cudaGraphNode_t last = nullptr;
-      for (int k = 0; k < 3; ++k) {
-        StageCoef coef = stage_coef(k);
-        void* recon_args[] = {cells.get(), &k};
-        void* tail_args[] = {tiles.get(), &k, &coef};
-        cudaKernelNodeParams np{};
-        np.func = reinterpret_cast<void*>(k == 0 ? recon_dt : recon);
-        np.gridDim = dim3(cells->first[n]);
-        np.blockDim = dim3(kTile);
-        np.sharedMemBytes = (unsigned)smem;
-        np.kernelParams = recon_args;
-        cudaGraphNode_t node;
-        AFAR_CUDA(cudaGraphAddKernelNode(&node, *graph, last ? &last : nullptr, last ? 1 : 0, &np));
-        np.func = reinterpret_cast<void*>(k == 0 ? tail_1 : tail_23);
-        np.gridDim = dim3(tiles->first[n]);
-        np.blockDim = dim3(kTailThreads);
-        np.sharedMemBytes = (unsigned)tail_bytes;
-        np.kernelParams = tail_args;
-        AFAR_CUDA(cudaGraphAddKernelNode(&last, *graph, &node, 1, &np));
-      }
+  std::unique_ptr<Table> cells(new Table), tiles(new Table);
+  long long blocks = 0;
+  for (const auto& m : tab) blocks += grid_for(m.Nc, kTile);
+  const bool early = blocks <= 4000 && !quads_one_wave(nfmax, blocks);
+  afar_status st = AFAR_OK;
+  for (size_t i0 = 0; i0 < tab.size() && !st; i0 += Table::kMembers) {
+    const int n = (int)std::min<size_t>(Table::kMembers, tab.size() - i0);
+    cells->n = tiles->n = n;
+    cells->first[0] = tiles->first[0] = 0;
+    for (int i = 0; i < n; ++i) {
+      const StageArgs<PolicyMixed>& m = tab[i0 + i];
+      cells->m[i] = tiles->m[i] = m;
+      cells->first[i + 1] = cells->first[i] + grid_for(m.Nc, kTile);
+      tiles->first[i + 1] = tiles->first[i] + m.nTail;
     }
-    return AFAR_OK;
-  };
-  st = build();
+    const auto chain = nfmax <= 3 ? (early ? add_fused_chain<3, true> : add_fused_chain<3, false>)
+                                  : (early ? add_fused_chain<4, true> : add_fused_chain<4, false>);
+    st = chain(*graph, b->device, *cells, *tiles, smem, tail_bytes);
+  }
   if (st) {
     cudaGraphDestroy(*graph);
     *graph = nullptr;

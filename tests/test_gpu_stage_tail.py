@@ -30,10 +30,10 @@ def case(name):
     return m, W, W[m.owner[m.n_internal_faces:]], CaseConfig(stencilType="edgeNeighbour", CFL=0.2)
 
 
-# quads: one cell, around one tile of 96, a remainder, either side of the change to tiles of 152 (14592 cells);
-# triangles: tiles of 192
+# quads: one cell, around one tile of 96, a remainder, either side of the change to tiles of 152 (4096 cells);
+# triangles: tiles of 192.  50,000 and 532,000 quads: the other ways its launches follow one another
 @pytest.mark.parametrize("name", [("quads", 1, 1), ("quads", 95, 1), ("quads", 12, 8), ("quads", 97, 1), ("quads", 61, 5),
-                                  ("quads", 152, 96), ("quads", 137, 107), ("triangles", 5000, 2), "corner_flow",
+                                  ("quads", 64, 64), ("quads", 241, 17), ("quads", 250, 200), ("quads", 760, 700), ("triangles", 5000, 2), "corner_flow",
                                   "ffs_tri", "mixed_riemann"], ids=str)
 def test_fused_run_is_the_separate_kernels(name):
     from afar_cudaeuler2dmixo3rk3solver_gb300 import Batch, CudaSolver, precompute
@@ -83,18 +83,18 @@ def test_fused_run_is_the_separate_kernels(name):
         s.close()
 
 
-# more members than one launch's parameters hold; cells of three and four faces together
-@pytest.mark.parametrize("members", [3, 48, 49])
-def test_fused_batch_is_the_separate_kernels(members):
+# more members than one launch's parameters hold; cells of three and four faces together; 380 to 608 blocks of quads
+@pytest.mark.parametrize("members,names", [(3, None), (48, None), (49, None), (6, [("quads", 100, 100)])], ids=str)
+def test_fused_batch_is_the_separate_kernels(members, names):
     from afar_cudaeuler2dmixo3rk3solver_gb300 import Batch, CudaSolver, precompute
 
     hfs = []
-    for name in ("ffs_tri", "mixed_riemann", ("quads", 17, 9)):
+    for name in names or ("ffs_tri", "mixed_riemann", ("quads", 17, 9)):
         m, W, Wb, cfg = case(name)
         hfs.append((precompute(m, cfg, W, Wb), cfg))
     out = []
     for schedule in ((0, 0), (128, 256)):
-        solvers = [CudaSolver(*hfs[i % 3], policy="mixed") for i in range(members)]
+        solvers = [CudaSolver(*hfs[i % len(hfs)], policy="mixed") for i in range(members)]
         batch = Batch("mixed")
         for i, s in enumerate(solvers):
             s.set_step_params(cfl=0.1 + 0.002 * i)
