@@ -53,21 +53,22 @@ __device__ __forceinline__ double undkey(const long long k) {
 }
 // Position along the Hilbert curve of order 13 over the centres' bounding square (cells of one key keep
 // the caller's order; a coordinate that is not finite counts as the smallest).
-__global__ void k_hilbert_keys(int n, const V2<double>* c, const long long* box, unsigned* key, int* id) {
+__global__ void k_hilbert_keys(int n, int bits, const V2<double>* c, const long long* box, unsigned* key, int* id) {
+  const unsigned top = (1u << bits) - 1u;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double x0 = undkey(box[0]), y0 = undkey(box[1]);
   const double ext = fmax(undkey(box[2]) - x0, undkey(box[3]) - y0);
-  const double scale = ext > 0.0 ? 8191.0 / ext : 0.0;
+  const double scale = ext > 0.0 ? (double)top / ext : 0.0;
   const double gx = (c[i].x - x0) * scale, gy = (c[i].y - y0) * scale;
-  unsigned x = gx >= 0.0 && gx <= 8191.0 ? (unsigned)gx : 0u, y = gy >= 0.0 && gy <= 8191.0 ? (unsigned)gy : 0u, d = 0;
-  for (unsigned s = 4096; s > 0; s >>= 1) {
+  unsigned x = gx >= 0.0 && gx <= (double)top ? (unsigned)gx : 0u, y = gy >= 0.0 && gy <= (double)top ? (unsigned)gy : 0u, d = 0;
+  for (unsigned s = (top + 1) >> 1; s > 0; s >>= 1) {
     const unsigned rx = (x & s) != 0, ry = (y & s) != 0;
     d += s * s * ((3 * rx) ^ ry);
     if (!ry) {
       if (rx) {
-        x = 8191 - x;
-        y = 8191 - y;
+        x = top - x;
+        y = top - y;
       }
       const unsigned t = x;
       x = y;
@@ -131,10 +132,25 @@ __global__ void __launch_bounds__(256) k_scan_apply(int n, int* a, const int* su
     run += total;
   }
 }
+// all of a short array in one block, 256 at a time
+__global__ void __launch_bounds__(256) k_scan_short(int n, int* a) {
+  int run = 0;
+  for (int k = 0; k < n; k += 256) {
+    const int i = k + threadIdx.x;
+    int total;
+    const int e = block_scan256(i < n ? a[i] : 0, &total);
+    if (i < n) a[i] = run + e;
+    run += total;
+  }
+}
 inline int scan_blocks(int n) { return (n + kScan - 1) / kScan; }
 inline void device_scan(int n, int* a, int* sums, cudaStream_t st) {  // sums: scan_blocks(n) ints
   const int b = scan_blocks(n);
   if (b == 0) return;
+  if (b == 1) {
+    k_scan_short<<<1, 256, 0, st>>>(n, a);
+    return;
+  }
   k_scan_sums<<<b, 256, 0, st>>>(n, a, sums);
   k_scan_top<<<1, 256, 0, st>>>(b, sums);
   k_scan_apply<<<b, 256, 0, st>>>(n, a, sums);
@@ -203,12 +219,17 @@ inline void hilbert_order(int n, const V2<double>* centre, int* perm, void* scra
   int* sums = cnt + 256 * (size_t)nb;
   k_box_init<<<1, 32, 0, st>>>(box);
   k_box<<<nb < 512 ? nb : 512, 256, 0, st>>>(n, centre, box);
-  k_hilbert_keys<<<(n + 255) / 256, 256, 0, st>>>(n, centre, box, key[0], id[0]);
-  for (int pass = 0; pass < 4; ++pass) {  // 26 bits
+  // A curve of 64 places or more a cell: a small mesh's set-up is a chain of launches, and every 8 bits of
+  // the key are three of them or five (1k cells: 9 launches, 23 with the 26 bits of a large mesh).
+  int bits = 4;
+  while (bits < 13 && (1ll << (2 * bits)) < 64ll * n) ++bits;
+  const int passes = (2 * bits + 7) / 8;
+  k_hilbert_keys<<<(n + 255) / 256, 256, 0, st>>>(n, bits, centre, box, key[0], id[0]);
+  for (int pass = 0; pass < passes; ++pass) {
     const int a = pass & 1, b = a ^ 1;
     k_sort_count<<<nb, 256, 0, st>>>(n, key[a], 8 * pass, cnt);
     device_scan(256 * nb, cnt, sums, st);
-    k_sort_scatter<<<nb, 256, 0, st>>>(n, key[a], id[a], 8 * pass, cnt, key[b], pass == 3 ? perm : id[b]);
+    k_sort_scatter<<<nb, 256, 0, st>>>(n, key[a], id[a], 8 * pass, cnt, key[b], pass == passes - 1 ? perm : id[b]);
   }
 }
 
