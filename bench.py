@@ -39,18 +39,19 @@ PEAKS_FILE = os.path.join(ROOT, "MEASURED_PEAKS.json")
 FALLBACK_HBM_GBS = 6800.0
 PROFILE_STEPS = 10
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one mixed-policy reconstruct launch
-# (tile-staged) per cell, by cell order, from ncu captures of the 500,094-cell version of this
-# workload (traffic grows with the cells of the tile stream); None when no capture matches the
-# current kernels (the tensor-map fetch; Hilbert order not captured with it).
-RECON_TRAFFIC_BYTES_PER_CELL = {"rcm": 398.2, "hilbert": None}
+# (tile-staged) per cell, the mean of a step's three (the first also reads the faces for the Courant
+# step: 433 and twice 395), from ncu captures of the 500,094-cell version of this workload (traffic
+# grows with the cells of the tile stream).  The kernels run in a device order of their own, whatever
+# the mesh's.
+RECON_TRAFFIC_BYTES_PER_CELL = {"rcm": 407.7, "hilbert": 407.7}
 # FP64 work per internal face of the fp64 policy's flux, averaged over a step's three launches (the
 # first also reduces the Courant step), from the ncu instruction counts
 # smsp__sass_thread_inst_executed_op_{dfma,dadd,dmul}_pred_on.sum of the three launches on the
 # 500,094-cell version of this workload (748,881 internal faces): instructions (DFMA + DADD + DMUL,
 # divisions and square roots counted as the DFMA sequences they run as) and floating-point
 # operations (2 per DFMA).  The FP64 pipe issues one such instruction per lane per cycle at its peak.
-FP64_FLUX_INST_PER_FACE = 243.77
-FP64_FLUX_FLOPS_PER_FACE = 360.17
+FP64_FLUX_INST_PER_FACE = 148.8
+FP64_FLUX_FLOPS_PER_FACE = 199.8
 
 
 def parse():
