@@ -2003,10 +2003,12 @@ void launch_flux(int block, int nblocks, const StageArgs<P>* t, const int2* map,
 std::mutex g_batch_tune_mu;
 std::map<std::tuple<int, int, int, int>, std::pair<int, int>> g_batch_tune;
 
-// A chain of six kernels in a graph for up to a MemberTable's worth of members of a fused batch.
+// A chain of six kernels in a graph for up to a MemberTable's worth of members of a fused batch, after *end
+// if that is a node; *end is its last kernel then.
 template <int NF, bool EARLY>
 afar_status add_fused_chain(cudaGraph_t graph, int device, const MemberTable<PolicyMixed>& cells,
-                            const MemberTable<PolicyMixed>& tiles, size_t smem, size_t tail_bytes) {
+                            const MemberTable<PolicyMixed>& tiles, size_t smem, size_t tail_bytes,
+                            cudaGraphNode_t* end) {
   const auto recon = kp_reconstruct_tile<NF, false, EARLY>, recon_dt = kp_reconstruct_tile<NF, true, EARLY>;
   const auto tail_1 = kp_tail<NF, true, EARLY>, tail_23 = kp_tail<NF, false, EARLY>;
   afar_status st;
@@ -2019,7 +2021,7 @@ afar_status add_fused_chain(cudaGraph_t graph, int device, const MemberTable<Pol
     edge.from_port = cudaGraphKernelNodePortProgrammatic;
     edge.type = cudaGraphDependencyTypeProgrammatic;
   }
-  cudaGraphNode_t last = nullptr;
+  cudaGraphNode_t last = *end;
   for (int k = 0; k < 3; ++k) {
     StageCoef coef = stage_coef(k);
     void* recon_args[] = {const_cast<MemberTable<PolicyMixed>*>(&cells), &k};
@@ -2041,10 +2043,13 @@ afar_status add_fused_chain(cudaGraph_t graph, int device, const MemberTable<Pol
     AFAR_CUDA(cudaGraphAddKernelNode(&last, graph, nullptr, 0, &np));
     AFAR_CUDA(cudaGraphAddDependencies(graph, &node, &last, &edge, 1));
   }
+  *end = last;
   return AFAR_OK;
 }
 
-// One fused step of a batch as a graph.  The chains do not depend on one another.  Early starts (see
+// One fused step of a batch as a graph.  The chains work on different members: side by side they fill the
+// GPU where one is less than a wave, one after another they leave it to one kernel at a time (256 ramps of
+// 5k to 200k quads: 8.93 ms a step side by side, 8.49 in turn, 8.59 as separate kernels).  Early starts (see
 // stage_early) where the members together are no more than 4000 blocks of 128 cells; us a step without / with:
 // four members of 4k quads 48 / 43, twelve of 41k triangles 296 / 292, twelve of 121k 727 / 731.
 afar_status capture_fused(afar_batch* b, const std::vector<StageArgs<PolicyMixed>>& tab, int nfmax, size_t smem,
@@ -2056,6 +2061,7 @@ afar_status capture_fused(afar_batch* b, const std::vector<StageArgs<PolicyMixed
   for (const auto& m : tab) blocks += grid_for(m.Nc, kTile);
   const bool early = blocks <= 4000 && !quads_one_wave(nfmax, blocks);
   afar_status st = AFAR_OK;
+  cudaGraphNode_t end = nullptr;
   for (size_t i0 = 0; i0 < tab.size() && !st; i0 += Table::kMembers) {
     const int n = (int)std::min<size_t>(Table::kMembers, tab.size() - i0);
     cells->n = tiles->n = n;
@@ -2068,7 +2074,8 @@ afar_status capture_fused(afar_batch* b, const std::vector<StageArgs<PolicyMixed
     }
     const auto chain = nfmax <= 3 ? (early ? add_fused_chain<3, true> : add_fused_chain<3, false>)
                                   : (early ? add_fused_chain<4, true> : add_fused_chain<4, false>);
-    st = chain(*graph, b->device, *cells, *tiles, smem, tail_bytes);
+    if (cells->first[n] <= 4 * 152) end = nullptr;
+    st = chain(*graph, b->device, *cells, *tiles, smem, tail_bytes, &end);
   }
   if (st) {
     cudaGraphDestroy(*graph);
