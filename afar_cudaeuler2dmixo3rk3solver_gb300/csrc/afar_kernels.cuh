@@ -106,9 +106,8 @@ struct StageArgs {
   float Rf, Cvf, gRf;  // R, Cv and gamma*R as floats (mixed)
   double px, py;       // periods of a periodic mesh (0: none); setup kernels only
   const V2<float>* dtgf;  // Nf (delta r, fraction) as floats (mixed Courant estimate)
-  // the optional multi-point face flux (ng > 0 points per face; 0: the face-centre flux)
   // mixed: the fused stage tail (tail_body)
-  const struct TailTile* tail;   // the tiles of 192 cells
+  const struct TailTile* tail;   // its tiles of tailT cells
   const int* thalo;              // [tile][kTailHalo] the cells across each tile's border
   const int* thcode;             // [tile][4][kTailHalo] the faces of their slots (see tail_body)
   const V2<typename P::G>* thsg; // [tile][4][kTailHalo] and sg of each
@@ -118,6 +117,7 @@ struct StageArgs {
   unsigned* wflag;               // a bit for each cell: troubled (written by the reconstruct)
   V4<typename P::W>* W3[3];      // the state's buffers: W, and the outputs of the first two stages
   int nTail, tailT;              // its tiles and the cells of one
+  // the optional multi-point face flux (ng > 0 points per face; 0: the face-centre flux)
   int ng;
   const S* wg;       // [(maxM*ng)*(maxS+1)][ldc] O3 weights at the face Gauss points, per cell slot
   const V2<G>* sgk;  // [maxM*ng][ldc] point minus cell centre, per cell slot
