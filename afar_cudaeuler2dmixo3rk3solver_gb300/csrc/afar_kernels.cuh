@@ -17,6 +17,7 @@
 #pragma once
 
 #include "afar_policy.cuh"
+#include "afar_tail_layout.h"
 
 namespace afar {
 
@@ -2216,8 +2217,6 @@ __device__ __forceinline__ void finish_one(StepCtl* ctl) {
 // 65k quads 66 / 52, 500k triangles 380 / 345, 2.0M triangles 1165 / 1026, 4.0M quads 2460 / 2297
 // (the tail itself 437 us a step at 2.0M triangles: 1.5 TB/s; its blocks wait, on the halo's gathers and at
 // their two barriers).
-constexpr int kTailThreads = 256, kTailBlocks = 4;
-constexpr int kTailHalo = 128, kTailExtra = 192, kTailList = 32;  // most of each that a tile may have
 struct TailTile {
   int fstart;  // the tile's own faces are fstart .. fstart + nOwn - 1
   int nOwn;
@@ -2292,8 +2291,9 @@ __device__ __forceinline__ void tail_body(const StageArgs<PolicyMixed>& a, const
     nM = a.nM[c];
     nS = a.nS[c];
   } else {
-    c = a.thalo[(size_t)blk * kTailHalo + (tid - T)];
-    load_slots(tid - T);
+    const int h = tail_first_halo(tid, T);
+    c = a.thalo[(size_t)blk * kTailHalo + h];
+    load_slots(h);
   }
   pdl_wait<EARLY>();
   if (own0) load_cell();
