@@ -2246,9 +2246,8 @@ __host__ __device__ inline TailSmem tail_smem(const int nf, const int cells) {
 constexpr int kNoFace = -1, kWall = -2, kElsewhere = 0x10000;
 
 template <int NF, bool E, bool EARLY = true>
-__device__ __forceinline__ void tail_body(const StageArgs<PolicyMixed>& a, const V4<float>* __restrict__ Win,
-                                          V4<float>* __restrict__ Wout, const int blk, const StageCoef& k,
-                                          unsigned char* sm) {
+__device__ __forceinline__ void tail_body(const StageArgs<PolicyMixed>& a, const V4<float>* Win, V4<float>* Wout,
+                                          const int blk, const StageCoef& k, unsigned char* sm) {
   __shared__ int s_go, s_extra[kTailExtra];
   __shared__ float s_bdt;
   const int tid = threadIdx.x, ldc = a.ldc;
