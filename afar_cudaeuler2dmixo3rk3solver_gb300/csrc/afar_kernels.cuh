@@ -460,12 +460,14 @@ __device__ __forceinline__ void recon_reg_body(const StageArgs<P>& a, const V4<t
 // stencil gathers, which hit L2.  One load per array rather than one per row: the fetch was bound
 // by the number of copies issued, not by their bytes.
 constexpr int kTile = 128;
-// Test hooks of the tile's bounded waits (afar_debug_wait_injection): the wait limit in SM clocks,
-// and bytes added to the transaction count the first barrier of every tile expects (never issued,
-// so that barrier cannot complete and its wait runs out).  2^31 clocks and no extra bytes in normal
-// operation.
+// Test hooks of the tiles' bounded waits (afar_debug_wait_injection_at): the wait limit in SM clocks,
+// and bytes added to the transaction count that a barrier of every tile expects (never issued, so
+// that barrier cannot complete and its wait runs out): x, y of the reconstruct's two, z, w of the
+// stage tail's.  g_tail_late_tx: bytes that the tail counts as arrived once its first wait has run out,
+// as a copy does that lands after it.  2^31 clocks and no bytes in normal operation.
 static __device__ long long g_tile_wait_limit = 1ll << 31;
-static __device__ unsigned g_tile_extra_tx = 0;
+static __device__ uint4 g_tile_extra_tx = {0, 0, 0, 0};
+static __device__ unsigned g_tail_late_tx = 0;
 // Tensor maps of the mixed policy's slot-major operator rows, one tiled TMA load per array and
 // tile: face ids [maxM][ldc] and the LS / face-geometry rows (float pairs, as 2 ldc floats), boxes
 // of 128 cells x maxM rows; stencil ids, a box of 128 cells x S rows for each stencil size S; O3
@@ -536,8 +538,8 @@ __device__ __forceinline__ void recon_tile_fetch(const StageArgs<P>& a, const V4
   const TileMaps* tm = a.tmaps;
   if (lane == 0) {
     const unsigned nw = (unsigned)min(kTile, a.Nc - c0);  // cells of the tile
-    mbar_arrive_expect_tx(bar, kTile * 4 * (M + S) + nw * 16 + g_tile_extra_tx);
-    mbar_arrive_expect_tx(bar + 1, kTile * 8 * 3 * M + kTile * 4 * S * M);
+    mbar_arrive_expect_tx(bar, kTile * 4 * (M + S) + nw * 16 + g_tile_extra_tx.x);
+    mbar_arrive_expect_tx(bar + 1, kTile * 8 * 3 * M + kTile * 4 * S * M + g_tile_extra_tx.y);
   }
   __syncwarp();
   switch (lane) {
@@ -2259,6 +2261,8 @@ __device__ __forceinline__ void tail_body(const StageArgs<PolicyMixed>& a, const
   const int4 hdr = reinterpret_cast<const int4*>(a.tail)[blk];
   const int xid = tid < kTailExtra ? a.textra[(size_t)blk * kTailExtra + tid] : 0;
   const int reach = tid < kTailList ? a.tlist[(size_t)blk * kTailList + tid] : 0;
+  uint2 extra_tx{0, 0};  // a test's (see g_tile_extra_tx)
+  if (tid == 0) extra_tx = reinterpret_cast<const uint2*>(&g_tile_extra_tx)[1];
   int c = c0 + (own0 && tid < nc ? tid : 0), nM = 0, nS = 0;
   int lf[NF];
   V2<float> d[NF];
@@ -2310,12 +2314,12 @@ __device__ __forceinline__ void tail_body(const StageArgs<PolicyMixed>& a, const
   if (tid == 0) {
     mbar_init(bar, 1);
     mbar_init(bar + 1, 1);
-    mbar_arrive_expect_tx(bar, (unsigned)nOwn * 48u);
+    mbar_arrive_expect_tx(bar, (unsigned)nOwn * 48u + extra_tx.x);
     if (nOwn) {
       bulk_to_smem(st, a.fv + 2 * (size_t)fstart, (unsigned)nOwn * 32u, bar);
       bulk_to_smem(sfs, a.fs + fstart, (unsigned)nOwn * 16u, bar);
     }
-    mbar_arrive_expect_tx(bar + 1, (unsigned)nc * (k.first ? 32u : 64u));
+    mbar_arrive_expect_tx(bar + 1, (unsigned)nc * (k.first ? 32u : 64u) + extra_tx.y);
     bulk_to_smem(sm + S.u0, a.U0 + c0, (unsigned)nc * 32u, bar + 1);
     if (!k.first) bulk_to_smem(sm + S.u, a.U + c0, (unsigned)nc * 32u, bar + 1);
   }
@@ -2370,7 +2374,13 @@ __device__ __forceinline__ void tail_body(const StageArgs<PolicyMixed>& a, const
     s_go = gt_zero(dt);
     s_bdt = (float)(k.b3 * dt);
   }
-  if (tid == 0 && !mbar_wait_bounded(bar, 0, limit)) near = 1;  // one thread polls, the block's barrier tells
+  // One thread polls, the block's barriers tell.  A wait that runs out marks the step invalid at once, since the
+  // copy may land before the next barrier; where it has not by then, the block leaves there.
+  if (tid == 0 && !mbar_wait_bounded(bar, 0, limit)) {
+    near = 1;
+    atomicOr(&a.ctl->err, 1u);
+    if (g_tail_late_tx) mbar_complete_tx(bar, g_tail_late_tx);
+  }
   near = __syncthreads_or(near);
   int lfs[NF];  // of this thread's own cell: local face of each slot, bit 15: the neighbour side; -1: none
 #pragma unroll

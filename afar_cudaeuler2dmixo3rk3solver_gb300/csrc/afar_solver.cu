@@ -2419,9 +2419,20 @@ extern "C" afar_status afar_batch_get_schedule(afar_batch* b, int* tileMembers, 
 }
 
 extern "C" afar_status afar_debug_wait_injection(int device, unsigned extraBytes, long long limitClocks) {
+  return afar_debug_wait_injection_at(device, AFAR_WAIT_RECONSTRUCT_IDS, extraBytes, 0, limitClocks);
+}
+
+extern "C" afar_status afar_debug_wait_injection_at(int device, int where, unsigned extraBytes, int late,
+                                                    long long limitClocks) {
+  if (where < AFAR_WAIT_RECONSTRUCT_IDS || where > AFAR_WAIT_TAIL_STATES || (late && where != AFAR_WAIT_TAIL_FACES))
+    return (set_error("afar_debug_wait_injection_at: unknown wait %d, or late at another than the tail's first", where),
+            AFAR_ERR_ARGUMENT);
   AFAR_CUDA(cudaSetDevice(device));
   const long long lim = limitClocks > 0 ? limitClocks : (1ll << 31);
-  AFAR_CUDA(cudaMemcpyToSymbol(g_tile_extra_tx, &extraBytes, sizeof(extraBytes)));
+  unsigned extra[4] = {0, 0, 0, 0}, lateBytes = late ? extraBytes : 0;
+  extra[where] = extraBytes;
+  AFAR_CUDA(cudaMemcpyToSymbol(g_tile_extra_tx, extra, sizeof(extra)));
+  AFAR_CUDA(cudaMemcpyToSymbol(g_tail_late_tx, &lateBytes, sizeof(lateBytes)));
   AFAR_CUDA(cudaMemcpyToSymbol(g_tile_wait_limit, &lim, sizeof(lim)));
   AFAR_CUDA(cudaDeviceSynchronize());
   return AFAR_OK;

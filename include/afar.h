@@ -503,6 +503,16 @@ afar_status afar_measure_fp64_peak(int device, double* gflops, float* ms);
  * operation.  Affects every solver and batch on the device until then. */
 afar_status afar_debug_wait_injection(int device, unsigned extraBytes, long long limitClocks);
 
+/* The same at one of the mixed policy's waits: the reconstruct's for its ids and states (the one above)
+ * and for its operator rows, the fused stage tail's for its faces and for its conserved states.  late != 0
+ * (AFAR_WAIT_TAIL_FACES only): once that wait has run out, the bytes are counted as arrived, as those
+ * of a copy that lands just after.  The call that meets the wait reports AFAR_ERR_CUDA either way. */
+#define AFAR_WAIT_RECONSTRUCT_IDS 0
+#define AFAR_WAIT_RECONSTRUCT_ROWS 1
+#define AFAR_WAIT_TAIL_FACES 2
+#define AFAR_WAIT_TAIL_STATES 3
+afar_status afar_debug_wait_injection_at(int device, int where, unsigned extraBytes, int late, long long limitClocks);
+
 /* The multi-point face flux (no counterpart in the reference, whose flux uses the face centre; off
  * by default since it changes results).  After afar_setDeviceFieldDataStencil, policies fp64 and
  * mixed: the flux of every internal face becomes the weighted sum of the fluxes at its nPoints (1-4)
