@@ -582,13 +582,14 @@ __device__ __forceinline__ void recon_tile_body(const StageArgs<P>& a, const V4<
   const int nS = c < a.Nc ? a.nS[c] : 0, nM = c < a.Nc ? a.nM[c] : 0;
   pdl_wait<EARLY>();
   const long long limit = g_tile_wait_limit;
-  // leaving: every copy into this block's shared memory must have landed first
+  // Leaving: every copy into this block's shared memory must have landed first.  The lanes of a warp leave
+  // together, though each polls by its own clock: those that stay meet again below (courant_min, put_troubled).
   auto give_up = [&]() {
     if (t == 0) atomicOr(&a.ctl->err, 1u);
     mbar_wait_bounded(bar, 0, limit);
     mbar_wait_bounded(bar + 1, 0, limit);
   };
-  if (!mbar_wait_bounded(bar, 0, limit)) return give_up();
+  if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar, 0, limit))) return give_up();
   if (c >= a.Nc) {
     if (!mbar_wait_bounded(bar + 1, 0, limit)) give_up();
     return;
@@ -618,7 +619,7 @@ __device__ __forceinline__ void recon_tile_body(const StageArgs<P>& a, const V4<
     if (u < nS) wj[u] = W[s_sten[u * kTile + t]];
   CourantFaces<NF> cour;
   if constexpr (DT) courant_load<NF>(cour, a, fid, inner);
-  if (!mbar_wait_bounded(bar + 1, 0, limit)) return give_up();
+  if (!__all_sync(cell_lanes(c, a.Nc), mbar_wait_bounded(bar + 1, 0, limit))) return give_up();
   if constexpr (DT) courant_min<NF>(cour, a, c, fid, inner, wc, wj);
   // O3 weights of boundary-face and missing slots are zero in the operator rows (setup), so only
   // slots past this mesh's largest cell (a batch may stage fewer rows than NF) are skipped
