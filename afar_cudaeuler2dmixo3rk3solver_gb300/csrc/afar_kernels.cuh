@@ -579,19 +579,21 @@ __device__ __forceinline__ void recon_tile_body(const StageArgs<P>& a, const V4<
   __syncthreads();
   if (t < 32) recon_tile_fetch<EARLY>(a, W, blk, L, sm, bar);
   const int c = blk * kTile + t;
-  const int nS = c < a.Nc ? a.nS[c] : 0, nM = c < a.Nc ? a.nM[c] : 0;
+  int nS = c < a.Nc ? a.nS[c] : 0, nM = c < a.Nc ? a.nM[c] : 0;
   pdl_wait<EARLY>();
   const long long limit = g_tile_wait_limit;
-  // Leaving: every copy into this block's shared memory must have landed first.  The lanes of a warp leave
-  // together, though each polls by its own clock: those that stay meet again below (courant_min, put_troubled).
-  auto give_up = [&]() {
-    if (t == 0) atomicOr(&a.ctl->err, 1u);
-    mbar_wait_bounded(bar, 0, limit);
-    mbar_wait_bounded(bar + 1, 0, limit);
+  // A lane whose wait runs out (each polls by its own clock) marks the step invalid, waits once more, since every
+  // copy into the block's shared memory must have landed before the block ends, and goes on with the others of its
+  // warp, whom it meets below (courant_min, put_troubled): without stencil and faces where the lists are still
+  // missing, so that it follows no index that is not one.
+  auto arrived = [&](unsigned long long* b) {
+    if (mbar_wait_bounded(b, 0, limit)) return true;
+    atomicOr(&a.ctl->err, 1u);
+    return mbar_wait_bounded(b, 0, limit);
   };
-  if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar, 0, limit))) return give_up();
+  if (!arrived(bar)) nS = nM = 0;
   if (c >= a.Nc) {
-    if (!mbar_wait_bounded(bar + 1, 0, limit)) give_up();
+    arrived(bar + 1);
     return;
   }
   const int* s_cf = reinterpret_cast<const int*>(sm + L.off_cf);
@@ -619,7 +621,7 @@ __device__ __forceinline__ void recon_tile_body(const StageArgs<P>& a, const V4<
     if (u < nS) wj[u] = W[s_sten[u * kTile + t]];
   CourantFaces<NF> cour;
   if constexpr (DT) courant_load<NF>(cour, a, fid, inner);
-  if (!__all_sync(cell_lanes(c, a.Nc), mbar_wait_bounded(bar + 1, 0, limit))) return give_up();
+  arrived(bar + 1);
   if constexpr (DT) courant_min<NF>(cour, a, c, fid, inner, wc, wj);
   // O3 weights of boundary-face and missing slots are zero in the operator rows (setup), so only
   // slots past this mesh's largest cell (a batch may stage fewer rows than NF) are skipped
