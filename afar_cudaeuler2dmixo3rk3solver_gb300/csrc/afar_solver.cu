@@ -635,7 +635,8 @@ void enqueue_tail(const Stage<P>& st) {
 }
 
 // What the separate BVD kernel leaves behind, after a fused stage: for the accessors of the limiter and
-// of the switch types.  A pending head no longer fits its tail then (the tail transforms the limiter).
+// of the switch types, and before anything replaces what it reads (a head's state, a stage's limiter, face
+// values and flags).  A pending head no longer fits its tail then (the tail transforms the limiter).
 afar_status settle_bvd(afar_solver* s) {
   if (s->bvd_pending < 0) return AFAR_OK;
   Stage<PolicyMixed> st;
@@ -824,6 +825,9 @@ static afar_status put_state(afar_solver* s, const afar_basicFieldData* FD, cons
                       const afar_conservedFieldData* cFDold) {
   const size_t Nc = s->Nc, Nb = s->Nb;
   const bool mixed = s->policy == AFAR_POLICY_MIXED;
+  if (FD && s->bvd_pending == 0) {  // (a later stage's state is in a buffer of its own)
+    if (afar_status st = settle_bvd(s)) return st;
+  }
   if (FD) {
     if (mixed) {
       AFAR_CUDA(cudaMemcpyAsync(s->xfer, FD, sizeof(V4<double>) * (Nc + Nb), cudaMemcpyHostToDevice, s->stream));
@@ -980,8 +984,8 @@ static afar_status tune_reconstruct(afar_solver* s) {
     }
   }
   Stage<PolicyMixed> sg;
-  afar_status st = make_stage<PolicyMixed>(s, false, &sg);
-  if (st) return st;
+  afar_status st = settle_bvd(s);
+  if (st || (st = make_stage<PolicyMixed>(s, false, &sg))) return st;
   cudaEvent_t e0, e1;
   AFAR_CUDA(cudaEventCreate(&e0));
   AFAR_CUDA(cudaEventCreate(&e1));
@@ -1783,6 +1787,9 @@ extern "C" afar_status afar_state_snapshot(afar_solver* s, int op) {
     if (st) return st;
   }
   if (!s->snap) return (set_error("restore without a saved snapshot"), AFAR_ERR_STATE);
+  if (op == AFAR_SNAPSHOT_RESTORE && s->bvd_pending == 0) {  // as in put_state
+    if (afar_status st = settle_bvd(s)) return st;
+  }
   char* p = static_cast<char*>(s->snap);
   void* dst[4] = {p, p + wb, p + wb + ub, p + wb + 2 * ub};
   void* src[4] = {s->W, s->U, s->U0, s->ctl};
@@ -2214,6 +2221,8 @@ afar_status batch_build(afar_batch* b) {
     // reconstruct once so that the BVD and flux read this step's intermediates, then time each
     // candidate: a warm-up and the best of three launches (both kernels are functions of the state
     // and the stage's intermediates; they change neither the state nor the step control)
+    for (afar_solver* m : b->members)
+      if ((st = settle_bvd(m))) return st;
     reconstruct();
     cudaEvent_t e0, e1;
     AFAR_CUDA(cudaEventCreate(&e0));
