@@ -1403,13 +1403,15 @@ extern "C" afar_status afar_adjustTimeStep(afar_solver* s, int facesNum, double 
     if ((st = ensure_graph(s, kGraphHead)) || (st = ensure_graph(s, kGraphTail))) return st;
     {
       k_set_ctl<<<1, 32, 0, s->stream>>>(s->ctl, 0.0, CFL, 0.0);
-      AFAR_CUDA(cudaMemcpyAsync(&s->ctl->dt_bits, &init, sizeof(init), cudaMemcpyHostToDevice, s->stream));
       AFAR_CUDA(cudaGraphLaunch(s->graph_head, s->stream));
       s->bvd_pending = fused_step(s) ? 0 : -1;
       StepCtl c;
       AFAR_CUDA(cudaMemcpyAsync(&c, s->ctl, sizeof(c), cudaMemcpyDeviceToHost, s->stream));
       AFAR_CUDA(cudaStreamSynchronize(s->stream));
       AFAR_CUDA(cudaGetLastError());
+      // the minimum is armed again at once, as at the end of a step: whichever step follows starts anew (the
+      // tail has its step size from the caller)
+      AFAR_CUDA(cudaMemcpyAsync(&s->ctl->dt_bits, &init, sizeof(init), cudaMemcpyHostToDevice, s->stream));
       if (c.err) {  // a bounded device wait gave up, in this head or in the step before it
         AFAR_CUDA(cudaMemsetAsync(&s->ctl->err, 0, sizeof(c.err), s->stream));
         AFAR_CUDA(cudaStreamSynchronize(s->stream));
