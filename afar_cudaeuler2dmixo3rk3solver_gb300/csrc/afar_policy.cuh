@@ -216,7 +216,7 @@ __device__ __forceinline__ double half64(const double x) {
 }
 // c1*a + c2*b of two conditions, one true: the chosen one, as the sum leaves it (a negative zero stays
 // one only next to a negative operand); anything not finite takes the sum.
-__device__ __noinline__ double blend64_sum(const bool c1, const bool c2, const double a, const double b) {
+static __device__ __noinline__ double blend64_sum(const bool c1, const bool c2, const double a, const double b) {
   return __dadd_rn(__dmul_rn((double)c1, a), __dmul_rn((double)c2, b));
 }
 __device__ __forceinline__ double blend64(const bool c1, const bool c2, const double a, const double b) {

@@ -513,6 +513,24 @@ afar_status afar_debug_wait_injection(int device, unsigned extraBytes, long long
 #define AFAR_WAIT_TAIL_STATES 3
 afar_status afar_debug_wait_injection_at(int device, int where, unsigned extraBytes, int late, long long limitClocks);
 
+/* Test hook: one of the functions by which the kernels do FP64 arithmetic off the FP64 pipe, over n pairs
+ * (a, b) of host arrays: 1/a, 1/sqrt(a), a/b, a as a float, (float)a as a double, a/2, the first or the second
+ * of a blend, fmax, fmin, a as a float to 20 bits, and the bits (a > 0) + 2 (a <= 0) + 4 (|a| < b) +
+ * 8 (|a| >= b) + 16 (a is not a number). */
+#define AFAR_ARITH_RCP 0
+#define AFAR_ARITH_RSQRT 1
+#define AFAR_ARITH_DIV 2
+#define AFAR_ARITH_TO_FLOAT 3
+#define AFAR_ARITH_TO_DOUBLE 4
+#define AFAR_ARITH_HALF 5
+#define AFAR_ARITH_BLEND_FIRST 6
+#define AFAR_ARITH_BLEND_SECOND 7
+#define AFAR_ARITH_MAX 8
+#define AFAR_ARITH_MIN 9
+#define AFAR_ARITH_TOP_FLOAT 10
+#define AFAR_ARITH_COMPARE 11
+afar_status afar_debug_arithmetic(int device, int op, int n, const double* a, const double* b, double* out);
+
 /* The multi-point face flux (no counterpart in the reference, whose flux uses the face centre; off
  * by default since it changes results).  After afar_setDeviceFieldDataStencil, policies fp64 and
  * mixed: the flux of every internal face becomes the weighted sum of the fluxes at its nPoints (1-4)
