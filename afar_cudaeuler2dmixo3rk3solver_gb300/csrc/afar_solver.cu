@@ -2149,9 +2149,11 @@ afar_status batch_build(afar_batch* b) {
   }
 
   std::vector<int2> mp_tile, mp_reg, mp_cell;
-  batch_map(b->members, kTile, false, &is_tile, mp_tile);
-  batch_map(b->members, kTile, false, &is_reg, mp_reg);
-  batch_map(b->members, kCellBlock, false, nullptr, mp_cell);
+  if (!fused) {  // (the fused stage finds its members from its own arguments)
+    batch_map(b->members, kTile, false, &is_tile, mp_tile);
+    batch_map(b->members, kTile, false, &is_reg, mp_reg);
+    batch_map(b->members, kCellBlock, false, nullptr, mp_cell);
+  }
   // candidate maps for the timing: BVD in 64/128/256-cell blocks, flux in 128/256-face blocks
   const int bvd_sizes[3] = {64, 128, 256}, flux_sizes[2] = {128, 256};
   std::vector<int2> mp_bvd[3], mp_face[2];
@@ -2183,7 +2185,7 @@ afar_status batch_build(afar_batch* b) {
   if ((st = grow(&b->tab, &b->tab_bytes, std::max<size_t>(1, tab.size()) * sizeof(StageArgs<P>)))) return st;
   if ((st = grow(reinterpret_cast<void**>(&b->maps), &cap_m, std::max<size_t>(1, all.size()) * sizeof(int2)))) return st;
   b->maps_n = cap_m / sizeof(int2);
-  if (!tab.empty()) {
+  if (!tab.empty() && !fused) {
     AFAR_CUDA(cudaMemcpyAsync(b->tab, tab.data(), tab.size() * sizeof(StageArgs<P>), cudaMemcpyHostToDevice, b->stream));
     AFAR_CUDA(cudaMemcpyAsync(b->maps, all.data(), all.size() * sizeof(int2), cudaMemcpyHostToDevice, b->stream));
   }
