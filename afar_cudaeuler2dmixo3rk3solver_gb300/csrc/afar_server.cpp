@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "afar_internal.h"
+#include "afar_tail_layout.h"
 
 namespace {
 
@@ -51,7 +52,7 @@ size_t estimate_bytes(const afar_fieldSizes& z, int policy) {
                           snapshot + res_dump + staging;
   const double per_face = 8 * g + 4 * g + 48 + 16 + 8;
   if (policy == AFAR_POLICY_MIXED) {  // the device order, two further state buffers, the fused stage's lists
-    const double tile = m <= 3 ? 192 : nc <= 4096 ? 96 : 152;
+    const double tile = afar::tail_tile_cells(z.maxCompactStencilSize, z.cellsNum);
     return (size_t)(nc * (per_cell + 8 + 8 * g + 2 * m + 7600 / tile) + (nf + nb) * (per_face + 8) + nb * (48 + 8 * g) +
                     (64u << 20));
   }

@@ -49,6 +49,7 @@ namespace {
 constexpr int kCellBlock = 128;
 constexpr size_t kMaxDynamicSmem = 227 * 1024;  // per CTA on sm_103a
 constexpr int kFaceBlock = 256;
+constexpr int kSMs = 152;  // GB300
 constexpr int kFaceBlock64 = 128;  // ref and fp64: smaller blocks, an evener last wave over the SMs' FP64 pipes
 // GPUevolve.cu:223-225: the reference's truncated SSP-RK3 coefficients
 constexpr double kBeta1[3] = {1.0, 0.75, 0.333333};
@@ -380,8 +381,10 @@ void reorder(afar_solver* s, T* a, size_t n) {
 // Cells of a tile of the fused stage tail: as many as its 256 threads take with the halo in one pass (192
 // triangles, 152 quads), fewer quads where a mesh is a few blocks and a block's time is the kernel's.  us a
 // step at 96 / 152 / 192 cells: triangles 1.1k 41 / 43 / 41, 99k 72 / 73 / 68, 998k 588 / 512 / 497; quads 1.0k 42 / 45 / 58,
-// 10k 46.5 / 47.2 / 61, 66k 70 / 62 / 72, 1.0M 670 / 584 / 631; six members of 10k quads in a batch 73 / 65.
-int tail_cells(const afar_solver* s) { return s->maxM <= 3 ? 192 : s->Nc <= 4096 ? 96 : 152; }
+// 10k 46.5 / 47.2 / 61, 66k 70 / 62 / 72, 1.0M 670 / 584 / 631.  The line is where batches of such meshes begin to
+// lose: 96 / 152 cells, 4096 quads alone 32.8 / 33.0, six, twelve and 24 members 40.7 / 41.0, 51.2 / 52.4, 85.8 / 84.0; 5041
+// alone 32.8 / 34.8, six and twelve members 42.8 / 44.3, 66.4 / 55.3; 10k alone 33.4 / 34.8, six members 65.3 / 54.7.
+int tail_cells(const afar_solver* s) { return tail_tile_cells(s->maxM, s->Nc); }
 
 template <class P>
 StageArgs<P> make_args(afar_solver* s) {
@@ -483,9 +486,8 @@ afar_status raise_smem_limit(K kernel, int device, size_t bytes) {
 template <class P>
 int block_for(long long n, int full) {
   if constexpr (P::id == PolicyMixed::id) return full;
-  constexpr long long kSMs = 152;
   int b = full;
-  while (b > 32 && n < 8 * kSMs * b) b /= 2;
+  while (b > 32 && n < 8ll * kSMs * b) b /= 2;
   return b;
 }
 
@@ -505,13 +507,18 @@ inline bool fused_step(const afar_solver* s) { return s->fused && s->ng == 0; }
 // kernel and runs the reference-layout flux; fp64 reconstructs staged, mixed in registers.
 // The fused stage's kernels start before the one ahead is complete (pdl_next near its end): their
 // barriers, lists and operator rows are on the way when its results are there.  us a step, without / with:
-// 1k quads 43.6 / 39.2, 10k 47 / 41, 250k 191 / 186; 10k triangles 46 / 40, 202k 130 / 121, 2.0M 946 / 937.  (Saying
-// pdl_next first thing: 4.0M quads 2308, 2.0M triangles 1003: the next kernel's waiting blocks take the places
-// of blocks that have work.)  Not meshes of many quads (4.0M 2167 / 2164), and not the tail where a quad mesh's
-// reconstruct is one wave of 2.5 to 4 blocks a SM: its blocks crowd where that ends first (65k quads 62.7 with
-// both early, 59.5 with the reconstruct alone; 48k 55.6 against 55.5 and 78k 67.6 against 70.5 on either side).
-inline bool quads_one_wave(int maxM, long long reconBlocks) { return maxM > 3 && reconBlocks > 380 && reconBlocks <= 608; }
-inline bool stage_early(int maxM, long long reconBlocks) { return maxM <= 3 || reconBlocks <= 4000; }
+// 1k quads 43.6 / 39.2, 10k 47 / 41, 256k 161.6 / 155.7, 640k 361 / 354, 1.5M 784 / 778, 4.0M 1961 / 1954 (face-neighbour
+// stencils 197.6 / 191.6, 422.6 / 419.5, 908 / 901, 2223 / 2217); 10k triangles 46 / 40, 202k 130 / 121, 2.0M 946 / 937.
+// (Saying pdl_next first thing: 4.0M quads 2308, 2.0M triangles 1003: the next kernel's waiting blocks take the
+// places of blocks that have work.)
+// Not the tail where a quad mesh's reconstruct has 2 to 3.5 blocks a SM: its blocks crowd where that ends first.
+// us a step with the tail early / on completion, edge- and face-neighbour stencils: 250 blocks 39.0 / 38.8 and
+// 51.0 / 51.2, 300 41.7 / 39.8 and 54.0 / 51.9, 350 42.8 / 41.0 and 58.8 / 54.1, 400 45.4 / 45.1 and 59.9 / 57.4, 450 47.1 / 46.0
+// and 61.7 / 57.4, 500 47.1 / 45.3 and 62.8 / 59.3, 549 47.2 / 49.2 and 64.0 / 61.3, 574 48.2 / 51.2 and 65.0 / 63.5,
+// 600 48.8 / 51.2 and 65.2 / 65.3, 650 55.2 / 57.2 and 71.7 / 75.0, 800 70.6 / 73.8 and 87.9 / 90.3.
+inline bool tail_early(int maxM, long long reconBlocks) {
+  return maxM <= 3 || reconBlocks <= 2 * kSMs || 2 * reconBlocks > 7 * kSMs;
+}
 
 // Launches a kernel, with pdl as the programmatic dependent of the one before it on the stream.
 template <class... A, class... B>
@@ -617,9 +624,9 @@ void enqueue_tail(const Stage<P>& st) {
   if (st.fused()) {
     Stage<P> d = st;
     for (int k = 0; k < 3; ++k) {
-      d.pdl = stage_early(st.s->maxM, d.gc());
+      d.pdl = true;
       if (k > 0) d.at(k).reconstruct();
-      d.pdl = d.pdl && !quads_one_wave(st.s->maxM, d.gc());
+      d.pdl = tail_early(st.s->maxM, d.gc());
       d.at(k).tail(k);
     }
     return;
@@ -2059,8 +2066,10 @@ afar_status add_fused_chain(cudaGraph_t graph, int device, const MemberTable<Pol
 // One fused step of a batch as a graph.  The chains work on different members: side by side they fill the
 // GPU where one is less than a wave, one after another they leave it to one kernel at a time (256 ramps of
 // 5k to 200k quads: 8.93 ms a step side by side, 8.49 in turn, 8.59 as separate kernels).  Early starts (see
-// stage_early) where the members together are no more than 4000 blocks of 128 cells; us a step without / with:
-// four members of 4k quads 48 / 43, twelve of 41k triangles 296 / 292, twelve of 121k 727 / 731.
+// tail_early) where the members together are no more than 4000 blocks of 128 cells; us a step without / with:
+// four members of 4k quads 48 / 43, twelve of 41k triangles 296 / 292, twelve of 121k 727 / 731, ten of 160k quads 1%
+// slower with.  The single solve's exception for quads is not one here: 450 to 480 blocks without / with, four
+// members of 14k 56.1 / 56.8 (edge-neighbour stencils 49.2 / 48.2), six of 10k 55.3 / 53.1 (51.2 / 48.6).
 afar_status capture_fused(afar_batch* b, const std::vector<StageArgs<PolicyMixed>>& tab, int nfmax, size_t smem,
                           size_t tail_bytes, cudaGraph_t* graph) {
   using Table = MemberTable<PolicyMixed>;
@@ -2068,7 +2077,7 @@ afar_status capture_fused(afar_batch* b, const std::vector<StageArgs<PolicyMixed
   std::unique_ptr<Table> cells(new Table), tiles(new Table);
   long long blocks = 0;
   for (const auto& m : tab) blocks += grid_for(m.Nc, kTile);
-  const bool early = blocks <= 4000 && !quads_one_wave(nfmax, blocks);
+  const bool early = blocks <= 4000;
   afar_status st = AFAR_OK;
   cudaGraphNode_t end = nullptr;
   for (size_t i0 = 0; i0 < tab.size() && !st; i0 += Table::kMembers) {
@@ -2083,7 +2092,7 @@ afar_status capture_fused(afar_batch* b, const std::vector<StageArgs<PolicyMixed
     }
     const auto chain = nfmax <= 3 ? (early ? add_fused_chain<3, true> : add_fused_chain<3, false>)
                                   : (early ? add_fused_chain<4, true> : add_fused_chain<4, false>);
-    if (cells->first[n] <= 4 * 152) end = nullptr;
+    if (cells->first[n] <= 4 * kSMs) end = nullptr;  // less than a wave of four blocks a SM
     st = chain(*graph, b->device, *cells, *tiles, smem, tail_bytes, &end);
   }
   if (st) {

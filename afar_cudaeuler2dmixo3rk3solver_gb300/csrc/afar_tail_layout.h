@@ -19,4 +19,9 @@ AFAR_HOST_DEVICE constexpr int tail_first_halo(const int thread, const int cells
   return thread - cells < kTailHalo ? thread - cells : kTailHalo - 1;
 }
 
+// Cells of a tile (see tail_cells) of a mesh with at most maxM faces a cell.
+AFAR_HOST_DEVICE constexpr int tail_tile_cells(const int maxM, const int cells) {
+  return maxM <= 3 ? 192 : cells <= 4096 ? 96 : 152;
+}
+
 }  // namespace afar
