@@ -74,7 +74,7 @@ struct StageArgs {
   const int2* on;             // Nf (owner, neighbour)
   const V4<G>* fd;            // Nf (xf-x_own, yf-y_own, xf-x_nei, yf-y_nei)
   const V4<G>* fs;            // Nf+Nb (Sfx, Sfy, magSf, 1/magSf; ref: 0)
-  const V2<double>* dtg;      // Nf (delta r, fraction) of the CFL estimate
+  const V2<double>* dtg;      // Nf (delta r, fraction) of the CFL estimate (mixed: with the multi-point flux)
   const V2<double>* bn;       // Nb unit normal of each boundary face
   const uint8_t* btype;       // Nb cudaEulerBCs label
   const double* vol;          // Nc
@@ -3237,7 +3237,9 @@ __global__ void k_setup_face_geom(StageArgs<P> a, const V4<double>* faceXY, cons
     const_cast<V4<G>*>(a.fd)[f] = V4<G>{(G)oxd, (G)oyd, (G)nxd, (G)nyd};
     const double deltaR = hypot(wrapd(cn.x - co.x, a.px), wrapd(cn.y - co.y, a.py));
     const double fraction = hypot(oxd, oyd) / deltaR;
-    const_cast<V2<double>*>(a.dtg)[f] = V2<double>{deltaR, fraction};
+    if (a.dtg) const_cast<V2<double>*>(a.dtg)[f] = V2<double>{deltaR, fraction};
+    if constexpr (P::id == PolicyMixed::id)
+      const_cast<V2<float>*>(a.dtgf)[f] = V2<float>{(float)deltaR, (float)fraction};
   } else {
     const int b = f - a.Nf;
     const_cast<V2<double>*>(a.bn)[b] = V2<double>{s.x / s.z, s.y / s.z};

@@ -17,7 +17,6 @@
 #include <vector>
 
 #include "afar_internal.h"
-#include "afar_tail_layout.h"
 
 namespace {
 
@@ -51,11 +50,6 @@ size_t estimate_bytes(const afar_fieldSizes& z, int policy) {
   const double per_cell = 4 * g + 64 + 8 * g + 4 * w + 2 + 4 * s + 4 * m + 8 * m * w + 2 * m * w + m * (s + 1) * w + 48 +
                           snapshot + res_dump + staging;
   const double per_face = 8 * g + 4 * g + 48 + 16 + 8;
-  if (policy == AFAR_POLICY_MIXED) {  // the device order, two further state buffers, the fused stage's lists
-    const double tile = afar::tail_tile_cells(z.maxCompactStencilSize, z.cellsNum);
-    return (size_t)(nc * (per_cell + 8 + 8 * g + 2 * m + 7600 / tile) + (nf + nb) * (per_face + 8) + nb * (48 + 8 * g) +
-                    (64u << 20));
-  }
   return (size_t)(nc * per_cell + (nf + nb) * per_face + nb * 48 + (64u << 20));
 }
 

@@ -159,7 +159,7 @@ __global__ void k_init_ctl(StepCtl* ctl) {
 __global__ void k_reciprocal(int n, const double* in, double* out, float* outf) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
-    out[i] = 1.0 / in[i];
+    if (out) out[i] = 1.0 / in[i];
     if (outf) outf[i] = (float)(1.0 / in[i]);
   }
 }
@@ -187,12 +187,6 @@ __global__ void k_df_to_double(int n, const DF4* in, V4<double>* out, DeviceOrde
 __global__ void k_flags_out(int Nc, int n, const int8_t* in, int8_t* out, DeviceOrder o) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) reinterpret_cast<char2*>(out)[i < Nc ? o.cell(i) : i] = reinterpret_cast<const char2*>(in)[i];
-}
-
-template <class A, class B>
-__global__ void k_convert2(int n, const V2<A>* in, V2<B>* out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = V2<B>{(B)in[i].x, (B)in[i].y};
 }
 
 // the primitive state (cells, then ghosts) into the device's cell order and out of it
@@ -694,7 +688,6 @@ afar_status setup_operators(afar_solver* s, const afar_fieldPointer* h, void* sc
   k_setup_slot_geom<P><<<gc, kCellBlock, 0, s->stream>>>(a, fxy);
   k_setup_face_geom<P><<<gF, kFaceBlock, 0, s->stream>>>(a, fxy, fsr);
   if constexpr (P::id == PolicyMixed::id) {
-    if (Nf > 0) k_convert2<double, float><<<grid_for(Nf, 256), 256, 0, s->stream>>>(Nf, s->dtg, s->dtgf);
   }
   AFAR_CUDA(cudaGetLastError());
   AFAR_CUDA(cudaStreamSynchronize(s->stream));
@@ -1061,21 +1054,27 @@ extern "C" afar_status afar_setDeviceFieldData(afar_solver* s, const afar_fieldP
   const size_t Nc = cellsNum, Nf = facesNum, Nb = totalBoundaryFacesNum;
   const size_t g = s->policy == AFAR_POLICY_MIXED ? sizeof(V4<float>) : sizeof(V4<double>);
   const size_t l = s->policy == AFAR_POLICY_FP64 ? sizeof(V4<double>) : sizeof(V4<float>);
-  int *perm = nullptr, *inv = nullptr;
+  const bool mixed = s->policy == AFAR_POLICY_MIXED;
+  int* perm = nullptr;
   afar_status st;
   if ((st = alloc_all(s, [&]() -> afar_status {
          afar_status st;
          if ((st = dalloc_t(s, &s->cellC, Nc + Nb))) return st;
          if ((st = dalloc_t(s, &s->faceRaw, Nf + Nb))) return st;
-         if ((st = dalloc_t(s, &s->vol, Nc))) return st;
-         if ((st = dalloc_t(s, &s->vinv, Nc))) return st;
-         if (s->policy == AFAR_POLICY_MIXED) {
+         if (mixed) {
            if ((st = dalloc_t(s, &s->vinvf, Nc))) return st;
-           if ((st = dalloc(s, &s->xfer, std::max(sizeof(V4<double>) * (Nc + Nb), order_scratch(cellsNum))))) return st;
+           // (the flux of a fused solver's rare separate kernels too, see afar_setDeviceFieldDataStencil)
+           if ((st = dalloc(s, &s->xfer, std::max({sizeof(V4<double>) * (Nc + Nb), sizeof(V4<float>) * (Nf + Nb),
+                                                   order_scratch(cellsNum)}))))
+             return st;
            if ((st = dalloc_t(s, &perm, Nc))) return st;
-           if ((st = dalloc_t(s, &inv, Nc))) return st;
            for (void*& w : s->Wb)
              if ((st = dalloc(s, &w, sizeof(V4<float>) * (Nc + Nb)))) return st;
+         } else {
+           if ((st = dalloc_t(s, &s->vol, Nc))) return st;
+           if ((st = dalloc_t(s, &s->vinv, Nc))) return st;
+           if ((st = dalloc(s, &s->flux, g * (Nf + Nb)))) return st;
+           if ((st = dalloc_t(s, &s->dtg, Nf))) return st;
          }
          if ((st = dalloc_t(s, &s->U, Nc))) return st;
          if ((st = dalloc_t(s, &s->U0, Nc))) return st;
@@ -1087,15 +1086,14 @@ extern "C" afar_status afar_setDeviceFieldData(afar_solver* s, const afar_fieldP
          if ((st = dalloc(s, &s->grad, g * 2 * Nc))) return st;
          if ((st = dalloc(s, &s->lim, l * Nc))) return st;
          if ((st = dalloc(s, &s->fv, g * 2 * Nf))) return st;
-         if ((st = dalloc(s, &s->flux, g * (Nf + Nb)))) return st;
-         if ((st = dalloc_t(s, &s->dtg, Nf))) return st;
          return dalloc_t(s, &s->bn, Nb);
        })))
     return st;
   AFAR_CUDA(cudaMemcpyAsync(s->cellC, h->CELL, sizeof(V2<double>) * (Nc + Nb), cudaMemcpyHostToDevice, s->stream));
   AFAR_CUDA(cudaMemcpyAsync(s->faceRaw, h->FACE, sizeof(FaceRaw) * (Nf + Nb), cudaMemcpyHostToDevice, s->stream));
-  AFAR_CUDA(cudaMemcpyAsync(s->vol, h->cellVolume, sizeof(double) * Nc, cudaMemcpyHostToDevice, s->stream));
-  if (s->policy == AFAR_POLICY_MIXED) {
+  double* const vol = mixed ? reinterpret_cast<double*>(s->U0) : s->vol;  // mixed: for the reciprocals alone
+  AFAR_CUDA(cudaMemcpyAsync(vol, h->cellVolume, sizeof(double) * Nc, cudaMemcpyHostToDevice, s->stream));
+  if (mixed) {
     // Cells along a Hilbert curve: a tile of consecutive cells is then a compact patch of the mesh,
     // whose stencils and faces reach few cells outside it, whatever order the caller numbers in
     // (reverse Cuthill-McKee fronts are strips: 128 cells reach ~620 others, a Hilbert patch ~96).
@@ -1103,13 +1101,11 @@ extern "C" afar_status afar_setDeviceFieldData(afar_solver* s, const afar_fieldP
     // Step, 2.0M triangles in RCM order: the reconstruct 0.60 -> 0.51 ms a step, the step 1.20 -> 1.10;
     // 4.0M quads and triangles, whose fronts are compact already: 2.19 -> 2.22.
     hilbert_order(cellsNum, s->cellC, perm, s->xfer, s->stream);
-    k_invert<<<grid_for(Nc, 256), 256, 0, s->stream>>>((int)Nc, perm, inv);
     s->order.perm = perm;
-    s->order.inv = inv;
     reorder(s, s->cellC, Nc);
-    reorder(s, s->vol, Nc);
+    reorder(s, vol, Nc);
   }
-  k_reciprocal<<<grid_for(Nc, 256), 256, 0, s->stream>>>((int)Nc, s->vol, s->vinv, s->vinvf);
+  k_reciprocal<<<grid_for(Nc, 256), 256, 0, s->stream>>>((int)Nc, vol, s->vinv, s->vinvf);
   AFAR_CUDA(cudaMemsetAsync(s->si, 0, 2 * (Nc + Nb), s->stream));
   if ((st = put_state(s, reinterpret_cast<const afar_basicFieldData*>(h->FD),
                       reinterpret_cast<const afar_conservedFieldData*>(h->cFD),
@@ -1257,7 +1253,7 @@ extern "C" afar_status afar_setDeviceFieldDataStencil(afar_solver* s, const afar
   const size_t wS = s->policy == AFAR_POLICY_FP64 ? 8 : 4, wG = s->policy == AFAR_POLICY_MIXED ? 4 : 8;
   const int ntile = (Nc + kTile - 1) / kTile;
   const size_t ntail = grid_for(Nc, tail_cells(s));
-  int *fperm = nullptr, *finv = nullptr;
+  int* fperm = nullptr;
   afar_status st;
   if ((st = alloc_all(s, [&]() -> afar_status {
          afar_status st;
@@ -1268,7 +1264,6 @@ extern "C" afar_status afar_setDeviceFieldDataStencil(afar_solver* s, const afar
          if ((st = dalloc_t(s, &s->sten, (size_t)s->maxS * ldc))) return st;
          if ((st = dalloc_t(s, &s->cf, (size_t)s->maxM * ldc))) return st;
          if ((st = dalloc_t(s, &s->tileS, (size_t)ntile))) return st;
-         if ((st = dalloc_t(s, &s->res_dbg, (size_t)Nc))) return st;
          if ((st = dalloc(s, &s->fd, 4 * wG * (size_t)Nf))) return st;
          if ((st = dalloc(s, &s->fs, 4 * wG * (size_t)(Nf + Nb)))) return st;
          if ((st = dalloc(s, &s->lsm, 2 * wS * (size_t)s->maxM * ldc))) return st;
@@ -1279,7 +1274,6 @@ extern "C" afar_status afar_setDeviceFieldDataStencil(afar_solver* s, const afar
            if ((st = dalloc_t(s, &s->dtgf, (size_t)Nf))) return st;
            if ((st = dalloc_t(s, &s->tmaps, 1))) return st;
            if ((st = dalloc_t(s, &fperm, (size_t)Nf))) return st;
-           if ((st = dalloc_t(s, &finv, (size_t)Nf))) return st;
            if ((st = dalloc_t(s, &s->tail, ntail))) return st;
            if ((st = dalloc_t(s, &s->thalo, ntail * kTailHalo))) return st;
            if ((st = dalloc_t(s, &s->thcode, ntail * 4 * kTailHalo))) return st;
@@ -1300,7 +1294,7 @@ extern "C" afar_status afar_setDeviceFieldDataStencil(afar_solver* s, const afar
   const size_t n_lists = n_dls + n_dext + (sizeof(int) * (size_t)s->maxM * Nc + 15) / 16 * 16;
   int tail_limits[2] = {0, 1};  // the most faces of a tile; a tile past the limits
   Scratch scratch;
-  AFAR_CUDA(cudaMalloc(&scratch.p, std::max({n_lists + sizeof(int2) * (size_t)Nf, nrbf * wS,
+  AFAR_CUDA(cudaMalloc(&scratch.p, std::max({n_lists + (sizeof(int2) + sizeof(int)) * (size_t)Nf + sizeof(int) * (size_t)Nc, nrbf * wS,
                                              2 * sizeof(V4<double>) * (size_t)(Nf + Nb + 1)})));
   AFAR_CUDA(cudaMemsetAsync(s->sten, 0, sizeof(int) * s->maxS * ldc, s->stream));
   AFAR_CUDA(cudaMemsetAsync(s->cf, 0, sizeof(int) * s->maxM * ldc, s->stream));
@@ -1324,9 +1318,15 @@ extern "C" afar_status afar_setDeviceFieldDataStencil(afar_solver* s, const afar
     AFAR_CUDA(cudaMemcpyAsync(dcf, h->cellFaces, sizeof(int) * (size_t)s->maxM * Nc, cudaMemcpyHostToDevice, s->stream));
     int2* raw = s->order.perm ? reinterpret_cast<int2*>(at + n_lists) : s->on;
     if (Nf) AFAR_CUDA(cudaMemcpyAsync(raw, h->neighbour, sizeof(int2) * Nf, cudaMemcpyHostToDevice, s->stream));
+    if (s->order.perm) {  // the way back to the device's order, for the set-up alone
+      int* inv = reinterpret_cast<int*>(at + n_lists + sizeof(int2) * (size_t)Nf);
+      k_invert<<<grid_for(Nc, 256), 256, 0, s->stream>>>(Nc, s->order.perm, inv);
+      s->order.inv = inv;
+    }
     if (s->order.perm && Nf) {
       if (paired) {  // (faces that are not keep the caller's order)
         int* start = static_cast<int*>(s->xfer);
+        int* finv = reinterpret_cast<int*>(at + n_lists + sizeof(int2) * (size_t)Nf) + Nc;
         for (int pass = 0; pass < 2; ++pass) {
           k_face_order<<<grid_for(Nc, 256), 256, 0, s->stream>>>(Nc, Nf, s->maxM, s->nM, dcf,
                                                                  reinterpret_cast<const int*>(raw), s->order, start,
@@ -1341,6 +1341,7 @@ extern "C" afar_status afar_setDeviceFieldDataStencil(afar_solver* s, const afar
     k_setup_lists<<<grid_for(Nc, kCellBlock), kCellBlock, 0, s->stream>>>(Nc, Nf, s->ldc, s->maxS, s->maxM, s->maxLB,
                                                                            s->nS, s->nM, dls, dext, dcf, s->sten, s->cf,
                                                                            s->order);
+    s->order.inv = s->order.finv = nullptr;
     if (s->policy == AFAR_POLICY_MIXED) {
       AFAR_CUDA(cudaMemsetAsync(s->wflag, 0, sizeof(unsigned) * (size_t)ntile * 4, s->stream));
     }
@@ -1369,6 +1370,12 @@ extern "C" afar_status afar_setDeviceFieldDataStencil(afar_solver* s, const afar
   s->bvd_pending = -1;
   s->fused = tail_limits[1] == 0 && tail_smem(tail_limits[0], tail_cells(s)).bytes <= kMaxDynamicSmem - 2048;
   s->tail_faces = tail_limits[0];
+  // The flux of the separate kernels: a solver that runs the fused stage has it in the transfer buffer, which
+  // nothing else uses between a flux and its update (afar_stage_debug; a batch with block sizes of its own).
+  if (s->policy == AFAR_POLICY_MIXED) {
+    s->flux = s->xfer;
+    if (!s->fused && (st = dalloc(s, &s->flux, sizeof(V4<float>) * (size_t)(Nf + Nb)))) return st;
+  }
   if (s->fused) {
     if ((st = raise_smem_limit(k_tail<3>, s->device, tail_smem(s->tail_faces, tail_cells(s)).bytes))) return st;
     if ((st = raise_smem_limit(k_tail<4>, s->device, tail_smem(s->tail_faces, tail_cells(s)).bytes))) return st;
@@ -1680,8 +1687,9 @@ extern "C" afar_status afar_stage_debug(afar_solver* s, int stage, double deltaT
   auto run = [&](auto tag) -> afar_status {
     using P = decltype(tag);
     Stage<P> sg;
-    afar_status r = make_stage<P>(s, true, &sg);
-    if (r) return r;
+    afar_status r = AFAR_OK;
+    if (!s->res_dbg && (r = dalloc_t(s, &s->res_dbg, Nc))) return r;
+    if ((r = make_stage<P>(s, true, &sg))) return r;
     s->bvd_pending = -1;
     sg.reconstruct();
     sg.bvd();
@@ -2488,6 +2496,12 @@ extern "C" afar_status afar_set_face_gauss_flux(afar_solver* s, int nPoints, con
   AFAR_CUDA(cudaMemsetAsync(s->sgk, 0, 2 * wG * (size_t)s->maxM * ng * s->ldc, s->stream));
   if ((st = dalloc(s, &s->fgk, 2 * wG * (size_t)Nf * ng))) return st;
   if ((st = dalloc(s, &s->fvg, 4 * wG * 2 * (size_t)Nf * ng))) return st;
+  if (mixed && s->flux == s->xfer) {  // its steps have a flux between the calls of the reference-shaped loop
+    void* flux = nullptr;
+    if ((st = dalloc(s, &flux, sizeof(V4<float>) * (size_t)(Nf + s->Nb)))) return st;
+    s->flux = flux;
+  }
+  if (mixed && !s->dtg && (st = dalloc_t(s, &s->dtg, (size_t)Nf))) return st;  // of its FP64 Courant step
   double *d_w = nullptr, *d_p = nullptr;
   V4<double>* fxy = nullptr;
   auto cleanup = [&]() {
@@ -2518,6 +2532,7 @@ extern "C" afar_status afar_set_face_gauss_flux(afar_solver* s, int nPoints, con
   auto setup = [&](auto tag) {
     using P = decltype(tag);
     StageArgs<P> a = make_args<P>(s);
+    if (mixed) k_setup_face_geom<P><<<gF, kFaceBlock, 0, s->stream>>>(a, fxy, fsr);  // (the same again, and dtg)
     k_setup_gauss<P><<<grid_for(s->Nc, kCellBlock), kCellBlock, 0, s->stream>>>(a, d_w, d_p, s->order.fperm);
     if (Nf > 0) k_setup_gauss_faces<P><<<grid_for((long long)Nf * ng, 256), 256, 0, s->stream>>>(a, d_p, fxy, s->order.fperm);
   };
