@@ -19,10 +19,11 @@ struct DeviceOrder {
 __global__ void k_box_init(long long* box) {
   if (threadIdx.x < 4) box[threadIdx.x] = threadIdx.x < 2 ? 0x7FFFFFFFFFFFFFFFll : -0x7FFFFFFFFFFFFFFFll;
 }
-// The smallest and largest finite coordinates, as ordered integers (dkey): (min x, min y, max x, max y).
-__global__ void __launch_bounds__(256) k_box(int n, const V2<double>* c, long long* box) {
+// The smallest and largest finite coordinates of centres i, i + stride, .., as ordered integers (dkey) into box:
+// (min x, min y, max x, max y).  All lanes of a warp take part.
+__device__ __forceinline__ void box_of(int i, const int stride, const int n, const V2<double>* c, long long* box) {
   long long lo[2] = {0x7FFFFFFFFFFFFFFFll, 0x7FFFFFFFFFFFFFFFll}, hi[2] = {-0x7FFFFFFFFFFFFFFFll, -0x7FFFFFFFFFFFFFFFll};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (; i < n; i += stride) {
     const V2<double> v = c[i];
     const double x[2] = {v.x, v.y};
 #pragma unroll
@@ -48,19 +49,19 @@ __global__ void __launch_bounds__(256) k_box(int n, const V2<double>* c, long lo
     }
   }
 }
+__global__ void __launch_bounds__(256) k_box(int n, const V2<double>* c, long long* box) {
+  box_of(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, n, c, box);
+}
 __device__ __forceinline__ double undkey(const long long k) {
   return __longlong_as_double(k ^ ((k >> 63) & 0x7FFFFFFFFFFFFFFFll));
 }
-// Position along the Hilbert curve of order 13 over the centres' bounding square (cells of one key keep
-// the caller's order; a coordinate that is not finite counts as the smallest).
-__global__ void k_hilbert_keys(int n, int bits, const V2<double>* c, const long long* box, unsigned* key, int* id) {
+// Position along the Hilbert curve of order `bits` over the square at (x0, y0) of side `ext` (a coordinate that
+// is not finite counts as the smallest).
+__device__ __forceinline__ unsigned hilbert_key(const int bits, const V2<double> c, const double x0, const double y0,
+                                                const double ext) {
   const unsigned top = (1u << bits) - 1u;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double x0 = undkey(box[0]), y0 = undkey(box[1]);
-  const double ext = fmax(undkey(box[2]) - x0, undkey(box[3]) - y0);
   const double scale = ext > 0.0 ? (double)top / ext : 0.0;
-  const double gx = (c[i].x - x0) * scale, gy = (c[i].y - y0) * scale;
+  const double gx = (c.x - x0) * scale, gy = (c.y - y0) * scale;
   unsigned x = gx >= 0.0 && gx <= (double)top ? (unsigned)gx : 0u, y = gy >= 0.0 && gy <= (double)top ? (unsigned)gy : 0u, d = 0;
   for (unsigned s = (top + 1) >> 1; s > 0; s >>= 1) {
     const unsigned rx = (x & s) != 0, ry = (y & s) != 0;
@@ -75,8 +76,47 @@ __global__ void k_hilbert_keys(int n, int bits, const V2<double>* c, const long 
       y = t;
     }
   }
-  key[i] = d;
+  return d;
+}
+// The keys over the centres' bounding square (cells of one key keep the caller's order).
+__global__ void k_hilbert_keys(int n, int bits, const V2<double>* c, const long long* box, unsigned* key, int* id) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double x0 = undkey(box[0]), y0 = undkey(box[1]);
+  key[i] = hilbert_key(bits, c[i], x0, y0, fmax(undkey(box[2]) - x0, undkey(box[3]) - y0));
   id[i] = i;
+}
+
+// The whole order of up to 4096 cells in one block: a curve of order 9 at most, so that key and cell fit 32
+// bits, sorted in shared memory.  Set-up of a mixed solver with this / as the launches of larger meshes: 1024
+// cells 465 / 505 us, 4096 707 / 735.
+constexpr int kOrderSmall = 4096;
+__global__ void __launch_bounds__(1024) k_hilbert_small(int n, int bits, const V2<double>* c, int* perm) {
+  __shared__ unsigned v[kOrderSmall];
+  __shared__ long long box[4];
+  const int t = threadIdx.x;
+  if (t < 4) box[t] = t < 2 ? 0x7FFFFFFFFFFFFFFFll : -0x7FFFFFFFFFFFFFFFll;
+  __syncthreads();
+  box_of(t, 1024, n, c, box);
+  __syncthreads();
+  const double x0 = undkey(box[0]), y0 = undkey(box[1]), ext = fmax(undkey(box[2]) - x0, undkey(box[3]) - y0);
+  const int N = n <= kOrderSmall / 2 ? kOrderSmall / 2 : kOrderSmall;
+  for (int i = t; i < N; i += 1024)
+    v[i] = i < n ? hilbert_key(bits, c[i], x0, y0, ext) << 12 | (unsigned)i : 0xFFFFFFFFu;
+  for (int k = 2; k <= N; k <<= 1)  // bitonic sort
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      __syncthreads();
+      for (int p = t; p < N / 2; p += 1024) {
+        const int lo = (p & ~(j - 1)) * 2 + (p & (j - 1)), hi = lo + j;
+        const unsigned a = v[lo], b = v[hi];
+        if ((a > b) == ((lo & k) == 0)) {
+          v[lo] = b;
+          v[hi] = a;
+        }
+      }
+    }
+  __syncthreads();
+  for (int i = t; i < n; i += 1024) perm[i] = (int)(v[i] & (kOrderSmall - 1));
 }
 
 // ---- exclusive scan of n ints in place: block sums (2048 a block), their scan by one block, the rest
@@ -209,6 +249,14 @@ inline size_t order_scratch(int n) {
   return 64 + 16 * (size_t)n + 4 * 256 * nb + 4 * (size_t)scan_blocks((int)(256 * nb)) + 64;
 }
 inline void hilbert_order(int n, const V2<double>* centre, int* perm, void* scratch, cudaStream_t st) {
+  // A curve of 64 places or more a cell: a small mesh's set-up is a chain of launches, and every 8 bits of
+  // the key are three of them or five (23 with the 26 bits of a large mesh).
+  int bits = 4;
+  while (bits < 13 && (1ll << (2 * bits)) < 64ll * n) ++bits;
+  if (n <= kOrderSmall) {
+    k_hilbert_small<<<1, 1024, 0, st>>>(n, bits, centre, perm);
+    return;
+  }
   long long* box = static_cast<long long*>(scratch);
   unsigned* key[2] = {reinterpret_cast<unsigned*>(box + 8), nullptr};
   key[1] = key[0] + n;
@@ -219,10 +267,6 @@ inline void hilbert_order(int n, const V2<double>* centre, int* perm, void* scra
   int* sums = cnt + 256 * (size_t)nb;
   k_box_init<<<1, 32, 0, st>>>(box);
   k_box<<<nb < 512 ? nb : 512, 256, 0, st>>>(n, centre, box);
-  // A curve of 64 places or more a cell: a small mesh's set-up is a chain of launches, and every 8 bits of
-  // the key are three of them or five (1k cells: 9 launches, 23 with the 26 bits of a large mesh).
-  int bits = 4;
-  while (bits < 13 && (1ll << (2 * bits)) < 64ll * n) ++bits;
   const int passes = (2 * bits + 7) / 8;
   k_hilbert_keys<<<(n + 255) / 256, 256, 0, st>>>(n, bits, centre, box, key[0], id[0]);
   for (int pass = 0; pass < passes; ++pass) {
@@ -233,14 +277,11 @@ inline void hilbert_order(int n, const V2<double>* centre, int* perm, void* scra
   }
 }
 
-__global__ void k_invert(int n, const int* perm, int* inv) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) inv[perm[i]] = i;
-}
+// Cells, and what follows them (ghosts) in place, from the caller's order into the device's.
 template <class T>
-__global__ void k_gather(int n, const int* perm, const T* in, T* out) {
+__global__ void k_gather(int Nc, int n, const T* in, T* out, DeviceOrder o) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = in[perm[i]];
+  if (i < n) out[i] = in[i < Nc ? o.cell(i) : i];
 }
 
 // The internal faces by their first cell in the device's order, then by the other (upper-triangular, as
@@ -283,13 +324,21 @@ __global__ void k_setup_owners(int Nf, const int2* raw, int2* on, DeviceOrder o)
   const int2 h = raw[o.face(f)];
   on[f] = o.inv ? int2{o.inv[h.x], o.inv[h.y]} : h;
 }
-// The largest stencil of each 128-cell tile (at least 1: the tile kernel loads the boxes of that size).
-__global__ void k_tile_stencils(int Nc, const uint8_t* nS, uint8_t* tileS) {
+// The cells' list lengths in the device's order, the way back to it (inv, where there is one), and the largest
+// stencil of each 128-cell tile (at least 1: the tile kernel loads the boxes of that size).
+__global__ void __launch_bounds__(128) k_setup_counts(int Nc, const uint8_t* nS0, const uint8_t* nM0, uint8_t* nS,
+                                                      uint8_t* nM, uint8_t* tileS, int* inv, DeviceOrder o) {
   __shared__ int m;
   if (threadIdx.x == 0) m = 1;
   __syncthreads();
   const int c = blockIdx.x * 128 + threadIdx.x;
-  if (c < Nc) atomicMax(&m, (int)nS[c]);
+  if (c < Nc) {
+    const int h = o.cell(c);
+    nS[c] = nS0[h];
+    nM[c] = nM0[h];
+    if (inv) inv[h] = c;
+    atomicMax(&m, (int)nS0[h]);
+  }
   __syncthreads();
   if (threadIdx.x == 0) tileS[blockIdx.x] = (uint8_t)m;
 }

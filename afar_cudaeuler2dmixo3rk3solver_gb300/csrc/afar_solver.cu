@@ -156,11 +156,12 @@ __global__ void k_init_ctl(StepCtl* ctl) {
   }
 }
 
-__global__ void k_reciprocal(int n, const double* in, double* out, float* outf) {
+__global__ void k_reciprocal(int n, const double* in, double* out, float* outf, DeviceOrder o) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
-    if (out) out[i] = 1.0 / in[i];
-    if (outf) outf[i] = (float)(1.0 / in[i]);
+    const double r = 1.0 / in[o.cell(i)];
+    if (out) out[i] = r;
+    if (outf) outf[i] = (float)r;
   }
 }
 
@@ -362,14 +363,6 @@ afar_status alloc_all(afar_solver* s, F&& f) {
 template <class T>
 afar_status dalloc_t(afar_solver* s, T** p, size_t n) {
   return dalloc(s, reinterpret_cast<void**>(p), n * sizeof(T));
-}
-
-// The first n <= Nc entries of a device array (at most 32 bytes each) from the caller's cell order into
-// the device's, through the transfer buffer; ordered on the solver's stream.
-template <class T>
-void reorder(afar_solver* s, T* a, size_t n) {
-  cudaMemcpyAsync(s->xfer, a, sizeof(T) * n, cudaMemcpyDeviceToDevice, s->stream);
-  k_gather<<<grid_for((long long)n, 256), 256, 0, s->stream>>>((int)n, s->order.perm, static_cast<const T*>(s->xfer), a);
 }
 
 // Cells of a tile of the fused stage tail: as many as its 256 threads take with the halo in one pass (192
@@ -1089,9 +1082,12 @@ extern "C" afar_status afar_setDeviceFieldData(afar_solver* s, const afar_fieldP
          return dalloc_t(s, &s->bn, Nb);
        })))
     return st;
-  AFAR_CUDA(cudaMemcpyAsync(s->cellC, h->CELL, sizeof(V2<double>) * (Nc + Nb), cudaMemcpyHostToDevice, s->stream));
+  // mixed: the caller's centres and volumes go to the state's buffers first, which put_state fills below
+  V2<double>* const centres = mixed ? static_cast<V2<double>*>(s->Wb[0]) : s->cellC;
+  static_assert(sizeof(V2<double>) == sizeof(V4<float>), "a centre in a state's place");
+  AFAR_CUDA(cudaMemcpyAsync(centres, h->CELL, sizeof(V2<double>) * (Nc + Nb), cudaMemcpyHostToDevice, s->stream));
   AFAR_CUDA(cudaMemcpyAsync(s->faceRaw, h->FACE, sizeof(FaceRaw) * (Nf + Nb), cudaMemcpyHostToDevice, s->stream));
-  double* const vol = mixed ? reinterpret_cast<double*>(s->U0) : s->vol;  // mixed: for the reciprocals alone
+  double* const vol = mixed ? reinterpret_cast<double*>(s->U0) : s->vol;
   AFAR_CUDA(cudaMemcpyAsync(vol, h->cellVolume, sizeof(double) * Nc, cudaMemcpyHostToDevice, s->stream));
   if (mixed) {
     // Cells along a Hilbert curve: a tile of consecutive cells is then a compact patch of the mesh,
@@ -1100,12 +1096,11 @@ extern "C" afar_status afar_setDeviceFieldData(afar_solver* s, const afar_fieldP
     // Each cell keeps its own order of stencil members and faces, so results do not change by a bit.
     // Step, 2.0M triangles in RCM order: the reconstruct 0.60 -> 0.51 ms a step, the step 1.20 -> 1.10;
     // 4.0M quads and triangles, whose fronts are compact already: 2.19 -> 2.22.
-    hilbert_order(cellsNum, s->cellC, perm, s->xfer, s->stream);
+    hilbert_order(cellsNum, centres, perm, s->xfer, s->stream);
     s->order.perm = perm;
-    reorder(s, s->cellC, Nc);
-    reorder(s, vol, Nc);
+    k_gather<<<grid_for(Nc + Nb, 256), 256, 0, s->stream>>>((int)Nc, (int)(Nc + Nb), centres, s->cellC, s->order);
   }
-  k_reciprocal<<<grid_for(Nc, 256), 256, 0, s->stream>>>((int)Nc, vol, s->vinv, s->vinvf);
+  k_reciprocal<<<grid_for(Nc, 256), 256, 0, s->stream>>>((int)Nc, vol, s->vinv, s->vinvf, s->order);
   AFAR_CUDA(cudaMemsetAsync(s->si, 0, 2 * (Nc + Nb), s->stream));
   if ((st = put_state(s, reinterpret_cast<const afar_basicFieldData*>(h->FD),
                       reinterpret_cast<const afar_conservedFieldData*>(h->cFD),
@@ -1294,39 +1289,34 @@ extern "C" afar_status afar_setDeviceFieldDataStencil(afar_solver* s, const afar
   const size_t n_lists = n_dls + n_dext + (sizeof(int) * (size_t)s->maxM * Nc + 15) / 16 * 16;
   int tail_limits[2] = {0, 1};  // the most faces of a tile; a tile past the limits
   Scratch scratch;
-  AFAR_CUDA(cudaMalloc(&scratch.p, std::max({n_lists + (sizeof(int2) + sizeof(int)) * (size_t)Nf + sizeof(int) * (size_t)Nc, nrbf * wS,
+  AFAR_CUDA(cudaMalloc(&scratch.p, std::max({n_lists + 12 * (size_t)Nf + 6 * (size_t)Nc, nrbf * wS,
                                              2 * sizeof(V4<double>) * (size_t)(Nf + Nb + 1)})));
   AFAR_CUDA(cudaMemsetAsync(s->sten, 0, sizeof(int) * s->maxS * ldc, s->stream));
   AFAR_CUDA(cudaMemsetAsync(s->cf, 0, sizeof(int) * s->maxM * ldc, s->stream));
   if (Nb) {
     AFAR_CUDA(cudaMemcpyAsync(s->btype, h->boundaryFacesType, Nb, cudaMemcpyHostToDevice, s->stream));
   }
-  AFAR_CUDA(cudaMemcpyAsync(s->nS, h->stencilSize, Nc, cudaMemcpyHostToDevice, s->stream));
-  AFAR_CUDA(cudaMemcpyAsync(s->nM, h->compactStencilSize, Nc, cudaMemcpyHostToDevice, s->stream));
-  if (s->order.perm) {
-    reorder(s, s->nS, (size_t)Nc);
-    reorder(s, s->nM, (size_t)Nc);
-  }
-  k_tile_stencils<<<ntile, kTile, 0, s->stream>>>(Nc, s->nS, s->tileS);
   {
     char* at = static_cast<char*>(scratch.p);
     uint16_t* dls = reinterpret_cast<uint16_t*>(at);
     int* dext = reinterpret_cast<int*>(at + n_dls);
     int* dcf = reinterpret_cast<int*>(at + n_dls + n_dext);
+    int* inv = reinterpret_cast<int*>(at + n_lists + sizeof(int2) * (size_t)Nf);  // then finv, for the set-up alone
+    uint8_t* counts = reinterpret_cast<uint8_t*>(inv + (size_t)Nc + Nf);
+    AFAR_CUDA(cudaMemcpyAsync(counts, h->stencilSize, Nc, cudaMemcpyHostToDevice, s->stream));
+    AFAR_CUDA(cudaMemcpyAsync(counts + Nc, h->compactStencilSize, Nc, cudaMemcpyHostToDevice, s->stream));
+    if (s->order.perm) s->order.inv = inv;
+    k_setup_counts<<<ntile, kTile, 0, s->stream>>>(Nc, counts, counts + Nc, s->nS, s->nM, s->tileS,
+                                                   s->order.perm ? inv : nullptr, s->order);
     AFAR_CUDA(cudaMemcpyAsync(dls, h->localStencil, sizeof(uint16_t) * (size_t)s->maxS * Nc, cudaMemcpyHostToDevice, s->stream));
     if (next) AFAR_CUDA(cudaMemcpyAsync(dext, h->extendStencil, sizeof(int) * next, cudaMemcpyHostToDevice, s->stream));
     AFAR_CUDA(cudaMemcpyAsync(dcf, h->cellFaces, sizeof(int) * (size_t)s->maxM * Nc, cudaMemcpyHostToDevice, s->stream));
     int2* raw = s->order.perm ? reinterpret_cast<int2*>(at + n_lists) : s->on;
     if (Nf) AFAR_CUDA(cudaMemcpyAsync(raw, h->neighbour, sizeof(int2) * Nf, cudaMemcpyHostToDevice, s->stream));
-    if (s->order.perm) {  // the way back to the device's order, for the set-up alone
-      int* inv = reinterpret_cast<int*>(at + n_lists + sizeof(int2) * (size_t)Nf);
-      k_invert<<<grid_for(Nc, 256), 256, 0, s->stream>>>(Nc, s->order.perm, inv);
-      s->order.inv = inv;
-    }
     if (s->order.perm && Nf) {
       if (paired) {  // (faces that are not keep the caller's order)
         int* start = static_cast<int*>(s->xfer);
-        int* finv = reinterpret_cast<int*>(at + n_lists + sizeof(int2) * (size_t)Nf) + Nc;
+        int* finv = inv + Nc;
         for (int pass = 0; pass < 2; ++pass) {
           k_face_order<<<grid_for(Nc, 256), 256, 0, s->stream>>>(Nc, Nf, s->maxM, s->nM, dcf,
                                                                  reinterpret_cast<const int*>(raw), s->order, start,
