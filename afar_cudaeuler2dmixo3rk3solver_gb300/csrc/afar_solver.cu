@@ -50,6 +50,7 @@ constexpr int kCellBlock = 128;
 constexpr size_t kMaxDynamicSmem = 227 * 1024;  // per CTA on sm_103a
 constexpr int kFaceBlock = 256;
 constexpr int kSMs = 152;  // GB300
+const unsigned long long kDtArmed = 0x40F86A0000000000ull;  // the Courant minimum before a step: bits of 1e5
 constexpr int kFaceBlock64 = 128;  // ref and fp64: smaller blocks, an evener last wave over the SMs' FP64 pipes
 // GPUevolve.cu:223-225: the reference's truncated SSP-RK3 coefficients
 constexpr double kBeta1[3] = {1.0, 0.75, 0.333333};
@@ -896,9 +897,9 @@ static afar_status get_state(afar_solver* s, afar_basicFieldData* FD, afar_conse
 // The project autotuner: the mixed reconstruct has two implementations whose speed depends on the
 // mesh (stencil size, faces per cell, size): the tile-staged kernel (TMA loads of each 128-cell
 // tile's operator rows into shared memory) and the register pass (no shared memory, more tiles per
-// SM).  At the stencil upload each is timed on the solver's own data (one warm-up, best of three
-// launches, CUDA events on its stream; the launches only write the stage's intermediates) and the
-// faster kept.  Decisions are cached per device and mesh class (faces per cell, stencil size, cell
+// SM).  At the stencil upload each is timed on the solver's own data (one warm-up, best of three times
+// the launches of a step, the first of a fused one with its Courant step; CUDA events on its stream; the
+// launches only write the stage's intermediates and that minimum) and the faster kept.  Decisions are cached per device and mesh class (faces per cell, stencil size, cell
 // count to a factor of two), so later solvers of the same class skip the timing.
 // cuTensorMapEncodeTiled, looked up once through the runtime (the library links no driver API).
 static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
@@ -985,20 +986,25 @@ static afar_status tune_reconstruct(afar_solver* s) {
   float best[2];
   for (int v = 0; v < 2; ++v) {
     s->recon_variant = v;
-    sg.reconstruct();  // warm-up
+    const auto step = [&] {
+      sg.reconstruct(sg.fused());
+      for (int k = 1; k < 3; ++k) sg.reconstruct();
+    };
+    step();  // warm-up
     best[v] = 1e30f;
     for (int k = 0; k < 3; ++k) {
       AFAR_CUDA(cudaEventRecord(e0, s->stream));
-      sg.reconstruct();
+      step();
       AFAR_CUDA(cudaEventRecord(e1, s->stream));
       AFAR_CUDA(cudaEventSynchronize(e1));
       float ms = 0.f;
       AFAR_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-      best[v] = std::min(best[v], ms);
+      best[v] = std::min(best[v], ms / 3.f);
     }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  AFAR_CUDA(cudaMemcpyAsync(&s->ctl->dt_bits, &kDtArmed, sizeof(kDtArmed), cudaMemcpyHostToDevice, s->stream));
   AFAR_CUDA(cudaGetLastError());
   if ((st = check_device_error(s))) return st;
   s->recon_variant = best[1] < best[0] ? 1 : 0;
@@ -1397,7 +1403,6 @@ extern "C" afar_status afar_adjustTimeStep(afar_solver* s, int facesNum, double 
     set_error("afar_adjustTimeStep: bad argument");
     return AFAR_ERR_ARGUMENT;
   }
-  const unsigned long long init = 0x40F86A0000000000ull;  // bits of 1e5
   // Outside a batch the Courant step comes from the head of the coming step -- stage 1 up to its
   // flux, whose fused reduction is the same Courant minimum over the internal faces (the ref
   // policy's head runs the reference-shaped Courant kernel itself) -- so no separate pass runs and
@@ -1415,7 +1420,7 @@ extern "C" afar_status afar_adjustTimeStep(afar_solver* s, int facesNum, double 
       AFAR_CUDA(cudaGetLastError());
       // the minimum is armed again at once, as at the end of a step: whichever step follows starts anew (the
       // tail has its step size from the caller)
-      AFAR_CUDA(cudaMemcpyAsync(&s->ctl->dt_bits, &init, sizeof(init), cudaMemcpyHostToDevice, s->stream));
+      AFAR_CUDA(cudaMemcpyAsync(&s->ctl->dt_bits, &kDtArmed, sizeof(kDtArmed), cudaMemcpyHostToDevice, s->stream));
       if (c.err) {  // a bounded device wait gave up, in this head or in the step before it
         AFAR_CUDA(cudaMemsetAsync(&s->ctl->err, 0, sizeof(c.err), s->stream));
         AFAR_CUDA(cudaStreamSynchronize(s->stream));
@@ -1427,7 +1432,7 @@ extern "C" afar_status afar_adjustTimeStep(afar_solver* s, int facesNum, double 
       return AFAR_OK;
     }
   }
-  AFAR_CUDA(cudaMemcpyAsync(s->dt_bits, &init, sizeof(init), cudaMemcpyHostToDevice, s->stream));
+  AFAR_CUDA(cudaMemcpyAsync(s->dt_bits, &kDtArmed, sizeof(kDtArmed), cudaMemcpyHostToDevice, s->stream));
   const int gf = grid_for(s->Nf, kFaceBlock);
   if (s->Nf > 0) {
     switch (s->policy) {

@@ -81,7 +81,13 @@ def test_the_tuner_s_launches_leave_the_switches():
     s.limiter64()
     assert np.array_equal(s.state()["shockIndicator"][1::2], before)
     assert before.any()
+    twin = CudaSolver(hf, cfg, policy="mixed")
+    for v in (s, twin):  # nor do they leave a Courant step
+        v.upload_state(FD=hf.FD, cFD=hf.cFD, cFDold=hf.cFD)
+        v.run(1)
+    assert s.time()[1] == twin.time()[1]
     s.close()
+    twin.close()
 
 
 def test_a_batch_s_timing_leaves_no_switch_pending():
