@@ -293,6 +293,7 @@ struct afar_solver {
   afar_batch* batch = nullptr;  // the batch this solver belongs to, if any
   StepCtl* ctl = nullptr;
   unsigned long long* dt_bits = nullptr;
+  unsigned long long* counters = nullptr;  // four, of afar_switch_counts
   // policy-typed device arrays (element size depends on the policy)
   void* W = nullptr;
   void* fd = nullptr;
@@ -1080,6 +1081,7 @@ extern "C" afar_status afar_setDeviceFieldData(afar_solver* s, const afar_fieldP
          if ((st = dalloc_t(s, &s->si, 2 * (Nc + Nb)))) return st;
          if ((st = dalloc_t(s, &s->ctl, 1))) return st;
          if ((st = dalloc_t(s, &s->dt_bits, 1))) return st;
+         if ((st = dalloc_t(s, &s->counters, 4))) return st;
          if ((st = dalloc(s, &s->W, w_size(s->policy) * (Nc + Nb)))) return st;
          // intermediates
          if ((st = dalloc(s, &s->grad, g * 2 * Nc))) return st;
@@ -1880,15 +1882,13 @@ extern "C" afar_status afar_switch_counts(afar_solver* s, long long counts[4]) {
   if (st) return st;
   if (!counts) return (set_error("null output"), AFAR_ERR_ARGUMENT);
   if (s->bvd_pending == 0 && (st = settle_bvd(s))) return st;  // a fused head: its stage's types
-  unsigned long long* d = nullptr;
-  AFAR_CUDA(cudaMalloc(&d, 4 * sizeof(unsigned long long)));
+  unsigned long long* const d = s->counters;
   AFAR_CUDA(cudaMemsetAsync(d, 0, 4 * sizeof(unsigned long long), s->stream));
   const int n = std::max(s->Nc, s->Nf);
   k_switch_counts<<<grid_for(n, 256), 256, 0, s->stream>>>(s->Nc, s->Nf, s->si, s->on, d);
   unsigned long long h[4];
   AFAR_CUDA(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, s->stream));
   AFAR_CUDA(cudaStreamSynchronize(s->stream));
-  AFAR_CUDA(cudaFree(d));
   for (int k = 0; k < 4; ++k) counts[k] = (long long)h[k];
   return AFAR_OK;
 }
