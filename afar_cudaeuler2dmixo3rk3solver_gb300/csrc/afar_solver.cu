@@ -261,6 +261,8 @@ struct afar_solver {
   // before: the state buffer of the last stage whose BVD the accessors still have to run (-1: none).
   int bvd_pending = -1;
   float tune_ms[2] = {0.f, 0.f};  // the autotuner's measured launch times (0: decision from the cache)
+  // Which ghosts the state's buffers hold, of all that were uploaded (mixed), and which the snapshot does.
+  long long ghosts = 0, ghosts_next = 0, snap_ghosts = 0;
   void* xfer = nullptr;    // mixed: staging for double <-> device-format copies, 32 B x (Nc + Nb)
   // The mixed policy keeps its cells along a Hilbert curve, its internal faces by their first cell in
   // that order (see setup_cell_order); everything that crosses the boundary is in the caller's order.
@@ -824,6 +826,7 @@ static afar_status put_state(afar_solver* s, const afar_basicFieldData* FD, cons
     if (afar_status st = settle_bvd(s)) return st;
   }
   if (FD) {
+    s->ghosts = ++s->ghosts_next;
     if (mixed) {
       AFAR_CUDA(cudaMemcpyAsync(s->xfer, FD, sizeof(V4<double>) * (Nc + Nb), cudaMemcpyHostToDevice, s->stream));
       k_state_in<<<grid_for(Nc + Nb, 256), 256, 0, s->stream>>>((int)Nc, (int)(Nc + Nb),
@@ -854,6 +857,7 @@ static afar_status put_state(afar_solver* s, const afar_basicFieldData* FD, cons
   return AFAR_OK;
 }
 
+// (the mixed policy's arrays leave through `xfer` one after another, in the stream's order)
 static afar_status get_state(afar_solver* s, afar_basicFieldData* FD, afar_conservedFieldData* cFD, int8_t* si) {
   const size_t Nc = s->Nc, Nb = s->Nb;
   const bool mixed = s->policy == AFAR_POLICY_MIXED;
@@ -863,7 +867,6 @@ static afar_status get_state(afar_solver* s, afar_basicFieldData* FD, afar_conse
                                                                  static_cast<const V4<float>*>(s->W),
                                                                  static_cast<V4<double>*>(s->xfer), s->order);
       AFAR_CUDA(cudaMemcpyAsync(FD, s->xfer, sizeof(V4<double>) * (Nc + Nb), cudaMemcpyDeviceToHost, s->stream));
-      AFAR_CUDA(cudaStreamSynchronize(s->stream));  // xfer is reused below
     } else {
       AFAR_CUDA(cudaMemcpyAsync(FD, s->W, sizeof(V4<double>) * (Nc + Nb), cudaMemcpyDeviceToHost, s->stream));
     }
@@ -883,7 +886,6 @@ static afar_status get_state(afar_solver* s, afar_basicFieldData* FD, afar_conse
     }
     const int8_t* from = s->si;
     if (mixed) {
-      if (cFD) AFAR_CUDA(cudaStreamSynchronize(s->stream));  // xfer is reused
       k_flags_out<<<grid_for(Nc + Nb, 256), 256, 0, s->stream>>>((int)Nc, (int)(Nc + Nb), s->si,
                                                                  static_cast<int8_t*>(s->xfer), s->order);
       from = static_cast<const int8_t*>(s->xfer);
@@ -1703,23 +1705,29 @@ extern "C" afar_status afar_stage_debug(afar_solver* s, int stage, double deltaT
   AFAR_CUDA(cudaGetLastError());
   AFAR_CUDA(cudaStreamSynchronize(s->stream));
   // copy out in the reference layout and the caller's order: `group` entries for each cell or face of
-  // `perm` (the caller's place of the device's), the rest in place
-  auto get4 = [&](void* dst, const void* src, size_t n, bool is_float, const std::vector<int>& perm,
-                  size_t group) -> afar_status {
-    std::vector<V4<double>> tmp(n);
-    if (!is_float) {
-      AFAR_CUDA(cudaMemcpy(tmp.data(), src, n * sizeof(V4<double>), cudaMemcpyDeviceToHost));
-    } else {
-      std::vector<V4<float>> t(n);
-      AFAR_CUDA(cudaMemcpy(t.data(), src, n * sizeof(V4<float>), cudaMemcpyDeviceToHost));
-      for (size_t i = 0; i < n; ++i) tmp[i] = V4<double>{t[i].x, t[i].y, t[i].z, t[i].w};
+  // `perm` (the caller's place of the device's; empty: the caller's order), the rest in place
+  auto get4 = [&](auto* dst, const auto* src, size_t n, const std::vector<int>& perm, size_t group) -> afar_status {
+    using D = std::remove_pointer_t<decltype(dst)>;
+    using S = std::remove_const_t<std::remove_pointer_t<decltype(src)>>;
+    if (std::is_same<D, S>::value && perm.empty()) {
+      AFAR_CUDA(cudaMemcpy(dst, src, n * sizeof(S), cudaMemcpyDeviceToHost));
+      return AFAR_OK;
     }
-    V4<double>* d = static_cast<V4<double>*>(dst);
-    for (size_t i = 0; i < n; ++i) {
-      const size_t g = i / group;
-      d[g < perm.size() ? (size_t)perm[g] * group + i % group : i] = tmp[i];
-    }
+    std::unique_ptr<S[]> t(new S[n]);
+    AFAR_CUDA(cudaMemcpy(t.get(), src, n * sizeof(S), cudaMemcpyDeviceToHost));
+    parallel_ranges((long long)n, 16384, [&](long long i0, long long i1) {
+      using E = decltype(dst->x);
+      for (size_t i = (size_t)i0; i < (size_t)i1; ++i) {
+        const size_t g = i / group;
+        dst[g < perm.size() ? (size_t)perm[g] * group + i % group : i] = D{(E)t[i].x, (E)t[i].y, (E)t[i].z, (E)t[i].w};
+      }
+    });
     return AFAR_OK;
+  };
+  auto get = [&](void* dst, const void* src, size_t n, const std::vector<int>& perm, size_t group) {
+    V4<double>* const d = static_cast<V4<double>*>(dst);
+    return mixed ? get4(d, static_cast<const V4<float>*>(src), n, perm, group)
+                 : get4(d, static_cast<const V4<double>*>(src), n, perm, group);
   };
   std::vector<int> perm, fperm;
   if (s->order.perm) {
@@ -1730,19 +1738,17 @@ extern "C" afar_status afar_stage_debug(afar_solver* s, int stage, double deltaT
     fperm.resize(Nf);
     AFAR_CUDA(cudaMemcpy(fperm.data(), s->order.fperm, sizeof(int) * Nf, cudaMemcpyDeviceToHost));
   }
-  if (out->faceFD && (st = get4(out->faceFD, s->fv, 2 * Nf, mixed, fperm, 2))) return st;
-  if (out->gradFD && (st = get4(out->gradFD, s->grad, 2 * Nc, mixed, perm, 2))) return st;
-  if (out->Flux && (st = get4(out->Flux, s->flux, Nf + Nb, mixed, fperm, 1))) return st;
+  if (out->faceFD && (st = get(out->faceFD, s->fv, 2 * Nf, fperm, 2))) return st;
+  if (out->gradFD && (st = get(out->gradFD, s->grad, 2 * Nc, perm, 2))) return st;
+  if (out->Flux && (st = get(out->Flux, s->flux, Nf + Nb, fperm, 1))) return st;
   if ((out->FD || out->cFD || out->shockIndicator) &&
       (st = get_state(s, out->FD, reinterpret_cast<afar_conservedFieldData*>(out->cFD), out->shockIndicator)))
     return st;
-  if (out->Res && (st = get4(out->Res, s->res_dbg, Nc, false, perm, 1))) return st;
-  if (out->limiter) {
-    std::vector<V4<double>> tmp(Nc);
-    if ((st = get4(tmp.data(), s->lim, Nc, !f64, perm, 1))) return st;
-    for (size_t i = 0; i < Nc; ++i)
-      out->limiter[i] = afar_limiterFieldData{(float)tmp[i].x, (float)tmp[i].y, (float)tmp[i].z, (float)tmp[i].w};
-  }
+  if (out->Res && (st = get4(reinterpret_cast<V4<double>*>(out->Res), s->res_dbg, Nc, perm, 1))) return st;
+  V4<float>* const lim = reinterpret_cast<V4<float>*>(out->limiter);
+  if (lim && (st = f64 ? get4(lim, static_cast<const V4<double>*>(s->lim), Nc, perm, 1)
+                       : get4(lim, static_cast<const V4<float>*>(s->lim), Nc, perm, 1)))
+    return st;
   return AFAR_OK;
 }
 
@@ -1754,12 +1760,16 @@ extern "C" afar_status afar_debug_limiter64(afar_solver* s, double* lim) {
   const size_t Nc = s->Nc;
   if (s->policy == AFAR_POLICY_FP64) {
     AFAR_CUDA(cudaMemcpy(lim, s->lim, Nc * sizeof(V4<double>), cudaMemcpyDeviceToHost));
+  } else if (s->policy == AFAR_POLICY_MIXED) {
+    k_state_out<<<grid_for((long long)Nc, 256), 256, 0, s->stream>>>((int)Nc, (int)Nc, static_cast<const V4<float>*>(s->lim),
+                                                                     static_cast<V4<double>*>(s->xfer), s->order);
+    AFAR_CUDA(cudaGetLastError());
+    AFAR_CUDA(cudaMemcpyAsync(lim, s->xfer, Nc * sizeof(V4<double>), cudaMemcpyDeviceToHost, s->stream));
+    AFAR_CUDA(cudaStreamSynchronize(s->stream));
   } else {
     std::vector<float> tmp(4 * Nc);
     AFAR_CUDA(cudaMemcpy(tmp.data(), s->lim, Nc * sizeof(V4<float>), cudaMemcpyDeviceToHost));
-    std::vector<int> perm(s->order.perm ? Nc : 0);
-    if (s->order.perm) AFAR_CUDA(cudaMemcpy(perm.data(), s->order.perm, sizeof(int) * Nc, cudaMemcpyDeviceToHost));
-    for (size_t i = 0; i < 4 * Nc; ++i) lim[perm.empty() ? i : 4 * (size_t)perm[i / 4] + i % 4] = tmp[i];
+    for (size_t i = 0; i < 4 * Nc; ++i) lim[i] = tmp[i];
   }
   return AFAR_OK;
 }
@@ -1814,10 +1824,13 @@ extern "C" afar_status afar_state_snapshot(afar_solver* s, int op) {
     else
       AFAR_CUDA(cudaMemcpyAsync(src[i], dst[i], n[i], cudaMemcpyDeviceToDevice, s->stream));
   }
-  if (op == AFAR_SNAPSHOT_RESTORE && s->policy == AFAR_POLICY_MIXED && s->Nb)  // the ghosts in every buffer
+  // The further buffers' ghosts are the last uploaded ones but for those that every stage writes.
+  if (op == AFAR_SNAPSHOT_SAVE) s->snap_ghosts = s->ghosts;
+  if (op == AFAR_SNAPSHOT_RESTORE && s->policy == AFAR_POLICY_MIXED && s->Nb && s->ghosts != s->snap_ghosts)
     for (void* b : s->Wb)
       AFAR_CUDA(cudaMemcpyAsync(static_cast<V4<float>*>(b) + s->Nc, static_cast<V4<float>*>(s->W) + s->Nc,
                                 sizeof(V4<float>) * (size_t)s->Nb, cudaMemcpyDeviceToDevice, s->stream));
+  if (op == AFAR_SNAPSHOT_RESTORE) s->ghosts = s->snap_ghosts;
   AFAR_CUDA(cudaStreamSynchronize(s->stream));
   return AFAR_OK;
 }
