@@ -202,11 +202,15 @@ __global__ void k_state_in(int Nc, int n, const V4<double>* in, V4<float>* out, 
   out[i] = w;
   if (i >= Nc) b[i] = c[i] = w;
 }
-__global__ void k_state_out(int Nc, int n, const V4<float>* in, V4<double>* out, DeviceOrder o) {
+// (and the switch flags with it, two a cell, where they are asked for)
+__global__ void k_state_out(int Nc, int n, const V4<float>* in, V4<double>* out, const int8_t* si, int8_t* si_out,
+                            DeviceOrder o) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const V4<float> v = in[i];
-  out[i < Nc ? o.cell(i) : i] = V4<double>{(double)v.x, (double)v.y, (double)v.z, (double)v.w};
+  const int at = i < Nc ? o.cell(i) : i;
+  out[at] = V4<double>{(double)v.x, (double)v.y, (double)v.z, (double)v.w};
+  if (si_out) reinterpret_cast<char2*>(si_out)[at] = reinterpret_cast<const char2*>(si)[i];
 }
 
 // A device buffer of one call.
@@ -859,38 +863,30 @@ static afar_status put_state(afar_solver* s, const afar_basicFieldData* FD, cons
 
 // (the mixed policy's arrays leave through `xfer` one after another, in the stream's order)
 static afar_status get_state(afar_solver* s, afar_basicFieldData* FD, afar_conservedFieldData* cFD, int8_t* si) {
-  const size_t Nc = s->Nc, Nb = s->Nb;
-  const bool mixed = s->policy == AFAR_POLICY_MIXED;
-  if (FD) {
-    if (mixed) {
-      k_state_out<<<grid_for(Nc + Nb, 256), 256, 0, s->stream>>>((int)Nc, (int)(Nc + Nb),
-                                                                 static_cast<const V4<float>*>(s->W),
-                                                                 static_cast<V4<double>*>(s->xfer), s->order);
-      AFAR_CUDA(cudaMemcpyAsync(FD, s->xfer, sizeof(V4<double>) * (Nc + Nb), cudaMemcpyDeviceToHost, s->stream));
-    } else {
-      AFAR_CUDA(cudaMemcpyAsync(FD, s->W, sizeof(V4<double>) * (Nc + Nb), cudaMemcpyDeviceToHost, s->stream));
-    }
+  const size_t Nc = s->Nc, Nb = s->Nb, n = Nc + Nb;
+  if (si && s->bvd_pending == 0) {  // a fused head: its stage's types
+    if (afar_status st = settle_bvd(s)) return st;
   }
+  const void *fd = s->W, *cfd = s->U;
+  const int8_t* flags = s->si;
+  const bool mixed = s->policy == AFAR_POLICY_MIXED;
+  if (mixed) {
+    int8_t* const to = si ? static_cast<int8_t*>(s->xfer) + sizeof(V4<double>) * n : nullptr;  // past the state's place
+    if (FD)
+      k_state_out<<<grid_for(n, 256), 256, 0, s->stream>>>((int)Nc, (int)n, static_cast<const V4<float>*>(s->W),
+                                                           static_cast<V4<double>*>(s->xfer), s->si, to, s->order);
+    else if (si)
+      k_flags_out<<<grid_for(n, 256), 256, 0, s->stream>>>((int)Nc, (int)n, s->si, to, s->order);
+    fd = cfd = s->xfer;
+    flags = to;
+  }
+  if (FD) AFAR_CUDA(cudaMemcpyAsync(FD, fd, sizeof(V4<double>) * n, cudaMemcpyDeviceToHost, s->stream));
+  if (si) AFAR_CUDA(cudaMemcpyAsync(si, flags, 2 * n, cudaMemcpyDeviceToHost, s->stream));
   if (cFD) {
-    if (mixed) {
+    if (mixed)
       k_df_to_double<<<grid_for(Nc, 256), 256, 0, s->stream>>>((int)Nc, reinterpret_cast<const DF4*>(s->U),
                                                                static_cast<V4<double>*>(s->xfer), s->order);
-      AFAR_CUDA(cudaMemcpyAsync(cFD, s->xfer, sizeof(V4<double>) * Nc, cudaMemcpyDeviceToHost, s->stream));
-    } else {
-      AFAR_CUDA(cudaMemcpyAsync(cFD, s->U, sizeof(V4<double>) * Nc, cudaMemcpyDeviceToHost, s->stream));
-    }
-  }
-  if (si) {
-    if (s->bvd_pending == 0) {  // a fused head: its stage's types
-      if (afar_status st = settle_bvd(s)) return st;
-    }
-    const int8_t* from = s->si;
-    if (mixed) {
-      k_flags_out<<<grid_for(Nc + Nb, 256), 256, 0, s->stream>>>((int)Nc, (int)(Nc + Nb), s->si,
-                                                                 static_cast<int8_t*>(s->xfer), s->order);
-      from = static_cast<const int8_t*>(s->xfer);
-    }
-    AFAR_CUDA(cudaMemcpyAsync(si, from, 2 * (Nc + Nb), cudaMemcpyDeviceToHost, s->stream));
+    AFAR_CUDA(cudaMemcpyAsync(cFD, cfd, sizeof(V4<double>) * Nc, cudaMemcpyDeviceToHost, s->stream));
   }
   AFAR_CUDA(cudaGetLastError());
   AFAR_CUDA(cudaStreamSynchronize(s->stream));
@@ -902,8 +898,9 @@ static afar_status get_state(afar_solver* s, afar_basicFieldData* FD, afar_conse
 // tile's operator rows into shared memory) and the register pass (no shared memory, more tiles per
 // SM).  At the stencil upload each is timed on the solver's own data (one warm-up, best of three times
 // the launches of a step, the first of a fused one with its Courant step; CUDA events on its stream; the
-// launches only write the stage's intermediates and that minimum) and the faster kept.  Decisions are cached per device and mesh class (faces per cell, stencil size, cell
-// count to a factor of two), so later solvers of the same class skip the timing.
+// launches only write the stage's intermediates and that minimum) and the faster kept.  Decisions are
+// cached per device and mesh class (faces per cell, stencil size, cell count to a factor of two), so later
+// solvers of the same class skip the timing.
 // cuTensorMapEncodeTiled, looked up once through the runtime (the library links no driver API).
 static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
@@ -1066,7 +1063,7 @@ extern "C" afar_status afar_setDeviceFieldData(afar_solver* s, const afar_fieldP
          if (mixed) {
            if ((st = dalloc_t(s, &s->vinvf, Nc))) return st;
            // (the flux of a fused solver's rare separate kernels too, see afar_setDeviceFieldDataStencil)
-           if ((st = dalloc(s, &s->xfer, std::max({sizeof(V4<double>) * (Nc + Nb), sizeof(V4<float>) * (Nf + Nb),
+           if ((st = dalloc(s, &s->xfer, std::max({(sizeof(V4<double>) + 2) * (Nc + Nb), sizeof(V4<float>) * (Nf + Nb),
                                                    order_scratch(cellsNum)}))))
              return st;
            if ((st = dalloc_t(s, &perm, Nc))) return st;
@@ -1762,7 +1759,7 @@ extern "C" afar_status afar_debug_limiter64(afar_solver* s, double* lim) {
     AFAR_CUDA(cudaMemcpy(lim, s->lim, Nc * sizeof(V4<double>), cudaMemcpyDeviceToHost));
   } else if (s->policy == AFAR_POLICY_MIXED) {
     k_state_out<<<grid_for((long long)Nc, 256), 256, 0, s->stream>>>((int)Nc, (int)Nc, static_cast<const V4<float>*>(s->lim),
-                                                                     static_cast<V4<double>*>(s->xfer), s->order);
+                                                                     static_cast<V4<double>*>(s->xfer), nullptr, nullptr, s->order);
     AFAR_CUDA(cudaGetLastError());
     AFAR_CUDA(cudaMemcpyAsync(lim, s->xfer, Nc * sizeof(V4<double>), cudaMemcpyDeviceToHost, s->stream));
     AFAR_CUDA(cudaStreamSynchronize(s->stream));

@@ -80,3 +80,50 @@ def test_fields_read_inside_a_step_do_not_change_it(kind):
         assert all(np.array_equal(x[f], y[f]) for f in ("Flux", "Res", "cFD"))
     a.close()
     b.close()
+
+
+def test_a_restored_snapshot_brings_its_fixed_ghosts():
+    """Ghosts that keep their uploaded state are in each of the state's buffers: a restored snapshot's are the
+    ones it was taken with, whatever was uploaded since, and an upload's its own."""
+    if not gpu_available():
+        pytest.skip("no CUDA device")
+    from afar_cudaeuler2dmixo3rk3solver_gb300 import CaseConfig, CudaSolver, precompute
+
+    m, W, Wb, st = small_cases()["corner_flow"]
+    cfg = CaseConfig(R=0.7142857, Cv=1.7857142857, CFL=0.08, stencilType=st, cOrder=7, fOrder=5)
+    hf = precompute(m, cfg, W, Wb)
+    other = hf.FD.copy()
+    other[hf.nc:, 0] *= 0.5  # another inlet
+    up = {"a": dict(FD=hf.FD, cFD=hf.cFD, cFDold=hf.cFD), "b": dict(FD=other, cFD=hf.cFD, cFDold=hf.cFD)}
+    want = {}
+    for k, u in up.items():
+        s = CudaSolver(hf, cfg, policy="mixed")
+        s.upload_state(**u)
+        s.run(4, dt=1e-4)
+        want[k] = s.state()["FD"]
+        s.close()
+    assert not np.array_equal(want["a"], want["b"])
+    s = CudaSolver(hf, cfg, policy="mixed")
+
+    def steps(k):
+        s.run(4, dt=1e-4)
+        assert np.array_equal(s.state()["FD"], want[k])
+
+    s.save()
+    steps("a")
+    s.upload_state(**up["b"])
+    steps("b")
+    s.restore()
+    steps("a")
+    s.restore()
+    steps("a")
+    s.upload_state(**up["b"])
+    s.save()
+    s.upload_state(**up["a"])
+    s.restore()
+    steps("b")
+    s.restore()
+    steps("b")
+    s.upload_state(**up["a"])
+    steps("a")
+    s.close()
