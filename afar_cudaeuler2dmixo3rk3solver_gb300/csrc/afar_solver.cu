@@ -2076,15 +2076,31 @@ afar_status add_fused_chain(cudaGraph_t graph, int device, const MemberTable<Pol
   return AFAR_OK;
 }
 
-// One fused step of a batch as a graph.  The chains work on different members: side by side they fill the
-// GPU where one is less than a wave, one after another they leave it to one kernel at a time (256 ramps of
-// 5k to 200k quads: 8.93 ms a step side by side, 8.49 in turn, 8.59 as separate kernels).  Early starts (see
+// Whether a batch of members with wide stencils (quads with their neighbours' neighbours, 12 members: the order
+// along the curve helps their reconstruct least) runs the fused stage: not many members of few cells, whose last
+// tiles and borders are much of the work.  us a step, fused / separate: 128 members of 6k quads 679 / 653, 10k
+// 1033 / 993, 20k 1870 / 1834; 256 of 4k 788 / 731, 6k 1344 / 1217, 10k 2053 / 1904; but 96 members of 4k 301 / 309, 10k 772 / 769,
+// 20k 1397 / 1405, 26k 1753 / 1747, and 128 of 40k 3505 / 3685.  Nor where the tiles are those of 96 cells and more than two
+// waves of them: 3.6k quads, 24 members 98 / 98, 48 190 / 170, 60 224 / 208.  Other stencils gain throughout: 256 members of
+// 4k quads (8 members a stencil) 657 / 679, 96 of 10k 550 / 692, 60 of 40k 1368 / 1572; quads and triangles (15), 256 of
+// 13k 2351 / 2379, 96 of 33k 2077 / 2221.
+bool fused_pays(long long members, long long cells, long long tiles, bool wide) {
+  if (!wide) return true;
+  if (members > 2 * MemberTable<PolicyMixed>::kMembers && cells < 32000 * members) return false;
+  return cells > 4096 * members || tiles <= 8 * kSMs;
+}
+
+// One fused step of a batch as a graph.  The chains work on different members: side by side they share their
+// kernels' ends, one after another they leave the GPU to one kernel at a time.  us a step side by side / in turn, by
+// the cells of a chain, wide stencils: 480k 486 / 524, 690k 667 / 691, 940k 890 / 898 (more members 1406 / 1384), 1.2M
+// 1127 / 1127 (1790 / 1740), 1.9M 1768 / 1678; others: 480k 350 / 399, 940k 1056 / 1091, 1.2M 1342 / 1381, 1.9M 1375 / 1377; 256
+// ramps of 5k to 200k quads 8930 / 8490.  Early starts (see
 // tail_early) where the members together are no more than 4000 blocks of 128 cells; us a step without / with:
 // four members of 4k quads 48 / 43, twelve of 41k triangles 296 / 292, twelve of 121k 727 / 731, ten of 160k quads 1%
 // slower with.  The single solve's exception for quads is not one here: 450 to 480 blocks without / with, four
 // members of 14k 56.1 / 56.8 (edge-neighbour stencils 49.2 / 48.2), six of 10k 55.3 / 53.1 (51.2 / 48.6).
 afar_status capture_fused(afar_batch* b, const std::vector<StageArgs<PolicyMixed>>& tab, int nfmax, size_t smem,
-                          size_t tail_bytes, cudaGraph_t* graph) {
+                          size_t tail_bytes, bool wide, cudaGraph_t* graph) {
   using Table = MemberTable<PolicyMixed>;
   AFAR_CUDA(cudaGraphCreate(graph, 0));
   std::unique_ptr<Table> cells(new Table), tiles(new Table);
@@ -2105,7 +2121,7 @@ afar_status capture_fused(afar_batch* b, const std::vector<StageArgs<PolicyMixed
     }
     const auto chain = nfmax <= 3 ? (early ? add_fused_chain<3, true> : add_fused_chain<3, false>)
                                   : (early ? add_fused_chain<4, true> : add_fused_chain<4, false>);
-    if (cells->first[n] <= 4 * kSMs) end = nullptr;  // less than a wave of four blocks a SM
+    if (cells->first[n] <= (wide ? 7000 : 12000)) end = nullptr;  // side by side
     st = chain(*graph, b->device, *cells, *tiles, smem, tail_bytes, &end);
   }
   if (st) {
@@ -2137,15 +2153,22 @@ afar_status batch_build(afar_batch* b) {
     }
   }
   // mixed: the fused stage (two kernels a stage) where every member has it, unless a member forces
-  // the register pass or block sizes of the separate BVD and flux kernels are asked for; the same
-  // bits either way
+  // the register pass or block sizes of the separate BVD and flux kernels are asked for, and where it
+  // pays; the same bits either way
   bool fused = P::id == PolicyMixed::id && !b->forced_bvd && !b->forced_flux && !tab.empty();
   size_t tail_bytes = 0;
+  long long tiles = 0;
+  int maxS = 0, maxM = 0;
   for (size_t i = 0; i < b->members.size(); ++i) {
     const afar_solver* s = b->members[i];
     fused = fused && fused_step(s) && is_tile[i];
     if (fused) tail_bytes = std::max<size_t>(tail_bytes, tail_smem(s->tail_faces, tail_cells(s)).bytes);
+    tiles += grid_for(s->Nc, tail_cells(s));
+    maxS = std::max(maxS, s->maxS);
+    maxM = std::max(maxM, s->maxM);
   }
+  const bool wide = maxM > 3 && maxS > 8;  // quads with their neighbours' neighbours
+  fused = fused && fused_pays((long long)b->members.size(), cells, tiles, wide);
   b->fused = fused;
   int lc = 0, lm = 0;
   while ((1ll << (lc + 1)) <= cells) ++lc;
@@ -2294,7 +2317,7 @@ afar_status batch_build(afar_batch* b) {
   cudaGraph_t g = nullptr;
   if constexpr (P::id == PolicyMixed::id) {
     if (fused) {
-      if ((st = capture_fused(b, tab, nfmax, smem, tail_bytes, &g))) return st;
+      if ((st = capture_fused(b, tab, nfmax, smem, tail_bytes, wide, &g))) return st;
     }
   }
   if (!fused) {
