@@ -126,6 +126,8 @@ def lib():
             "afar_device_bytes": (S, [_p, C.POINTER(C.c_size_t)]),
             "afar_measure_fp64_peak": (S, [C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_float)]),
             "afar_debug_wait_injection": (S, [C.c_int, C.c_uint, C.c_longlong]),
+            "afar_step_launches": (C.c_int, [_p]),
+            "afar_batch_step_launches": (S, [_p, C.POINTER(C.c_int)]),
             "afar_debug_arithmetic": (S, [C.c_int, C.c_int, C.c_int, _p, _p, _p]),
             "afar_debug_wait_injection_at": (S, [C.c_int, C.c_int, C.c_uint, C.c_int, C.c_longlong]),
             "afar_set_face_gauss_flux": (S, [_p, C.c_int, _p, _p, _p]),
@@ -186,5 +188,5 @@ EXPORTED = [
     "afar_set_write_interval", "afar_set_periodic", "afar_set_tuning", "afar_get_tuning", "afar_batch_create", "afar_batch_add", "afar_batch_remove", "afar_batch_size", "afar_batch_run",
     "afar_batch_destroy", "afar_batch_get_schedule", "afar_batch_set_schedule", "afar_server_create", "afar_server_submit", "afar_server_wait", "afar_server_get_stats",
     "afar_server_destroy", "afar_server_cancel", "afar_switch_counts", "afar_measure_fp64_peak",
-    "afar_debug_wait_injection", "afar_debug_wait_injection_at", "afar_debug_arithmetic", "afar_set_face_gauss_flux",
+    "afar_debug_wait_injection", "afar_debug_wait_injection_at", "afar_debug_arithmetic", "afar_step_launches", "afar_batch_step_launches", "afar_set_face_gauss_flux",
 ]

@@ -1362,7 +1362,8 @@ struct MixedSide {
 // is written out, in the pattern in which the compiler fuses those expressions in the separate flux
 // kernel (found by comparing results: each candidate rounding on 65k random faces, equal to the bit), so
 // that the kernels that call it agree bit for bit whatever the code around the call.  E: the energy flux's
-// sum of two products fused, as the compiler has it in the batched stage-1 flux (DT) and nowhere else.
+// sum of two products fused, as the compiler had it in the batched stage-1 flux (DT) and nowhere else when the
+// roundings were written out; kept, so that a batch's results stay what they were.
 __device__ __forceinline__ float fm_(const float a, const float b, const float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ float ml_(const float a, const float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float ad_(const float a, const float b) { return __fadd_rn(a, b); }

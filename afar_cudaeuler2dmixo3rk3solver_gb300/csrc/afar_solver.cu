@@ -1915,6 +1915,10 @@ extern "C" int afar_launches_per_step(afar_solver* s) {
   return s->ng > 0 ? 17 : 13;  // the multi-point flux: a Gauss-point reconstruct per stage, the Courant kernel
 }
 
+extern "C" int afar_step_launches(afar_solver* s) {
+  return s && s->policy == AFAR_POLICY_MIXED && fused_step(s) ? 6 : afar_launches_per_step(s);
+}
+
 extern "C" afar_status afar_freeFieldData(afar_solver* s) {
   if (!s) return AFAR_OK;
   if (s->batch) afar_batch_remove(s->batch, s);  // the batch forgets a freed member
@@ -1991,6 +1995,7 @@ struct afar_batch {
   BatchSchedule sched;
   int forced_bvd = 0, forced_flux = 0;  // afar_batch_set_schedule (0: autotune)
   cudaGraphExec_t graph = nullptr;
+  size_t launches = 0;  // kernels of it
   bool dirty = true;
 };
 
@@ -2334,7 +2339,8 @@ afar_status batch_build(afar_batch* b) {
     kb_finish_step<P><<<grid_for((long long)tab.size(), 128), 128, 0, b->stream>>>(t, (int)tab.size());
     AFAR_CUDA(cudaStreamEndCapture(b->stream, &g));
   }
-  const cudaError_t e = cudaGraphInstantiate(&b->graph, g, 0);
+  cudaError_t e = cudaGraphGetNodes(g, nullptr, &b->launches);
+  if (e == cudaSuccess) e = cudaGraphInstantiate(&b->graph, g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) {
     b->graph = nullptr;
@@ -2473,6 +2479,19 @@ extern "C" afar_status afar_batch_get_schedule(afar_batch* b, int* tileMembers, 
   if (fluxBlock) *fluxBlock = b->sched.flux_block;
   if (ms)
     for (int k = 0; k < 5; ++k) ms[k] = b->sched.ms[k];
+  return AFAR_OK;
+}
+
+extern "C" afar_status afar_batch_step_launches(afar_batch* b, int* launches) {
+  if (!b || !launches) return (set_error("null argument"), AFAR_ERR_ARGUMENT);
+  *launches = 0;
+  if (b->members.empty()) return AFAR_OK;
+  if (b->dirty) {
+    AFAR_CUDA(cudaSetDevice(b->device));
+    const afar_status st = b->policy == AFAR_POLICY_MIXED ? batch_build<PolicyMixed>(b) : batch_build<PolicyFP64>(b);
+    if (st) return st;
+  }
+  *launches = (int)b->launches;
   return AFAR_OK;
 }
 

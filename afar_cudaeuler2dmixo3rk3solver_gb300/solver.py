@@ -366,6 +366,10 @@ class CudaSolver:
     def launches_per_step(self) -> int:
         return lib().afar_launches_per_step(self.h)
 
+    def step_launches(self) -> int:
+        """Kernel launches of one step as the solver runs it (launches_per_step: as separate kernels)."""
+        return lib().afar_step_launches(self.h)
+
     def save(self):
         """In-device checkpoint of the state (bit-exact resume with restore())."""
         check(lib().afar_state_snapshot(self.h, 0))
@@ -511,6 +515,12 @@ class Batch:
         check(lib().afar_batch_get_schedule(self.h, C.byref(t), C.byref(r), C.byref(bb), C.byref(fb), ms))
         return {"tile_members": t.value, "register_members": r.value, "bvd_block": bb.value, "flux_block": fb.value,
                 "ms_bvd": {64: ms[0], 128: ms[1], 256: ms[2]}, "ms_flux": {128: ms[3], 256: ms[4]}}
+
+    def step_launches(self) -> int:
+        """Kernel launches of one step of the whole batch."""
+        n = C.c_int()
+        check(lib().afar_batch_step_launches(self.h, C.byref(n)))
+        return n.value
 
     def set_schedule(self, bvd_block: int = 0, flux_block: int = 0):
         """Forces the BVD and flux block sizes (0: autotune)."""

@@ -496,7 +496,7 @@ def run_ours(args, dist: Dist):
             st = s.state()
             W_ = st["FD"][:hf.nc]
             finite &= bool(np.isfinite(st["cFD"]).all() and (W_[:, 0] > 0).all() and (W_[:, 3] > 0).all())
-        results[pol] = {"ms": ms, "finite": finite, "launches": s.launches_per_step()}
+        results[pol] = {"ms": ms, "finite": finite, "launches": s.step_launches()}
     clocks = sampler.stop()
     for pol in policies:
         s = solvers[pol]
@@ -508,9 +508,6 @@ def run_ours(args, dist: Dist):
             for k, v in s.profile_step().items():
                 acc[k] = acc.get(k, 0.0) + v / PROFILE_STEPS
         results[pol]["kernels_ms"] = acc
-        # a step without BVD and flux kernels is the fused one: reconstruct and stage tail, three times
-        if acc["bvd"] == 0.0 and acc["flux"] == 0.0:
-            results[pol]["launches"] = 6
         results[pol]["device_bytes"] = s.device_bytes()
         if pol == "mixed":
             results[pol]["tuning"] = s.tuning()
@@ -1146,11 +1143,7 @@ def run_batch(args, dist: Dist):
         s.restore()
         solo_ms += s.run_timed(40) / 40.0
         s.restore()
-    # the fused step: reconstruct and stage tail, three times, for every 48 members (see the single solve)
-    fused = all(s.profile_step()["flux"] == 0.0 for s in solvers)
-    for s in solvers:
-        s.restore()
-    launches = 6 if fused else 13
+    solo_launches = sum(s.step_launches() for s in solvers)
     batch = Batch("mixed", device=dist.local)
     for s in solvers:
         s.set_step_params()
@@ -1160,7 +1153,7 @@ def run_batch(args, dist: Dist):
         s.restore()
     dist.barrier()
     ms = dist.max(batch.run(args.batch_steps))
-    schedule = batch.schedule()
+    schedule, launches = batch.schedule(), batch.step_launches()
     finite = all(bool(np.isfinite(s.state()["FD"]).all()) for s in solvers)
     batch.close()
     for s in solvers:
@@ -1173,11 +1166,11 @@ def run_batch(args, dist: Dist):
         "n_gpus": dist.world, "higher_is_better": True, "ms_per_step": ms / args.batch_steps,
         "data": "synthetic (compression ramps 5k-200k quads, Mach 1.5-4, 5-20 deg, vortex 0-5, seeded)",
         "config": {"workload": "batch_wedges", "solves": args.batch_solves, "cells": int(cells.sum()),
-                   "steps": args.batch_steps, "policy": "mixed", "launches_per_step": 6 * -(-len(solvers) // 48) if fused else 13, "setup_s": round(setup_s, 1)},
+                   "steps": args.batch_steps, "policy": "mixed", "launches_per_step": launches, "setup_s": round(setup_s, 1)},
         "schedule": schedule,
         "one_after_another": None if args.batch_no_solo else {
             "value": float(cells.sum()) / (solo_ms * 1e-3), "ms_per_step": solo_ms,
-            "launches_per_step": launches * args.batch_solves},
+            "launches_per_step": solo_launches},
         "finite": finite,
     }), flush=True)
 

@@ -358,12 +358,12 @@ afar_status afar_set_periodic(afar_solver* solver, double periodX, double period
 /* A batch steps all of its member solvers with one launch per stage kernel (13 per RK3 step; the
  * mixed policy's fused stage: six for every 48 members; replayed as one CUDA graph): every block works
  * on one member, so meshes of uneven size share the GPU without padding.  Each member keeps its own
- * device data, time step (fixed or CFL, with its own step params), end time and step count.  A member's result does not depend on which other
- * solves share its batch (bitwise); it agrees with afar_run of the same solve to the policy's
- * rounding (the batched kernels read their arguments from a device table, afar_run's from kernel
- * parameters, and the compiler may fuse a multiply-add differently in the two).  Members join and
- * leave between runs without moving their data.  Policies fp64 and mixed; all members of a batch
- * share the batch's policy and device; a solver belongs to at most one batch at a time and must
+ * device data, time step (fixed or CFL, with its own step params), end time and step count.  A member's
+ * result does not depend on which other solves share its batch (bitwise); it agrees with afar_run of
+ * the same solve to the policy's rounding (mixed: the batched first stage rounds the energy flux's sum of
+ * two products once, afar_run's twice; fp64: the compiler fuses some multiply-adds in one of the two
+ * only).  Members join and leave between runs without moving their data.  Policies fp64 and mixed; all
+ * members of a batch share the batch's policy and device; a solver belongs to at most one batch at a time and must
  * not be stepped on its own while it belongs to one.  Not thread-safe: one host thread per batch. */
 typedef struct afar_batch afar_batch;
 afar_status afar_batch_create(afar_batch** batch, int policy, int device);
@@ -381,14 +381,16 @@ afar_status afar_batch_destroy(afar_batch* batch);
  * member's result never depends on its batch-mates), and the BVD and flux kernels run in the block
  * size that timed fastest on the whole batch (BVD 64, 128 or 256 cells, flux 128 or 256 faces;
  * best of three launches each), cached per device, policy and batch shape (cells and members, each
- * to a factor of two).  A mixed batch whose members all have the fused
- * stage, and force neither, runs that and times nothing.  Block sizes do not change results.  afar_batch_get_schedule reports the
- * members on each reconstruct, the block sizes and the launch times measured (ms: BVD at 64, 128,
+ * to a factor of two).  A mixed batch whose members all have the fused stage, and force neither, runs
+ * that and times nothing, unless it is of many small members whom the separate kernels suit better.
+ * Block sizes do not change results.  afar_batch_get_schedule reports the members on each reconstruct, the block sizes and the launch times measured (ms: BVD at 64, 128,
  * 256, flux at 128, 256; zeros when the decision came from the cache or was forced);
  * afar_batch_set_schedule forces block sizes (0: autotune). */
 afar_status afar_batch_get_schedule(afar_batch* batch, int* tileMembers, int* registerMembers, int* bvdBlock,
                                     int* fluxBlock, float ms[5]);
 afar_status afar_batch_set_schedule(afar_batch* batch, int bvdBlock, int fluxBlock);
+/* The kernel launches of one step of the whole batch. */
+afar_status afar_batch_step_launches(afar_batch* batch, int* launches);
 
 /* ---- serving: a queue of solve requests on one GPU under a device-memory budget --------------- */
 /* No counterpart in the reference (it runs one case per process).  A server owns a worker thread
@@ -545,9 +547,11 @@ afar_status afar_debug_arithmetic(int device, int op, int n, const double* a, co
 afar_status afar_set_face_gauss_flux(afar_solver* solver, int nPoints, const double* points,
                                      const double* pointWeights, const double* rbfGauss);
 
-/* Number of kernel launches of one step as separate stage kernels (for accounting).  The mixed
- * policy's fused step (see afar_profile_step) issues six instead of its 13. */
+/* Number of kernel launches of one step as separate stage kernels (for accounting), and of the step
+ * that the solver's calls issue: six where the mixed policy runs its fused stage (see
+ * afar_profile_step), the same otherwise. */
 int afar_launches_per_step(afar_solver* solver);
+int afar_step_launches(afar_solver* solver);
 
 #ifdef __cplusplus
 }

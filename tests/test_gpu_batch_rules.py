@@ -10,9 +10,10 @@ pytestmark = pytest.mark.gpu
 
 
 # (members, quads a side, stencil): chains side by side; chains in turn; many small members; tiles of 96 cells
-@pytest.mark.parametrize("members,n,stencil", [(50, 33, "edgeNeighbour"), (50, 152, "faceNeighbour"),
-                                               (97, 24, "faceNeighbour"), (33, 61, "faceNeighbour")], ids=str)
-def test_every_way_is_the_separate_kernels(members, n, stencil):
+@pytest.mark.parametrize("members,n,stencil,launches", [(50, 33, "edgeNeighbour", 12), (50, 152, "faceNeighbour", 12),
+                                                        (97, 24, "faceNeighbour", 13), (33, 61, "faceNeighbour", 13)],
+                         ids=str)
+def test_every_way_is_the_separate_kernels(members, n, stencil, launches):
     if not gpu_available():
         pytest.skip("no CUDA device")
     from afar_cudaeuler2dmixo3rk3solver_gb300 import Batch, CaseConfig, CudaSolver, mesh as M, precompute
@@ -22,6 +23,7 @@ def test_every_way_is_the_separate_kernels(members, n, stencil):
     cfg = CaseConfig(stencilType=stencil, CFL=0.2)
     hf = precompute(m, cfg, W, Wb, device=0)
     solvers = [CudaSolver(hf, cfg, policy="mixed") for _ in range(members)]
+    assert solvers[0].step_launches() == 6 and solvers[0].launches_per_step() == 13
     out = []
     for schedule in ((0, 0), (128, 256)):
         batch = Batch("mixed")
@@ -30,7 +32,9 @@ def test_every_way_is_the_separate_kernels(members, n, stencil):
             s.set_time(0.0)
             s.set_step_params(cfl=0.1 + 0.001 * i)
             batch.add(s)
+        assert batch.step_launches() == launches
         batch.set_schedule(*schedule)
+        assert batch.step_launches() == (13 if schedule[0] else launches)
         batch.run(3)
         out.append([(s.state(), s.time()[0]) for s in solvers[:: max(1, members // 12)] + solvers[-1:]])
         batch.close()
