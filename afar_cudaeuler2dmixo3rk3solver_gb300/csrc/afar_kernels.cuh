@@ -2219,9 +2219,9 @@ __device__ __forceinline__ void finish_one(StepCtl* ctl) {
 // registers, border and boundary faces by the threads.  The stencils' troubled-cell flags are read only
 // where a 128-cell tile that they reach holds one (words of 32 flags, written by the reconstruct).
 // 256 threads: with its halo a tile of 192 triangles or 152 quads is mostly one pass of the block.  Four
-// blocks a SM (64 registers); five spilled and lost 8%.  us a step, separate kernels / fused: 986 quads 54 / 42,
-// 65k quads 66 / 52, 500k triangles 380 / 345, 2.0M triangles 1165 / 1026, 4.0M quads 2460 / 2297
-// (the tail itself 437 us a step at 2.0M triangles: 1.5 TB/s; its blocks wait, on the halo's gathers and at
+// blocks a SM (64 registers); five spilled and lost 8%.  us a step, separate kernels in the caller's order / fused,
+// with early starts: 2.5k quads 51 / 33, 65k 68 / 60, 4.0M 2276 / 2183; 2k triangles 53 / 35, 200k 147 / 120, 2.0M 1178 / 942
+// (the tail itself 443 us a step at 2.0M triangles: 1.5 TB/s; its blocks wait, on the halo's gathers and at
 // their two barriers).
 struct TailTile {
   int fstart;  // the tile's own faces are fstart .. fstart + nOwn - 1
