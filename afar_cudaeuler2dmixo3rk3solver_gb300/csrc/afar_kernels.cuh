@@ -180,11 +180,13 @@ __device__ __forceinline__ void limiter_process_ratio(LimiterRatio& r, double& p
 }
 // The four ratios of a cell from one reciprocal (simultaneous inversion, a few ulps from four
 // divisions).  Every den is 1, or 2 |d2| + 2e-10 >= 2e-5 with d2 a jump of the flow over a face: the
-// product of four stays far from the range limits of double.
+// product of four leaves the range of double only where one of them is not finite, or for jumps of 1e77: those
+// divide each, so that what is wrong with one variable stays with it.
 __device__ __forceinline__ V4<double> limiter_ratios(const LimiterRatio& a, const LimiterRatio& b,
                                                      const LimiterRatio& c, const LimiterRatio& d) {
-  const double ab = a.den * b.den, cd = c.den * d.den;
-  const double inv = rcp64(ab * cd);
+  const double ab = a.den * b.den, cd = c.den * d.den, all = ab * cd;
+  if (!pos_normal(all)) return V4<double>{a.num / a.den, b.num / b.den, c.num / c.den, d.num / d.den};
+  const double inv = rcp64(all);
   const double iab = inv * cd, icd = inv * ab;
   return V4<double>{a.num * (iab * b.den), b.num * (iab * a.den), c.num * (icd * d.den), d.num * (icd * c.den)};
 }

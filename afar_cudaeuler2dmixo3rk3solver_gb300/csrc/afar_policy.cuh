@@ -116,6 +116,10 @@ __device__ __forceinline__ bool le_zero(const double x) {
 __device__ __forceinline__ double flip_sign(const double x, const int bit) {
   return __hiloint2double(__double2hiint(x) ^ bit, __double2loint(x));
 }
+// positive, normal and finite, by the high word
+__device__ __forceinline__ bool pos_normal(const double x) {
+  return (unsigned)__double2hiint(x) - 0x00100000u < 0x7FE00000u;
+}
 __device__ __forceinline__ bool neg_(const double x) { return (long long)dbits(x) < 0; }  // the sign bit
 // fmin of two doubles without a sign (NaN loses, as in fmin)
 __device__ __forceinline__ double min_nonneg(const double a, const double b) { return dbits(b) < dbits(a) ? b : a; }
